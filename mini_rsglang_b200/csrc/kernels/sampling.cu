@@ -14,8 +14,7 @@
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
 
-#define SAMPLE_THREADS 1024
-#define SAMPLE_WARPS 32
+#define ARGMAX_THREADS 1024
 
 __device__ __forceinline__ unsigned ordered_key(float x) {
     const unsigned b = __float_as_uint(x);
@@ -42,10 +41,8 @@ __device__ __forceinline__ Best better(Best a, Best b) {
     return (b.value > a.value || (b.value == a.value && b.id < a.id)) ? b : a;
 }
 
-// Arg-max of one row by the whole block; result valid in every thread.
-__device__ Best block_argmax(const float* __restrict__ row, int vocab, Best* scratch) {
-    Best best = {-CUDART_INF_F, 0x7fffffff};
-    for (int i = threadIdx.x; i < vocab; i += blockDim.x) best = better(best, Best{row[i], i});
+// The best of the block's threads; result valid in every thread.
+__device__ Best block_best(Best best, Best* scratch) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         Best other = {__shfl_xor_sync(0xffffffffu, best.value, o), __shfl_xor_sync(0xffffffffu, best.id, o)};
@@ -68,10 +65,17 @@ __device__ Best block_argmax(const float* __restrict__ row, int vocab, Best* scr
     return scratch[32];
 }
 
+// Arg-max of one row by the whole block; result valid in every thread.
+__device__ Best block_argmax(const float* __restrict__ row, int vocab, Best* scratch) {
+    Best best = {-CUDART_INF_F, 0x7fffffff};
+    for (int i = threadIdx.x; i < vocab; i += blockDim.x) best = better(best, Best{row[i], i});
+    return block_best(best, scratch);
+}
+
 // One row per thread-block cluster: every block of the cluster takes a share of the row, block 0
 // gathers the shares' results through distributed shared memory.  A row of 150k logits is then
 // read by eight SMs instead of one.
-__global__ void __launch_bounds__(SAMPLE_THREADS) argmax_kernel(const float* __restrict__ logits, int* __restrict__ out,
+__global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const float* __restrict__ logits, int* __restrict__ out,
                                                                 int vocab) {
     __shared__ Best scratch[33];
     __shared__ Best shares[16];
@@ -99,7 +103,7 @@ MRS_EXPORT int mrs_argmax(const float* logits, int* out, int rows, int vocab, vo
     const unsigned blocks = vocab >= 65536 ? 8 : (vocab >= 16384 ? 4 : 1);
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(rows * blocks);
-    config.blockDim = dim3(SAMPLE_THREADS);
+    config.blockDim = dim3(ARGMAX_THREADS);
     config.stream = (cudaStream_t)stream;
     cudaLaunchAttribute attribute;
     attribute.id = cudaLaunchAttributeClusterDimension;
@@ -113,6 +117,25 @@ MRS_EXPORT int mrs_argmax(const float* logits, int* out, int rows, int vocab, vo
     MRS_RETURN_LAUNCH_STATUS();
 }
 
+// ------------------------------------------------------------------------------------------------
+// Sampling.  A row belongs to a thread-block cluster (1, 4 or 8 CTAs): every CTA brings its share of the row into shared
+// memory once, and everything after that (largest logit, the two thresholds, the draw) reads it there; the CTAs meet
+// through distributed shared memory.  What bounds it is the chain of those meetings: a row is read once (608 KB at
+// 151,936 logits), a threshold takes three digits of 11, 11 and 10 bits with two cluster barriers each.  One CTA a row,
+// which read the row from L2 some fifteen times with 8-bit digits, took 1,626 us for 24 rows of 151,936 logits (top-k and
+// top-p rows among them); this takes 87 us.
+//
+// The weights of the kept set are summed in 32 segments of a row, in id order, whatever the cluster's size: a row's token
+// does not depend on how many CTAs shared it.
+// ------------------------------------------------------------------------------------------------
+#define SAMPLE_CTA_THREADS 512
+#define SAMPLE_CTA_WARPS (SAMPLE_CTA_THREADS / 32)
+#define SAMPLE_SEGMENTS 32
+#define SAMPLE_BINS 2048
+#define SAMPLE_OWN_BINS (SAMPLE_BINS / SAMPLE_CTA_THREADS)     // bins a thread looks at when the edge is searched
+#define SAMPLE_SHARE_BYTES (96 * 1024)                         // of a row in a CTA's shared memory, at most: two CTAs an SM
+#define SAMPLE_NOT_KEPT (-1.0f)
+
 // Which elements are kept: keys above `low`, and the first `quota` ids among keys equal to `low`.
 struct Cut {
     unsigned low;
@@ -120,222 +143,368 @@ struct Cut {
 };
 
 struct SampleShared {
-    Best best[33];
-    float f[33];
-    unsigned count[256];
-    float weight[256];
-    int warp_ties[SAMPLE_WARPS];
-    int tie_base[SAMPLE_WARPS];
-    float warp_weight[SAMPLE_WARPS];
-    int sel;
-    int remaining;
-    float acc;
-    int pick_warp;
-    float pick_base;
+    Best warp_best[33];                              // block_argmax's
+    Best best;                                       // of this CTA's share; read by the whole cluster, as are the next five
+    int bad;
+    unsigned count[SAMPLE_BINS];                     // this CTA's histogram
+    float weight[SAMPLE_BINS];
+    unsigned slice_count[SAMPLE_BINS / 4];           // this CTA's slice of the bins, summed over the cluster
+    float slice_weight[SAMPLE_BINS / 4];
+    int seg_ties[SAMPLE_SEGMENTS];                   // this CTA's segments
+    float seg_weight[SAMPLE_SEGMENTS];
+    unsigned warp_count[SAMPLE_CTA_WARPS];           // scan over the bins
+    float warp_weight[SAMPLE_CTA_WARPS];
+    int first, lowest;                               // places in descending order of the bins
+    unsigned edge_count, above_count;
+    float above_weight;
+    int all_ties[SAMPLE_SEGMENTS];
+    float all_weight[SAMPLE_SEGMENTS];
 };
 
-// Per-warp exclusive offsets (in id order) of the elements whose key equals `key`.
-__device__ void tie_offsets(const float* __restrict__ row, int vocab, int per_warp, unsigned key, SampleShared& s) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int begin = warp * per_warp, end = min(vocab, begin + per_warp);
-    int ties = 0;
-    for (int i = begin + lane; i < end; i += 32) ties += ordered_key(row[i]) == key;
-    ties = (int)warp_sum((float)ties);   // counts stay far below 2^24
+// What the digit search knows: keys that match `prefix` under `mask` hold the edge, `above` of them (by count or weight)
+// lie above it.
+struct Edge {
+    unsigned prefix, mask, count;     // `count`: elements of the last digit's bin
+    unsigned above_count;
+    float above_weight, total;
+};
+
+// One digit.  `f(add)` walks this CTA's elements and calls add(key, weight) for those to be counted (the digit's place is
+// applied here); by weight the first bin (from the top) whose running weight reaches target(total of all bins) is chosen,
+// by count the first whose running count reaches `wanted`.  `extra_key`, `extra_weight`: a run of equal keys that the
+// elements leave out, added to its bin once.
+template <bool BY_WEIGHT, typename Walk, typename Target>
+__device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsigned rank, unsigned blocks, int shift, int bits, Edge& e,
+                             Walk walk_elements, Target target, unsigned wanted, bool has_extra, unsigned extra_key, float extra_weight) {
+    const unsigned digit = (1u << bits) - 1u;
+    for (int b = threadIdx.x; b < SAMPLE_BINS; b += SAMPLE_CTA_THREADS) {
+        s.count[b] = 0u;
+        if (BY_WEIGHT) s.weight[b] = 0.0f;
+    }
+    if (threadIdx.x == 0) s.first = 0x7fffffff, s.lowest = -1;
     __syncthreads();
-    if (lane == 0) s.warp_ties[warp] = ties;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int w = 0; w < SAMPLE_WARPS; ++w) {
-            s.tie_base[w] = run;
-            run += s.warp_ties[w];
+    walk_elements([&](unsigned key, float w) {
+        if ((key & e.mask) != e.prefix) return;
+        const unsigned b = (key >> shift) & digit;
+        atomicAdd(&s.count[b], 1u);
+        if (BY_WEIGHT) atomicAdd(&s.weight[b], w);
+    });
+    if (has_extra && rank == 0) {
+        __syncthreads();
+        if (threadIdx.x == 0 && (extra_key & e.mask) == e.prefix) {
+            s.count[(extra_key >> shift) & digit] += 1u;
+            if (BY_WEIGHT) s.weight[(extra_key >> shift) & digit] += extra_weight;
         }
     }
-    __syncthreads();
-}
-
-// Walks this warp's id range in order and calls f(i, x, kept) for every element.
-template <typename F>
-__device__ __forceinline__ void walk(const float* __restrict__ row, int vocab, int per_warp, Cut cut, int tie_base,
-                                     F f) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int begin = warp * per_warp, end = min(vocab, begin + per_warp);
-    int seen = tie_base;
-    for (int base = begin; base < end; base += 32) {
-        const int i = base + lane;
-        const bool live = i < end;
-        const float x = live ? row[i] : 0.0f;
-        const unsigned key = live ? ordered_key(x) : 0u;
-        const bool tie = live && key == cut.low;
-        const unsigned tie_mask = __ballot_sync(0xffffffffu, tie);
-        const int rank = seen + __popc(tie_mask & ((1u << lane) - 1u));
-        seen += __popc(tie_mask);
-        const bool kept = live && (key > cut.low || (tie && rank < cut.quota));
-        f(i, x, key, kept);
+    if (blocks > 1) {
+        cluster.sync();
+        const int slice = SAMPLE_BINS / blocks;
+        for (int i = threadIdx.x; i < slice; i += SAMPLE_CTA_THREADS) {
+            unsigned c = 0u;
+            float w = 0.0f;
+            for (unsigned r = 0; r < blocks; ++r) {
+                c += cluster.map_shared_rank(s.count, r)[rank * slice + i];
+                if (BY_WEIGHT) w += cluster.map_shared_rank(s.weight, r)[rank * slice + i];
+            }
+            s.slice_count[i] = c;
+            if (BY_WEIGHT) s.slice_weight[i] = w;
+        }
+        cluster.sync();
+    } else {
+        __syncthreads();
     }
+    // bins from the top: thread t has places 4 t .. 4 t + 3, place p is bin BINS - 1 - p
+    unsigned c[SAMPLE_OWN_BINS];
+    float w[SAMPLE_OWN_BINS];
+    unsigned c_sum = 0u;
+    float w_sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < SAMPLE_OWN_BINS; ++j) {
+        const int bin = SAMPLE_BINS - 1 - ((int)threadIdx.x * SAMPLE_OWN_BINS + j);
+        if (blocks > 1) {
+            const int slice = SAMPLE_BINS / blocks;
+            c[j] = cluster.map_shared_rank(s.slice_count, bin / slice)[bin % slice];
+            w[j] = BY_WEIGHT ? cluster.map_shared_rank(s.slice_weight, bin / slice)[bin % slice] : 0.0f;
+        } else {
+            c[j] = s.count[bin];
+            w[j] = BY_WEIGHT ? s.weight[bin] : 0.0f;
+        }
+        c_sum += c[j];
+        w_sum += w[j];
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned c_run = c_sum;
+    float w_run = w_sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned cu = __shfl_up_sync(0xffffffffu, c_run, o);
+        const float wu = __shfl_up_sync(0xffffffffu, w_run, o);
+        if (lane >= o) c_run += cu, w_run += wu;
+    }
+    if (lane == 31) s.warp_count[warp] = c_run, s.warp_weight[warp] = w_run;
+    unsigned c_at = __shfl_up_sync(0xffffffffu, c_run, 1);
+    float w_at = __shfl_up_sync(0xffffffffu, w_run, 1);
+    if (lane == 0) c_at = 0u, w_at = 0.0f;
+    __syncthreads();
+    unsigned c_before = 0u;
+    float w_before = 0.0f, w_total = 0.0f;
+    for (int i = 0; i < SAMPLE_CTA_WARPS; ++i) {
+        if (i == warp) c_before = c_at, w_before = w_total + w_at;
+        if (i < warp) c_at += s.warp_count[i];
+        w_total += s.warp_weight[i];
+    }
+    c_before = c_at;
+    if (e.mask == 0u) e.total = w_total;
+    const float goal = BY_WEIGHT ? target(e.total) - e.above_weight : 0.0f;
+    const unsigned need = wanted - e.above_count;
+    {
+        unsigned ca = c_before;
+        float wa = w_before;
+        int found = 0x7fffffff, last = -1;
+#pragma unroll
+        for (int j = 0; j < SAMPLE_OWN_BINS; ++j) {
+            if (c[j] == 0u) continue;
+            last = (int)threadIdx.x * SAMPLE_OWN_BINS + j;
+            if (found == 0x7fffffff && (BY_WEIGHT ? wa + w[j] >= goal : ca + c[j] >= need)) found = last;
+            ca += c[j];
+            wa += w[j];
+        }
+        if (found != 0x7fffffff) atomicMin(&s.first, found);
+        if (last >= 0) atomicMax(&s.lowest, last);
+    }
+    __syncthreads();
+    const int place = s.first != 0x7fffffff ? s.first : max(s.lowest, 0);      // rounding left the sum a hair short: the last bin holds the edge
+    if (place / SAMPLE_OWN_BINS == (int)threadIdx.x) {
+        unsigned ca = c_before, here = 0u;
+        float wa = w_before;
+#pragma unroll
+        for (int j = 0; j < SAMPLE_OWN_BINS; ++j) {
+            if ((int)threadIdx.x * SAMPLE_OWN_BINS + j < place) ca += c[j], wa += w[j];
+            if ((int)threadIdx.x * SAMPLE_OWN_BINS + j == place) here = c[j];
+        }
+        s.edge_count = here;
+        s.above_count = ca;
+        s.above_weight = wa;
+    }
+    __syncthreads();
+    e.prefix |= (unsigned)(SAMPLE_BINS - 1 - place) << shift;
+    e.mask |= digit << shift;
+    e.count = s.edge_count;
+    e.above_count += s.above_count;
+    e.above_weight += s.above_weight;
+    // the histogram is written again after the next barrier of the cluster's first kind: every CTA has read its slices by then
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
-    const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
+// IN_SHARED: the CTA's share of the row lies in shared memory (and gives its place to the weights of the kept set);
+// otherwise a row is too long for that and is read from memory each time.
+template <bool IN_SHARED>
+__global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
+    const float* __restrict__ logits, int vocab, int per_segment, const float* __restrict__ temperature,
     const int* __restrict__ top_k, const float* __restrict__ top_p, const unsigned long long* __restrict__ seed,
     const int* __restrict__ draw_index, int* __restrict__ out) {
     pdl_launch_dependents();
     pdl_wait();
+    extern __shared__ __align__(16) float share[];
     __shared__ SampleShared s;
-    const int r = blockIdx.x;
-    const float* row = logits + (size_t)r * vocab;
+    cg::cluster_group cluster = cg::this_cluster();
+    const unsigned rank = cluster.block_rank(), blocks = cluster.num_blocks();
+    const int r = blockIdx.x / blocks;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int own_segments = SAMPLE_SEGMENTS / blocks;
+    const int begin = min(vocab, (int)rank * own_segments * per_segment);
+    const int length = min(vocab, begin + own_segments * per_segment) - begin;      // of this CTA's share
+    const float* row = logits + (size_t)r * vocab + begin;
     const float temp = temperature[r];
     const int k_raw = top_k[r];
     const float p_raw = top_p[r];
 
     // Largest logit (also the greedy answer) and a check that the row is finite.
     int bad = 0;
-    for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
-        const float x = row[i];
+    Best mine = {-CUDART_INF_F, 0x7fffffff};
+    auto see = [&](float x, int i) {
         bad |= !(fabsf(x) <= 3.402823466e38f);
+        mine = better(mine, Best{x, i});
+    };
+    int vectors = 0;
+    if (((uintptr_t)row & 15) == 0) {
+        vectors = length / 4;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < vectors; i += SAMPLE_CTA_THREADS) {
+            const float4 v = reinterpret_cast<const float4*>(row)[i];
+            if (IN_SHARED) reinterpret_cast<float4*>(share)[i] = v;
+            see(v.x, begin + 4 * i), see(v.y, begin + 4 * i + 1), see(v.z, begin + 4 * i + 2), see(v.w, begin + 4 * i + 3);
+        }
+    }
+#pragma unroll 4
+    for (int i = 4 * vectors + threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) {
+        const float v = row[i];
+        if (IN_SHARED) share[i] = v;
+        see(v, begin + i);
     }
     bad = __syncthreads_or(bad);
-    const Best top = block_argmax(row, vocab, s.best);
-    if (bad) {
-        if (threadIdx.x == 0) out[r] = -1;
-        return;
+    mine = block_best(mine, s.warp_best);
+    if (threadIdx.x == 0) s.best = mine, s.bad = bad;
+    if (blocks > 1) cluster.sync();
+    else __syncthreads();
+    Best top = s.best;
+    for (unsigned q = 0; q < blocks; ++q) {
+        top = better(top, *cluster.map_shared_rank(&s.best, q));
+        bad |= *cluster.map_shared_rank(&s.bad, q);
     }
-    if (temp == 0.0f || k_raw == 1) {
-        if (threadIdx.x == 0) out[r] = top.id;
+    // the same in every CTA of the cluster: they leave together, and none while another still reads its shared memory
+    if (bad || temp == 0.0f || k_raw == 1) {
+        if (rank == 0 && threadIdx.x == 0) out[r] = bad ? -1 : top.id;
+        if (blocks > 1) cluster.sync();
         return;
     }
     const float inv_t = 1.0f / temp;
-    const int per_warp = (((vocab + SAMPLE_WARPS - 1) / SAMPLE_WARPS) + 31) & ~31;
+    const float* x = IN_SHARED ? share : row;
+    auto weight_of = [&](float v) { return expf((v - top.value) * inv_t); };
 
     // ---- top_k: the k-th largest key by count ------------------------------------------------
     Cut cut = {0u, 0x7fffffff};
-    if (k_raw > 0 && k_raw < vocab) {
-        unsigned prefix = 0u, mask = 0u;
-        int remaining = k_raw;
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            for (int b = threadIdx.x; b < 256; b += blockDim.x) s.count[b] = 0u;
-            __syncthreads();
-            for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
-                const unsigned key = ordered_key(row[i]);
-                if ((key & mask) == prefix) atomicAdd(&s.count[(key >> shift) & 255u], 1u);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int left = remaining, chosen = 0;
-                for (int b = 255; b >= 0; --b) {
-                    if ((int)s.count[b] >= left) { chosen = b; break; }
-                    left -= (int)s.count[b];
-                }
-                s.sel = chosen;
-                s.remaining = left;
-            }
-            __syncthreads();
-            prefix |= (unsigned)s.sel << shift;
-            mask |= 255u << shift;
-            remaining = s.remaining;
-            __syncthreads();
-        }
-        cut.low = prefix;
-        cut.quota = remaining;
+    int ties = 0;                                    // elements of the row whose key is cut.low
+    const bool by_count = k_raw > 0 && k_raw < vocab;
+    if (by_count) {
+        Edge e = {0u, 0u, 0u, 0u, 0.0f, 0.0f};
+        auto each = [&](auto add) {
+#pragma unroll 4
+            for (int i = threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) add(ordered_key(x[i]), 0.0f);
+        };
+        auto none = [](float) { return 0.0f; };
+        sample_digit<false>(cluster, s, rank, blocks, 21, 11, e, each, none, (unsigned)k_raw, false, 0u, 0.0f);
+        sample_digit<false>(cluster, s, rank, blocks, 10, 11, e, each, none, (unsigned)k_raw, false, 0u, 0.0f);
+        sample_digit<false>(cluster, s, rank, blocks, 0, 10, e, each, none, (unsigned)k_raw, false, 0u, 0.0f);
+        cut.low = e.prefix;
+        cut.quota = k_raw - (int)e.above_count;
+        ties = (int)e.count;
     }
-    tie_offsets(row, vocab, per_warp, cut.low, s);
-    int tie_base = s.tie_base[warp];
 
-    // ---- weight of the top_k set ----------------------------------------------------------------
-    float local = 0.0f;
-    walk(row, vocab, per_warp, cut, tie_base, [&](int, float x, unsigned, bool kept) {
-        if (kept) local += expf((x - top.value) * inv_t);
-    });
-    float total = block_sum(local, s.f);
-
-    // ---- top_p: the key at which the running weight reaches top_p * total -----------------------
+    // ---- top_p: the key at which the running weight reaches top_p times the top_k set's weight ---
     if (p_raw < 1.0f) {
-        const float target = p_raw * total;
-        unsigned prefix = 0u, mask = 0u;
-        float above = 0.0f;
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            for (int b = threadIdx.x; b < 256; b += blockDim.x) { s.weight[b] = 0.0f; s.count[b] = 0u; }
-            __syncthreads();
-            walk(row, vocab, per_warp, cut, tie_base, [&](int, float x, unsigned key, bool kept) {
-                if (kept && (key & mask) == prefix) {
-                    atomicAdd(&s.weight[(key >> shift) & 255u], expf((x - top.value) * inv_t));
-                    atomicAdd(&s.count[(key >> shift) & 255u], 1u);
-                }
-            });
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                float acc = above;
-                int chosen = -1, lowest = 0;
-                for (int b = 255; b >= 0; --b) {
-                    if (s.count[b] == 0u) continue;
-                    lowest = b;
-                    if (acc + s.weight[b] >= target) { chosen = b; break; }
-                    acc += s.weight[b];
-                }
-                if (chosen < 0) {          // rounding left the sum a hair short: the last bin holds the edge
-                    chosen = lowest;
-                    acc -= s.weight[lowest];
-                }
-                s.sel = chosen;
-                s.acc = acc;
+        Edge e = {0u, 0u, 0u, 0u, 0.0f, 0.0f};
+        const unsigned low = cut.low;
+        const float low_weight = by_count ? weight_of(key_value(low)) * (float)cut.quota : 0.0f;       // the kept ones among equals
+        auto each = [&](auto add) {
+#pragma unroll 4
+            for (int i = threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) {
+                const float v = x[i];
+                const unsigned key = ordered_key(v);
+                if (key > low && (key & e.mask) == e.prefix) add(key, weight_of(v));
             }
-            __syncthreads();
-            prefix |= (unsigned)s.sel << shift;
-            mask |= 255u << shift;
-            above = s.acc;
-            __syncthreads();
-        }
-        const float each = expf((key_value(prefix) - top.value) * inv_t);
-        int need = (int)ceilf((target - above) / each);
+        };
+        auto target = [&](float total) { return p_raw * total; };
+        sample_digit<true>(cluster, s, rank, blocks, 21, 11, e, each, target, 0u, by_count, low, low_weight);
+        sample_digit<true>(cluster, s, rank, blocks, 10, 11, e, each, target, 0u, by_count, low, low_weight);
+        sample_digit<true>(cluster, s, rank, blocks, 0, 10, e, each, target, 0u, by_count, low, low_weight);
+        const float one = weight_of(key_value(e.prefix));
+        int need = (int)ceilf((p_raw * e.total - e.above_weight) / one);
         if (need < 1) need = 1;
-        if (prefix == cut.low) {
+        if (by_count && e.prefix == cut.low) {
             cut.quota = min(cut.quota, need);
         } else {
-            cut.low = prefix;
+            cut.low = e.prefix;
             cut.quota = need;
-            tie_offsets(row, vocab, per_warp, cut.low, s);
-            tie_base = s.tie_base[warp];
+            ties = (int)e.count;
         }
     }
 
-    // ---- inverse CDF over the kept set in id order ------------------------------------------------
-    local = 0.0f;
-    walk(row, vocab, per_warp, cut, tie_base, [&](int, float x, unsigned, bool kept) {
-        if (kept) local += expf((x - top.value) * inv_t);
-    });
-    local = warp_sum(local);
-    __syncthreads();
-    if (lane == 0) s.warp_weight[warp] = local;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float retained = 0.0f;
-        for (int w = 0; w < SAMPLE_WARPS; ++w) retained += s.warp_weight[w];
-        const float u = uniform_from_counter(seed[r], (unsigned long long)draw_index[r]) * retained;
-        float run = 0.0f;
-        int chosen = -1, last = 0;
-        for (int w = 0; w < SAMPLE_WARPS; ++w) {
-            if (s.warp_weight[w] <= 0.0f) continue;
-            last = w;
-            if (run + s.warp_weight[w] > u) { chosen = w; break; }
-            run += s.warp_weight[w];
+    // ---- the kept set's weights, segment by segment in id order -------------------------------------
+    // Where only some of the equals at the cut are kept (the first ids), a segment has to know how many come before it.
+    const bool ranked = cut.quota < ties;
+    const int first_segment = (int)rank * own_segments;
+    auto share_segments = [&]() {                     // every CTA gets all segments' numbers
+        if (blocks > 1) cluster.sync();
+        else __syncthreads();
+    };
+    if (ranked) {
+        for (int g = warp; g < own_segments; g += SAMPLE_CTA_WARPS) {
+            const int from = g * per_segment, to = min(length, from + per_segment);
+            int n = 0;
+            for (int i = from + lane; i < to; i += 32) n += ordered_key(x[i]) == cut.low;
+            n = __reduce_add_sync(0xffffffffu, n);
+            if (lane == 0) s.seg_ties[g] = n;
         }
-        if (chosen < 0) {
-            chosen = last;
-            run -= s.warp_weight[last];
-        }
-        s.pick_warp = chosen;
-        s.pick_base = run;
-        s.acc = u;
+        share_segments();
+        if (threadIdx.x < SAMPLE_SEGMENTS) s.all_ties[threadIdx.x] = cluster.map_shared_rank(s.seg_ties, threadIdx.x / own_segments)[threadIdx.x % own_segments];
+        __syncthreads();
     }
-    __syncthreads();
-    if (warp != s.pick_warp) return;
-    const float u = s.acc;
-    float run = s.pick_base;
+    // f(i, weight or SAMPLE_NOT_KEPT) for 32 neighbouring elements of segment g at a time
+    auto walk = [&](int g, auto f) {
+        const int from = g * per_segment, to = min(length, from + per_segment);
+        int seen = 0;
+        if (ranked)
+            for (int j = 0; j < first_segment + g; ++j) seen += s.all_ties[j];
+        for (int base = from; base < to; base += 32) {
+            const int i = base + lane;
+            const bool live = i < to;
+            const float v = live ? x[i] : 0.0f;
+            const unsigned key = live ? ordered_key(v) : 0u;
+            bool kept = live && key >= cut.low;
+            if (ranked) {
+                const bool tie = live && key == cut.low;
+                const unsigned tie_mask = __ballot_sync(0xffffffffu, tie);
+                if (tie) kept = seen + __popc(tie_mask & ((1u << lane) - 1u)) < cut.quota;
+                seen += __popc(tie_mask);
+            }
+            f(i, live, kept ? weight_of(v) : SAMPLE_NOT_KEPT);
+        }
+    };
+    if (IN_SHARED) {                                  // the weights take the logits' place
+        if (ranked) {
+            for (int g = warp; g < own_segments; g += SAMPLE_CTA_WARPS)
+                walk(g, [&](int i, bool live, float w) { if (live) share[i] = w; });
+        } else {
+#pragma unroll 4
+            for (int i = threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) {
+                const float v = share[i];
+                share[i] = ordered_key(v) >= cut.low ? weight_of(v) : SAMPLE_NOT_KEPT;
+            }
+        }
+        __syncthreads();
+    }
+    auto weights = [&](int g, auto f) {
+        if constexpr (IN_SHARED) {
+            const int from = g * per_segment, to = min(length, from + per_segment);
+#pragma unroll 8
+            for (int base = from; base < to; base += 32) f(base + lane, base + lane < to, base + lane < to ? share[base + lane] : SAMPLE_NOT_KEPT);
+        } else {
+            walk(g, f);
+        }
+    };
+    for (int g = warp; g < own_segments; g += SAMPLE_CTA_WARPS) {
+        float local = 0.0f;
+        weights(g, [&](int, bool, float w) { local += w >= 0.0f ? w : 0.0f; });
+        local = warp_sum(local);
+        if (lane == 0) s.seg_weight[g] = local;
+    }
+    share_segments();
+    if (threadIdx.x < SAMPLE_SEGMENTS) s.all_weight[threadIdx.x] = cluster.map_shared_rank(s.seg_weight, threadIdx.x / own_segments)[threadIdx.x % own_segments];
+    if (blocks > 1) cluster.sync();                   // behind it no CTA reads another's shared memory
+    else __syncthreads();
+
+    // ---- inverse CDF over the kept set in id order ------------------------------------------------
+    if (warp != 0) return;
+    float retained = 0.0f;
+    for (int g = 0; g < SAMPLE_SEGMENTS; ++g) retained += s.all_weight[g];
+    const float u = uniform_from_counter(seed[r], (unsigned long long)draw_index[r]) * retained;
+    float run = 0.0f;
+    int chosen = -1, last = 0;
+    for (int g = 0; g < SAMPLE_SEGMENTS; ++g) {
+        if (s.all_weight[g] <= 0.0f) continue;
+        last = g;
+        if (run + s.all_weight[g] > u) { chosen = g; break; }
+        run += s.all_weight[g];
+    }
+    if (chosen < 0) {
+        chosen = last;
+        run -= s.all_weight[last];
+    }
+    if (chosen / own_segments != (int)rank) return;
     int picked = -1, last_kept = -1;
-    walk(row, vocab, per_warp, cut, tie_base, [&](int i, float x, unsigned, bool kept) {
-        const float e = kept ? expf((x - top.value) * inv_t) : 0.0f;
-        float cum = e;
+    weights(chosen % own_segments, [&](int i, bool, float w) {
+        const bool kept = w >= 0.0f;
+        float cum = kept ? w : 0.0f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float up = __shfl_up_sync(0xffffffffu, cum, o);
@@ -343,22 +512,47 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(
         }
         const unsigned hit = __ballot_sync(0xffffffffu, kept && run + cum > u);
         const unsigned kept_mask = __ballot_sync(0xffffffffu, kept);
-        if (picked < 0 && hit) picked = i - lane + (__ffs(hit) - 1);
-        if (kept_mask) last_kept = i - lane + (31 - __clz(kept_mask));
+        if (picked < 0 && hit) picked = begin + i - lane + (__ffs(hit) - 1);
+        if (kept_mask) last_kept = begin + i - lane + (31 - __clz(kept_mask));
         run += __shfl_sync(0xffffffffu, cum, 31);
     });
     if (lane == 0) out[r] = picked >= 0 ? picked : last_kept;
 }
 
-// One row per block.  temperature, top_k (<= 0: off), top_p, seed and draw_index are per row.
+// temperature, top_k (<= 0: off), top_p, seed and draw_index are per row.
 // out[r] = the token, or -1 when the row holds a NaN or an infinity.
 MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float* temperature, const int* top_k,
                           const float* top_p, const unsigned long long* seed, const int* draw_index, int* out,
                           void* stream) {
     if (rows <= 0) return 0;
     if (vocab <= 0) return MRS_BAD_ARGUMENT;
-    MRS_LAUNCH(sample_kernel, rows, SAMPLE_THREADS, 0, stream,
-        logits, vocab, temperature, top_k, top_p, seed,
-                                                                     draw_index, out);
+    const int per_segment = (int)((((long long)vocab + SAMPLE_SEGMENTS - 1) / SAMPLE_SEGMENTS + 31) & ~31LL);
+    // short rows gain nothing from more CTAs: their meetings cost more than the walks
+    const int blocks = vocab >= 65536 ? 8 : (vocab >= 8192 ? 4 : 1);
+    if (rows > 0x7fffffff / 8) return MRS_BAD_ARGUMENT;
+    const size_t share = (size_t)per_segment * (SAMPLE_SEGMENTS / blocks) * sizeof(float);
+    const bool in_shared = share <= SAMPLE_SHARE_BYTES;
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SHARE_BYTES);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((unsigned)rows * blocks);
+    config.blockDim = dim3(SAMPLE_CTA_THREADS);
+    config.dynamicSmemBytes = in_shared ? share : 0;
+    config.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = blocks, attributes[0].val.clusterDim.y = 1, attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    static const bool plain = getenv("MRS_PLAIN_LAUNCH") != nullptr;
+    config.attrs = attributes;
+    config.numAttrs = plain ? 1 : 2;
+    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out)
+                                    : cudaLaunchKernelEx(&config, sample_kernel<false>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out);
+    if (e != cudaSuccess) return (int)e;
     MRS_RETURN_LAUNCH_STATUS();
 }

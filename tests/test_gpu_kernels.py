@@ -809,6 +809,46 @@ def test_sampler_support_and_repeatability(vocab):
     assert set(sampler.sample(logits.expand(20, vocab).contiguous(), [tiny] * 20, list(range(20)))) == {int(logits[0].argmax())}
 
 
+@pytest.mark.parametrize("vocab", [1, 32, 1025, 8191, 8192, 32768, 65535, 65536, 151936, 196608, 196640, 200003])
+def test_sampler_rows_that_several_ctas_share(vocab):
+    """One row a cluster of 1, 4 or 8 CTAs, in shared memory or (from 196,609 logits on) read from memory; rows that start off a
+    16-byte boundary; equal logits across the shares' edges, of which a cut by count or by weight keeps the first ids; every row
+    against the draw restated in float64.  A draw may differ only where u falls within 1e-5 of the weight between two tokens (float32
+    sums of at most 200,003 weights in 1,024 runs), which at most one row in twenty does."""
+    sampler = Sampler(torch.device(DEV))
+    g = torch.Generator().manual_seed(vocab)
+    settings = [SamplingParams(temperature=0.8, top_p=0.95, seed=1), SamplingParams(temperature=0.7, top_k=50, top_p=0.9, seed=2),
+                SamplingParams(temperature=1.0, seed=3), SamplingParams(temperature=0.6, top_k=20, seed=4), SamplingParams(temperature=0.0),
+                SamplingParams(temperature=5.0, top_p=0.6, seed=5), SamplingParams(temperature=1.0, top_k=max(1, vocab - 1), top_p=0.7, seed=6)]
+    params = [settings[i % len(settings)] for i in range(21)]
+    logits = torch.randn(21, vocab, generator=g) * 2
+    logits[7:14] = (logits[7:14] * 2).round() / 2          # a few dozen values: long runs of equals at every cut
+    logits[14:] = logits[14:].clamp(max=1.5)
+    got = sampler.sample(logits.to(DEV), params, list(range(21)))
+    # the restated draw as tensors: the support by a stable sort, then the inverse CDF in id order
+    wrong = 0
+    for row, p, i, token in zip(logits.double(), params, range(21), got):
+        if p.is_greedy():
+            assert token == int(row.argmax())
+            continue
+        order = torch.sort(row, descending=True, stable=True).indices[:p.top_k]
+        weight = torch.exp((row[order] - row[order[0]]) / p.temperature)
+        # the shortest prefix that reaches top_p; equals at its edge by a count that float32 sums may get one off in 1e5
+        keep = len(order) if p.top_p >= 1.0 else int((torch.cumsum(weight, 0) < p.top_p * weight.sum() * (1 - 1e-12)).sum()) + 1
+        kept = torch.sort(order[:keep]).values
+        running = torch.cumsum(torch.exp((row[kept] - row.max()) / p.temperature), 0)
+        u = uniform_from_counter(p.seed, i)
+        place = int(torch.searchsorted(running, u * running[-1], right=True))
+        if token != int(kept[min(place, len(kept) - 1)]):
+            near = running / running[-1]
+            at = torch.searchsorted(kept, torch.tensor(token))
+            assert at < len(kept) + 1 and (near - u).abs().min() < 1e-5, f"row {i}: {token} with {p}"
+            wrong += 1
+    assert wrong <= 1, wrong
+    again = sampler.sample(logits.to(DEV), params, list(range(21)))
+    assert sum(a != b for a, b in zip(got, again)) <= 1
+
+
 def test_sampler_distribution_ties_and_bad_rows():
     sampler = Sampler(torch.device(DEV))
     logits = torch.tensor([[0.0, 2.0, 1.0, -1.0, 0.5]], device=DEV)

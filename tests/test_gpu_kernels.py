@@ -123,6 +123,29 @@ def test_gemm_f32_is_true_float32(m, n, k):
     assert torch.equal(whole[69:70], alone)
 
 
+@pytest.mark.parametrize("m", [1, 4, 5, 8, 9, 31, 33, 64, 65, 700, 2100])
+@pytest.mark.parametrize("n,k", [(16, 128), (1, 4), (33, 132), (1000, 1020), (257, 1026), (64, 37), (4100, 96)])
+def test_gemm_f32_sizes_keep_a_rows_bits(m, n, k):
+    """Every kernel that the sizes choose (few rows, three tile shapes, sixteen- and four-byte copies), at whole and ragged
+    tiles and stages: within the rounding of a chain of k multiply-adds of the 64-bit product, and every element the same bits
+    as the product of its row alone (a chain in ascending order whatever the kernel)."""
+    g = torch.Generator(device=DEV).manual_seed(m * 7 + n + k)
+    x, w = torch.randn(m, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    out = torch.full((m, n), float("nan"), device=DEV)
+    kernels.gemm_f32(x, w, out)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert ((out.double() - want).abs() <= size * k * 2.0 ** -24).all()
+    for row in {0, m // 2, m - 1}:
+        alone = torch.empty(1, n, device=DEV)
+        kernels.gemm_f32(x[row:row + 1].clone(), w, alone)
+        assert torch.equal(out[row:row + 1], alone)
+    shifted = torch.empty(m * k + 1, device=DEV)[1:].view(m, k)           # off a 16-byte boundary: four-byte copies
+    shifted.copy_(x)
+    other = torch.empty_like(out)
+    kernels.gemm_f32(shifted, w, other)
+    assert torch.equal(out, other)
+
+
 def plain_qk(qkv, positions, q_w, k_w, eps, theta, nq, nkv, d):
     """q and k after head norm and rotation, v untouched, from the plain implementation's parts."""
     ar = P.Arith(None)

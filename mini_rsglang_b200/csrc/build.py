@@ -168,7 +168,7 @@ def host_library() -> ctypes.CDLL:
     return _load("host_sanitized" if sanitize else "host", builder)
 
 
-GENERIC_KERNEL_SOURCES = ("elementwise.cu", "attention_simt.cu", "gemm_f32.cu", "sampling.cu")
+GENERIC_KERNEL_SOURCES = ("elementwise.cu", "attention_simt.cu", "attention_f32.cu", "gemm_f32.cu", "sampling.cu")
 
 
 def kernel_library() -> ctypes.CDLL:

@@ -1,0 +1,419 @@
+// Paged causal grouped-query attention in float32 for heads of a multiple of 4 elements: the attention of the 32-bit path.
+// (attention_simt.cu takes the other sizes, and bfloat16.)                                   (reference: ops.cu:101-147)
+//
+// A block takes one tile of rows, up to 64 (token, head of one key/value head's group) pairs of consecutive tokens of one
+// request, and walks their keys in blocks of 32 through shared memory: scores, then the row's maximum, exponentials and sum,
+// then the weighted values, all float32 multiply-adds.  The copies of the next keys run beside the exponentials and the values,
+// those of the next values beside the scores.  Tiles begin where a request's position is a multiple of the tile's tokens, found
+// by each block from the step's positions, so that no list has to be planned.
+//
+// A row's result has the same bits however its request is cut into steps and whatever lies beside it: a score is one chain over
+// d in ascending order, blocks of keys begin at multiples of 32, keys are taken in chunks that begin at multiples of CHUNK, and
+// the chunks' results (maximum, sum, weighted values) are joined in ascending order by the same arithmetic whether one block
+// walked them all or each had a block of its own (few rows with long contexts; a second kernel then joins them).
+//
+// Bound by the multiply-add pipe and shared memory for prompts, by the cache's bytes for decoded tokens.  Alone, 16 query and
+// 8 key/value heads of 128, one warp a (token, head) before and now: a prompt of 777 tokens 2,661 -> 190 us, of 2,000 16,388 -> 719
+// (23 TFLOP/s), 512 tokens behind 1,536 8,094 -> 366; one token behind 4,000 2,120 -> 105, 8 tokens behind 2,000 1,723 -> 130,
+// 64 tokens behind 256 325 -> 127.
+#include "common.cuh"
+
+#include <type_traits>
+
+namespace {
+
+constexpr int ROWS = 64, KEYS = 32, CHUNK = 512, THREADS = 256, FEW_ROWS = 8;
+constexpr int P_PITCH = KEYS + 4;
+
+template <int D> constexpr int smem_floats() { return ROWS * (D + 4) + KEYS * (D + 4) + KEYS * D + ROWS * P_PITCH; }
+
+__device__ __forceinline__ void copy16(float* to, const float* from, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from), "r"(live ? 16 : 0));
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+// exp(a - b) where a may be -inf (nothing there): 0
+__device__ __forceinline__ float ratio(float a, float b) { return a == -CUDART_INF_F ? 0.0f : expf(a - b); }
+// what both ways of joining chunks compute for an element
+__device__ __forceinline__ float join(float total, float keep, float part, float take) { return fmaf(part, take, total * keep); }
+
+struct Args {
+    const float *q, *k, *v;
+    const int *positions, *seq_of_token, *table;
+    float *out, *part_o, *part_ml;               // [tokens, nq, chunks, d], [tokens, nq, chunks, 2]
+    int tokens, nq, nkv, d, page_size, table_width, window, tile_tokens, chunks;
+    float scale;
+};
+
+// SPLIT: a block takes one chunk (blockIdx.z) of its tiles' keys and leaves its parts in part_o and part_ml; otherwise all of them.
+template <int D, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kernel(const Args A) {
+    constexpr int PITCH = D + 4, COLS = D / 16;          // columns of the output a thread has (rows in fours)
+    extern __shared__ __align__(16) float smem[];
+    float* q_s = smem;                                   // [ROWS][PITCH]
+    float* k_s = q_s + ROWS * PITCH;                     // [KEYS][PITCH]
+    float* v_s = k_s + KEYS * PITCH;                     // [KEYS][D]
+    float* p_s = v_s + KEYS * D;                         // [ROWS][P_PITCH]
+    float* total_s = p_s + ROWS * P_PITCH;               // !SPLIT: [4 * COLS][THREADS], a thread's own
+    __shared__ float keep_s[ROWS], take_s[ROWS];
+    __shared__ int found[2], warp_count[THREADS / 32];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = blockIdx.y, group = A.nq / A.nkv, d = A.d;
+    auto begins = [&](int t) {
+        if (t >= A.tokens) return true;
+        const int pos = A.positions[t];
+        return t == 0 || pos % A.tile_tokens == 0 || A.seq_of_token[t] != A.seq_of_token[t - 1] || pos != A.positions[t - 1] + 1;
+    };
+    for (int tile = blockIdx.x;; tile += gridDim.x) {
+        // ---- the tile-th of the step's tiles from the end (late tiles walk the most keys: they start first) ------------------
+        __syncthreads();                                 // what the tile before used has been read
+        if (tid == 0) found[0] = -1;
+        __syncthreads();
+        int before = 0;
+        for (int base = (A.tokens - 1) / THREADS * THREADS; base >= 0; base -= THREADS) {
+            const int t = base + tid;
+            const bool first = t < A.tokens && begins(t);
+            const int here = __syncthreads_count(first);
+            if (before + here > tile) {
+                const int wanted = here - 1 - (tile - before);           // from the front of these
+                const unsigned mask = __ballot_sync(0xffffffffu, first);
+                if (lane == 0) warp_count[warp] = __popc(mask);
+                __syncthreads();
+                int ahead = 0;
+                for (int w = 0; w < warp; ++w) ahead += warp_count[w];
+                if (first && ahead + __popc(mask & ((1u << lane) - 1u)) == wanted) found[0] = t;
+                break;
+            }
+            before += here;
+        }
+        __syncthreads();
+        const int t0 = found[0];
+        if (t0 < 0) return;
+        if (tid < 32) {                                  // tokens of the tile
+            int count = A.tile_tokens;
+            for (int i = 1 + lane; i < A.tile_tokens; i += 32)
+                if (begins(t0 + i)) { count = i; break; }
+            count = __reduce_min_sync(0xffffffffu, count);
+            if (lane == 0) found[1] = count;
+        }
+        __syncthreads();
+        const int tokens = found[1], rows = tokens * group;
+        const int pos0 = A.positions[t0], end_key = pos0 + tokens;
+        int begin = A.window > 0 ? max(0, pos0 + 1 - A.window) : 0, end = end_key;       // keys that some row sees
+        if (SPLIT) {
+            begin = max(begin, (int)blockIdx.z * CHUNK);     // keys beyond the last chunk that was planned go with it
+            if ((int)blockIdx.z + 1 < A.chunks) end = min(end, ((int)blockIdx.z + 1) * CHUNK);
+            if (begin >= end) continue;
+        }
+        const int* pages = A.table + (size_t)A.seq_of_token[t0] * A.table_width;
+        // row r: token t0 + r / group, head g * group + r % group
+        for (int i = tid; i < rows * (D / 4); i += THREADS) {
+            const int r = i / (D / 4), c = i % (D / 4) * 4;
+            float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (c < d) x = *reinterpret_cast<const float4*>(A.q + ((size_t)(t0 + r / group) * A.nq + g * group + r % group) * d + c);
+            *reinterpret_cast<float4*>(q_s + r * PITCH + c) = x;
+        }
+        // keys (or values) of the block that begins at key `at`, zeros outside begin .. end
+        auto fetch = [&](const float* __restrict__ cache, float* to, int pitch, int at) {
+            if (at < end) {
+                for (int i = tid; i < KEYS * (D / 4); i += THREADS) {
+                    const int j = i / (D / 4), c = i % (D / 4) * 4, p = at + j;
+                    const bool live = p >= begin && p < end && c < d;
+                    const float* from = cache;
+                    if (live) from += (((size_t)pages[p / A.page_size] * A.nkv + g) * A.page_size + p % A.page_size) * d + c;
+                    copy16(to + j * pitch + c, from, live);
+                }
+            }
+            copies_commit();
+        };
+        const bool few = rows <= FEW_ROWS;
+        // scores: a warp has 16 rows x 16 keys, lanes 4 x 8; few rows: a warp a row, a lane a key
+        const int s_row = (warp >> 1) * 16 + (lane >> 3), s_key = (warp & 1) * 16 + (lane & 7);
+        // values: a thread has rows o_row .. o_row + 3 and COLS columns in pieces of 4, 64 apart; few rows: a column of every
+        // FEW_STEP-th row
+        const int o_row = (warp * 2 + (lane >> 4)) * 4, o_col = (lane & 15) * 4;
+        constexpr int FEW_STEP = THREADS / D, FEW_OWN = FEW_ROWS / FEW_STEP;
+        const int f_col = tid % D, f_row = tid / D;
+        float o[4][COLS];                                // few rows: o_few[i] is row f_row + i * FEW_STEP
+        float* o_few = &o[0][0];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) {
+                o[i][c] = 0.0f;
+                if (!SPLIT) total_s[(i * COLS + c) * THREADS + tid] = 0.0f;
+            }
+        // a row's maximum and sum: four threads a row, eight keys of a block each
+        const int m_row = tid >> 2, m_key = (tid & 3) * 8;
+        float m = -CUDART_INF_F, l = 0.0f, m_all = -CUDART_INF_F, l_all = 0.0f;
+        const int m_pos = m_row < rows ? pos0 + m_row / group : -1;      // rows beyond the last see nothing
+        const int m_first = A.window > 0 ? max(0, m_pos + 1 - A.window) : 0;
+
+        int at = begin / KEYS * KEYS;
+        fetch(A.k, k_s, PITCH, at);
+        fetch(A.v, v_s, D, at);
+        for (; at < end; at += KEYS) {
+            copies_wait<1>();
+            __syncthreads();                             // the keys are there (and q)
+            if (few) {
+                if (warp < rows) {
+                    float s = 0.0f;
+#pragma unroll 8
+                    for (int e = 0; e < D; e += 4) {
+                        const float4 x = *reinterpret_cast<const float4*>(q_s + warp * PITCH + e), y = *reinterpret_cast<const float4*>(k_s + lane * PITCH + e);
+                        s = fmaf(x.x, y.x, s), s = fmaf(x.y, y.y, s), s = fmaf(x.z, y.z, s), s = fmaf(x.w, y.w, s);
+                    }
+                    p_s[warp * P_PITCH + lane] = s;
+                }
+            } else if ((warp >> 1) * 16 < rows) {
+                float s[4][2] = {};
+#pragma unroll 4
+                for (int e = 0; e < D; e += 4) {
+                    float4 y[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) y[j] = *reinterpret_cast<const float4*>(k_s + (s_key + 8 * j) * PITCH + e);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float4 x = *reinterpret_cast<const float4*>(q_s + (s_row + 4 * i) * PITCH + e);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.x, y[j].x, s[i][j]);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.y, y[j].y, s[i][j]);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.z, y[j].z, s[i][j]);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.w, y[j].w, s[i][j]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) p_s[(s_row + 4 * i) * P_PITCH + s_key + 8 * j] = s[i][j];
+            }
+            __syncthreads();                             // the scores are there, the keys have been read
+            fetch(A.k, k_s, PITCH, at + KEYS);
+            if (m_row < rows || !few) {
+                float* p = p_s + m_row * P_PITCH + m_key;
+                float x[8], top = -CUDART_INF_F;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int key = at + m_key + u;
+                    x[u] = key <= m_pos && key >= m_first ? p[u] * A.scale : -CUDART_INF_F;
+                    top = fmaxf(top, x[u]);
+                }
+                // the four threads of a row lie in one warp and take this branch together
+                const unsigned quad = 0xfu << (lane & 28);
+                top = fmaxf(top, __shfl_xor_sync(quad, top, 1));
+                top = fmaxf(top, __shfl_xor_sync(quad, top, 2));
+                const float next = fmaxf(m, top), alpha = m == next ? 1.0f : ratio(m, next);
+                float sum = 0.0f;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const float e = ratio(x[u], next);
+                    p[u] = e;
+                    sum += e;
+                }
+                sum += __shfl_xor_sync(quad, sum, 1);
+                sum += __shfl_xor_sync(quad, sum, 2);
+                l = l * alpha + sum;
+                m = next;
+                if ((tid & 3) == 0) keep_s[m_row] = alpha;
+            }
+            copies_wait<1>();
+            __syncthreads();                             // the weights and the values are there
+            // where some row does not see all of the block's keys, weights of zero are skipped: a value that a row does not
+            // see never reaches it, not even one that is no number
+            const bool masked = at + KEYS > pos0 + 1 || (A.window > 0 && at < end_key - A.window);
+            if (few) {
+                const int live = min(KEYS, end - at);
+                float f[FEW_OWN];
+#pragma unroll
+                for (int i = 0; i < FEW_OWN; ++i) f[i] = f_row + i * FEW_STEP < rows ? o_few[i] * keep_s[f_row + i * FEW_STEP] : 0.0f;
+                for (int j = 0; j < live; ++j) {
+                    const float y = v_s[j * D + f_col];
+#pragma unroll
+                    for (int i = 0; i < FEW_OWN; ++i) {
+                        const int r = f_row + i * FEW_STEP;
+                        if (r >= rows) continue;
+                        const float w = p_s[r * P_PITCH + j];
+                        if (!masked || w != 0.0f) f[i] = fmaf(w, y, f[i]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < FEW_OWN; ++i) o_few[i] = f[i];
+            } else if (o_row < rows) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float alpha = keep_s[o_row + i];
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) o[i][c] *= alpha;
+                }
+                auto keys = [&](auto skip) {
+#pragma unroll 2
+                    for (int j = 0; j < KEYS; j += 4) {
+                        float w[4][4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(p_s + (o_row + i) * P_PITCH + j);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+#pragma unroll
+                            for (int c = 0; c < COLS; c += 4) {
+                                float y[4];
+                                *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(v_s + (j + u) * D + o_col + 16 * c);
+#pragma unroll
+                                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                                    for (int b = 0; b < 4; ++b)
+                                        if (!decltype(skip)::value || w[i][u] != 0.0f) o[i][c + b] = fmaf(w[i][u], y[b], o[i][c + b]);
+                            }
+                    }
+                };
+                if (masked) keys(std::true_type{});
+                else keys(std::false_type{});
+            }
+            if (!SPLIT && (at + KEYS >= end || (at + KEYS) % CHUNK == 0)) {
+                // the chunk joins those before it
+                __syncthreads();                         // keep_s has been read
+                if ((tid & 3) == 0) {
+                    const float next = fmaxf(m_all, m), keep = m_all == next ? 1.0f : ratio(m_all, next), take = ratio(m, next);
+                    l_all = join(l_all, keep, l, take);
+                    m_all = next;
+                    keep_s[m_row] = keep;
+                    take_s[m_row] = take;
+                }
+                m = -CUDART_INF_F, l = 0.0f;
+                __syncthreads();
+#pragma unroll
+                for (int i = 0; i < 4 * COLS; ++i) {
+                    if (few && i >= FEW_OWN) continue;
+                    const int r = few ? min(f_row + i * FEW_STEP, ROWS - 1) : o_row + i / COLS;
+                    float& total = total_s[i * THREADS + tid];
+                    total = join(total, keep_s[r], o[i / COLS][i % COLS], take_s[r]);
+                    o[i / COLS][i % COLS] = 0.0f;
+                }
+            }
+            __syncthreads();                             // values, weights and factors have been read
+            fetch(A.v, v_s, D, at + KEYS);
+        }
+        copies_wait<0>();
+        auto row_of = [&](int r) { return (size_t)(t0 + r / group) * A.nq + g * group + r % group; };
+        if (SPLIT) {
+            auto place = [&](int r) { return row_of(r) * A.chunks + blockIdx.z; };
+            if ((tid & 3) == 0 && m_row < rows) {
+                A.part_ml[2 * place(m_row)] = m;
+                A.part_ml[2 * place(m_row) + 1] = l;
+            }
+            if (few) {
+#pragma unroll
+                for (int i = 0; i < FEW_OWN; ++i)
+                    if (f_row + i * FEW_STEP < rows && f_col < d) A.part_o[place(f_row + i * FEW_STEP) * d + f_col] = o_few[i];
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (o_row + i >= rows) continue;
+#pragma unroll
+                    for (int c = 0; c < COLS; c += 4)
+                        if (o_col + 16 * c < d)
+                            *reinterpret_cast<float4*>(A.part_o + place(o_row + i) * d + o_col + 16 * c) = make_float4(o[i][c], o[i][c + 1], o[i][c + 2], o[i][c + 3]);
+                }
+            }
+            continue;
+        }
+        __syncthreads();
+        if ((tid & 3) == 0) keep_s[m_row] = 1.0f / l_all;
+        __syncthreads();
+        if (few) {
+#pragma unroll
+            for (int i = 0; i < FEW_OWN; ++i) {
+                const int r = f_row + i * FEW_STEP;
+                if (r < rows && f_col < d) A.out[row_of(r) * d + f_col] = total_s[i * THREADS + tid] * keep_s[r];
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (o_row + i >= rows) continue;
+                const float inv = keep_s[o_row + i];
+#pragma unroll
+                for (int c = 0; c < COLS; c += 4) {
+                    if (o_col + 16 * c >= d) continue;
+                    float x[4];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) x[b] = total_s[(i * COLS + c + b) * THREADS + tid] * inv;
+                    *reinterpret_cast<float4*>(A.out + row_of(o_row + i) * d + o_col + 16 * c) = make_float4(x[0], x[1], x[2], x[3]);
+                }
+            }
+        }
+    }
+}
+
+// Joins a row's chunks in ascending order: a warp a (token, head).
+__global__ void attention_f32_join_kernel(const Args A) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= (long long)A.tokens * A.nq) return;
+    const int pos = A.positions[row / A.nq];
+    const int first = min((A.window > 0 ? max(0, pos + 1 - A.window) : 0) / CHUNK, A.chunks - 1), last = min(pos / CHUNK, A.chunks - 1);
+    const float* ml = A.part_ml + 2 * row * A.chunks;
+    float m_all = -CUDART_INF_F, l_all = 0.0f, total[8] = {};
+    for (int c = first; c <= last; ++c) {
+        const float m = ml[2 * c], next = fmaxf(m_all, m), keep = m_all == next ? 1.0f : ratio(m_all, next), take = ratio(m, next);
+        l_all = join(l_all, keep, ml[2 * c + 1], take);
+        m_all = next;
+        const float* o = A.part_o + (row * A.chunks + c) * A.d;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (lane + 32 * i < A.d) total[i] = join(total[i], keep, o[lane + 32 * i], take);
+    }
+    const float inv = 1.0f / l_all;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        if (lane + 32 * i < A.d) A.out[row * A.d + lane + 32 * i] = total[i] * inv;
+}
+
+template <int D, bool SPLIT>
+int launch(const Args& A, int tiles, void* stream) {
+    constexpr int SMEM = (smem_floats<D>() + (SPLIT ? 0 : THREADS * D / 4)) * (int)sizeof(float);
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    MRS_LAUNCH((attention_f32_kernel<D, SPLIT>), dim3(tiles, A.nkv, SPLIT ? A.chunks : 1), THREADS, SMEM, stream, A);
+    MRS_RETURN_LAUNCH_STATUS();
+}
+
+}  // namespace
+
+MRS_EXPORT int mrs_attention_f32_chunk() { return CHUNK; }
+
+// `parts`: null, or scratch of tokens * nq * chunks * (d + 2) floats; then every chunk of mrs_attention_f32_chunk() keys of a tile has
+// a block of its own (keys beyond `chunks` of them go with the last one: right, but no longer the same bits as in one walk).  `sequences`: rows of the block table.
+MRS_EXPORT int mrs_attention_f32(const float* q, const float* k_cache, const float* v_cache, const int* positions, const int* seq_of_token,
+                                 const int* block_table, float* out, float* parts, int chunks, int tokens, int sequences, int nq, int nkv, int d,
+                                 int page_size, int table_width, float scale, int window, void* stream) {
+    if (tokens <= 0) return 0;
+    if (d <= 0 || d % 4 || d > 256 || nkv <= 0 || nkv > 65535 || nq <= 0 || nq % nkv || nq / nkv > ROWS || page_size <= 0 || sequences < 0 ||
+        (parts && (chunks <= 0 || chunks > 65535)) || (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out | (uintptr_t)parts) & 15))
+        return MRS_BAD_ARGUMENT;
+    Args A = {};
+    A.q = q, A.k = k_cache, A.v = v_cache, A.positions = positions, A.seq_of_token = seq_of_token, A.table = block_table, A.out = out;
+    A.tokens = tokens, A.nq = nq, A.nkv = nkv, A.d = d, A.page_size = page_size, A.table_width = table_width, A.window = window, A.scale = scale;
+    A.tile_tokens = ROWS / (nq / nkv);
+    A.chunks = parts ? chunks : 1;
+    A.part_o = parts, A.part_ml = parts ? parts + (size_t)tokens * nq * chunks * d : nullptr;
+    // a request's rows make at most two tiles that are not whole; rows that lie otherwise make more, and blocks take several
+    const long long most = (long long)tokens / A.tile_tokens + 2LL * sequences + 1;
+    const int tiles = (int)(most < tokens ? most : tokens);
+    const int code = d <= 64 ? (parts ? launch<64, true>(A, tiles, stream) : launch<64, false>(A, tiles, stream))
+                   : d <= 128 ? (parts ? launch<128, true>(A, tiles, stream) : launch<128, false>(A, tiles, stream))
+                              : (parts ? launch<256, true>(A, tiles, stream) : launch<256, false>(A, tiles, stream));
+    if (code != 0 || !parts) return code;
+    MRS_LAUNCH(attention_f32_join_kernel, (unsigned)(((long long)tokens * nq + 3) / 4), 128, 0, stream, A);
+    MRS_RETURN_LAUNCH_STATUS();
+}

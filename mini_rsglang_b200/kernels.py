@@ -28,6 +28,9 @@ _SIGNATURES = {
     "mrs_silu_mul": [_c_int, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_vp],
     "mrs_attention_simt": [_c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int,
                            _c_int, _c_int, _c_float, _c_int, _c_vp],
+    "mrs_attention_f32": [_c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
+                          _c_int, _c_int, _c_float, _c_int, _c_vp],
+    "mrs_attention_f32_chunk": [],
     "mrs_gemm_f32": [_c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_vp],
     "mrs_argmax": [_c_vp, _c_vp, _c_int, _c_int, _c_vp],
     "mrs_sample": [_c_vp, _c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp],
@@ -238,10 +241,17 @@ def silu_mul(gate_up: torch.Tensor, out: torch.Tensor, block: int = 0) -> None:
                                   _stream()), "silu_mul")
 
 
+ATTENTION_F32_PARTS_BYTES = 64 << 20       # scratch up to which the chunks of a row's keys get blocks of their own
+
+
 def attention_simt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, positions: torch.Tensor,
                    seq_of_token: torch.Tensor, block_table: torch.Tensor, out: torch.Tensor, nq: int, nkv: int,
-                   d: int, window: int = 0, scale: float | None = None) -> None:
-    """Causal paged attention; one warp per (token, head); any sizes; float32 or bfloat16."""
+                   d: int, window: int = 0, scale: float | None = None, longest: int = 0) -> None:
+    """Causal paged attention on the CUDA cores; any sizes; float32 or bfloat16.  float32 with heads of a multiple of 4
+    elements and up to 64 query heads a key/value head takes tiles of rows (`attention_f32.cu`), the rest one warp a (token,
+    head).  `longest`: keys of the longest row as far as the host knows (0: the block table's width); with few rows and long
+    contexts the keys are then shared among blocks in chunks, and a second kernel joins them."""
+    global launch_count
     tokens = q.shape[0]
     _need(q, None, "q", (tokens, nq * d))
     _need(k_cache, q.dtype, "k cache")
@@ -253,11 +263,26 @@ def attention_simt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
     page_size = k_cache.shape[2]
     if tuple(k_cache.shape[1:]) != (nkv, page_size, d):
         raise InvalidRequest("attention: cache shape does not match heads/head_dim")
-    _check(library().mrs_attention_simt(_is_bf16(q.dtype), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
-                                        positions.data_ptr(), seq_of_token.data_ptr(), block_table.data_ptr(),
-                                        out.data_ptr(), tokens, nq, nkv, d, page_size, block_table.shape[1],
-                                        float(scale if scale is not None else 1.0 / math.sqrt(d)), int(window),
-                                        _stream()), "attention_simt")
+    scale = float(scale if scale is not None else 1.0 / math.sqrt(d))
+    lib = library()
+    if q.dtype is torch.float32 and d % 4 == 0 and d <= 256 and nkv > 0 and nq % nkv == 0 and nq // nkv <= 64 and \
+            not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) & 15:
+        # A prompt of 777 rows of 16 heads walks at most two chunks: 26 tiles x 8 heads are 1.4 rounds of SMs, with blocks a
+        # chunk 2.1 shorter ones.  Many rows have blocks enough, and their parts would cost more than they bring.
+        chunks = -(-(longest or block_table.shape[1] * page_size) // int(lib.mrs_attention_f32_chunk()))
+        floats = tokens * nq * chunks * (d + 2)
+        parts = None
+        if chunks > 1 and 4 * floats <= ATTENTION_F32_PARTS_BYTES:
+            parts = torch.empty(floats, dtype=torch.float32, device=q.device)
+            launch_count += 1
+        _check(lib.mrs_attention_f32(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), positions.data_ptr(), seq_of_token.data_ptr(),
+                                     block_table.data_ptr(), out.data_ptr(), _ptr(parts), chunks, tokens, block_table.shape[0], nq, nkv, d,
+                                     page_size, block_table.shape[1], scale, int(window), _stream()), "attention_f32")
+        return
+    _check(lib.mrs_attention_simt(_is_bf16(q.dtype), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+                                  positions.data_ptr(), seq_of_token.data_ptr(), block_table.data_ptr(),
+                                  out.data_ptr(), tokens, nq, nkv, d, page_size, block_table.shape[1],
+                                  scale, int(window), _stream()), "attention_simt")
 
 
 def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:

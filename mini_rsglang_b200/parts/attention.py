@@ -258,7 +258,8 @@ def paged_attention(q, cache, ctx, out, nq: int, nkv: int, d: int, window: int, 
     if (scale is not None or cap or sinks is not None) and (q.dtype is not torch.bfloat16 or not fast_kernels_take(d, group, cache.k.shape[2])):
         raise InvalidRequest("a scale of its own, a soft cap or sinks need the kernels that are fed by bulk tensor copies")
     if q.dtype is not torch.bfloat16 or not kernels.attention_mma_supported(d, group):
-        kernels.attention_simt(q, cache.k, cache.v, ctx.positions, ctx.seq_of_token, table, out, nq, nkv, d, window)
+        kernels.attention_simt(q, cache.k, cache.v, ctx.positions, ctx.seq_of_token, table, out, nq, nkv, d, window,
+                               longest=ctx.max_context_len)
         return
     page_size = cache.k.shape[2]
     sms = kernels.sm_count(q.device)

@@ -338,6 +338,35 @@ def test_attention_simt(dtype, nq, nkv, d, page):
     close(case.run_simt(), case.plain(), dtype, "attention_simt")
 
 
+@pytest.mark.parametrize("nq,nkv,d,page,window", [(4, 2, 128, 16, 0), (16, 8, 128, 16, 0), (5, 1, 64, 8, 0), (12, 1, 96, 4, 0), (64, 1, 36, 16, 0),
+                                                  (3, 3, 256, 32, 0), (4, 2, 128, 16, 700), (2, 1, 20, 4, 37)])
+def test_attention_f32_gives_a_row_the_same_bits_in_every_cut(monkeypatch, nq, nkv, d, page, window):
+    """Tiles of rows that begin and end anywhere, single tokens, contexts on both sides of a chunk's and a block's end; a row's
+    bits are the same as a single token, inside a prompt, beside other requests, with a chunk's keys in blocks of their own or
+    in one walk; a value behind a row's last key does not reach it, not even one that is no number."""
+    spans = [(0, 1), (511, 2), (0, 130), (1030, 1), (480, 77), (1535, 1), (96, 1), (31, 33)]
+    case = PagedCase(torch.float32, nq, nkv, d, page, spans, seed=d + window, window=window)
+    got = case.run_simt()
+    close(got, case.plain(), torch.float32, "attention_f32")
+    monkeypatch.setattr(kernels, "ATTENTION_F32_PARTS_BYTES", 0)
+    assert torch.equal(got, case.run_simt())
+    monkeypatch.undo()
+    q, table = case.dev(case.q.reshape(-1, nq * d)), case.dev(case.table)
+    for row in (0, 2, 3, 130, 133, 134, 150, 210, 211, 212, 213, 230, q.shape[0] - 1):
+        seq, position = int(case.seq[row]), int(case.positions[row])
+        kc, vc = case.kc.clone(), case.vc.clone()
+        length = spans[seq][0] + spans[seq][1]
+        for p in range(position + 1, length):                      # what the request's later tokens left behind this one
+            kc[case.table[seq, p // page], :, p % page] = float("inf")
+            vc[case.table[seq, p // page], :, p % page] = float("nan")
+        first = max(0, row - (position - spans[seq][0]))             # the request's rows up to this one, in one step
+        for rows in (slice(row, row + 1), slice(first, row + 1), slice(first, case.q_start[seq + 1])):
+            out = torch.empty(rows.stop - rows.start, nq * d, device=DEV)
+            kernels.attention_simt(q[rows].clone(), case.dev(kc), case.dev(vc), case.dev(case.positions)[rows].clone(), case.dev(case.seq)[rows].clone(),
+                                   table, out, nq, nkv, d, window, longest=length)
+            assert torch.equal(out[row - rows.start], got[row]), (row, rows)
+
+
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_attention_window_edges(window):
     for dtype in DTYPES:

@@ -185,7 +185,7 @@ def kernel_library() -> ctypes.CDLL:
 
 HYBRID_KERNEL_SOURCES = ("hybrid_elementwise.cu", "ssm_scan.cu")
 LATENT_KERNEL_SOURCES = ("latent_elementwise.cu",)
-EXPERT_KERNEL_SOURCES = ("experts.cu", "experts_mma.cu")
+EXPERT_KERNEL_SOURCES = ("experts.cu", "experts_few.cu", "experts_mma.cu")
 PARALLEL_KERNEL_SOURCES = ("parallel_elementwise.cu",)
 DELTA_KERNEL_SOURCES = ("delta_rule.cu",)
 LINEAR_SCAN_KERNEL_SOURCES = ("linear_scan.cu",)

@@ -16,7 +16,7 @@
 //                  the first product is the ungated one over gathered rows with an activation on its sums, written at the
 //                  rows' places in the lists (`act` >= 0): act[row] = activation(W_up[e] x_rows[row]);
 //                  one kernel for every size (the 32-bit path), one for few rows an expert (decode steps: the
-//                  weights streamed once); the tensor-core versions are experts_mma.cu and experts_tc.cu
+//                  weights streamed once); the tensor-core versions are experts_few.cu, experts_mma.cu and experts_tc.cu
 //   moe_combine    out[token] = sum over its choices of weight * (y[pair] or, for an expert without weights, the
 //                  input itself) + shared gate * shared expert's output
 //

@@ -1483,6 +1483,7 @@ _EXPERT_SIGNATURES = {
     "mrs_moe_align": [_c_vp, _c_int, _c_int, _c_int, _c_vp, _c_vp, _c_int, _c_vp],
     "mrs_moe_product_simt": [_c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_vp],
     "mrs_moe_product_rows": [_c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_vp],
+    "mrs_moe_product_few": [_c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_vp],
     "mrs_moe_gather_rows": [_c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_vp],
     "mrs_moe_gather_scaled_rows": [_c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_vp],
     "mrs_moe_product_mma": [_c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_vp],
@@ -1680,6 +1681,13 @@ def moe_rows_supported(x: torch.Tensor, inner: int) -> bool:
     return x.shape[1] % piece == 0 and inner % piece == 0
 
 
+def moe_few_tile(pairs: int, routed: int) -> int:
+    """Rows of a tile of the tensor-core product for few rows: 8 up to 8 pairs an expert on average, 16 up to 16, else 32.  Both
+    products of 32 experts, tiles of 8, 16 and 32 rows: width 4,096, inner 1,536, 2 pairs an expert 189, 208 and 281 us, 8 pairs
+    230, 231 and 313, 12 pairs 284, 245 and 322, 24 pairs 440, 377 and 348."""
+    return 8 if pairs <= 8 * routed else (16 if pairs <= 16 * routed else 32)
+
+
 def moe_mma_supported(x: torch.Tensor, inner: int) -> bool:
     """bfloat16 with rows on 16-byte boundaries in both products: the width and the experts' inner size multiples of 8."""
     return x.dtype is torch.bfloat16 and x.shape[1] % 8 == 0 and inner % 8 == 0
@@ -1700,7 +1708,8 @@ def moe_product(x: torch.Tensor, sorted_rows: torch.Tensor, tile_expert: torch.T
                 top: int, gated: bool, kernel: str = "simt", block: int = 0, activation: str | None = None) -> None:
     """One product of the experts over the lists of `moe_align`: `kernel` "simt" (CUDA cores, tiles of `moe_simt_tile()`
     rows, every size), "rows" (CUDA cores, few rows an expert: tiles of `moe_rows_tile()` rows, the weights streamed once;
-    rows of a multiple of 16 bytes) or "mma" (mma.sync, bfloat16, k a multiple of 8, tiles of `moe_mma_tile()` rows).
+    rows of a multiple of 16 bytes), "few" (mma.sync on weights that go straight to registers, bfloat16, few rows an expert,
+    k a multiple of 8, tiles of 8, 16 or 32 rows) or "mma" (mma.sync, bfloat16, k a multiple of 8, tiles of `moe_mma_tile()` rows).
     `gated`: x [tokens, k], weight [experts, 2 n, k] (all gate rows, then all up rows; with `block`, blocks of that many
     gate rows each followed by the matching up rows), out [capacity, n] = silu(gate) * up of every listed pair's token;
     else x [capacity, k], weight [experts, n, k], out [pairs, n] written at the pair; or, with `activation` (one of
@@ -1722,6 +1731,12 @@ def moe_product(x: torch.Tensor, sorted_rows: torch.Tensor, tile_expert: torch.T
                                                     weight.data_ptr(), out.data_ptr(), capacity, n, k, top, int(block) if gated else 0,
                                                     act, _stream()), "moe_product_mma")
         return
+    if kernel == "few":
+        _need(x, torch.bfloat16, "expert input")
+        _check(expert_library().mrs_moe_product_few(int(gated), x.data_ptr(), sorted_rows.data_ptr(), tile_expert.data_ptr(),
+                                                    weight.data_ptr(), out.data_ptr(), capacity, capacity // (tile_expert.shape[0] - 1), n, k,
+                                                    top, int(block) if gated else 0, act, _stream()), "moe_product_few")
+        return
     if kernel == "rows":
         _check(expert_library().mrs_moe_product_rows(_is_bf16(x.dtype), int(gated), x.data_ptr(), sorted_rows.data_ptr(),
                                                      tile_expert.data_ptr(), weight.data_ptr(), out.data_ptr(), capacity, n, k, top,
@@ -1737,6 +1752,29 @@ def moe_product(x: torch.Tensor, sorted_rows: torch.Tensor, tile_expert: torch.T
 MOE_TC_BLOCK = 64              # gate rows of a block in the layout of the product for many rows; the 64 matching up rows follow
 MOE_TC_MIN_PAIRS = int(os.environ.get("MRS_MOE_TC_MIN_PAIRS", "1024"))      # the variables: for measuring other crossovers
 MOE_ROWS_MAX_PAIRS = int(os.environ.get("MRS_MOE_ROWS_MAX_PAIRS", "128"))
+
+
+def moe_kernel(x: torch.Tensor, pairs: int, routed: int, inner: int, tc: bool) -> str:
+    """Which kernel multiplies `pairs` (token, choice) pairs with `routed` experts; `tc`: the tcgen05 one takes these sizes.
+    bfloat16: tcgen05 from MOE_TC_MIN_PAIRS pairs on, up to 32 pairs an expert the weights straight to registers, mma.sync
+    between them; else the CUDA cores, with the weights streamed once up to 4 * MOE_ROWS_MAX_PAIRS pairs.  16 tokens x 4 choices
+    of 32 experts, width 4,096, inner 1,536: both products 189 us straight to registers, 298 on the CUDA cores, 503 with
+    mma.sync from shared memory (168 us for the weights' bytes)."""
+    if tc and pairs >= MOE_TC_MIN_PAIRS:
+        return "tc"
+    if moe_mma_supported(x, inner):
+        return "few" if pairs <= 32 * routed else "mma"
+    if moe_rows_supported(x, inner) and pairs <= 4 * MOE_ROWS_MAX_PAIRS:
+        return "rows"
+    return "simt"
+
+
+def _moe_tile(kernel: str, pairs: int, routed: int) -> int:
+    if kernel == "few":
+        return moe_few_tile(pairs, routed)
+    return 128 if kernel == "tc" else {"mma": moe_mma_tile, "simt": moe_simt_tile, "rows": moe_rows_tile}[kernel]()
+
+
 _moe_tc_lib = None
 _moe_tc_maps: dict[tuple, tuple] = {}
 
@@ -1837,13 +1875,8 @@ def moe_plain_experts(h: torch.Tensor, chosen: torch.Tensor, weights: torch.Tens
     tokens, top = chosen.shape
     inner = down.shape[2]
     if kernel is None:
-        if tokens * top <= MOE_ROWS_MAX_PAIRS and moe_rows_supported(h, inner):
-            kernel = "rows"
-        elif tokens * top >= MOE_TC_MIN_PAIRS and moe_plain_tc_supported(h, up, down):
-            kernel = "tc"
-        else:
-            kernel = "mma" if moe_mma_supported(h, inner) else ("rows" if moe_rows_supported(h, inner) and tokens * top <= 4 * MOE_ROWS_MAX_PAIRS else "simt")
-    tile = {"tc": 128, "mma": moe_mma_tile(), "simt": moe_simt_tile(), "rows": moe_rows_tile()}[kernel]
+        kernel = moe_kernel(h, tokens * top, routed, inner, moe_plain_tc_supported(h, up, down))
+    tile = _moe_tile(kernel, tokens * top, routed)
     capacity = moe_capacity(tokens * top, routed, tile)
     sorted_rows = torch.empty((capacity,), dtype=torch.int32, device=h.device)
     tile_expert = torch.empty((capacity // tile + 1,), dtype=torch.int32, device=h.device)
@@ -1876,19 +1909,13 @@ def moe_experts(h: torch.Tensor, chosen: torch.Tensor, gate_up: torch.Tensor, do
     choice] is one of the first `routed`; the other rows of y are left as they are.  `gate_up` [routed, 2 inner, width]
     (all gate rows, then all up rows; with `block`, blocks of that many gate rows each followed by the matching up rows),
     `down` [routed, width, inner].  `kernel`: "simt" (CUDA cores, every size and both dtypes), "rows" (CUDA cores, few rows
-    an expert, rows of a multiple of 16 bytes), "mma" (mma.sync, bfloat16, sizes of a multiple of 8), "tc" (tcgen05, bfloat16,
-    blocks of 64); None: up to MOE_ROWS_MAX_PAIRS pairs "rows", from MOE_TC_MIN_PAIRS pairs on "tc", between them "mma",
-    wherever they apply, else "simt"."""
+    an expert, rows of a multiple of 16 bytes), "few" (mma.sync, bfloat16, few rows an expert, sizes of a multiple of 8), "mma"
+    (mma.sync, bfloat16, sizes of a multiple of 8), "tc" (tcgen05, bfloat16, blocks of 64); None: `moe_kernel`'s choice."""
     tokens, top = chosen.shape
     inner = down.shape[2]
     if kernel is None:
-        if tokens * top <= MOE_ROWS_MAX_PAIRS and moe_rows_supported(h, inner):
-            kernel = "rows"
-        elif tokens * top >= MOE_TC_MIN_PAIRS and moe_tc_supported(h, gate_up, down, block):
-            kernel = "tc"
-        else:
-            kernel = "mma" if moe_mma_supported(h, inner) else ("rows" if moe_rows_supported(h, inner) and tokens * top <= 4 * MOE_ROWS_MAX_PAIRS else "simt")
-    tile = {"tc": 128, "mma": moe_mma_tile(), "simt": moe_simt_tile(), "rows": moe_rows_tile()}[kernel]
+        kernel = moe_kernel(h, tokens * top, routed, inner, moe_tc_supported(h, gate_up, down, block))
+    tile = _moe_tile(kernel, tokens * top, routed)
     capacity = moe_capacity(tokens * top, routed, tile)
     sorted_rows = torch.empty((capacity,), dtype=torch.int32, device=h.device)
     tile_expert = torch.empty((capacity // tile + 1,), dtype=torch.int32, device=h.device)

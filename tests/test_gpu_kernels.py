@@ -928,3 +928,43 @@ def test_sampler_distribution_ties_and_bad_rows():
     bad[0, 2] = float("inf")
     with pytest.raises(BackendError, match="nonfinite"):
         sampler.sample(bad, [params], [0])
+
+
+@pytest.mark.parametrize("per_expert", [1, 8, 9, 16, 17, 40])
+@pytest.mark.parametrize("experts,width,inner,block", [(3, 72, 40, 0), (2, 136, 64, 64), (4, 1032, 200, 0), (2, 4104, 128, 64), (1, 2048, 1032, 0)])
+def test_experts_for_few_rows(per_expert, experts, width, inner, block):
+    """The tensor-core product for few rows an expert over whole and filled-up tiles of 8, 16 and 32 rows, K split among 1, 2, 4
+    and 8 warps with a ragged end, columns beyond the last group, an expert without rows: silu(gate) * up and the down product
+    within bfloat16 rounding of the 64-bit result; ungated experts that read gathered rows likewise; a row's bits do not
+    depend on the other rows of its tile."""
+    g = torch.Generator(device=DEV).manual_seed(per_expert * 31 + width)
+    top = 2 if experts > 1 else 1
+    tokens = max(1, per_expert * experts // top)
+    h = torch.randn(tokens, width, device=DEV, generator=g).bfloat16()
+    gate, up = ((torch.randn(experts, inner, width, device=DEV, generator=g) * width ** -0.5).bfloat16() for _ in range(2))
+    down = (torch.randn(experts, width, inner, device=DEV, generator=g) * inner ** -0.5).bfloat16()
+    chosen = torch.stack([torch.randperm(experts, generator=g, device=DEV)[:top] for _ in range(tokens)]).int()
+    if experts > 3:
+        chosen = chosen % 3                                   # an expert without rows (and tokens that choose one twice)
+    if block:
+        laid = torch.stack([gate.view(experts, -1, block, width), up.view(experts, -1, block, width)], dim=2).reshape(experts, 2 * inner, width)
+    else:
+        laid = torch.cat([gate, up], dim=1)
+    y = torch.full((tokens * top, width), 77.0, device=DEV).bfloat16()
+    kernels.moe_experts(h, chosen, laid.contiguous(), down, y, experts, kernel="few", block=block)
+    plain = torch.full_like(y, 77.0)
+    kernels.moe_plain_experts(h, chosen, None, up, down, plain, experts, "relu", kernel="few")
+    pairs = chosen.view(-1).long()
+    x = h.repeat_interleave(top, dim=0).double()
+    z = torch.einsum("pw,piw->pi", x, gate.double()[pairs]).bfloat16().double()
+    u = torch.einsum("pw,piw->pi", x, up.double()[pairs])
+    act = (z * torch.sigmoid(z) * u.bfloat16().double()).bfloat16().double()
+    # three bfloat16 roundings on the way (gate, up, their product) and one at the end, each 2^-9 of its value
+    for got, inner_rows in ((y, act), (plain, torch.relu(u).bfloat16().double())):
+        want = torch.einsum("pi,pwi->pw", inner_rows, down.double()[pairs])
+        size = torch.einsum("pi,pwi->pw", inner_rows.abs(), down.double()[pairs].abs())
+        assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -7).all()
+    alone = torch.empty((top, width), device=DEV).bfloat16()
+    last = tokens - 1
+    kernels.moe_experts(h[last:].clone(), chosen[last:].clone(), laid.contiguous(), down, alone, experts, kernel="few", block=block)
+    assert torch.equal(alone, y[last * top:])

@@ -24,10 +24,13 @@ constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + (2 * STAGES 
 
 // x_map: the gathered rows [capacity, K]; w_map: the weights [experts * N, K]; N: weight rows an expert.
 // tile_expert [capacity / 128 + 1]: the expert of every tile of rows, then the number of tiles in use.
-template <bool GATED>
+// ACT: the activation's number, or -1.  It is a parameter of the kernel: chosen at run time, its five forms stood 256 times in the
+// unrolled epilogue, and jumping over them took a tile some 45 us of instruction fetches (128 tokens with
+// 4 of 32 experts: the down product of 2,048 x 1,024 106 -> 27 us, of 4,096 x 1,536 235 -> 73).
+template <bool GATED, int ACT>
 __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
     const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const int* __restrict__ tile_expert,
-    const int* __restrict__ sorted_rows, bf16* __restrict__ out, int m_tiles_all, int N, int K, int act) {
+    const int* __restrict__ sorted_rows, bf16* __restrict__ out, int m_tiles_all, int N, int K) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -161,8 +164,8 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
                     }
                 }
             } else {
-                bf16* dst = out + (size_t)(pair < 0 ? 0 : (act >= 0 ? m0 + row : pair)) * N + n0;
-#pragma unroll
+                bf16* dst = out + (size_t)(pair < 0 ? 0 : (ACT >= 0 ? m0 + row : pair)) * N + n0;
+#pragma unroll 2
                 for (int c = 0; c < BN; c += 32) {
                     float v[32];
                     tmem_load_32_async(acc + c, v);
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
                             uint32_t w[4];
 #pragma unroll
                             for (int p = 0; p < 4; ++p) {
-                                __nv_bfloat162 two = act >= 0 ? __floats2bfloat162_rn(mrs_activate(v[e + 2 * p], act), mrs_activate(v[e + 2 * p + 1], act))
+                                __nv_bfloat162 two = ACT >= 0 ? __floats2bfloat162_rn(mrs_activate(v[e + 2 * p], ACT), mrs_activate(v[e + 2 * p + 1], ACT))
                                                               : __floats2bfloat162_rn(v[e + 2 * p], v[e + 2 * p + 1]);
                                 w[p] = *reinterpret_cast<uint32_t*>(&two);
                             }
@@ -194,6 +197,19 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
         tcgen05_fence_after_sync();
         tmem_dealloc(tmem_base, TMEM_COLUMNS);
     }
+}
+
+template <bool GATED, int ACT>
+int launch(const CUtensorMap& x, const CUtensorMap& w, const int* tile_expert, const int* sorted_rows, void* out, int m_tiles, int N, int K,
+           int grid, void* stream) {
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(moe_product_tc_kernel<GATED, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    MRS_LAUNCH((moe_product_tc_kernel<GATED, ACT>), grid, THREADS, SMEM_BYTES, stream, x, w, tile_expert, sorted_rows, (bf16*)out, m_tiles, N, K);
+    MRS_RETURN_LAUNCH_STATUS();
 }
 
 }  // namespace
@@ -221,23 +237,19 @@ MRS_EXPORT int mrs_moe_product_tc(int gated, const void* x_map, const void* w_ma
     if (capacity % BM || K <= 0 || K % 8 || N <= 0 || (gated ? N % 128 : N % 8) || ctas < 1 || !x_map || !w_map || !out ||
         ((uintptr_t)out & 15) || act > 4 || (gated && act >= 0))
         return MRS_BAD_ARGUMENT;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(moe_product_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(moe_product_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
     const int m_tiles = capacity / BM;
     const long long tiles = (long long)m_tiles * ((N + BN - 1) / BN);
     const int grid = (int)(ctas < tiles ? ctas : tiles);
-    if (gated)
-        MRS_LAUNCH(moe_product_tc_kernel<true>, grid, THREADS, SMEM_BYTES, stream, *reinterpret_cast<const CUtensorMap*>(x_map),
-                   *reinterpret_cast<const CUtensorMap*>(w_map), tile_expert, sorted_rows, (bf16*)out, m_tiles, N, K, act);
-    else
-        MRS_LAUNCH(moe_product_tc_kernel<false>, grid, THREADS, SMEM_BYTES, stream, *reinterpret_cast<const CUtensorMap*>(x_map),
-                   *reinterpret_cast<const CUtensorMap*>(w_map), tile_expert, sorted_rows, (bf16*)out, m_tiles, N, K, act);
-    MRS_RETURN_LAUNCH_STATUS();
+    const CUtensorMap &x = *reinterpret_cast<const CUtensorMap*>(x_map), &w = *reinterpret_cast<const CUtensorMap*>(w_map);
+    if (gated) return launch<true, -1>(x, w, tile_expert, sorted_rows, out, m_tiles, N, K, grid, stream);
+    switch (act) {
+        case 0: return launch<false, 0>(x, w, tile_expert, sorted_rows, out, m_tiles, N, K, grid, stream);
+        case 1: return launch<false, 1>(x, w, tile_expert, sorted_rows, out, m_tiles, N, K, grid, stream);
+        case 2: return launch<false, 2>(x, w, tile_expert, sorted_rows, out, m_tiles, N, K, grid, stream);
+        case 3: return launch<false, 3>(x, w, tile_expert, sorted_rows, out, m_tiles, N, K, grid, stream);
+        case 4: return launch<false, 4>(x, w, tile_expert, sorted_rows, out, m_tiles, N, K, grid, stream);
+    }
+    return launch<false, -1>(x, w, tile_expert, sorted_rows, out, m_tiles, N, K, grid, stream);
 }
 
 MRS_EXPORT int mrs_moe_tc_take_error(unsigned int* word) { return mrs_take_error_word(word); }

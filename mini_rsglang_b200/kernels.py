@@ -1756,11 +1756,14 @@ MOE_ROWS_MAX_PAIRS = int(os.environ.get("MRS_MOE_ROWS_MAX_PAIRS", "128"))
 
 def moe_kernel(x: torch.Tensor, pairs: int, routed: int, inner: int, tc: bool) -> str:
     """Which kernel multiplies `pairs` (token, choice) pairs with `routed` experts; `tc`: the tcgen05 one takes these sizes.
-    bfloat16: tcgen05 from MOE_TC_MIN_PAIRS pairs on, up to 32 pairs an expert the weights straight to registers, mma.sync
+    bfloat16: tcgen05 from MOE_TC_MIN_PAIRS pairs on, or from 8 pairs an expert on where its tiles (128 inner columns an expert)
+    are as many as the SMs (both products of 32 experts, tcgen05 against the weights straight to registers: 4 pairs an expert
+    219 against 211 us at width 4,096, inner 1,536 and 86 against 78 at 2,048 and 1,024; 8 pairs 221 against 232 and 87 against
+    86; 12 pairs 222 against 247 and 87 against 92); up to 32 pairs an expert the weights straight to registers; mma.sync
     between them; else the CUDA cores, with the weights streamed once up to 4 * MOE_ROWS_MAX_PAIRS pairs.  16 tokens x 4 choices
     of 32 experts, width 4,096, inner 1,536: both products 189 us straight to registers, 298 on the CUDA cores, 503 with
     mma.sync from shared memory (168 us for the weights' bytes)."""
-    if tc and pairs >= MOE_TC_MIN_PAIRS:
+    if tc and (pairs >= MOE_TC_MIN_PAIRS or (pairs > 8 * routed and routed * (inner // 128) >= sm_count(x.device))):
         return "tc"
     if moe_mma_supported(x, inner):
         return "few" if pairs <= 32 * routed else "mma"

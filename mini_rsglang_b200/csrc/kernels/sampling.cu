@@ -123,17 +123,20 @@ MRS_EXPORT int mrs_argmax(const float* logits, int* out, int rows, int vocab, vo
 // through distributed shared memory.  What bounds it is the chain of those meetings: a row is read once (608 KB at
 // 151,936 logits), a threshold takes three digits of 11, 11 and 10 bits with two cluster barriers each.  One CTA a row,
 // which read the row from L2 some fifteen times with 8-bit digits, took 1,626 us for 24 rows of 151,936 logits (top-k and
-// top-p rows among them); this takes 87 us.
+// top-p rows among them); a cluster with weights added as floats and one warp that walked the drawn segment took 87 us,
+// whole numbers of 2^-34 and all warps at the segment take 81 (all 24 rows with top-k and top-p: 86; top-k alone 40, temperature
+// alone 25, greedy 10).
 //
 // The weights of the kept set are summed in 32 segments of a row, in id order, whatever the cluster's size: a row's token
 // does not depend on how many CTAs shared it.
 // ------------------------------------------------------------------------------------------------
 #define SAMPLE_CTA_THREADS 512
 #define SAMPLE_CTA_WARPS (SAMPLE_CTA_THREADS / 32)
+#define SAMPLE_MAX_BLOCKS 8
 #define SAMPLE_SEGMENTS 32
 #define SAMPLE_BINS 2048
 #define SAMPLE_OWN_BINS (SAMPLE_BINS / SAMPLE_CTA_THREADS)     // bins a thread looks at when the edge is searched
-#define SAMPLE_SHARE_BYTES (96 * 1024)                         // of a row in a CTA's shared memory, at most: two CTAs an SM
+#define SAMPLE_SHARE_BYTES (160 * 1024)                        // of a row in a CTA's shared memory, at most (up to 77 KB two CTAs fit an SM)
 #define SAMPLE_NOT_KEPT (-1.0f)
 
 // Which elements are kept: keys above `low`, and the first `quota` ids among keys equal to `low`.
@@ -142,21 +145,31 @@ struct Cut {
     int quota;
 };
 
+// A weight (0 .. 1) as a whole number of 2^-(2 bits): a high and a low part of `bits` bits each, whose sums over a CTA's share fit
+// 32 bits (native additions in shared memory; sums of whole numbers do not depend on their order).
+struct Fixed {
+    unsigned high, low;
+};
+__device__ __forceinline__ Fixed fixed_weight(float w, float scale) {
+    const float x = w * scale, whole = floorf(x);                       // scale is a power of two: both exact
+    return Fixed{(unsigned)whole, __float2uint_rn((x - whole) * scale)};
+}
+
 struct SampleShared {
-    Best warp_best[33];                              // block_argmax's
-    Best best;                                       // of this CTA's share; read by the whole cluster, as are the next five
+    Best warp_best[33];                              // block_best's
+    Best best;                                       // of this CTA's share; read by the whole cluster, as are the next nine
     int bad;
     unsigned count[SAMPLE_BINS];                     // this CTA's histogram
-    float weight[SAMPLE_BINS];
+    unsigned high[SAMPLE_BINS], low[SAMPLE_BINS];
     unsigned slice_count[SAMPLE_BINS / 4];           // this CTA's slice of the bins, summed over the cluster
-    float slice_weight[SAMPLE_BINS / 4];
+    unsigned long long slice_weight[SAMPLE_BINS / 4];
     int seg_ties[SAMPLE_SEGMENTS];                   // this CTA's segments
     float seg_weight[SAMPLE_SEGMENTS];
     unsigned warp_count[SAMPLE_CTA_WARPS];           // scan over the bins
-    float warp_weight[SAMPLE_CTA_WARPS];
+    unsigned long long warp_weight[SAMPLE_CTA_WARPS];
     int first, lowest;                               // places in descending order of the bins
     unsigned edge_count, above_count;
-    float above_weight;
+    unsigned long long above_weight;
     int all_ties[SAMPLE_SEGMENTS];
     float all_weight[SAMPLE_SEGMENTS];
 };
@@ -166,106 +179,110 @@ struct SampleShared {
 struct Edge {
     unsigned prefix, mask, count;     // `count`: elements of the last digit's bin
     unsigned above_count;
-    float above_weight, total;
+    unsigned long long above_weight, total;
+    double target;                    // weight, in the same units, that the edge has to reach
 };
 
-// One digit.  `f(add)` walks this CTA's elements and calls add(key, weight) for those to be counted (the digit's place is
-// applied here); by weight the first bin (from the top) whose running weight reaches target(total of all bins) is chosen,
-// by count the first whose running count reaches `wanted`.  `extra_key`, `extra_weight`: a run of equal keys that the
-// elements leave out, added to its bin once.
-template <bool BY_WEIGHT, typename Walk, typename Target>
+// One digit.  `walk_elements(add)` walks this CTA's elements and calls add(key, w) for those to be counted, w() being an element's
+// weight (the digit's place is applied here); by weight the first bin (from the top) whose running weight reaches
+// `share` of all the weight (a float32 product) is chosen, by count the first whose running count reaches `wanted`.  `extra_key`, `extra_weight`: a
+// run of equal keys that the elements leave out, added to its bin once.
+template <bool BY_WEIGHT, typename Walk>
 __device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsigned rank, unsigned blocks, int shift, int bits, Edge& e,
-                             Walk walk_elements, Target target, unsigned wanted, bool has_extra, unsigned extra_key, float extra_weight) {
+                             Walk walk_elements, int weight_bits, float share, unsigned wanted, bool has_extra, unsigned extra_key,
+                             unsigned long long extra_weight) {
     const unsigned digit = (1u << bits) - 1u;
+    const float scale = (float)(1u << weight_bits);
+    const double unit = 1.0 / ((double)scale * (double)scale);
     for (int b = threadIdx.x; b < SAMPLE_BINS; b += SAMPLE_CTA_THREADS) {
         s.count[b] = 0u;
-        if (BY_WEIGHT) s.weight[b] = 0.0f;
+        if (BY_WEIGHT) s.high[b] = 0u, s.low[b] = 0u;
     }
     if (threadIdx.x == 0) s.first = 0x7fffffff, s.lowest = -1;
     __syncthreads();
-    walk_elements([&](unsigned key, float w) {
+    walk_elements([&](unsigned key, auto weight) {
         if ((key & e.mask) != e.prefix) return;
         const unsigned b = (key >> shift) & digit;
         atomicAdd(&s.count[b], 1u);
-        if (BY_WEIGHT) atomicAdd(&s.weight[b], w);
-    });
-    if (has_extra && rank == 0) {
-        __syncthreads();
-        if (threadIdx.x == 0 && (extra_key & e.mask) == e.prefix) {
-            s.count[(extra_key >> shift) & digit] += 1u;
-            if (BY_WEIGHT) s.weight[(extra_key >> shift) & digit] += extra_weight;
+        if (BY_WEIGHT) {
+            const Fixed w = fixed_weight(weight(), scale);
+            if (w.high) atomicAdd(&s.high[b], w.high);
+            if (w.low) atomicAdd(&s.low[b], w.low);
         }
-    }
+    });
+    const bool extra = BY_WEIGHT && has_extra && (extra_key & e.mask) == e.prefix;
+    const int extra_bin = (int)((extra_key >> shift) & digit);
     if (blocks > 1) {
         cluster.sync();
         const int slice = SAMPLE_BINS / blocks;
         for (int i = threadIdx.x; i < slice; i += SAMPLE_CTA_THREADS) {
             unsigned c = 0u;
-            float w = 0.0f;
-            for (unsigned r = 0; r < blocks; ++r) {
+            unsigned long long high = 0ull, low = 0ull;
+#pragma unroll
+            for (unsigned r = 0; r < SAMPLE_MAX_BLOCKS; ++r) {       // all loads under way together
+                if (r >= blocks) continue;
                 c += cluster.map_shared_rank(s.count, r)[rank * slice + i];
-                if (BY_WEIGHT) w += cluster.map_shared_rank(s.weight, r)[rank * slice + i];
+                if (BY_WEIGHT) high += cluster.map_shared_rank(s.high, r)[rank * slice + i], low += cluster.map_shared_rank(s.low, r)[rank * slice + i];
             }
             s.slice_count[i] = c;
-            if (BY_WEIGHT) s.slice_weight[i] = w;
+            if (BY_WEIGHT) s.slice_weight[i] = (high << weight_bits) + low;
         }
         cluster.sync();
     } else {
         __syncthreads();
     }
     // bins from the top: thread t has places 4 t .. 4 t + 3, place p is bin BINS - 1 - p
-    unsigned c[SAMPLE_OWN_BINS];
-    float w[SAMPLE_OWN_BINS];
-    unsigned c_sum = 0u;
-    float w_sum = 0.0f;
+    unsigned c[SAMPLE_OWN_BINS], c_sum = 0u;
+    unsigned long long w[SAMPLE_OWN_BINS], w_sum = 0ull;
 #pragma unroll
     for (int j = 0; j < SAMPLE_OWN_BINS; ++j) {
         const int bin = SAMPLE_BINS - 1 - ((int)threadIdx.x * SAMPLE_OWN_BINS + j);
+        w[j] = 0ull;
         if (blocks > 1) {
             const int slice = SAMPLE_BINS / blocks;
             c[j] = cluster.map_shared_rank(s.slice_count, bin / slice)[bin % slice];
-            w[j] = BY_WEIGHT ? cluster.map_shared_rank(s.slice_weight, bin / slice)[bin % slice] : 0.0f;
+            if (BY_WEIGHT) w[j] = cluster.map_shared_rank(s.slice_weight, bin / slice)[bin % slice];
         } else {
             c[j] = s.count[bin];
-            w[j] = BY_WEIGHT ? s.weight[bin] : 0.0f;
+            if (BY_WEIGHT) w[j] = ((unsigned long long)s.high[bin] << weight_bits) + s.low[bin];
         }
+        if (extra && bin == extra_bin) c[j] += 1u, w[j] += extra_weight;
         c_sum += c[j];
         w_sum += w[j];
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned c_run = c_sum;
-    float w_run = w_sum;
+    unsigned long long w_run = w_sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const unsigned cu = __shfl_up_sync(0xffffffffu, c_run, o);
-        const float wu = __shfl_up_sync(0xffffffffu, w_run, o);
-        if (lane >= o) c_run += cu, w_run += wu;
+        if (lane >= o) c_run += cu;
+        if (BY_WEIGHT) {
+            const unsigned long long wu = __shfl_up_sync(0xffffffffu, w_run, o);
+            if (lane >= o) w_run += wu;
+        }
     }
     if (lane == 31) s.warp_count[warp] = c_run, s.warp_weight[warp] = w_run;
-    unsigned c_at = __shfl_up_sync(0xffffffffu, c_run, 1);
-    float w_at = __shfl_up_sync(0xffffffffu, w_run, 1);
-    if (lane == 0) c_at = 0u, w_at = 0.0f;
     __syncthreads();
-    unsigned c_before = 0u;
-    float w_before = 0.0f, w_total = 0.0f;
+    unsigned c_before = c_run - c_sum;
+    unsigned long long w_before = w_run - w_sum, w_total = 0ull;
     for (int i = 0; i < SAMPLE_CTA_WARPS; ++i) {
-        if (i == warp) c_before = c_at, w_before = w_total + w_at;
-        if (i < warp) c_at += s.warp_count[i];
-        w_total += s.warp_weight[i];
+        if (i < warp) c_before += s.warp_count[i], w_before += s.warp_weight[i];
+        if (BY_WEIGHT) w_total += s.warp_weight[i];
     }
-    c_before = c_at;
     if (e.mask == 0u) e.total = w_total;
-    const float goal = BY_WEIGHT ? target(e.total) - e.above_weight : 0.0f;
+    if (BY_WEIGHT && e.mask == 0u) e.target = (double)(share * (float)((double)e.total * unit)) / unit;
+    const double goal = BY_WEIGHT ? e.target - (double)e.above_weight : 0.0;
     const unsigned need = wanted - e.above_count;
     {
         unsigned ca = c_before;
-        float wa = w_before;
+        unsigned long long wa = w_before;
         int found = 0x7fffffff, last = -1;
 #pragma unroll
         for (int j = 0; j < SAMPLE_OWN_BINS; ++j) {
             if (c[j] == 0u) continue;
             last = (int)threadIdx.x * SAMPLE_OWN_BINS + j;
-            if (found == 0x7fffffff && (BY_WEIGHT ? wa + w[j] >= goal : ca + c[j] >= need)) found = last;
+            if (found == 0x7fffffff && (BY_WEIGHT ? (double)(wa + w[j]) >= goal : ca + c[j] >= need)) found = last;
             ca += c[j];
             wa += w[j];
         }
@@ -276,7 +293,7 @@ __device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsign
     const int place = s.first != 0x7fffffff ? s.first : max(s.lowest, 0);      // rounding left the sum a hair short: the last bin holds the edge
     if (place / SAMPLE_OWN_BINS == (int)threadIdx.x) {
         unsigned ca = c_before, here = 0u;
-        float wa = w_before;
+        unsigned long long wa = w_before;
 #pragma unroll
         for (int j = 0; j < SAMPLE_OWN_BINS; ++j) {
             if ((int)threadIdx.x * SAMPLE_OWN_BINS + j < place) ca += c[j], wa += w[j];
@@ -299,7 +316,7 @@ __device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsign
 // otherwise a row is too long for that and is read from memory each time.
 template <bool IN_SHARED>
 __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
-    const float* __restrict__ logits, int vocab, int per_segment, const float* __restrict__ temperature,
+    const float* __restrict__ logits, int vocab, int per_segment, int weight_bits, const float* __restrict__ temperature,
     const int* __restrict__ top_k, const float* __restrict__ top_p, const unsigned long long* __restrict__ seed,
     const int* __restrict__ draw_index, int* __restrict__ out) {
     pdl_launch_dependents();
@@ -347,7 +364,9 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     if (blocks > 1) cluster.sync();
     else __syncthreads();
     Best top = s.best;
-    for (unsigned q = 0; q < blocks; ++q) {
+#pragma unroll
+    for (unsigned q = 0; q < SAMPLE_MAX_BLOCKS; ++q) {
+        if (q >= blocks) continue;
         top = better(top, *cluster.map_shared_rank(&s.best, q));
         bad |= *cluster.map_shared_rank(&s.bad, q);
     }
@@ -362,45 +381,53 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     auto weight_of = [&](float v) { return expf((v - top.value) * inv_t); };
 
     // ---- top_k: the k-th largest key by count ------------------------------------------------
+    // Kept are the keys from cut.low on; of those equal to it, where there are more than `quota`, the first ids.
     Cut cut = {0u, 0x7fffffff};
-    int ties = 0;                                    // elements of the row whose key is cut.low
-    const bool by_count = k_raw > 0 && k_raw < vocab;
-    if (by_count) {
-        Edge e = {0u, 0u, 0u, 0u, 0.0f, 0.0f};
+    int ties = 0;                                    // elements of the row whose key is cut.low, where some of them may be left out
+    if (k_raw > 0 && k_raw < vocab) {
+        Edge e = {0u, 0u, 0u, 0u, 0ull, 0ull, 0.0};
         auto each = [&](auto add) {
 #pragma unroll 4
-            for (int i = threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) add(ordered_key(x[i]), 0.0f);
+            for (int i = threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) add(ordered_key(x[i]), [] { return 0.0f; });
         };
-        auto none = [](float) { return 0.0f; };
-        sample_digit<false>(cluster, s, rank, blocks, 21, 11, e, each, none, (unsigned)k_raw, false, 0u, 0.0f);
-        sample_digit<false>(cluster, s, rank, blocks, 10, 11, e, each, none, (unsigned)k_raw, false, 0u, 0.0f);
-        sample_digit<false>(cluster, s, rank, blocks, 0, 10, e, each, none, (unsigned)k_raw, false, 0u, 0.0f);
-        cut.low = e.prefix;
-        cut.quota = k_raw - (int)e.above_count;
-        ties = (int)e.count;
+        sample_digit<false>(cluster, s, rank, blocks, 21, 11, e, each, 0, 0.0f, (unsigned)k_raw, false, 0u, 0ull);
+        sample_digit<false>(cluster, s, rank, blocks, 10, 11, e, each, 0, 0.0f, (unsigned)k_raw, false, 0u, 0ull);
+        if (e.above_count + e.count == (unsigned)k_raw) {
+            cut.low = e.prefix;                      // all keys of the bin are kept, whatever their last digit
+        } else {
+            sample_digit<false>(cluster, s, rank, blocks, 0, 10, e, each, 0, 0.0f, (unsigned)k_raw, false, 0u, 0ull);
+            cut.low = e.prefix;
+            cut.quota = k_raw - (int)e.above_count;
+            ties = (int)e.count;
+        }
     }
 
     // ---- top_p: the key at which the running weight reaches top_p times the top_k set's weight ---
     if (p_raw < 1.0f) {
-        Edge e = {0u, 0u, 0u, 0u, 0.0f, 0.0f};
+        Edge e = {0u, 0u, 0u, 0u, 0ull, 0ull, 0.0};
+        const float scale = (float)(1u << weight_bits);
+        auto units = [&](float w) {
+            const Fixed f = fixed_weight(w, scale);
+            return ((unsigned long long)f.high << weight_bits) + f.low;
+        };
+        const bool some = cut.quota < ties;          // only some of the equals at the cut: they are added as one
         const unsigned low = cut.low;
-        const float low_weight = by_count ? weight_of(key_value(low)) * (float)cut.quota : 0.0f;       // the kept ones among equals
+        const unsigned long long low_weight = some ? units(weight_of(key_value(low))) * (unsigned long long)cut.quota : 0ull;
         auto each = [&](auto add) {
 #pragma unroll 4
             for (int i = threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) {
                 const float v = x[i];
                 const unsigned key = ordered_key(v);
-                if (key > low && (key & e.mask) == e.prefix) add(key, weight_of(v));
+                if (some ? key > low : key >= low) add(key, [&] { return weight_of(v); });
             }
         };
-        auto target = [&](float total) { return p_raw * total; };
-        sample_digit<true>(cluster, s, rank, blocks, 21, 11, e, each, target, 0u, by_count, low, low_weight);
-        sample_digit<true>(cluster, s, rank, blocks, 10, 11, e, each, target, 0u, by_count, low, low_weight);
-        sample_digit<true>(cluster, s, rank, blocks, 0, 10, e, each, target, 0u, by_count, low, low_weight);
-        const float one = weight_of(key_value(e.prefix));
-        int need = (int)ceilf((p_raw * e.total - e.above_weight) / one);
-        if (need < 1) need = 1;
-        if (by_count && e.prefix == cut.low) {
+        sample_digit<true>(cluster, s, rank, blocks, 21, 11, e, each, weight_bits, p_raw, 0u, some, low, low_weight);
+        sample_digit<true>(cluster, s, rank, blocks, 10, 11, e, each, weight_bits, p_raw, 0u, some, low, low_weight);
+        sample_digit<true>(cluster, s, rank, blocks, 0, 10, e, each, weight_bits, p_raw, 0u, some, low, low_weight);
+        const unsigned long long one = units(weight_of(key_value(e.prefix)));
+        const double missing = (e.target - (double)e.above_weight) / (double)one;
+        const int need = missing < 2147483647.0 ? max(1, (int)ceil(missing)) : 0x7fffffff;        // a weight of nothing: all its equals
+        if (some && e.prefix == cut.low) {
             cut.quota = min(cut.quota, need);
         } else {
             cut.low = e.prefix;
@@ -484,7 +511,6 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     else __syncthreads();
 
     // ---- inverse CDF over the kept set in id order ------------------------------------------------
-    if (warp != 0) return;
     float retained = 0.0f;
     for (int g = 0; g < SAMPLE_SEGMENTS; ++g) retained += s.all_weight[g];
     const float u = uniform_from_counter(seed[r], (unsigned long long)draw_index[r]) * retained;
@@ -501,22 +527,60 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
         run -= s.all_weight[last];
     }
     if (chosen / own_segments != (int)rank) return;
-    int picked = -1, last_kept = -1;
-    weights(chosen % own_segments, [&](int i, bool, float w) {
-        const bool kept = w >= 0.0f;
-        float cum = kept ? w : 0.0f;
+    chosen %= own_segments;
+    // running weights of 32 neighbouring elements
+    auto scan = [&](float w) {
+        float cum = w >= 0.0f ? w : 0.0f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float up = __shfl_up_sync(0xffffffffu, cum, o);
             if (lane >= o) cum += up;
         }
-        const unsigned hit = __ballot_sync(0xffffffffu, kept && run + cum > u);
-        const unsigned kept_mask = __ballot_sync(0xffffffffu, kept);
-        if (picked < 0 && hit) picked = begin + i - lane + (__ffs(hit) - 1);
-        if (kept_mask) last_kept = begin + i - lane + (31 - __clz(kept_mask));
-        run += __shfl_sync(0xffffffffu, cum, 31);
-    });
-    if (lane == 0) out[r] = picked >= 0 ? picked : last_kept;
+        return cum;
+    };
+    if constexpr (IN_SHARED) {
+        // Every warp scans some of the segment's groups of 32; one thread then adds the groups' weights in order and stops at the
+        // group that u falls into: some kept element's running weight is above it, which the largest tells.
+        const int from = chosen * per_segment, to = min(length, from + per_segment), groups = (to - from + 31) / 32;      // at most BINS
+        float *weight = reinterpret_cast<float*>(s.high), *largest = reinterpret_cast<float*>(s.low);
+        for (int g = warp; g < groups; g += SAMPLE_CTA_WARPS) {
+            const int i = from + 32 * g + lane;
+            const float w = i < to ? share[i] : SAMPLE_NOT_KEPT, cum = scan(w);
+            const float top_cum = warp_max(w >= 0.0f ? cum : -1.0f);
+            if (lane == 31) weight[g] = cum, largest[g] = top_cum;
+        }
+        __syncthreads();
+        if (warp != 0) return;
+        int group = -1, last_group = 0;
+        for (int base = 0; base < groups && group < 0; base += 32) {         // 32 groups' numbers in the lanes; every lane adds them
+            const float mine = base + lane < groups ? weight[base + lane] : 0.0f, top_mine = base + lane < groups ? largest[base + lane] : -1.0f;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) {
+                const float step = __shfl_sync(0xffffffffu, mine, k), top_step = __shfl_sync(0xffffffffu, top_mine, k);
+                if (group >= 0) continue;
+                if (top_step >= 0.0f) {
+                    last_group = base + k;
+                    if (run + top_step > u) group = base + k;
+                }
+                if (group < 0) run += step;
+            }
+        }
+        const int g = group >= 0 ? group : last_group, i = from + 32 * g + lane;
+        const float w = i < to ? share[i] : SAMPLE_NOT_KEPT, cum = scan(w);
+        const unsigned hit = __ballot_sync(0xffffffffu, w >= 0.0f && run + cum > u), kept = __ballot_sync(0xffffffffu, w >= 0.0f);
+        if (lane == 0) out[r] = begin + from + 32 * g + (group >= 0 ? __ffs(hit) - 1 : 31 - __clz(kept));
+    } else {
+        if (warp != 0) return;
+        int picked = -1, last_kept = -1;
+        walk(chosen, [&](int i, bool, float w) {
+            const float cum = scan(w);
+            const unsigned hit = __ballot_sync(0xffffffffu, w >= 0.0f && run + cum > u), kept = __ballot_sync(0xffffffffu, w >= 0.0f);
+            if (picked < 0 && hit) picked = begin + i - lane + (__ffs(hit) - 1);
+            if (kept) last_kept = begin + i - lane + (31 - __clz(kept));
+            run += __shfl_sync(0xffffffffu, cum, 31);
+        });
+        if (lane == 0) out[r] = picked >= 0 ? picked : last_kept;
+    }
 }
 
 // temperature, top_k (<= 0: off), top_p, seed and draw_index are per row.
@@ -532,6 +596,8 @@ MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float*
     if (rows > 0x7fffffff / 8) return MRS_BAD_ARGUMENT;
     const size_t share = (size_t)per_segment * (SAMPLE_SEGMENTS / blocks) * sizeof(float);
     const bool in_shared = share <= SAMPLE_SHARE_BYTES;
+    int weight_bits = 17;                             // so that a share's weights, at most one each, sum up to less than 2^32
+    while (weight_bits > 1 && (unsigned long long)(share / sizeof(float)) << weight_bits >= (1ull << 32)) --weight_bits;
     static bool configured = false;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SHARE_BYTES);
@@ -551,8 +617,8 @@ MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float*
     static const bool plain = getenv("MRS_PLAIN_LAUNCH") != nullptr;
     config.attrs = attributes;
     config.numAttrs = plain ? 1 : 2;
-    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out)
-                                    : cudaLaunchKernelEx(&config, sample_kernel<false>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out);
+    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true>, logits, vocab, per_segment, weight_bits, temperature, top_k, top_p, seed, draw_index, out)
+                                    : cudaLaunchKernelEx(&config, sample_kernel<false>, logits, vocab, per_segment, weight_bits, temperature, top_k, top_p, seed, draw_index, out);
     if (e != cudaSuccess) return (int)e;
     MRS_RETURN_LAUNCH_STATUS();
 }

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 from typing import Sequence
 
+import numpy as np
 import torch
 
 from .. import kernels
@@ -40,6 +41,21 @@ class Sampler:
         self.device = device
         self._pinned: list[torch.Tensor] = []       # host buffers that take turns: two results may be outstanding
         self._turn = 0
+        self._staging: list = []                    # (pinned host buffer, event of its last copy out), taken in turn
+        self._staged = 0
+
+    def _stage(self, rows: int):
+        """A pinned host buffer for the parameters of `rows` rows whose last copy to the device has finished."""
+        self._staged = (self._staged + 1) % 3
+        while len(self._staging) < 3:
+            self._staging.append(None)
+        held = self._staging[self._staged]
+        if held is None or held[0].numel() < 24 * rows:
+            held = (torch.empty(24 * max(64, 2 * rows), dtype=torch.uint8, pin_memory=True), torch.cuda.Event())
+            self._staging[self._staged] = held
+        else:
+            held[1].synchronize()
+        return held
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], draw_index: Sequence[int]) -> list[int]:
         """One token per row of `logits` [rows, vocab] (float32, on the device)."""
@@ -63,16 +79,21 @@ class Sampler:
         if all(p.is_greedy() for p in params):
             kernels.argmax(logits, out)
         else:
-            # seeds are sent as signed 64-bit patterns of the unsigned value
-            seeds = torch.tensor([p.seed - (1 << 64) if p.seed >= (1 << 63) else p.seed for p in params],
-                                 dtype=torch.int64)
-            temperature = torch.tensor([0.0 if p.is_greedy() else float(p.temperature) for p in params],
-                                       dtype=torch.float32)
-            top_k = torch.tensor([p.top_k or 0 for p in params], dtype=torch.int32)
-            top_p = torch.tensor([float(p.top_p) for p in params], dtype=torch.float32)
-            draws = torch.tensor(list(draw_index), dtype=torch.int32)
-            dev = self.device
-            kernels.sample(logits, temperature.to(dev), top_k.to(dev), top_p.to(dev), seeds.to(dev), draws.to(dev), out)
+            # One copy from pinned memory carries every row's parameters: five pageable ones waited for the stream each.
+            # Seeds are 64-bit patterns of the unsigned value; then temperature, top_k, top_p and draw index, 32 bits each.
+            host, copied = self._stage(rows)
+            packed = np.empty(6 * rows, dtype=np.int32)
+            packed[:2 * rows].view(np.uint64)[:] = np.array([p.seed for p in params], dtype=np.uint64)
+            packed[2 * rows:3 * rows].view(np.float32)[:] = [0.0 if p.is_greedy() else p.temperature for p in params]
+            packed[3 * rows:4 * rows] = [p.top_k or 0 for p in params]
+            packed[4 * rows:5 * rows].view(np.float32)[:] = [p.top_p for p in params]
+            packed[5 * rows:] = draw_index
+            host.numpy()[:24 * rows] = packed.view(np.uint8)
+            words = torch.empty(6 * rows, dtype=torch.int32, device=self.device)
+            words.view(torch.uint8).copy_(host[:24 * rows], non_blocking=True)
+            copied.record()
+            temperature, top_k, top_p, draws = (words[k * rows:(k + 1) * rows] for k in range(2, 6))
+            kernels.sample(logits, temperature.view(torch.float32), top_k, top_p.view(torch.float32), words[:2 * rows].view(torch.int64), draws, out)
         while len(self._pinned) < 3:
             self._pinned.append(torch.empty(max(256, rows), dtype=torch.int32, pin_memory=True))
         self._turn = (self._turn + 1) % 3

@@ -861,12 +861,12 @@ def test_sampler_support_and_repeatability(vocab):
     assert set(sampler.sample(logits.expand(20, vocab).contiguous(), [tiny] * 20, list(range(20)))) == {int(logits[0].argmax())}
 
 
-@pytest.mark.parametrize("vocab", [1, 32, 1025, 8191, 8192, 32768, 65535, 65536, 151936, 196608, 196640, 200003])
+@pytest.mark.parametrize("vocab", [1, 32, 1025, 8191, 8192, 32768, 65535, 65536, 151936, 196640, 327680, 327681])
 def test_sampler_rows_that_several_ctas_share(vocab):
-    """One row a cluster of 1, 4 or 8 CTAs, in shared memory or (from 196,609 logits on) read from memory; rows that start off a
+    """One row a cluster of 1, 4 or 8 CTAs, in shared memory or (from 327,681 logits on) read from memory; rows that start off a
     16-byte boundary; equal logits across the shares' edges, of which a cut by count or by weight keeps the first ids; every row
     against the draw restated in float64.  A draw may differ only where u falls within 1e-5 of the weight between two tokens (float32
-    sums of at most 200,003 weights in 1,024 runs), which at most one row in twenty does."""
+    sums of at most 327,681 weights in 1,024 runs), which at most one row in twenty does."""
     sampler = Sampler(torch.device(DEV))
     g = torch.Generator().manual_seed(vocab)
     settings = [SamplingParams(temperature=0.8, top_p=0.95, seed=1), SamplingParams(temperature=0.7, top_k=50, top_p=0.9, seed=2),

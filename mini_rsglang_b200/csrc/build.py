@@ -279,4 +279,5 @@ SPECIALISED_BUILDS = tuple((lambda d=d: specialised_kernel_library("attention_mm
      lambda: specialised_kernel_library("attention_biased_mma.cu", {"MRS_HEAD_DIM": 64, "MRS_VALUE_DIM": 32}),
      lambda: specialised_kernel_library("attention_biased_mma.cu", {"MRS_HEAD_DIM": 288, "MRS_VALUE_DIM": 256, "MRS_VALUES_IN_KEYS": 1}),
      lambda: specialised_kernel_library("attention_biased_mma.cu", {"MRS_HEAD_DIM": 80, "MRS_VALUE_DIM": 64, "MRS_VALUES_IN_KEYS": 1}),
+     lambda: specialised_kernel_library("attention_latent_tc.cu", {"MRS_LATENT": 256, "MRS_ROTARY": 32}),
      lambda: specialised_kernel_library("experts_tc.cu", {}))

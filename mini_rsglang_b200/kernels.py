@@ -1467,6 +1467,85 @@ def attention_biased_mma(q, k_cache, v_cache, positions, block_table, tiles, out
 
 
 # ------------------------------------------------------------------------------------------------
+# tcgen05 attention over cached latents for prompt portions, one library per (latent, rotated) sizes
+# ------------------------------------------------------------------------------------------------
+_latent_tc_libs: dict[tuple[int, int], ctypes.CDLL] = {}
+LATENT_TC_ROWS = 128           # query rows of a tile: 128 // heads tokens times all heads
+
+
+def attention_latent_tc_supported(latent: int, rotated: int, heads: int, page_size: int) -> bool:
+    """Latents of 64 to 256 elements in steps of 64 with 0, 32 or 64 rotated ones, rows of at most 288 (a tile's queries and four
+    blocks of 64 rows fill a CTA's shared memory), up to 128 heads, pages of 8 rows and more (a power of two)."""
+    return (latent % 64 == 0 and 64 <= latent <= 256 and rotated in (0, 32, 64) and latent + rotated <= 288
+            and 1 <= heads <= LATENT_TC_ROWS and page_size >= 8 and page_size & (page_size - 1) == 0)
+
+
+def attention_latent_tc_library(latent: int, rotated: int) -> ctypes.CDLL:
+    key = (latent, rotated)
+    if key not in _latent_tc_libs:
+        if not torch.cuda.is_available():
+            raise BackendError("no CUDA device: the engine has no CPU path")
+        lib = specialised_kernel_library("attention_latent_tc.cu", {"MRS_LATENT": latent, "MRS_ROTARY": rotated})
+        lib.mrs_attention_latent_tc_cache_maps.argtypes = [_c_vp, ctypes.c_longlong, _c_int, _c_vp]
+        lib.mrs_attention_latent_tc_query_maps.argtypes = [_c_vp, ctypes.c_longlong, _c_int, _c_vp]
+        lib.mrs_attention_latent_tc.argtypes = [_c_vp] * 4 + [_c_int, _c_vp, _c_int, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_float, _c_int, _c_vp]
+        lib.mrs_attention_latent_tc_take_error.argtypes = [ctypes.POINTER(ctypes.c_uint)]
+        for name in ("cache_maps", "query_maps", "take_error", "rows"):
+            getattr(lib, f"mrs_attention_latent_tc_{name}").restype = _c_int
+        lib.mrs_attention_latent_tc.restype = _c_int
+        lib.mrs_attention_latent_tc_error_string.argtypes = [_c_int]
+        lib.mrs_attention_latent_tc_error_string.restype = ctypes.c_char_p
+        if lib.mrs_attention_latent_tc_rows() != LATENT_TC_ROWS:
+            raise BackendError(f"attention_latent_tc takes {lib.mrs_attention_latent_tc_rows()} rows a CTA, the planner expects {LATENT_TC_ROWS}")
+        _latent_tc_libs[key] = lib
+        _register_error_word(f"attention_latent_tc (latent {latent} + {rotated})", lib, "mrs_attention_latent_tc")
+    return _latent_tc_libs[key]
+
+
+def attention_latent_tc(q, cache, positions, block_table, tiles, out, heads: int, latent: int, rotated: int, scale: float, window: int = 0,
+                        gate: torch.Tensor | None = None, sink_logits: torch.Tensor | None = None) -> None:
+    """Attention of all heads over the same cached rows [pages, 1, page_size, latent + rotated], whose first `latent` elements are
+    the values too, on the tcgen05 tensor cores: q [tokens, heads * (latent + rotated)], out [tokens, heads * latent], tiles
+    [n, 4] (sequence, first row, up to 128 // heads tokens, 0).  `window` 0: every earlier key is seen; `gate` [tokens, heads]
+    float32 multiplies a head's result; `sink_logits` [heads] float32: one more term exp(sink) in the denominator."""
+    global launch_count
+    tokens, row, page_size = q.shape[0], latent + rotated, cache.shape[2]
+    _need(q, torch.bfloat16, "q", (tokens, heads * row))
+    _need(cache, torch.bfloat16, "cached rows", (cache.shape[0], 1, page_size, row))
+    _need(out, torch.bfloat16, "attention out", (tokens, heads * latent))
+    _need(positions, torch.int32, "positions", (tokens,))
+    _need(block_table, torch.int32, "block_table")
+    _need(tiles, torch.int32, "tiles")
+    if tiles.dim() != 2 or tiles.shape[1] != 4:
+        raise InvalidRequest("attention tiles must be [n, 4] (sequence, first token, tokens, 0)")
+    if not attention_latent_tc_supported(latent, rotated, heads, page_size):
+        raise InvalidRequest(f"attention_latent_tc: a latent of {latent} + {rotated} with {heads} heads and pages of {page_size} is not built")
+    if gate is not None:
+        _need(gate, torch.float32, "attention gate", (tokens, heads))
+    if sink_logits is not None:
+        _need(sink_logits, torch.float32, "sink logits", (heads,))
+    lib = attention_latent_tc_library(latent, rotated)
+
+    def fail(code, what):
+        raise BackendError(f"{what}: {lib.mrs_attention_latent_tc_error_string(code).decode()} (code {code})")
+
+    keep, maps = _aligned_block(512, 64)                 # two maps of the cache, two of the queries
+    code = lib.mrs_attention_latent_tc_cache_maps(cache.data_ptr(), cache.shape[0], page_size, maps)
+    if code != 0:
+        fail(code, "tensor maps of the cache")
+    code = lib.mrs_attention_latent_tc_query_maps(q.data_ptr(), tokens, heads, maps + 256)
+    if code != 0:
+        fail(code, "tensor maps of the queries")
+    launch_count += 1
+    code = lib.mrs_attention_latent_tc(maps + 256, maps, positions.data_ptr(), block_table.data_ptr(),
+                                       block_table.shape[1], tiles.data_ptr(), tiles.shape[0], out.data_ptr(), _ptr(gate), _ptr(sink_logits),
+                                       heads, page_size, float(scale), int(window), _stream())
+    del keep                          # the maps were copied into the launch
+    if code != 0:
+        fail(code, "attention_latent_tc")
+
+
+# ------------------------------------------------------------------------------------------------
 # layer norms with bias, latent attention, routed experts
 # ------------------------------------------------------------------------------------------------
 _LATENT_SIGNATURES = {

@@ -968,3 +968,54 @@ def test_experts_for_few_rows(per_expert, experts, width, inner, block):
     last = tokens - 1
     kernels.moe_experts(h[last:].clone(), chosen[last:].clone(), laid.contiguous(), down, alone, experts, kernel="few", block=block)
     assert torch.equal(alone, y[last * top:])
+
+
+@pytest.mark.parametrize("heads,latent,rotated,page,window", [(16, 256, 32, 16, 1024), (16, 256, 32, 16, 0), (32, 256, 32, 8, 100), (5, 192, 64, 64, 0),
+                                                              (3, 128, 0, 128, 70), (64, 64, 32, 32, 0), (1, 256, 0, 16, 65), (128, 64, 64, 16, 64)])
+def test_attention_latent_tc(heads, latent, rotated, page, window):
+    """The tcgen05 latent attention over tiles of 128 rows: whole and ragged tiles, heads that do not divide 128, portions behind
+    contexts on both sides of a block's and a page's end, rings gone round several times, windows that begin inside a block with
+    the pages before them given back, gates and sinks; entries without tokens are left out."""
+    spans = [(0, 1), (0, 130), (63, 2), (64, 65), (500, 40), (1100, 9), (2047, 1)]
+    row, per_tile = latent + rotated, 128 // heads
+    g = torch.Generator(device=DEV).manual_seed(heads + latent + page)
+    pages = [-(-(c + n) // page) for c, n in spans]
+    cache = torch.randn(sum(pages) + 3, 1, page, row, device=DEV, generator=g).bfloat16()
+    order = torch.randperm(cache.shape[0], generator=g, device=DEV).int().tolist()
+    table = torch.full((len(spans), max(pages)), -1, dtype=torch.int32)
+    tiles, positions, first = [], [], 0
+    for i, (c, n) in enumerate(spans):
+        taken = [order.pop() for _ in range(pages[i])]
+        gone = max(0, c - window + 1) // page if window else 0
+        table[i, :pages[i]] = torch.tensor([-1] * gone + taken[gone:], dtype=torch.int32)
+        tiles += [(i, first + s, min(per_tile, n - s), 0) for s in range(0, n, per_tile)] + [(0, 0, 0, 0)]
+        positions += range(c, c + n)
+        first += n
+    q = torch.randn(first, heads * row, device=DEV, generator=g).bfloat16()
+    gate, sinks = torch.rand(first, heads, device=DEV, generator=g), torch.randn(heads, device=DEV, generator=g) * 3
+    scale = 1.7 * row ** -0.5
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).to(DEV)      # noqa: E731
+    for use_gate, use_sinks in ((True, True), (False, False)):
+        out = torch.full((first, heads * latent), 77.0, device=DEV).bfloat16()
+        kernels.attention_latent_tc(q, cache, i32(positions), i32(table), i32(tiles), out, heads, latent, rotated, scale, window=window,
+                                    gate=gate if use_gate else None, sink_logits=sinks if use_sinks else None)
+        kernels.check_device_errors(certain=True)
+        at = 0
+        for i, (c, n) in enumerate(spans):
+            slots = torch.arange(c + n, device=DEV)
+            keys = cache[table[i].to(DEV).long()[slots // page].clamp(min=0), 0, slots % page].double()
+            scores = torch.einsum("thd,kd->thk", q[at:at + n].view(n, heads, row).double(), keys) * scale
+            query, key = torch.arange(c, c + n, device=DEV)[:, None], slots[None]
+            seen = (key <= query) & ((key > query - window) if window else True)
+            scores = scores.masked_fill(~seen[:, None], -float("inf"))
+            if use_sinks:
+                scores = torch.cat([scores, sinks.double()[None, :, None].expand(n, heads, 1)], dim=2)
+            weights = torch.softmax(scores, dim=2)[:, :, :c + n]
+            want = torch.einsum("thk,ke->the", weights, keys[:, :latent])
+            size = torch.einsum("thk,ke->the", weights, keys[:, :latent].abs())
+            if use_gate:
+                want, size = want * gate[at:at + n].double()[..., None], size * gate[at:at + n].double()[..., None]
+            got = out[at:at + n].view(n, heads, latent).double()
+            # a weight and the result rounded to bfloat16 (2^-9 each), the scores' float32 sums far below
+            assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -8 + 1e-6).all(), (i, use_gate)
+            at += n

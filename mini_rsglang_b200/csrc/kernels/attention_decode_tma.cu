@@ -74,26 +74,6 @@ __device__ __forceinline__ void store_cluster(uint32_t address, float2 v) {
 __device__ __forceinline__ void arrive_in_cluster(uint32_t barrier_address) {          // after this thread's (and, through a CTA barrier, its CTA's) stores
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(barrier_address) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return done != 0;
-}
-// Bounded like mbar_wait; sees what the arriving CTAs of the cluster stored.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    const long long start = clock64();
-    unsigned int spins = 0;
-    while (!mbar_try_wait_cluster(bar, parity)) {
-        if ((++spins & 255u) == 0 && *reinterpret_cast<volatile unsigned int*>(&mrs_error_word) != 0) return false;
-        if (clock64() - start > MRS_WAIT_CYCLES) {
-            mrs_raise(MRS_ERR_BARRIER_TIMEOUT);
-            return false;
-        }
-    }
-    return true;
-}
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

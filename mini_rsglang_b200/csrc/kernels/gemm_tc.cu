@@ -14,9 +14,16 @@
 // while the last one is stored.
 //
 // K is cut into `splits` ranges so that the units fill all SMs evenly.  The cut depends on N
-// and K alone and partial sums are added in the order of the ranges by whichever CTA finishes
-// a tile last, so a row's result does not depend on M or on what else is in the batch, bit for
-// bit.                       (reference: cuBLAS in 32-row blocks, crates/kernels/src/lib.rs:241-322)
+// and K alone (and the GPU) and partial sums are added in the order of the ranges, by the first
+// CTA of a tile's cluster where its ranges run as one, else by whichever CTA finishes a tile last,
+// so a row's result does not depend on M or on what else is in the batch, bit for bit.
+//
+// Small products (0.6B shape, 2 to 6 MB of weights) are bound by the trips one after another: the
+// previous kernel's end, x, the MMAs, the ranges' meeting, the store.  Ranges that meet in a cluster,
+// and rings no longer than a CTA's range (two kernels' CTAs then share an SM, and the next one's
+// weights come in under this one): q/k/v 9.1 -> 7.9 us, o and down 7.8 -> 6.5, gate/up 8.5 -> 7.5
+// alone; a step of one token through 4 layers and the head 210 -> 191 us, a decode step of 8 requests
+// at the 8B shape 629 -> 616 us.                       (reference: cuBLAS in 32-row blocks, crates/kernels/src/lib.rs:241-322)
 #include "tcgen05.cuh"
 
 namespace {
@@ -33,6 +40,8 @@ constexpr int W_TILE_BYTES = TILE_N * BLOCK_K * 2;
 #define MRS_GEMM_TC_RING 8
 #endif
 
+constexpr size_t MAX_SMEM_BYTES = 227 * 1024 - 64;          // what a CTA may have, less its static words
+
 template <int MPAD> struct Shape {
     static constexpr int X_TILE_BYTES = MPAD * BLOCK_K * 2;
     static constexpr int BLOCK_BYTES = W_TILE_BYTES + X_TILE_BYTES;          // a block of K: its weight tile, then its rows of x
@@ -44,10 +53,12 @@ template <int MPAD> struct Shape {
     // 4.51, 4.35, 4.27, 4.27, 4.32, 4.38, 4.42 ms
     static constexpr int STAGES = (MPAD <= 32 ? MRS_GEMM_TC_RING : (MPAD <= 64 ? 6 : 5)) / BLOCKS;
     static constexpr int TMEM_COLUMNS = 2 * MPAD < 32 ? 32 : 2 * MPAD;
-    static constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * sizeof(uint64_t) + 16 +
+    // beside the ring and what a cluster's first CTA receives
+    static constexpr size_t FIXED_BYTES = 1024 + (2 * STAGES + 6) * sizeof(uint64_t) + 16 +
                                          (size_t)MPAD * (MPAD <= 32 ? 128 : 64) * sizeof(float) + 4 * MPAD * sizeof(float) +
                                          (MPAD <= 32 ? (size_t)MPAD * (128 + 1) * sizeof(float) : 0) +   // cosines, sines, write slots
                                          MPAD * sizeof(float);                                           // the rows' norm factors
+    static constexpr size_t SMEM_BYTES = FIXED_BYTES + (size_t)STAGES * STAGE_BYTES;
 };
 
 // How K is cut, as one number: ranges a tile (low 8 bits) for the first `tiles_first` tiles (bits 16 and up), and,
@@ -77,6 +88,24 @@ __device__ __forceinline__ void unit_place(const Ranges& r, int unit, int& tile,
         tile = r.tiles_first + u / r.rest, split = u % r.rest, splits = r.rest;
     }
 }
+
+// ---- a tile's ranges as one thread-block cluster
+// Partial sums that travel through global memory cost the CTA that finishes a tile a store, a fence, an atomic and a
+// load one after another, each a trip to L2.  Where every range of every tile has a CTA of its own, the CTAs of a
+// tile are a cluster instead (as long as the GPU holds all clusters at once: 74 of 2, 45 of 3, 33 of 4, 15 of 8, 7 of 12
+// here; a cluster that waits for SMs would cost more than the trips): they send their sums into the shared memory of the first, each packet counted by that
+// CTA's barrier, and it adds them in the order of the ranges, as before.
+__device__ __forceinline__ uint32_t in_first_cta(uint32_t local_address) {      // the same place in the cluster's CTA 0
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(local_address));
+    return a;
+}
+__device__ __forceinline__ void send_float4(uint32_t address, uint32_t barrier, float4 v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(address),
+                 "r"(barrier), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 2, 128;" ::: "memory"); }
 
@@ -119,17 +148,22 @@ template <int MPAD, typename OutT, int EPI>
 __global__ void __launch_bounds__(THREADS, 1) gemm_small_m_kernel(
     const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, OutT* __restrict__ out,
     float* __restrict__ partials, int* __restrict__ counters, int M, int N, int K, int splits, const HeadEpilogue heads,
-    const NormLink link) {
+    const NormLink link, int ring_stages, int receive_bytes) {
     using S = Shape<MPAD>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::STAGES * S::STAGE_BYTES);
+    // The ring has no more stages than this launch's CTAs have steps.  `receive_bytes` > 0: the tile's ranges are a cluster.
+    const bool in_cluster = receive_bytes > 0;
+    float4* received = reinterpret_cast<float4*>(smem + ring_stages * S::STAGE_BYTES);       // [ranges - 1][float4s of M][TILE_N]
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + ring_stages * S::STAGE_BYTES + receive_bytes);
     uint64_t* empty = full + S::STAGES;
     uint64_t* acc_full = empty + S::STAGES;
     uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* received_bar = acc_empty + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(received_bar + 2);
     float* exchange = reinterpret_cast<float*>(tmem_slot + 4);        // rows of a tile meet here: [MPAD][64] gated, [MPAD][128] + [4][MPAD] heads (up to 32 rows)
     __shared__ int is_last;
+    bool gave_up = false;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
@@ -146,7 +180,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_small_m_kernel(
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 4);
         }
+        mbar_init(received_bar, 1);
         mbar_fence_init();
+        if (in_cluster && blockIdx.x % ranges.first == 0) mbar_arrive_expect_tx(received_bar, receive_bytes);
     }
     if (warp == 1) {
         tmem_alloc(tmem_slot, S::TMEM_COLUMNS);
@@ -156,6 +192,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_small_m_kernel(
     __syncthreads();
     tcgen05_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    if (in_cluster) cluster_arrive();          // this CTA's barrier stands; everyone waits for everyone's before the first packet
     pdl_launch_dependents();
 
     if (warp == 0) {
@@ -298,7 +335,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_small_m_kernel(
             // needed only by the CTA that finishes the tile
             float stream_old[EPI == EPI_RESIDUAL ? MPAD : 1];
             float next_weight = 0.0f;
-            if (EPI == EPI_RESIDUAL) {
+            if (EPI == EPI_RESIDUAL && (!in_cluster || split == 0)) {
                 const int column = tile * TILE_N + row;
                 if (column < N) next_weight = __ldg(link.next_weight + column);
 #pragma unroll
@@ -317,7 +354,32 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_small_m_kernel(
 
             const int n = tile * TILE_N + row;
             bool finished = of == 1;                      // does this CTA hold the tile's final sums?
-            if (of > 1) {
+            if (in_cluster) {
+                const int m4 = (M + 3) >> 2;
+                cluster_wait();                                       // begun at the kernel's start: long complete
+                finished = split == 0;
+                if (!finished) {
+                    const uint32_t bar = in_first_cta(smem_u32(received_bar));
+                    const uint32_t to = in_first_cta(smem_u32(received + (size_t)(split - 1) * m4 * TILE_N + row));
+#pragma unroll
+                    for (int j = 0; j < MPAD / 4; ++j)
+                        if (j < m4) send_float4(to + j * TILE_N * 16, bar, make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]));
+                } else {
+                    if (!mbar_wait_cluster(received_bar, 0)) gave_up = true;
+#pragma unroll
+                    for (int m = 0; m < MPAD; ++m) acc[m] = 0.0f + acc[m];          // as the sum below begins
+                    for (int s = 0; s < of - 1; ++s)
+#pragma unroll
+                        for (int j = 0; j < MPAD / 4; ++j)
+                            if (j < m4) {
+                                const float4 v = received[(s * m4 + j) * TILE_N + row];
+                                acc[4 * j] += v.x;
+                                acc[4 * j + 1] += v.y;
+                                acc[4 * j + 2] += v.z;
+                                acc[4 * j + 3] += v.w;
+                            }
+                }
+            } else if (of > 1) {
                 // partial sums of this range of K, then: the CTA that finishes the tile last adds all ranges in order
                 constexpr int V = MPAD / 4;                                   // float4s of a padded row
                 constexpr int RANGES_AT_ONCE = MPAD == 16 ? 4 : (MPAD == 32 ? 2 : 1);
@@ -468,26 +530,90 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_small_m_kernel(
             epilogue_sync();                               // `is_last` is rewritten in the next round
         }
     }
+    if (in_cluster && warp < 2) cluster_wait();
     tcgen05_fence_before_sync();
-    __syncthreads();
+    const bool peers_unknown = __syncthreads_or(gave_up);
     if (warp == 1) {
         tcgen05_fence_after_sync();
         tmem_dealloc(tmem_base, S::TMEM_COLUMNS);
     }
+    if (peers_unknown) {                       // a wait ran out: packets may still be on their way here, so this CTA
+        cluster_arrive();                      // outlives its peers (those that have ended count as arrived)
+        cluster_wait();
+    }
+}
+
+// Clusters of `ranges` CTAs that the GPU holds at once with one CTA an SM (0: none), asked of the driver once a size.
+int resident_clusters(int ranges) {
+    using S = Shape<16>;
+    static int known[17] = {};
+    if (ranges < 2 || ranges > 16) return 0;
+    if (known[ranges] == 0) {
+        int clusters = 0;
+        const auto kernel = gemm_small_m_kernel<16, bf16, EPI_PLAIN>;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES) == cudaSuccess &&
+            (ranges <= 8 || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
+            cudaLaunchConfig_t probe = {};
+            probe.gridDim = dim3(ranges * 64), probe.blockDim = dim3(THREADS), probe.dynamicSmemBytes = S::SMEM_BYTES;
+            cudaLaunchAttribute shape;
+            shape.id = cudaLaunchAttributeClusterDimension;
+            shape.val.clusterDim.x = ranges, shape.val.clusterDim.y = 1, shape.val.clusterDim.z = 1;
+            probe.attrs = &shape, probe.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &probe) != cudaSuccess || clusters < 0) clusters = 0;
+        }
+        (void)cudaGetLastError();
+        known[ranges] = clusters > 0 ? clusters : -1;
+    }
+    return known[ranges] > 0 ? known[ranges] : 0;
 }
 
 template <int MPAD, typename OutT, int EPI>
 int launch(const CUtensorMap* w_map, const CUtensorMap* x_map, void* out, float* partials, int* counters, int M, int N,
            int K, int splits, int ctas, cudaStream_t stream, const NormLink& link, const HeadEpilogue& heads = HeadEpilogue{}) {
     using S = Shape<MPAD>;
+    const auto kernel = gemm_small_m_kernel<MPAD, OutT, EPI>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_small_m_kernel<MPAD, OutT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    return mrs_launch(gemm_small_m_kernel<MPAD, OutT, EPI>, dim3(ctas), dim3(THREADS), S::SMEM_BYTES, stream, *w_map, *x_map,
-                      (OutT*)out, partials, counters, M, N, K, splits, heads, link);
+    const int n_tiles = (N + TILE_N - 1) / TILE_N, k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
+    const Ranges ranges = ranges_of(splits, n_tiles);
+    int ring_stages = S::STAGES, receive_bytes = 0;
+    if (units_of(ranges, n_tiles) <= ctas) {
+        // One unit a CTA: a ring of as many stages as the longest unit has steps, so that a CTA of the next kernel finds
+        // room beside this one's and fetches its weights under it.
+        const int fewest = ranges.rest > 0 && ranges.rest < ranges.first ? ranges.rest : ranges.first;
+        const int steps = ((k_blocks + fewest - 1) / fewest + S::BLOCKS - 1) / S::BLOCKS;
+        if (steps < ring_stages) ring_stages = steps;
+        // The ranges of a tile as a cluster, where all clusters are resident at once and the sums find room.
+        const size_t receive = (size_t)(ranges.first - 1) * TILE_N * ((M + 3) / 4) * sizeof(float4);
+        if (ranges.first > 1 && ranges.tiles_first == n_tiles && n_tiles <= resident_clusters(ranges.first) &&
+            S::FIXED_BYTES + (size_t)ring_stages * S::STAGE_BYTES + receive <= MAX_SMEM_BYTES)
+            receive_bytes = (int)receive;
+    }
+    const size_t smem = S::FIXED_BYTES + (size_t)ring_stages * S::STAGE_BYTES + receive_bytes;
+    if (receive_bytes == 0)
+        return mrs_launch(kernel, dim3(ctas), dim3(THREADS), smem, stream, *w_map, *x_map, (OutT*)out, partials, counters, M, N, K,
+                          splits, heads, link, ring_stages, receive_bytes);
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(n_tiles * ranges.first);
+    config.blockDim = dim3(THREADS);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = ranges.first, attributes[0].val.clusterDim.y = 1, attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    static const bool plain = getenv("MRS_PLAIN_LAUNCH") != nullptr;
+    config.attrs = attributes;
+    config.numAttrs = plain ? 1 : 2;
+    return (int)cudaLaunchKernelEx(&config, kernel, *w_map, *x_map, (OutT*)out, partials, counters, M, N, K, splits, heads, link,
+                                   ring_stages, receive_bytes);
 }
 
 }  // namespace
@@ -504,8 +630,10 @@ MRS_EXPORT int mrs_gemm_tc_map(const void* base, long long rows, long long cols,
 // Ranges of K for a weight matrix [N, K] on a GPU with `sms` SMs, by a count of the time an SM
 // spends: rounds of units x (64-column blocks of a unit + a unit's fixed cost + the cost of
 // leaving and adding partial sums when there are several ranges), the costs in blocks' worth of
-// time.  It depends on N, K and the GPU alone, never on the rows of the product.  The costs 4 and 8
-// were measured in decode steps (with 2 and 2 the gate/up product of the 8B shape took 3 ranges
+// time.  It depends on N, K and the GPU alone, never on the rows of the product.  Ranges that can meet
+// in a cluster cost 3: with 8 for them too, the 0.6B shape's gate/up took 3 ranges and its down product 12, neither a
+// set of clusters that the GPU holds at once, and a step of one token 203 us against 191.  The costs
+// 4 and 8 were measured in decode steps (with 2 and 2 the gate/up product of the 8B shape took 3 ranges
 // instead of 2: batch 8 4.155 against 4.104 ms a step, batch 16 5.129 against 4.997 ms; 14B shape
 // at batch 16 8.83 against 8.61 ms; 1 and 1, 3 and 4, 6 and 12, 4 and 16, 8 and 8 all slower).
 MRS_EXPORT int mrs_gemm_tc_splits(int N, int K, int sms) {
@@ -516,7 +644,8 @@ MRS_EXPORT int mrs_gemm_tc_splits(int N, int K, int sms) {
     long long best_cost = -1;
     for (int s = 1; s <= limit; ++s) {
         const long long rounds = ((long long)n_tiles * s + sms - 1) / sms;
-        const long long cost = rounds * ((k_blocks + s - 1) / s + 4 + (s > 1 ? 8 : 0));
+        const bool in_cluster = s > 1 && n_tiles <= resident_clusters(s);
+        const long long cost = rounds * ((k_blocks + s - 1) / s + 4 + (s == 1 ? 0 : (in_cluster ? 3 : 8)));
         if (best_cost < 0 || cost < best_cost) best = s, best_cost = cost;
     }
     // A last round of units that fills the GPU partly (after at least one full round): its tiles take as many ranges
@@ -545,6 +674,7 @@ static bool ranges_fit(int splits, int N, int K) {
     const Ranges r = ranges_of(splits, (N + TILE_N - 1) / TILE_N);
     return splits > 0 && r.first >= 1 && r.first <= k_blocks && r.rest <= k_blocks && r.tiles_first >= 0;
 }
+MRS_EXPORT int mrs_gemm_tc_resident_clusters(int ranges) { return resident_clusters(ranges); }
 MRS_EXPORT int mrs_gemm_tc_counters(int N) { return (N + TILE_N - 1) / TILE_N; }
 
 // out[M, N] = x . w^T.  `w_map`: mrs_gemm_tc_map(w, N, K, 128); `x_map`: mrs_gemm_tc_map(x, M, K, mpad) with

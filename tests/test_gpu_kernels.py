@@ -778,6 +778,37 @@ def test_gemm_tc_gated_and_heads_finish_a_norm(m):
     close(vc.cpu()[slot // page, :, slot % page], v, torch.bfloat16, "v in the cache")
 
 
+@pytest.mark.parametrize("m", [1, 7, 16, 20, 64, 100])
+@pytest.mark.parametrize("n,k,splits", [(1024, 2048, 8), (1024, 3072, 12), (4096, 1024, 4), (6144, 4096, 3), (4096, 4096, 4), (300, 1032, 2),
+                                        (128, 8192, 16), (384, 8192, 5), (24576, 4096, 2)])
+def test_gemm_tc_ranges_merged_in_a_cluster(m, n, k, splits, monkeypatch):
+    """Where every range has a CTA of its own the ranges of a tile meet in a cluster's shared memory: the same bits as
+    with fewer CTAs, whose partial sums go through global memory (both add the ranges in their order)."""
+    torch.manual_seed(31)
+    x = torch.randn(m, k, dtype=torch.bfloat16, device=DEV)
+    w = torch.randn(n, k, dtype=torch.bfloat16, device=DEV) / k ** 0.5
+    state = kernels._gemm_device_state(x.device)
+    results = []
+    for sms in (state["sms"], 5):
+        monkeypatch.setitem(state, "sms", sms)
+        stream = torch.linspace(-2, 2, m * n, device=DEV).view(m, n).contiguous()
+        plain, folded = torch.empty(m, n, device=DEV), torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+        for _ in range(3):                       # back to back: a launch begins under the one before it
+            kernels.gemm_tc(x, w, plain, splits=splits)
+        out = [plain]
+        if n % 128 == 0:
+            gated = torch.empty(m, n // 2, dtype=torch.bfloat16, device=DEV)
+            kernels.gemm_tc(x, w, gated, gated=True, splits=splits)
+            out.append(gated)
+        if m <= 32:
+            sums = kernels.gemm_tc(x, w, folded, splits=splits, residual=(stream, torch.ones(n, device=DEV)))
+            out += [folded, stream, sums[:, :m]]
+        results.append(out)
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    close(results[0][0], x.double() @ w.double().T, torch.float32, f"gemm_tc {m}x{n}x{k} in {splits} ranges")
+
+
 def test_gemm_tc_rows_do_not_depend_on_the_batch():
     """The same row alone, among 8 and among 100 others: equal bit for bit, twice in a row (the
     counters of the ranges of K are left ready for the next launch)."""

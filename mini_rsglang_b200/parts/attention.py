@@ -86,12 +86,14 @@ def attention_tile_lists(facts: StepFacts, group: int, wide_rows: int, kv_heads:
             blocks = -(-(begin + tokens) // key_block) - first_key // key_block
             found.append((i, first + start, tokens, begin, blocks))
     # CTAs an entry may become.  Beside decoded tokens the kernel for few rows runs at the same time and wants SMs
-    # of its own: the wide entries then share WIDE_SHARE_BESIDE_NARROW of them.
+    # of its own: the wide entries are then cut into tiles for WIDE_SHARE_BESIDE_NARROW of them, and into shares of
+    # their keys where their walks would end long after the narrow tiles.
     room = int(sms * WIDE_SHARE_BESIDE_NARROW) if narrow else sms
     spare = room // max(len(found) * kv_heads, 1) if tensor_core else 1
+    beside = shares_beside_narrow(found, lengths, facts.start_pos, narrow, kv_heads, window, sms) if tensor_core and narrow else 0
     wide = []
     shared = False
-    if tensor_core and tiles == 2 and spare < 2 and len(found) * kv_heads <= room and not window and PAIR_FAR_TILES:
+    if tensor_core and tiles == 2 and spare < 2 and beside < 2 and len(found) * kv_heads <= room and not window and PAIR_FAR_TILES:
         # One round of CTAs, more than half the SMs: what is left to gain is their balance.  The tiles of a portion
         # walk 1, 2, 3, ... blocks of keys more than the first, and a CTA holds two tiles: the first with the last,
         # the second with the last but one, and so on, so that every CTA has the same work; the early tile is done
@@ -123,7 +125,7 @@ def attention_tile_lists(facts: StepFacts, group: int, wide_rows: int, kv_heads:
         wide = [t[:4] for t in wide]
         found = []
     for i, first, tokens, begin, blocks in found:
-        shares = min(spare, blocks // 4, 255) if spare >= 2 else 1
+        shares = min(max(beside, spare), blocks // 4, 255)
         if shares >= 2:
             shared = True
             wide += [(i, first, tokens, s | shares << 8, begin) for s in range(shares)]
@@ -141,6 +143,28 @@ def attention_tile_lists(facts: StepFacts, group: int, wide_rows: int, kv_heads:
         lists.wide_cap = max(16, 1 << (len(wide) - 1).bit_length()) if wide else 0
     facts.plans[key] = lists
     return lists
+
+
+def shares_beside_narrow(found: list, lengths: list, start_pos, narrow: list, kv_heads: int, window: int, sms: int) -> int:
+    """Shares of its keys that an entry for the kernel for wide tiles is cut into while the kernel for few rows runs beside it.
+    Times in blocks of keys of a CTA's two tiles (2.3 us): a walk is its blocks, and 6 more where shares have to be merged; the
+    narrow tiles take 2.6 and one for every 15 MB of their keys and values (heads of 128), stretched where the wide CTAs leave
+    them fewer than 0.6 of the SMs.  The count with the shortest time for both is taken.  Measured, steps of 4 layers, one portion
+    under a budget of 512 tokens, 1, 2, 3 and 4 shares (0.6B shape: 32 CTAs a share): 27 requests at 1,100 beside a portion behind
+    1,500 tokens 504, 476, 467, 468 us, behind 7,000 tokens 834, 641, 568, 551; 64 requests at 1,000, behind 512 tokens 553, 554,
+    552, 556, behind 3,000 638, 587, 591, 606; 16 at 4,000, behind 1,500 528, 546, 588, 590.  1 and 2 shares (8B shape: 64 CTAs a
+    share): 27 at 1,100, behind 1,500 1,215, 1,228, behind 7,000 1,538, 1,372; 16 at 4,000, behind 3,000 1,323, 1,421."""
+    ctas = max(len(found) * kv_heads, 1)
+    longest = max((entry[4] for entry in found), default=0)
+    keys = sum(min(start_pos[i] + lengths[i], window + lengths[i]) if window else start_pos[i] + lengths[i] for i, *_ in narrow)
+    few = 2.6 + keys * kv_heads * 512 / 15e6
+    best, best_time = 1, max(longest, few)
+    for shares in range(2, min(sms // ctas, longest // 4, 255) + 1):
+        walk = longest / shares + 6
+        time = walk + max(0.0, few - walk * min(1.0, (sms - ctas * shares) / (0.6 * sms)))
+        if time < 0.97 * best_time:
+            best, best_time = shares, time
+    return best
 
 
 def plan_attention_tiles(ctx, group: int, wide_rows: int, kv_heads: int = 1, window: int = 0, key_block: int = 128,
@@ -303,7 +327,8 @@ def paged_attention(q, cache, ctx, out, nq: int, nkv: int, d: int, window: int, 
 SIDE_BY_SIDE = os.environ.get("MRS_ATTENTION_SIDE_BY_SIDE", "1") == "1"      # the variable: for measuring
 # Continuous batching, 64 requests of 16 to 2,048 prompt tokens and 64 generated ones, portions under 512 tokens a
 # step: 0.6B shape 143.7k tokens/s one kernel after the other, 159.9k side by side, 162.4k with the wide entries cut
-# for a quarter of the SMs only (the same with no cutting at all); 8B shape 45.6k, 47.0k, 47.3k.
+# for a quarter of the SMs only (the same with no cutting at all); 8B shape 45.6k, 47.0k, 47.3k.  (Shares of the keys:
+# `shares_beside_narrow`.)
 WIDE_SHARE_BESIDE_NARROW = float(os.environ.get("MRS_WIDE_SHARE", "0.25"))
 PAIR_FAR_TILES = os.environ.get("MRS_PAIR_FAR_TILES", "1") == "1"      # the variable: for measuring
 

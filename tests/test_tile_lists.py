@@ -120,3 +120,15 @@ def test_one_round_of_entries_pairs_early_tiles_with_late_ones():
     assert not any(gaps([2048], [0]))               # more CTAs than SMs: the rounds balance themselves
     assert not any(gaps([1024], [0], window=256))   # with a window every tile walks the same few blocks
     assert not any(gaps([256], [4096]))             # few CTAs: shares of the keys instead
+
+
+@pytest.mark.parametrize("decodes,context,behind,shares", [(27, 1100, 512, 1), (27, 1100, 3000, 3), (64, 1000, 1500, 1), (64, 1000, 7000, 3),
+                                                           (4, 2000, 0, 1), (4, 2000, 7000, 4)])
+def test_a_long_walk_beside_decoded_tokens_is_cut_into_shares(decodes, context, behind, shares):
+    """A portion far behind its request's start becomes shares of its keys when its walk would outlast the decoded tokens beside it,
+    and never more CTAs than one round of the SMs."""
+    facts = facts_of([1] * decodes + [512 - decodes], [context] * decodes + [behind])
+    lists = attention_tile_lists(facts, 2, kernels.PREFILL_TC_ROWS, 8, 0, 128, 148)
+    assert lists.shared == (shares > 1) and len(lists.narrow) == decodes
+    assert {max(share >> 8 & 0xFF, 1) for *_, share in lists.wide} == {shares}
+    assert len(lists.wide) * 8 <= 148

@@ -14,7 +14,7 @@
 // while the last one is stored.
 //
 // K is cut into `splits` ranges so that the units fill all SMs evenly.  The cut depends on N
-// and K alone (and the GPU) and partial sums are added in the order of the ranges, by the first
+// and K alone (and the count of SMs) and partial sums are added in the order of the ranges, by the first
 // CTA of a tile's cluster where its ranges run as one, else by whichever CTA finishes a tile last,
 // so a row's result does not depend on M or on what else is in the batch, bit for bit.
 //
@@ -93,8 +93,8 @@ __device__ __forceinline__ void unit_place(const Ranges& r, int unit, int& tile,
 // Partial sums that travel through global memory cost the CTA that finishes a tile a store, a fence, an atomic and a
 // load one after another, each a trip to L2.  Where every range of every tile has a CTA of its own, the CTAs of a
 // tile are a cluster instead (as long as the GPU holds all clusters at once: 74 of 2, 45 of 3, 33 of 4, 15 of 8, 7 of 12
-// here; a cluster that waits for SMs would cost more than the trips): they send their sums into the shared memory of the first, each packet counted by that
-// CTA's barrier, and it adds them in the order of the ranges, as before.
+// on one GPU; a cluster that waits for SMs would cost more than the trips): they send their sums into the shared memory
+// of the first, each packet counted by that CTA's barrier, and it adds them in the order of the ranges: the same bits.
 __device__ __forceinline__ uint32_t in_first_cta(uint32_t local_address) {      // the same place in the cluster's CTA 0
     uint32_t a;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(local_address));
@@ -630,10 +630,11 @@ MRS_EXPORT int mrs_gemm_tc_map(const void* base, long long rows, long long cols,
 // Ranges of K for a weight matrix [N, K] on a GPU with `sms` SMs, by a count of the time an SM
 // spends: rounds of units x (64-column blocks of a unit + a unit's fixed cost + the cost of
 // leaving and adding partial sums when there are several ranges), the costs in blocks' worth of
-// time.  It depends on N, K and the GPU alone, never on the rows of the product.  Ranges that can meet
-// in a cluster cost 3: with 8 for them too, the 0.6B shape's gate/up took 3 ranges and its down product 12, neither a
-// set of clusters that the GPU holds at once, and a step of one token 203 us against 191.  The costs
-// 4 and 8 were measured in decode steps (with 2 and 2 the gate/up product of the 8B shape took 3 ranges
+// time.  It depends on N, K and the count of SMs alone, never on the rows of the product, nor on how many clusters this very
+// GPU holds (that differs from one to the next; ranks that repeat a product have to cut it alike).  Ranges that
+// can meet in a cluster on all of them (2, 4 or 8 ranges and a CTA for each on seven eighths of the SMs) cost 3: with 8
+// for them too, the 0.6B shape's gate/up took 3 ranges and its down product 12, neither a set of clusters that was
+// held at once, and a step of one token 203 us against 191.  The costs 4 and 8 were measured in decode steps (with 2 and 2 the gate/up product of the 8B shape took 3 ranges
 // instead of 2: batch 8 4.155 against 4.104 ms a step, batch 16 5.129 against 4.997 ms; 14B shape
 // at batch 16 8.83 against 8.61 ms; 1 and 1, 3 and 4, 6 and 12, 4 and 16, 8 and 8 all slower).
 MRS_EXPORT int mrs_gemm_tc_splits(int N, int K, int sms) {
@@ -644,7 +645,7 @@ MRS_EXPORT int mrs_gemm_tc_splits(int N, int K, int sms) {
     long long best_cost = -1;
     for (int s = 1; s <= limit; ++s) {
         const long long rounds = ((long long)n_tiles * s + sms - 1) / sms;
-        const bool in_cluster = s > 1 && n_tiles <= resident_clusters(s);
+        const bool in_cluster = (s == 2 || s == 4 || s == 8) && (long long)n_tiles * s * 8 <= (long long)sms * 7;
         const long long cost = rounds * ((k_blocks + s - 1) / s + 4 + (s == 1 ? 0 : (in_cluster ? 3 : 8)));
         if (best_cost < 0 || cost < best_cost) best = s, best_cost = cost;
     }

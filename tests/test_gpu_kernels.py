@@ -787,6 +787,8 @@ def test_gemm_tc_ranges_merged_in_a_cluster(m, n, k, splits, monkeypatch):
     torch.manual_seed(31)
     x = torch.randn(m, k, dtype=torch.bfloat16, device=DEV)
     w = torch.randn(n, k, dtype=torch.bfloat16, device=DEV) / k ** 0.5
+    lib = kernels.gemm_tc_library()
+    assert lib.mrs_gemm_tc_splits(6144, 1024, 148) == 2 and lib.mrs_gemm_tc_splits(1024, 3072, 148) == 8     # by N, K and SMs alone
     state = kernels._gemm_device_state(x.device)
     results = []
     for sms in (state["sms"], 5):

@@ -543,7 +543,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_small_m_kernel(
     }
 }
 
-// Clusters of `ranges` CTAs that the GPU holds at once with one CTA an SM (0: none), asked of the driver once a size.
+// Clusters of `ranges` CTAs that the GPU holds at once with one CTA an SM (0: none), asked of the driver once a size.  The kernel
+// that is asked about is launched too: its limit of shared memory is set to what a launch sets, never below.
 int resident_clusters(int ranges) {
     using S = Shape<16>;
     static int known[17] = {};
@@ -551,7 +552,7 @@ int resident_clusters(int ranges) {
     if (known[ranges] == 0) {
         int clusters = 0;
         const auto kernel = gemm_small_m_kernel<16, bf16, EPI_PLAIN>;
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES) == cudaSuccess &&
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM_BYTES) == cudaSuccess &&
             (ranges <= 8 || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
             cudaLaunchConfig_t probe = {};
             probe.gridDim = dim3(ranges * 64), probe.blockDim = dim3(THREADS), probe.dynamicSmemBytes = S::SMEM_BYTES;
@@ -567,6 +568,30 @@ int resident_clusters(int ranges) {
     return known[ranges] > 0 ? known[ranges] : 0;
 }
 
+// How a launch lays out its shared memory: stages of the ring, and bytes that the first CTA of a tile's cluster receives (0: the
+// ranges of a tile are no cluster).
+struct Layout {
+    int ring_stages, receive_bytes;
+};
+template <int MPAD> Layout layout_of(int M, int N, int K, int splits, int ctas) {
+    using S = Shape<MPAD>;
+    const int n_tiles = (N + TILE_N - 1) / TILE_N, k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
+    const Ranges ranges = ranges_of(splits, n_tiles);
+    Layout layout{S::STAGES, 0};
+    if (units_of(ranges, n_tiles) > ctas) return layout;
+    // One unit a CTA: a ring of as many stages as the longest unit has steps, so that a CTA of the next kernel finds
+    // room beside this one's and fetches its weights under it.
+    const int fewest = ranges.rest > 0 && ranges.rest < ranges.first ? ranges.rest : ranges.first;
+    const int steps = ((k_blocks + fewest - 1) / fewest + S::BLOCKS - 1) / S::BLOCKS;
+    if (steps < layout.ring_stages) layout.ring_stages = steps;
+    // The ranges of a tile as a cluster, where all clusters are resident at once and the sums find room.
+    const size_t receive = (size_t)(ranges.first - 1) * TILE_N * ((M + 3) / 4) * sizeof(float4);
+    if (ranges.first > 1 && ranges.tiles_first == n_tiles && n_tiles <= resident_clusters(ranges.first) &&
+        S::FIXED_BYTES + (size_t)layout.ring_stages * S::STAGE_BYTES + receive <= MAX_SMEM_BYTES)
+        layout.receive_bytes = (int)receive;
+    return layout;
+}
+
 template <int MPAD, typename OutT, int EPI>
 int launch(const CUtensorMap* w_map, const CUtensorMap* x_map, void* out, float* partials, int* counters, int M, int N,
            int K, int splits, int ctas, cudaStream_t stream, const NormLink& link, const HeadEpilogue& heads = HeadEpilogue{}) {
@@ -580,21 +605,9 @@ int launch(const CUtensorMap* w_map, const CUtensorMap* x_map, void* out, float*
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    const int n_tiles = (N + TILE_N - 1) / TILE_N, k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
+    const int n_tiles = (N + TILE_N - 1) / TILE_N;
     const Ranges ranges = ranges_of(splits, n_tiles);
-    int ring_stages = S::STAGES, receive_bytes = 0;
-    if (units_of(ranges, n_tiles) <= ctas) {
-        // One unit a CTA: a ring of as many stages as the longest unit has steps, so that a CTA of the next kernel finds
-        // room beside this one's and fetches its weights under it.
-        const int fewest = ranges.rest > 0 && ranges.rest < ranges.first ? ranges.rest : ranges.first;
-        const int steps = ((k_blocks + fewest - 1) / fewest + S::BLOCKS - 1) / S::BLOCKS;
-        if (steps < ring_stages) ring_stages = steps;
-        // The ranges of a tile as a cluster, where all clusters are resident at once and the sums find room.
-        const size_t receive = (size_t)(ranges.first - 1) * TILE_N * ((M + 3) / 4) * sizeof(float4);
-        if (ranges.first > 1 && ranges.tiles_first == n_tiles && n_tiles <= resident_clusters(ranges.first) &&
-            S::FIXED_BYTES + (size_t)ring_stages * S::STAGE_BYTES + receive <= MAX_SMEM_BYTES)
-            receive_bytes = (int)receive;
-    }
+    const auto [ring_stages, receive_bytes] = layout_of<MPAD>(M, N, K, splits, ctas);
     const size_t smem = S::FIXED_BYTES + (size_t)ring_stages * S::STAGE_BYTES + receive_bytes;
     if (receive_bytes == 0)
         return mrs_launch(kernel, dim3(ctas), dim3(THREADS), smem, stream, *w_map, *x_map, (OutT*)out, partials, counters, M, N, K,
@@ -675,7 +688,17 @@ static bool ranges_fit(int splits, int N, int K) {
     const Ranges r = ranges_of(splits, (N + TILE_N - 1) / TILE_N);
     return splits > 0 && r.first >= 1 && r.first <= k_blocks && r.rest <= k_blocks && r.tiles_first >= 0;
 }
-MRS_EXPORT int mrs_gemm_tc_resident_clusters(int ranges) { return resident_clusters(ranges); }
+// Whether a product's ranges would meet in clusters (the sums are the same either way).
+MRS_EXPORT int mrs_gemm_tc_in_cluster(int M, int N, int K, int splits, int mpad, int ctas) {
+    if (M <= 0 || N <= 0 || K <= 0 || M > mpad || !ranges_fit(splits, N, K)) return 0;
+    switch (mpad) {
+        case 16: return layout_of<16>(M, N, K, splits, ctas).receive_bytes > 0;
+        case 32: return layout_of<32>(M, N, K, splits, ctas).receive_bytes > 0;
+        case 64: return layout_of<64>(M, N, K, splits, ctas).receive_bytes > 0;
+        case 128: return layout_of<128>(M, N, K, splits, ctas).receive_bytes > 0;
+    }
+    return 0;
+}
 MRS_EXPORT int mrs_gemm_tc_counters(int N) { return (N + TILE_N - 1) / TILE_N; }
 
 // out[M, N] = x . w^T.  `w_map`: mrs_gemm_tc_map(w, N, K, 128); `x_map`: mrs_gemm_tc_map(x, M, K, mpad) with

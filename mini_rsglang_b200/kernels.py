@@ -661,6 +661,8 @@ def gemm_tc_library() -> ctypes.CDLL:
         lib.mrs_gemm_tc_partial_floats.restype = ctypes.c_longlong
         lib.mrs_gemm_tc_counters.argtypes = [_c_int]
         lib.mrs_gemm_tc_counters.restype = _c_int
+        lib.mrs_gemm_tc_in_cluster.argtypes = [_c_int] * 6
+        lib.mrs_gemm_tc_in_cluster.restype = _c_int
         lib.mrs_gemm_tc_small_m.argtypes = [_c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int,
                                             _c_int, _c_int, _c_vp, _c_vp]
         lib.mrs_gemm_tc_small_m.restype = _c_int

@@ -2,6 +2,10 @@
 at sizes other than the engine's tiny configurations (widths and vocabularies that are no power
 of two, head sizes in steps of 16, odd numbers of heads and groups)."""
 
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -783,13 +787,17 @@ def test_gemm_tc_gated_and_heads_finish_a_norm(m):
                                         (128, 8192, 16), (384, 8192, 5), (24576, 4096, 2)])
 def test_gemm_tc_ranges_merged_in_a_cluster(m, n, k, splits, monkeypatch):
     """Where every range has a CTA of its own the ranges of a tile meet in a cluster's shared memory: the same bits as
-    with fewer CTAs, whose partial sums go through global memory (both add the ranges in their order)."""
+    with fewer CTAs, whose partial sums go through global memory (both add the ranges in their order), in every epilogue."""
     torch.manual_seed(31)
     x = torch.randn(m, k, dtype=torch.bfloat16, device=DEV)
     w = torch.randn(n, k, dtype=torch.bfloat16, device=DEV) / k ** 0.5
     lib = kernels.gemm_tc_library()
     assert lib.mrs_gemm_tc_splits(6144, 1024, 148) == 2 and lib.mrs_gemm_tc_splits(1024, 3072, 148) == 8     # by N, K and SMs alone
     state = kernels._gemm_device_state(x.device)
+    mpad = 16 if m <= 16 else (32 if m <= 32 else (64 if m <= 64 else 128))
+    if (n, k, splits) in ((1024, 2048, 8), (300, 1032, 2)) and m <= 20:      # few tiles, sums that find room: clusters for certain
+        assert lib.mrs_gemm_tc_in_cluster(m, n, k, splits, mpad, state["sms"])
+    assert not lib.mrs_gemm_tc_in_cluster(m, n, k, splits, mpad, 5)
     results = []
     for sms in (state["sms"], 5):
         monkeypatch.setitem(state, "sms", sms)
@@ -797,7 +805,10 @@ def test_gemm_tc_ranges_merged_in_a_cluster(m, n, k, splits, monkeypatch):
         plain, folded = torch.empty(m, n, device=DEV), torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
         for _ in range(3):                       # back to back: a launch begins under the one before it
             kernels.gemm_tc(x, w, plain, splits=splits)
-        out = [plain]
+        rounded = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+        kernels.gemm_tc(x, w, rounded, splits=splits)
+        assert torch.equal(rounded, plain.bfloat16())
+        out = [plain, rounded]
         if n % 128 == 0:
             gated = torch.empty(m, n // 2, dtype=torch.bfloat16, device=DEV)
             kernels.gemm_tc(x, w, gated, gated=True, splits=splits)
@@ -809,6 +820,30 @@ def test_gemm_tc_ranges_merged_in_a_cluster(m, n, k, splits, monkeypatch):
     for a, b in zip(*results):
         assert torch.equal(a, b)
     close(results[0][0], x.double() @ w.double().T, torch.float32, f"gemm_tc {m}x{n}x{k} in {splits} ranges")
+
+
+FIRST_PRODUCTS = """
+import torch
+from mini_rsglang_b200 import kernels
+lib, sms = kernels.gemm_tc_library(), kernels.sm_count(torch.device("cuda", 0))
+g = torch.Generator(device="cuda").manual_seed(4)
+for n, k in ((4096, 4096), (1024, 3072), (3072, 2048), (4096, 4096)):      # 4, 8 and 4 ranges: each new count is asked about in between
+    x, w = torch.randn(16, k, device="cuda", generator=g).bfloat16(), (torch.randn(n, k, device="cuda", generator=g) / k ** 0.5).bfloat16()
+    assert lib.mrs_gemm_tc_splits(n, k, sms) > 1
+    for m in (1, 16):
+        out = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
+        kernels.gemm_tc(x[:m].contiguous(), w, out)
+        want = x[:m].double() @ w.double().T
+        assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all(), (n, k, m)
+"""
+
+
+def test_gemm_tc_plain_bfloat16_product_as_a_process_first():
+    """Asking how many clusters the GPU holds leaves the limits of shared memory as the launches set them: bfloat16 products of full
+    rings and clusters are taken as a process's first ones, and after another count of ranges was asked about."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", FIRST_PRODUCTS], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
 
 
 def test_gemm_tc_rows_do_not_depend_on_the_batch():

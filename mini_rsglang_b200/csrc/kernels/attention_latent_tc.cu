@@ -13,6 +13,10 @@
 //   warps 4-7  softmax, one thread a query row: scores from tensor memory, mask, running maximum and sum in float32,
 //              probabilities back as pairs of bfloat16; the accumulator is rescaled only when a row's maximum grew by more
 //              than 2^8, after the last P.V issued has been added.
+// A weight of 0 does not keep a row out of P.V when the row is not finite (0 x inf is no number), so the rows that no query of the
+// tile sees are zeros in shared memory: pages behind the last key or given back are copied from behind the cache, where the copy
+// fills zeros, and the others' rows before the window and behind the last key are cleared once the scores were made.  (A row that
+// one token of a tile sees reaches the tile's other tokens when it is not finite.)
 // Two warps issue because a commit holds its issuer some 400 clocks and a block's MMAs run 1,300: 18 of 45 clocks for the
 // scores (N 64), 4 of 128 for the values (N 256), 82% of the tensor cores' rate.  Four stages and four score buffers let scores run
 // ahead of softmax, which is as long.  A prompt of 2,048 tokens, 16 heads, R 256, r 32, a window of 1,024: 50 us
@@ -75,7 +79,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_latent_kernel(
     const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap q_tail_map, const __grid_constant__ CUtensorMap k_map,
     const __grid_constant__ CUtensorMap k_tail_map, const int* __restrict__ positions, const int* __restrict__ block_table, int table_width,
     const Tile* __restrict__ tiles, bf16* __restrict__ out, const float* __restrict__ gate, const float* __restrict__ sinks, int heads,
-    int page_size, int page_shift, float scale_log2, int window) {
+    int page_size, int page_shift, int cache_pages, float scale_log2, int window) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* q_smem = smem;                                // [chunk][128 rows][64], then [128 rows][32]
@@ -119,7 +123,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_latent_kernel(
     const Tile work = tiles[blockIdx.x];
     const int tokens = min(work.tokens, BM / heads);
     const int first_pos = tokens > 0 ? positions[work.first_token] : 0, key_end = first_pos + tokens;
-    const int block_first = (window > 0 ? max(0, first_pos - window + 1) : 0) / BN;
+    const int first_seen = window > 0 ? max(0, first_pos - window + 1) : 0, block_first = first_seen / BN;
     const int blocks = tokens > 0 ? (key_end + BN - 1) / BN - block_first : 0;
     const int* pages = block_table + (size_t)work.seq * table_width;
 
@@ -132,8 +136,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_latent_kernel(
         }
         __syncwarp();
         const int rows_per_copy = min(page_size, BN), copies = BN / rows_per_copy;       // pages of a block: 1 to 8
-        // lane p reads the number of a block's page p a block ahead; keys past the end, before the window or on a page that was
-        // given back are masked by their position: their copy reads page 0, which always exists and holds finite numbers
+        // lane p reads the number of a block's page p a block ahead; where there is none (keys past the end, a page that was given
+        // back) the copy takes the page behind the cache's last: zeros
         auto page_of = [&](int j) {
             const int key = (block_first + j) * BN + lane * rows_per_copy;
             return (lane < copies && key < key_end) ? pages[key >> page_shift] : -1;
@@ -153,9 +157,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_latent_kernel(
                 const int idx = base + lane, p = idx % copies, c = idx / copies;
                 const int page = __shfl_sync(0xffffffffu, pages_here, p);
                 if (idx >= copies * PARTS) continue;
-                const int key = (block_first + j) * BN + p * rows_per_copy, row = page < 0 ? 0 : key & (page_size - 1);
-                if (c < CHUNKS) tma_load_3d(stage + c * K_CHUNK + p * rows_per_copy * 128, &k_map, &bars->k_full[s], c * 64, row, max(page, 0));
-                else tma_load_3d(stage + CHUNKS * K_CHUNK + p * rows_per_copy * 64, &k_tail_map, &bars->k_full[s], 0, row, max(page, 0));
+                const int key = (block_first + j) * BN + p * rows_per_copy, row = key & (page_size - 1), from = page < 0 ? cache_pages : page;
+                if (c < CHUNKS) tma_load_3d(stage + c * K_CHUNK + p * rows_per_copy * 128, &k_map, &bars->k_full[s], c * 64, row, from);
+                else tma_load_3d(stage + CHUNKS * K_CHUNK + p * rows_per_copy * 64, &k_tail_map, &bars->k_full[s], 0, row, from);
             }
             __syncwarp();
         }
@@ -223,6 +227,18 @@ __global__ void __launch_bounds__(THREADS, 1) attention_latent_kernel(
             mbar_wait(&bars->s_full[s], (j / STAGES) & 1);
             __syncwarp();                                        // the loads below are collective: the warp goes on together
             tcgen05_fence_after_sync();
+            // rows of the block that no query of the tile sees: before the window of the first, behind the last key
+            const int live_from = max(0, first_seen - key0), live_to = min(BN, key_end - key0);
+            if (live_from > 0 || live_to < BN) {                 // the scores have read the keys, and P.V waits for this warp below
+                mbar_wait(&bars->k_full[s], (j / STAGES) & 1);   // complete: the copies' writes come before those here
+                for (int idx = threadIdx.x - 128; idx < (R / 64) * BN * 8; idx += 128) {
+                    const int c = idx / (BN * 8), row_of = idx / 8 % BN;     // a row's 128 bytes of a chunk stay its own in the swizzle
+                    if (row_of < live_from || row_of >= live_to)
+                        *reinterpret_cast<uint4*>(k_smem + s * K_BYTES + c * K_CHUNK + idx % (BN * 8) * 16) = make_uint4(0, 0, 0, 0);
+                }
+                fence_async_shared();
+                __syncwarp();
+            }
             const bool edge = key0 + BN - 1 > first_pos || (window > 0 && key0 < key_end - window);
             float x[BN];
 #pragma unroll
@@ -362,12 +378,15 @@ MRS_EXPORT int mrs_attention_latent_tc_query_maps(const void* q, long long token
 
 // Tiles of up to 128 / heads consecutive tokens of one request each: (sequence, first token, tokens, 0).  out [tokens, heads, R];
 // `gate` [tokens, heads] or null multiplies a head's result; `sinks` [heads] or null: one more term exp(sink) in the denominator.
+// `cache_pages`: the pages that the cache's maps cover.
 MRS_EXPORT int mrs_attention_latent_tc(const void* query_maps, const void* cache_maps, const int* positions, const int* block_table,
                                        int table_width, const int* tiles, int num_tiles, void* out, const float* gate, const float* sinks,
-                                       int heads, int page_size, float scale, int window, void* stream) {
+                                       int heads, int page_size, long long cache_pages, float scale, int window, void* stream) {
     if (num_tiles <= 0) return 0;
     const int shift = page_shift_of(page_size);
-    if (shift < 0 || page_size < 8 || heads <= 0 || heads > BM || !(scale > 0.0f) || window < 0 || ((uintptr_t)out & 15)) return MRS_BAD_ARGUMENT;
+    if (shift < 0 || page_size < 8 || cache_pages <= 0 || cache_pages >= 0x7fffffff || heads <= 0 || heads > BM ||
+        !(scale > 0.0f) || window < 0 || ((uintptr_t)out & 15))
+        return MRS_BAD_ARGUMENT;
     static bool configured = false;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(attention_latent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
@@ -376,7 +395,7 @@ MRS_EXPORT int mrs_attention_latent_tc(const void* query_maps, const void* cache
     }
     const CUtensorMap *q = reinterpret_cast<const CUtensorMap*>(query_maps), *k = reinterpret_cast<const CUtensorMap*>(cache_maps);
     MRS_LAUNCH(attention_latent_kernel, num_tiles, THREADS, SMEM_BYTES, stream, q[0], q[TAIL ? 1 : 0], k[0], k[TAIL ? 1 : 0], positions, block_table,
-               table_width, (const Tile*)tiles, (bf16*)out, gate, sinks, heads, page_size, shift, scale * LOG2E, window);
+               table_width, (const Tile*)tiles, (bf16*)out, gate, sinks, heads, page_size, shift, (int)cache_pages, scale * LOG2E, window);
     MRS_RETURN_LAUNCH_STATUS();
 }
 

@@ -1490,7 +1490,8 @@ def attention_latent_tc_library(latent: int, rotated: int) -> ctypes.CDLL:
         lib = specialised_kernel_library("attention_latent_tc.cu", {"MRS_LATENT": latent, "MRS_ROTARY": rotated})
         lib.mrs_attention_latent_tc_cache_maps.argtypes = [_c_vp, ctypes.c_longlong, _c_int, _c_vp]
         lib.mrs_attention_latent_tc_query_maps.argtypes = [_c_vp, ctypes.c_longlong, _c_int, _c_vp]
-        lib.mrs_attention_latent_tc.argtypes = [_c_vp] * 4 + [_c_int, _c_vp, _c_int, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_float, _c_int, _c_vp]
+        lib.mrs_attention_latent_tc.argtypes = [_c_vp] * 4 + [_c_int, _c_vp, _c_int, _c_vp, _c_vp, _c_vp, _c_int, _c_int, ctypes.c_longlong, _c_float, _c_int,
+                                                              _c_vp]
         lib.mrs_attention_latent_tc_take_error.argtypes = [ctypes.POINTER(ctypes.c_uint)]
         for name in ("cache_maps", "query_maps", "take_error", "rows"):
             getattr(lib, f"mrs_attention_latent_tc_{name}").restype = _c_int
@@ -1541,7 +1542,7 @@ def attention_latent_tc(q, cache, positions, block_table, tiles, out, heads: int
     launch_count += 1
     code = lib.mrs_attention_latent_tc(maps + 256, maps, positions.data_ptr(), block_table.data_ptr(),
                                        block_table.shape[1], tiles.data_ptr(), tiles.shape[0], out.data_ptr(), _ptr(gate), _ptr(sink_logits),
-                                       heads, page_size, float(scale), int(window), _stream())
+                                       heads, page_size, cache.shape[0], float(scale), int(window), _stream())
     del keep                          # the maps were copied into the launch
     if code != 0:
         fail(code, "attention_latent_tc")

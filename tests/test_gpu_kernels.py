@@ -1087,3 +1087,85 @@ def test_attention_latent_tc(heads, latent, rotated, page, window):
             # a weight and the result rounded to bfloat16 (2^-9 each), the scores' float32 sums far below
             assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -8 + 1e-6).all(), (i, use_gate)
             at += n
+
+
+@pytest.mark.parametrize("heads,latent,rotated,page,window", [(16, 256, 32, 16, 0), (16, 256, 32, 16, 100), (32, 256, 32, 8, 1024), (5, 192, 64, 64, 70),
+                                                              (3, 128, 0, 128, 0), (64, 64, 32, 32, 33)])
+def test_attention_latent_tc_leaves_out_rows_that_no_query_sees(heads, latent, rotated, page, window):
+    """Rows behind a portion's last key, before its window, on pages of other requests, on the cache's first page (which no table names
+    here) and on pages that were given back are no numbers: the results are those over a clean cache, bit for bit."""
+    spans = [(0, 1), (0, 130), (63, 1), (64, 65), (500, 3), (1100, 9)]
+    row, per_tile = latent + rotated, 128 // heads
+    g = torch.Generator(device=DEV).manual_seed(heads + page)
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).to(DEV)      # noqa: E731
+    scale = row ** -0.5
+    for c, n in spans:
+        pages = -(-(c + n) // page)
+        clean = torch.randn(2 * pages + 3, 1, page, row, device=DEV, generator=g).bfloat16()
+        order = (1 + torch.randperm(clean.shape[0] - 1, generator=g, device=DEV)[:pages]).tolist()
+        # one portion of a tile's tokens at a time: which of its rows nobody sees is then the portion's own matter
+        for start in {0, (n - 1) // per_tile * per_tile}:
+            tokens, first = min(per_tile, n - start), c + start
+            seen = max(0, first - window + 1) if window else 0
+            q = torch.randn(tokens, heads * row, device=DEV, generator=g).bfloat16()
+            dirty = torch.full_like(clean, float("nan"))
+            dirty[::2] = float("inf")
+            slots = torch.arange(seen, first + tokens, device=DEV)
+            pages_of = torch.tensor(order, device=DEV)[slots // page]
+            dirty[pages_of, 0, slots % page] = clean[pages_of, 0, slots % page]
+            results = []
+            for cache, gone in ((clean, 0), (dirty, 0), (dirty, seen // page)):
+                out = torch.full((tokens, heads * latent), 77.0, device=DEV).bfloat16()
+                kernels.attention_latent_tc(q, cache, i32(list(range(first, first + tokens))), i32([[-1] * gone + order[gone:]]), i32([(0, 0, tokens, 0)]), out,
+                                            heads, latent, rotated, scale, window=window)
+                kernels.check_device_errors(certain=True)
+                results.append(out)
+            assert torch.isfinite(results[0].float()).all()
+            assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2]), (c, n, start)
+
+
+def test_attention_latent_tc_scores_that_are_no_numbers():
+    """A query that is no number gives its own (token, head) no number and no other one; rows whose scores are all -inf have no
+    weights and give zeros; a score of +inf gives no number, as its softmax does."""
+    heads, latent, rotated, page, n = 16, 256, 32, 16, 8
+    row = latent + rotated
+    g = torch.Generator(device=DEV).manual_seed(3)
+    cache = torch.randn(9, 1, page, row, device=DEV, generator=g).bfloat16()
+    cache[..., latent:] = cache[..., latent:].abs() + 1               # the last elements tell the sign of an infinite score
+    q = torch.randn(n, heads, row, device=DEV, generator=g).bfloat16()
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).to(DEV)      # noqa: E731
+
+    def attend(q):
+        out = torch.full((n, heads * latent), 77.0, device=DEV).bfloat16()
+        kernels.attention_latent_tc(q.reshape(n, -1).contiguous(), cache, i32(list(range(100, 100 + n))), i32([[3, 1, 4, 8, 5, 0, 2]]), i32([(0, 0, n, 0)]), out,
+                                    heads, latent, rotated, row ** -0.5)
+        kernels.check_device_errors(certain=True)
+        return out.view(n, heads, latent)
+
+    clean, odd = attend(q), q.clone()
+    odd[2, 3, 7] = float("nan")
+    odd[5, 0, row - 1] = -float("inf")
+    odd[6, 9, row - 1] = float("inf")
+    got = attend(odd)
+    assert torch.isnan(got[2, 3]).all() and torch.isnan(got[6, 9]).all() and (got[5, 0] == 0).all()
+    for token, head in ((2, 3), (5, 0), (6, 9)):
+        got[token, head] = clean[token, head]
+    assert torch.equal(got, clean)
+
+
+def test_attention_f32_keeps_what_is_no_number_in_its_row():
+    """A query that is no number gives its own (token, head) no number and no other one, in tiles of rows, single tokens and with the
+    keys in chunks."""
+    nq, nkv, d, page = 4, 2, 64, 16
+    case = PagedCase(torch.float32, nq, nkv, d, page, [(0, 90), (700, 3), (1200, 1)], seed=5)
+    clean = case.run_simt().view(-1, nq, d)
+    odd = case.q.clone().view(-1, nq, d)
+    marks = ((0, 1), (70, 2), (91, 0), (93, 3))
+    for token, head in marks:
+        odd[token, head, 5] = float("nan")
+    case.q = odd.view(case.q.shape)
+    got = case.run_simt().view(-1, nq, d)
+    for token, head in marks:
+        assert torch.isnan(got[token, head]).all()
+        got[token, head] = clean[token, head]
+    assert torch.equal(got, clean)

@@ -123,9 +123,9 @@ MRS_EXPORT int mrs_argmax(const float* logits, int* out, int rows, int vocab, vo
 // through distributed shared memory.  What bounds it is the chain of those meetings: a row is read once (608 KB at
 // 151,936 logits), a threshold takes three digits of 11, 11 and 10 bits with two cluster barriers each.  One CTA a row,
 // which read the row from L2 some fifteen times with 8-bit digits, took 1,626 us for 24 rows of 151,936 logits (top-k and
-// top-p rows among them); a cluster with weights added as floats and one warp that walked the drawn segment took 87 us,
-// whole numbers of 2^-34 and all warps at the segment take 81 (all 24 rows with top-k and top-p: 86; top-k alone 40, temperature
-// alone 25, greedy 10).
+// top-p rows among them); a cluster with weights added as floats and one warp that walked the drawn segment took 87 us.  With weights
+// as whole numbers, all warps at the segment and counts only in the digits that need them, 24 rows with top-k and top-p take 68 us,
+// with top-p alone 69, top-k alone 35, temperature alone 23, greedy 8 (one row: 47, 48, 25, 17, 6).
 //
 // The weights of the kept set are summed in 32 segments of a row, in id order, whatever the cluster's size: a row's token
 // does not depend on how many CTAs shared it.
@@ -135,9 +135,10 @@ MRS_EXPORT int mrs_argmax(const float* logits, int* out, int rows, int vocab, vo
 #define SAMPLE_MAX_BLOCKS 8
 #define SAMPLE_SEGMENTS 32
 #define SAMPLE_BINS 2048
-#define SAMPLE_OWN_BINS (SAMPLE_BINS / SAMPLE_CTA_THREADS)     // bins a thread looks at when the edge is searched
 #define SAMPLE_SHARE_BYTES (160 * 1024)                        // of a row in a CTA's shared memory, at most (up to 77 KB two CTAs fit an SM)
+#define SAMPLE_PIECE 32768                                     // elements of a longer share whose weights are added at a time
 #define SAMPLE_NOT_KEPT (-1.0f)
+static_assert(SAMPLE_SHARE_BYTES / 4 <= 65535 && SAMPLE_PIECE <= 65535, "parts of weights fit 32 bits");
 
 // Which elements are kept: keys above `low`, and the first `quota` ids among keys equal to `low`.
 struct Cut {
@@ -145,31 +146,37 @@ struct Cut {
     int quota;
 };
 
-// A weight (0 .. 1) as a whole number of 2^-(2 bits): a high and a low part of `bits` bits each, whose sums over a CTA's share fit
-// 32 bits (native additions in shared memory; sums of whole numbers do not depend on their order).
+// A weight (0 .. 1) as a whole number of 2^-48 in three parts of 16 bits, whose sums over up to 65,535 elements fit 32 bits each
+// (native additions in shared memory; sums of whole numbers do not depend on their order).  A float32 from 2^-25 on is such a number
+// itself; a smaller one is off by 2^-49 at most, a million of them together by 2^-29 of the largest weight.  Bins are added up
+// across CTAs and along the row in float64, in a fixed order.
 struct Fixed {
-    unsigned high, low;
+    unsigned high, mid, low;
 };
-__device__ __forceinline__ Fixed fixed_weight(float w, float scale) {
-    const float x = w * scale, whole = floorf(x);                       // scale is a power of two: both exact
-    return Fixed{(unsigned)whole, __float2uint_rn((x - whole) * scale)};
+__device__ __forceinline__ Fixed fixed_weight(float w) {
+    const float x = w * 65536.0f, high = floorf(x), y = (x - high) * 65536.0f, mid = floorf(y);      // all exact
+    return Fixed{(unsigned)high, (unsigned)mid, __float2uint_rn((y - mid) * 65536.0f)};
+}
+__device__ __forceinline__ double fixed_value(unsigned high, unsigned mid, unsigned low) {
+    return (double)(((unsigned long long)high << 32) + ((unsigned long long)mid << 16) + low) * (1.0 / 281474976710656.0);
 }
 
 struct SampleShared {
     Best warp_best[33];                              // block_best's
-    Best best;                                       // of this CTA's share; read by the whole cluster, as are the next nine
+    Best best;                                       // of this CTA's share; read by the whole cluster, as are the next eight
     int bad;
-    unsigned count[SAMPLE_BINS];                     // this CTA's histogram
-    unsigned high[SAMPLE_BINS], low[SAMPLE_BINS];
+    // This CTA's histogram.  By count it is `high`; by weight it is the three parts, which give their place (`high` and `mid`) to the
+    // words of a float64 when the walk is over; the last digit, of half as many bins, also counts, in the upper half of `high`.
+    unsigned high[SAMPLE_BINS], mid[SAMPLE_BINS], low[SAMPLE_BINS];
     unsigned slice_count[SAMPLE_BINS / 4];           // this CTA's slice of the bins, summed over the cluster
-    unsigned long long slice_weight[SAMPLE_BINS / 4];
+    double slice_weight[SAMPLE_BINS / 4];
     int seg_ties[SAMPLE_SEGMENTS];                   // this CTA's segments
     float seg_weight[SAMPLE_SEGMENTS];
     unsigned warp_count[SAMPLE_CTA_WARPS];           // scan over the bins
-    unsigned long long warp_weight[SAMPLE_CTA_WARPS];
+    double warp_weight[SAMPLE_CTA_WARPS];
     int first, lowest;                               // places in descending order of the bins
     unsigned edge_count, above_count;
-    unsigned long long above_weight;
+    double above_weight;
     int all_ties[SAMPLE_SEGMENTS];
     float all_weight[SAMPLE_SEGMENTS];
 };
@@ -179,72 +186,96 @@ struct SampleShared {
 struct Edge {
     unsigned prefix, mask, count;     // `count`: elements of the last digit's bin
     unsigned above_count;
-    unsigned long long above_weight, total;
-    double target;                    // weight, in the same units, that the edge has to reach
+    double above_weight, target;      // `target`: the weight that the edge has to reach
 };
 
-// One digit.  `walk_elements(add)` walks this CTA's elements and calls add(key, w) for those to be counted, w() being an element's
-// weight (the digit's place is applied here); by weight the first bin (from the top) whose running weight reaches
-// `share` of all the weight (a float32 product) is chosen, by count the first whose running count reaches `wanted`.  `extra_key`, `extra_weight`: a
-// run of equal keys that the elements leave out, added to its bin once.
-template <bool BY_WEIGHT, typename Walk>
-__device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsigned rank, unsigned blocks, int shift, int bits, Edge& e,
-                             Walk walk_elements, int weight_bits, float share, unsigned wanted, bool has_extra, unsigned extra_key,
-                             unsigned long long extra_weight) {
-    const unsigned digit = (1u << bits) - 1u;
-    const float scale = (float)(1u << weight_bits);
-    const double unit = 1.0 / ((double)scale * (double)scale);
-    for (int b = threadIdx.x; b < SAMPLE_BINS; b += SAMPLE_CTA_THREADS) {
-        s.count[b] = 0u;
-        if (BY_WEIGHT) s.high[b] = 0u, s.low[b] = 0u;
+// One digit of BITS bits.  `walk_elements(piece, add)` walks this CTA's elements of a piece (at most 65,535 of them) and calls
+// add(key, w) for those to be counted, w() being an element's weight (the digit's place is applied here); by weight the first bin (from
+// the top) whose running weight reaches `share` of all the weight (a float32 product) is chosen, by count the first whose running
+// count reaches `wanted`.  By weight a bin without weight counts as empty.  `extra_key`, `extra_weight`: a run of equal keys that the
+// elements leave out, added to its bin once.
+template <bool BY_WEIGHT, int BITS, typename Walk>
+__device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsigned rank, unsigned blocks, int shift, Edge& e,
+                             Walk walk_elements, int pieces, float share, unsigned wanted, bool has_extra, unsigned extra_key,
+                             double extra_weight) {
+    constexpr int BINS = 1 << BITS, OWN = BINS / SAMPLE_CTA_THREADS;      // bins, and bins a thread looks at when the edge is searched
+    constexpr bool COUNTED = !BY_WEIGHT || 2 * BINS <= SAMPLE_BINS;
+    static_assert(BINS <= SAMPLE_BINS && OWN * SAMPLE_CTA_THREADS == BINS, "whole bins a thread");
+    unsigned* count = BY_WEIGHT ? s.high + SAMPLE_BINS / 2 : s.high;
+    double held[OWN];                                // weights of bins threadIdx.x, + CTA_THREADS, ...
+#pragma unroll
+    for (int j = 0; j < OWN; ++j) {
+        const int b = threadIdx.x + j * SAMPLE_CTA_THREADS;
+        held[j] = 0.0;
+        if (COUNTED) count[b] = 0u;
+        if (BY_WEIGHT) s.high[b] = 0u, s.mid[b] = 0u, s.low[b] = 0u;
     }
     if (threadIdx.x == 0) s.first = 0x7fffffff, s.lowest = -1;
     __syncthreads();
-    walk_elements([&](unsigned key, auto weight) {
-        if ((key & e.mask) != e.prefix) return;
-        const unsigned b = (key >> shift) & digit;
-        atomicAdd(&s.count[b], 1u);
-        if (BY_WEIGHT) {
-            const Fixed w = fixed_weight(weight(), scale);
-            if (w.high) atomicAdd(&s.high[b], w.high);
-            if (w.low) atomicAdd(&s.low[b], w.low);
+    for (int piece = 0; piece < pieces; ++piece) {
+        walk_elements(piece, [&](unsigned key, auto weight) {
+            if ((key & e.mask) != e.prefix) return;
+            const unsigned b = (key >> shift) & (BINS - 1u);
+            if (COUNTED) atomicAdd(&count[b], 1u);
+            if (BY_WEIGHT) {
+                const Fixed w = fixed_weight(weight());
+                if (w.high) atomicAdd(&s.high[b], w.high);
+                if (w.mid) atomicAdd(&s.mid[b], w.mid);
+                if (w.low) atomicAdd(&s.low[b], w.low);
+            }
+        });
+        if (!BY_WEIGHT) continue;
+        __syncthreads();
+        const bool last = piece + 1 == pieces;
+#pragma unroll
+        for (int j = 0; j < OWN; ++j) {
+            const int b = threadIdx.x + j * SAMPLE_CTA_THREADS;
+            held[j] += fixed_value(s.high[b], s.mid[b], s.low[b]);
+            s.high[b] = last ? (unsigned)__double2hiint(held[j]) : 0u;
+            s.mid[b] = last ? (unsigned)__double2loint(held[j]) : 0u;
+            s.low[b] = 0u;
         }
-    });
+        if (!last) __syncthreads();
+    }
     const bool extra = BY_WEIGHT && has_extra && (extra_key & e.mask) == e.prefix;
-    const int extra_bin = (int)((extra_key >> shift) & digit);
+    const int extra_bin = (int)((extra_key >> shift) & (BINS - 1u));
+    auto weight_in = [&](unsigned r, int bin) {
+        return __hiloint2double((int)cluster.map_shared_rank(s.high, r)[bin], (int)cluster.map_shared_rank(s.mid, r)[bin]);
+    };
+    const int slice = BINS / blocks;
     if (blocks > 1) {
         cluster.sync();
-        const int slice = SAMPLE_BINS / blocks;
-        for (int i = threadIdx.x; i < slice; i += SAMPLE_CTA_THREADS) {
+        if ((int)threadIdx.x < slice) {
+            const int b = (int)rank * slice + (int)threadIdx.x;
             unsigned c = 0u;
-            unsigned long long high = 0ull, low = 0ull;
+            double w = 0.0;
 #pragma unroll
             for (unsigned r = 0; r < SAMPLE_MAX_BLOCKS; ++r) {       // all loads under way together
                 if (r >= blocks) continue;
-                c += cluster.map_shared_rank(s.count, r)[rank * slice + i];
-                if (BY_WEIGHT) high += cluster.map_shared_rank(s.high, r)[rank * slice + i], low += cluster.map_shared_rank(s.low, r)[rank * slice + i];
+                if (COUNTED) c += cluster.map_shared_rank(count, r)[b];
+                if (BY_WEIGHT) w += weight_in(r, b);
             }
-            s.slice_count[i] = c;
-            if (BY_WEIGHT) s.slice_weight[i] = (high << weight_bits) + low;
+            s.slice_count[threadIdx.x] = c;
+            if (BY_WEIGHT) s.slice_weight[threadIdx.x] = w;
         }
         cluster.sync();
     } else {
         __syncthreads();
     }
-    // bins from the top: thread t has places 4 t .. 4 t + 3, place p is bin BINS - 1 - p
-    unsigned c[SAMPLE_OWN_BINS], c_sum = 0u;
-    unsigned long long w[SAMPLE_OWN_BINS], w_sum = 0ull;
+    // bins from the top: thread t has places OWN t .. OWN t + OWN - 1, place p is bin BINS - 1 - p
+    unsigned c[OWN], c_sum = 0u;
+    double w[OWN], w_sum = 0.0;
 #pragma unroll
-    for (int j = 0; j < SAMPLE_OWN_BINS; ++j) {
-        const int bin = SAMPLE_BINS - 1 - ((int)threadIdx.x * SAMPLE_OWN_BINS + j);
-        w[j] = 0ull;
+    for (int j = 0; j < OWN; ++j) {
+        const int bin = BINS - 1 - ((int)threadIdx.x * OWN + j);
+        c[j] = 0u;
+        w[j] = 0.0;
         if (blocks > 1) {
-            const int slice = SAMPLE_BINS / blocks;
-            c[j] = cluster.map_shared_rank(s.slice_count, bin / slice)[bin % slice];
+            if (COUNTED) c[j] = cluster.map_shared_rank(s.slice_count, bin / slice)[bin % slice];
             if (BY_WEIGHT) w[j] = cluster.map_shared_rank(s.slice_weight, bin / slice)[bin % slice];
         } else {
-            c[j] = s.count[bin];
-            if (BY_WEIGHT) w[j] = ((unsigned long long)s.high[bin] << weight_bits) + s.low[bin];
+            if (COUNTED) c[j] = count[bin];
+            if (BY_WEIGHT) w[j] = weight_in(0, bin);
         }
         if (extra && bin == extra_bin) c[j] += 1u, w[j] += extra_weight;
         c_sum += c[j];
@@ -252,37 +283,43 @@ __device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsign
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned c_run = c_sum;
-    unsigned long long w_run = w_sum;
+    double w_run = w_sum, w_before = 0.0, w_total = 0.0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const unsigned cu = __shfl_up_sync(0xffffffffu, c_run, o);
-        if (lane >= o) c_run += cu;
-        if (BY_WEIGHT) {
-            const unsigned long long wu = __shfl_up_sync(0xffffffffu, w_run, o);
+        if (!BY_WEIGHT) {
+            const unsigned cu = __shfl_up_sync(0xffffffffu, c_run, o);
+            if (lane >= o) c_run += cu;
+        } else {
+            const double wu = __shfl_up_sync(0xffffffffu, w_run, o);
             if (lane >= o) w_run += wu;
         }
+    }
+    if (BY_WEIGHT) {
+        w_before = __shfl_up_sync(0xffffffffu, w_run, 1);
+        if (lane == 0) w_before = 0.0;
     }
     if (lane == 31) s.warp_count[warp] = c_run, s.warp_weight[warp] = w_run;
     __syncthreads();
     unsigned c_before = c_run - c_sum;
-    unsigned long long w_before = w_run - w_sum, w_total = 0ull;
     for (int i = 0; i < SAMPLE_CTA_WARPS; ++i) {
-        if (i < warp) c_before += s.warp_count[i], w_before += s.warp_weight[i];
-        if (BY_WEIGHT) w_total += s.warp_weight[i];
+        if (!BY_WEIGHT && i < warp) c_before += s.warp_count[i];
+        if (BY_WEIGHT) {
+            if (i == warp) w_before += w_total;
+            w_total += s.warp_weight[i];
+        }
     }
-    if (e.mask == 0u) e.total = w_total;
-    if (BY_WEIGHT && e.mask == 0u) e.target = (double)(share * (float)((double)e.total * unit)) / unit;
-    const double goal = BY_WEIGHT ? e.target - (double)e.above_weight : 0.0;
+    if (BY_WEIGHT && e.mask == 0u) e.target = (double)(share * (float)w_total);
+    const double goal = BY_WEIGHT ? e.target - e.above_weight : 0.0;
     const unsigned need = wanted - e.above_count;
     {
         unsigned ca = c_before;
-        unsigned long long wa = w_before;
+        double wa = w_before;
         int found = 0x7fffffff, last = -1;
 #pragma unroll
-        for (int j = 0; j < SAMPLE_OWN_BINS; ++j) {
-            if (c[j] == 0u) continue;
-            last = (int)threadIdx.x * SAMPLE_OWN_BINS + j;
-            if (found == 0x7fffffff && (BY_WEIGHT ? (double)(wa + w[j]) >= goal : ca + c[j] >= need)) found = last;
+        for (int j = 0; j < OWN; ++j) {
+            if (BY_WEIGHT ? w[j] == 0.0 : c[j] == 0u) continue;
+            last = (int)threadIdx.x * OWN + j;
+            if (found == 0x7fffffff && (BY_WEIGHT ? wa + w[j] >= goal : ca + c[j] >= need)) found = last;
             ca += c[j];
             wa += w[j];
         }
@@ -291,23 +328,23 @@ __device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsign
     }
     __syncthreads();
     const int place = s.first != 0x7fffffff ? s.first : max(s.lowest, 0);      // rounding left the sum a hair short: the last bin holds the edge
-    if (place / SAMPLE_OWN_BINS == (int)threadIdx.x) {
+    if (place / OWN == (int)threadIdx.x) {
         unsigned ca = c_before, here = 0u;
-        unsigned long long wa = w_before;
+        double wa = w_before;
 #pragma unroll
-        for (int j = 0; j < SAMPLE_OWN_BINS; ++j) {
-            if ((int)threadIdx.x * SAMPLE_OWN_BINS + j < place) ca += c[j], wa += w[j];
-            if ((int)threadIdx.x * SAMPLE_OWN_BINS + j == place) here = c[j];
+        for (int j = 0; j < OWN; ++j) {
+            if ((int)threadIdx.x * OWN + j < place) ca += c[j], wa += w[j];
+            if ((int)threadIdx.x * OWN + j == place) here = c[j];
         }
         s.edge_count = here;
         s.above_count = ca;
         s.above_weight = wa;
     }
     __syncthreads();
-    e.prefix |= (unsigned)(SAMPLE_BINS - 1 - place) << shift;
-    e.mask |= digit << shift;
+    e.prefix |= (unsigned)(BINS - 1 - place) << shift;
+    e.mask |= (BINS - 1u) << shift;
     e.count = s.edge_count;
-    e.above_count += s.above_count;
+    if (!BY_WEIGHT) e.above_count += s.above_count;
     e.above_weight += s.above_weight;
     // the histogram is written again after the next barrier of the cluster's first kind: every CTA has read its slices by then
 }
@@ -316,7 +353,7 @@ __device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsign
 // otherwise a row is too long for that and is read from memory each time.
 template <bool IN_SHARED>
 __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
-    const float* __restrict__ logits, int vocab, int per_segment, int weight_bits, const float* __restrict__ temperature,
+    const float* __restrict__ logits, int vocab, int per_segment, const float* __restrict__ temperature,
     const int* __restrict__ top_k, const float* __restrict__ top_p, const unsigned long long* __restrict__ seed,
     const int* __restrict__ draw_index, int* __restrict__ out) {
     pdl_launch_dependents();
@@ -371,12 +408,12 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
         bad |= *cluster.map_shared_rank(&s.bad, q);
     }
     // the same in every CTA of the cluster: they leave together, and none while another still reads its shared memory
-    if (bad || temp == 0.0f || k_raw == 1) {
+    const float inv_t = 1.0f / temp;                 // beyond a float's range: as temperature 0
+    if (bad || temp == 0.0f || k_raw == 1 || isinf(inv_t)) {
         if (rank == 0 && threadIdx.x == 0) out[r] = bad ? -1 : top.id;
         if (blocks > 1) cluster.sync();
         return;
     }
-    const float inv_t = 1.0f / temp;
     const float* x = IN_SHARED ? share : row;
     auto weight_of = [&](float v) { return expf((v - top.value) * inv_t); };
 
@@ -385,17 +422,17 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     Cut cut = {0u, 0x7fffffff};
     int ties = 0;                                    // elements of the row whose key is cut.low, where some of them may be left out
     if (k_raw > 0 && k_raw < vocab) {
-        Edge e = {0u, 0u, 0u, 0u, 0ull, 0ull, 0.0};
-        auto each = [&](auto add) {
+        Edge e = {0u, 0u, 0u, 0u, 0.0, 0.0};
+        auto each = [&](int, auto add) {
 #pragma unroll 4
             for (int i = threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) add(ordered_key(x[i]), [] { return 0.0f; });
         };
-        sample_digit<false>(cluster, s, rank, blocks, 21, 11, e, each, 0, 0.0f, (unsigned)k_raw, false, 0u, 0ull);
-        sample_digit<false>(cluster, s, rank, blocks, 10, 11, e, each, 0, 0.0f, (unsigned)k_raw, false, 0u, 0ull);
+        sample_digit<false, 11>(cluster, s, rank, blocks, 21, e, each, 1, 0.0f, (unsigned)k_raw, false, 0u, 0.0);
+        sample_digit<false, 11>(cluster, s, rank, blocks, 10, e, each, 1, 0.0f, (unsigned)k_raw, false, 0u, 0.0);
         if (e.above_count + e.count == (unsigned)k_raw) {
             cut.low = e.prefix;                      // all keys of the bin are kept, whatever their last digit
         } else {
-            sample_digit<false>(cluster, s, rank, blocks, 0, 10, e, each, 0, 0.0f, (unsigned)k_raw, false, 0u, 0ull);
+            sample_digit<false, 10>(cluster, s, rank, blocks, 0, e, each, 1, 0.0f, (unsigned)k_raw, false, 0u, 0.0);
             cut.low = e.prefix;
             cut.quota = k_raw - (int)e.above_count;
             ties = (int)e.count;
@@ -404,28 +441,29 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
 
     // ---- top_p: the key at which the running weight reaches top_p times the top_k set's weight ---
     if (p_raw < 1.0f) {
-        Edge e = {0u, 0u, 0u, 0u, 0ull, 0ull, 0.0};
-        const float scale = (float)(1u << weight_bits);
-        auto units = [&](float w) {
-            const Fixed f = fixed_weight(w, scale);
-            return ((unsigned long long)f.high << weight_bits) + f.low;
+        Edge e = {0u, 0u, 0u, 0u, 0.0, 0.0};
+        auto counted = [&](float w) {                // a weight as the histograms count it
+            const Fixed f = fixed_weight(w);
+            return fixed_value(f.high, f.mid, f.low);
         };
         const bool some = cut.quota < ties;          // only some of the equals at the cut: they are added as one
         const unsigned low = cut.low;
-        const unsigned long long low_weight = some ? units(weight_of(key_value(low))) * (unsigned long long)cut.quota : 0ull;
-        auto each = [&](auto add) {
+        const double low_weight = some ? counted(weight_of(key_value(low))) * cut.quota : 0.0;
+        const int pieces = IN_SHARED ? 1 : (length + SAMPLE_PIECE - 1) / SAMPLE_PIECE;
+        auto each = [&](int piece, auto add) {
+            const int from = IN_SHARED ? 0 : piece * SAMPLE_PIECE, to = IN_SHARED ? length : min(length, from + SAMPLE_PIECE);
 #pragma unroll 4
-            for (int i = threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) {
+            for (int i = from + threadIdx.x; i < to; i += SAMPLE_CTA_THREADS) {
                 const float v = x[i];
                 const unsigned key = ordered_key(v);
                 if (some ? key > low : key >= low) add(key, [&] { return weight_of(v); });
             }
         };
-        sample_digit<true>(cluster, s, rank, blocks, 21, 11, e, each, weight_bits, p_raw, 0u, some, low, low_weight);
-        sample_digit<true>(cluster, s, rank, blocks, 10, 11, e, each, weight_bits, p_raw, 0u, some, low, low_weight);
-        sample_digit<true>(cluster, s, rank, blocks, 0, 10, e, each, weight_bits, p_raw, 0u, some, low, low_weight);
-        const unsigned long long one = units(weight_of(key_value(e.prefix)));
-        const double missing = (e.target - (double)e.above_weight) / (double)one;
+        sample_digit<true, 11>(cluster, s, rank, blocks, 21, e, each, pieces, p_raw, 0u, some, low, low_weight);
+        sample_digit<true, 11>(cluster, s, rank, blocks, 10, e, each, pieces, p_raw, 0u, some, low, low_weight);
+        sample_digit<true, 10>(cluster, s, rank, blocks, 0, e, each, pieces, p_raw, 0u, some, low, low_weight);
+        const double one = counted(weight_of(key_value(e.prefix)));
+        const double missing = (e.target - e.above_weight) / one;
         const int need = missing < 2147483647.0 ? max(1, (int)ceil(missing)) : 0x7fffffff;        // a weight of nothing: all its equals
         if (some && e.prefix == cut.low) {
             cut.quota = min(cut.quota, need);
@@ -596,8 +634,6 @@ MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float*
     if (rows > 0x7fffffff / 8) return MRS_BAD_ARGUMENT;
     const size_t share = (size_t)per_segment * (SAMPLE_SEGMENTS / blocks) * sizeof(float);
     const bool in_shared = share <= SAMPLE_SHARE_BYTES;
-    int weight_bits = 17;                             // so that a share's weights, at most one each, sum up to less than 2^32
-    while (weight_bits > 1 && (unsigned long long)(share / sizeof(float)) << weight_bits >= (1ull << 32)) --weight_bits;
     static bool configured = false;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SHARE_BYTES);
@@ -617,8 +653,8 @@ MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float*
     static const bool plain = getenv("MRS_PLAIN_LAUNCH") != nullptr;
     config.attrs = attributes;
     config.numAttrs = plain ? 1 : 2;
-    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true>, logits, vocab, per_segment, weight_bits, temperature, top_k, top_p, seed, draw_index, out)
-                                    : cudaLaunchKernelEx(&config, sample_kernel<false>, logits, vocab, per_segment, weight_bits, temperature, top_k, top_p, seed, draw_index, out);
+    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out)
+                                    : cudaLaunchKernelEx(&config, sample_kernel<false>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out);
     if (e != cudaSuccess) return (int)e;
     MRS_RETURN_LAUNCH_STATUS();
 }

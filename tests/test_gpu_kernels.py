@@ -6,6 +6,7 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 import torch
 
@@ -933,8 +934,8 @@ def test_sampler_support_and_repeatability(vocab):
 def test_sampler_rows_that_several_ctas_share(vocab):
     """One row a cluster of 1, 4 or 8 CTAs, in shared memory or (from 327,681 logits on) read from memory; rows that start off a
     16-byte boundary; equal logits across the shares' edges, of which a cut by count or by weight keeps the first ids; every row
-    against the draw restated in float64.  A draw may differ only where u falls within 1e-5 of the weight between two tokens (float32
-    sums of at most 327,681 weights in 1,024 runs), which at most one row in twenty does."""
+    against the draw restated in float64.  A draw may differ only where u falls within 1e-5 of the weight of its token's interval (float32
+    sums of at most 327,681 weights in 1,024 runs), which at most one row in twenty does; the same call again gives the same tokens."""
     sampler = Sampler(torch.device(DEV))
     g = torch.Generator().manual_seed(vocab)
     settings = [SamplingParams(temperature=0.8, top_p=0.95, seed=1), SamplingParams(temperature=0.7, top_k=50, top_p=0.9, seed=2),
@@ -945,28 +946,69 @@ def test_sampler_rows_that_several_ctas_share(vocab):
     logits[7:14] = (logits[7:14] * 2).round() / 2          # a few dozen values: long runs of equals at every cut
     logits[14:] = logits[14:].clamp(max=1.5)
     got = sampler.sample(logits.to(DEV), params, list(range(21)))
-    # the restated draw as tensors: the support by a stable sort, then the inverse CDF in id order
-    wrong = 0
-    for row, p, i, token in zip(logits.double(), params, range(21), got):
-        if p.is_greedy():
-            assert token == int(row.argmax())
-            continue
-        order = torch.sort(row, descending=True, stable=True).indices[:p.top_k]
-        weight = torch.exp((row[order] - row[order[0]]) / p.temperature)
-        # the shortest prefix that reaches top_p; equals at its edge by a count that float32 sums may get one off in 1e5
-        keep = len(order) if p.top_p >= 1.0 else int((torch.cumsum(weight, 0) < p.top_p * weight.sum() * (1 - 1e-12)).sum()) + 1
-        kept = torch.sort(order[:keep]).values
-        running = torch.cumsum(torch.exp((row[kept] - row.max()) / p.temperature), 0)
-        u = uniform_from_counter(p.seed, i)
-        place = int(torch.searchsorted(running, u * running[-1], right=True))
-        if token != int(kept[min(place, len(kept) - 1)]):
-            near = running / running[-1]
-            at = torch.searchsorted(kept, torch.tensor(token))
-            assert at < len(kept) + 1 and (near - u).abs().min() < 1e-5, f"row {i}: {token} with {p}"
-            wrong += 1
+    wrong = sum(not drawn(row, p, i, token, 1e-5) for row, p, i, token in zip(logits.double(), params, range(21), got))
     assert wrong <= 1, wrong
-    again = sampler.sample(logits.to(DEV), params, list(range(21)))
-    assert sum(a != b for a, b in zip(got, again)) <= 1
+    assert sampler.sample(logits.to(DEV), params, list(range(21))) == got          # whole numbers and fixed orders: the same bits
+
+
+def drawn(row, p, index, token, tolerance) -> bool:
+    """Whether `token` is the draw restated in float64: the support by a stable sort, then the inverse CDF in id order.  A token that is
+    not has to be one that float32 sums may give instead: u within `tolerance` of the kept weight of that token's own interval, and the
+    token kept, or the next one at the edge of the support (which one it is hangs on a float32 product: 2^-23 of the weight)."""
+    if p.is_greedy():
+        assert token == int(row.argmax())
+        return True
+    order = torch.sort(row, descending=True, stable=True).indices[:p.top_k]
+    weight = torch.exp((row[order] - row[order[0]]) / p.temperature)
+    total = weight.sum()
+    keep = len(order) if p.top_p >= 1.0 else int((torch.cumsum(weight, 0) < p.top_p * total * (1 - 1e-12)).sum()) + 1
+    more = 0 if p.top_p >= 1.0 else 1 + int(total * 2.0 ** -23 / weight[min(keep, len(order)) - 1])
+    kept = torch.sort(order[:keep]).values
+    running = torch.cumsum(torch.exp((row[kept] - row.max()) / p.temperature), 0)
+    u = uniform_from_counter(p.seed, index)
+    place = int(torch.searchsorted(running, u * running[-1], right=True))
+    if token == int(kept[min(place, len(kept) - 1)]):
+        return True
+    kept = torch.sort(order[:keep + more]).values
+    at = int(torch.searchsorted(kept, torch.tensor(token)))
+    assert at < len(kept) and int(kept[at]) == token, f"{token} is not kept by {p}"
+    running = torch.cumsum(torch.exp((row[kept] - row.max()) / p.temperature), 0) / running[-1]
+    before = running[at - 1] if at else 0.0
+    assert before - tolerance <= u <= running[at] + tolerance, f"u {u} lies off {token}'s interval, {before} to {running[at]}, with {p}"
+    return False
+
+
+@pytest.mark.parametrize("vocab", [151936, 262144, 1000003])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_sampler_counts_a_long_tail_of_small_weights(vocab, ragged):
+    """One large logit (the last id) and a long tail whose weights are a 2^-35 to 2^-31 of it and together 2.75e-5: the cut by weight at
+    1 - 2^-16 keeps the tail's first 1.22e-5 (of equal weights the first ids), so that draws with a small u are tokens of the tail, each
+    the one that u names to 2^-23 (the cut's weight is a float32 product; a tail that ends a little earlier or later moves the others)."""
+    g = torch.Generator().manual_seed(vocab)
+    tail = torch.full((vocab,), 2.75e-5 / vocab, dtype=torch.float64)
+    if ragged:
+        tail *= torch.rand(vocab, generator=g, dtype=torch.float64) * 1.2 + 0.4
+    tail[-1] = 1.0
+    logits = torch.log(tail).float()
+    p = SamplingParams(temperature=1.0, top_p=1.0 - 2.0 ** -16, seed=77)
+    index = torch.arange(1 << 21)
+    u = uniforms(p.seed, index)
+    small = index[(u > 1e-6) & (u < 1.1e-5)][:8].tolist()
+    assert len(small) == 8 and u[small[0]] == uniform_from_counter(p.seed, small[0])
+    got = Sampler(torch.device(DEV)).sample(logits.expand(8, vocab).contiguous().to(DEV), [p] * 8, small)
+    for i, token in zip(small, got):
+        assert token != vocab - 1
+        drawn(logits.double(), p, i, token, 2.0 ** -23)
+    assert Sampler(torch.device(DEV)).sample(logits[None].to(DEV), [SamplingParams(temperature=1e-42)], [0]) == [vocab - 1]
+
+
+def uniforms(seed, index):
+    """`uniform_from_counter` of many draw indices."""
+    with np.errstate(over="ignore"):
+        z = np.uint64(seed) + np.uint64(0x9E3779B97F4A7C15) * (index.numpy().astype(np.uint64) + np.uint64(1))
+        z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+        z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+    return torch.from_numpy(((z ^ (z >> np.uint64(31))) >> np.uint64(40)).astype(np.float64)) / 16777216.0
 
 
 def test_sampler_distribution_ties_and_bad_rows():

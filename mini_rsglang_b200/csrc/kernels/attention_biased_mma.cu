@@ -507,13 +507,13 @@ MRS_EXPORT int mrs_attention_biased_mma(int narrow, const void* q, const void* k
     Extras x;
     x.bias = bias, x.gate = gate, x.bias_rows = bias_rows, x.scale = scale, x.cap = cap, x.window = window, x.keep_first = keep_first;
     x.sink = sink, x.sink_logits = sink_logits, x.sink_heads = sink_heads, x.chunk = chunk;
-    static bool configured[2] = {false, false};
-    if (!configured[narrow ? 1 : 0]) {
+    static PerDevice configured[2];
+    if (!configured[narrow ? 1 : 0].get()) {
         cudaError_t e = narrow
             ? cudaFuncSetAttribute(attention_biased_keys_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_keys)
             : cudaFuncSetAttribute(attention_biased_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows);
         if (e != cudaSuccess) return (int)e;
-        configured[narrow ? 1 : 0] = true;
+        configured[narrow ? 1 : 0].set(1);
     }
     if (narrow) {
         float* part_o = scratch;

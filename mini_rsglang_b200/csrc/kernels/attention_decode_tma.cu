@@ -482,18 +482,19 @@ MRS_EXPORT int mrs_attention_decode_tma(const void* k_map, const void* v_map, co
     if (shift < 0 || page_size < 8 || nkv <= 0 || nq % nkv || nq / nkv > ROWS || splits < 1 || splits > 256)
         return MRS_BAD_ARGUMENT;
     if (splits > 1 && (!scratch || !counters)) return MRS_BAD_ARGUMENT;
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     float* part_o = scratch;
     float* part_ml = scratch ? scratch + (size_t)num_tiles * nkv * splits * ROWS * D : nullptr;
     const float scale_log2 = scale * 1.4426950408889634f;
     // 2, 4, 8 or 16 splits whose slices of the head's columns are whole float4s run as one cluster and merge among themselves
-    static int largest_cluster = -1;
-    if (largest_cluster < 0) {
+    static PerDevice largest;
+    int largest_cluster = largest.get();
+    if (largest_cluster == 0) {
         largest_cluster = 8;
         if (cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             cudaLaunchConfig_t probe = {};
@@ -506,6 +507,7 @@ MRS_EXPORT int mrs_attention_decode_tma(const void* k_map, const void* v_map, co
             if (cudaOccupancyMaxActiveClusters(&clusters, attention_decode_kernel, &probe) == cudaSuccess && clusters > 0) largest_cluster = 16;
         }
         (void)cudaGetLastError();
+        largest.set(largest_cluster);
     }
     const bool in_cluster = splits > 1 && (splits & (splits - 1)) == 0 && splits <= largest_cluster && D % (4 * splits) == 0;
     if (in_cluster) {
@@ -537,10 +539,11 @@ MRS_EXPORT int mrs_attention_decode_tma(const void* k_map, const void* v_map, co
 // Thread-block clusters of `splits` CTAs of this kernel that the GPU holds at once (0: no such cluster): what a
 // plan may count on when it wants every share of every tile resident together.  Asked of the driver once a size.
 MRS_EXPORT int mrs_attention_decode_tma_resident_clusters(int splits) {
-    static int known[17] = {};
+    static PerDevice known[17];              // clusters, or -1
     if (splits < 2 || splits > 16 || (splits & (splits - 1))) return 0;
-    if (known[splits] == 0) {
-        known[splits] = -1;
+    int held = known[splits].get();
+    if (held == 0) {
+        held = -1;
         if (cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES) == cudaSuccess &&
             (splits <= 8 || cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
             cudaLaunchConfig_t probe = {};
@@ -550,11 +553,12 @@ MRS_EXPORT int mrs_attention_decode_tma_resident_clusters(int splits) {
             shape.val.clusterDim.x = 1, shape.val.clusterDim.y = 1, shape.val.clusterDim.z = splits;
             probe.attrs = &shape, probe.numAttrs = 1;
             int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, attention_decode_kernel, &probe) == cudaSuccess && clusters > 0) known[splits] = clusters;
+            if (cudaOccupancyMaxActiveClusters(&clusters, attention_decode_kernel, &probe) == cudaSuccess && clusters > 0) held = clusters;
         }
         (void)cudaGetLastError();
+        known[splits].set(held);
     }
-    return known[splits] > 0 ? known[splits] : 0;
+    return held > 0 ? held : 0;
 }
 
 // Reads and clears this library's error word (waits for the device).  0: no kernel gave up a wait.

@@ -378,11 +378,11 @@ __global__ void attention_f32_join_kernel(const Args A) {
 template <int D, bool SPLIT>
 int launch(const Args& A, int tiles, void* stream) {
     constexpr int SMEM = (smem_floats<D>() + (SPLIT ? 0 : THREADS * D / 4)) * (int)sizeof(float);
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     MRS_LAUNCH((attention_f32_kernel<D, SPLIT>), dim3(tiles, A.nkv, SPLIT ? A.chunks : 1), THREADS, SMEM, stream, A);
     MRS_RETURN_LAUNCH_STATUS();

@@ -387,11 +387,11 @@ MRS_EXPORT int mrs_attention_latent_tc(const void* query_maps, const void* cache
     if (shift < 0 || page_size < 8 || cache_pages <= 0 || cache_pages >= 0x7fffffff || heads <= 0 || heads > BM ||
         !(scale > 0.0f) || window < 0 || ((uintptr_t)out & 15))
         return MRS_BAD_ARGUMENT;
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         const cudaError_t e = cudaFuncSetAttribute(attention_latent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     const CUtensorMap *q = reinterpret_cast<const CUtensorMap*>(query_maps), *k = reinterpret_cast<const CUtensorMap*>(cache_maps);
     MRS_LAUNCH(attention_latent_kernel, num_tiles, THREADS, SMEM_BYTES, stream, q[0], q[TAIL ? 1 : 0], k[0], k[TAIL ? 1 : 0], positions, block_table,

@@ -462,11 +462,11 @@ MRS_EXPORT int mrs_attention_mma_rows_mode(const void* q, const void* k_cache, c
     if (num_tiles <= 0) return 0;
     const int shift = page_shift_of(page_size);
     if (shift < 0 || nkv <= 0 || nq % nkv || nq / nkv > ROWS_WIDE) return MRS_BAD_ARGUMENT;
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     MRS_LAUNCH(attention_rows_kernel, dim3(num_tiles, nkv), THREADS, smem_rows, stream,
         (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, positions, block_table, table_width,
@@ -484,11 +484,11 @@ MRS_EXPORT int mrs_attention_mma_keys_mode(const void* q, const void* k_cache, c
     const int shift = page_shift_of(page_size);
     if (shift < 0 || nkv <= 0 || nq % nkv || nq / nkv > ROWS_NARROW || splits < 1 || splits > 65535) return MRS_BAD_ARGUMENT;
     if (splits > 1 && !scratch) return MRS_BAD_ARGUMENT;
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(attention_keys_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_keys);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     float* part_o = scratch;
     float* part_ml = scratch ? scratch + (size_t)num_tiles * nkv * splits * ROWS_NARROW * D : nullptr;

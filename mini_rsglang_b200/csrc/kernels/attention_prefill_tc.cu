@@ -554,12 +554,12 @@ MRS_EXPORT int mrs_attention_prefill_tc(const void* q_map, const void* k_map, co
     const float cap_in = cap > 0.0f ? 2.0f * scale * 1.4426950408889634f / cap : 0.0f, cap_out = cap * 1.4426950408889634f;
     const int shift = page_shift_of(page_size);
     if (shift < 0 || page_size < 8 || nkv <= 0 || nq % nkv || nq / nkv > BM) return MRS_BAD_ARGUMENT;
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(attention_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     for (int done = 0; done < num_tiles; done += 65535) {         // a grid's second dimension ends at 65,535
         const int now = num_tiles - done < 65535 ? num_tiles - done : 65535;

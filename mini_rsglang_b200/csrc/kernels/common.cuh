@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include "per_device.h"
+
 typedef __nv_bfloat16 bf16;
 
 template <typename T> __device__ __forceinline__ float to_float(T x);
@@ -67,15 +69,13 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // Multiprocessors of the current device (asked once per device and kept): grids that loop over their
 // work are capped by a multiple of it.
 static inline int mrs_sm_count() {
-    static int counts[64] = {};
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 1;
-    if (counts[device] == 0) {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) n = 1;
-        counts[device] = n;
+    static PerDevice counts;
+    int n = counts.get(), device = 0;
+    if (n == 0) {
+        if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) return 1;
+        counts.set(n);
     }
-    return counts[device];
+    return n;
 }
 
 template <typename... KernelArgs, typename... Args>

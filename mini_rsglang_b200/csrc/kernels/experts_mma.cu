@@ -147,13 +147,13 @@ MRS_EXPORT int mrs_moe_product_mma(int gated, const void* x, const int* sorted_r
     if (capacity % BM || n <= 0 || k <= 0 || k % 8 || top <= 0 || (((uintptr_t)x | (uintptr_t)weight) & 15) || block < 0 ||
         (block && (!gated || n % block)) || act > 4 || (gated && act >= 0))
         return MRS_BAD_ARGUMENT;
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(moe_product_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<true>());
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(moe_product_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<false>());
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     const dim3 grid(capacity / BM, (n + BN - 1) / BN);
     if (gated)

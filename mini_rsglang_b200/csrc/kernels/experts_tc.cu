@@ -202,11 +202,11 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
 template <bool GATED, int ACT>
 int launch(const CUtensorMap& x, const CUtensorMap& w, const int* tile_expert, const int* sorted_rows, void* out, int m_tiles, int N, int K,
            int grid, void* stream) {
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         const cudaError_t e = cudaFuncSetAttribute(moe_product_tc_kernel<GATED, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     MRS_LAUNCH((moe_product_tc_kernel<GATED, ACT>), grid, THREADS, SMEM_BYTES, stream, x, w, tile_expert, sorted_rows, (bf16*)out, m_tiles, N, K);
     MRS_RETURN_LAUNCH_STATUS();

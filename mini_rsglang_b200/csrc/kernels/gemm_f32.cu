@@ -186,12 +186,12 @@ __global__ void __launch_bounds__(FEW_THREADS) gemm_f32_few_kernel(const float* 
 template <int BM, int BN, int TM, int TN, int BK, int STAGES, int MIN_CTAS, bool VEC>
 int launch_tiles(const float* A, const float* W, float* C, int M, int N, int K, void* stream) {
     constexpr int SMEM = STAGES * (BM + BN) * (BK + 4) * (int)sizeof(float);
-    static bool configured = false;
+    static PerDevice configured;
     auto kernel = gemm_f32_tiles_kernel<BM, BN, TM, TN, BK, STAGES, MIN_CTAS, VEC>;
-    if (!configured) {
+    if (!configured.get()) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return MRS_BAD_ARGUMENT;
@@ -212,11 +212,11 @@ int launch_shape(int shape, const float* A, const float* W, float* C, int M, int
 template <int R>
 int launch_few(const float* A, const float* W, float* C, int M, int N, int K, void* stream) {
     constexpr int SMEM = FEW_STAGES * (FEW_COLS + 4 * R) * FEW_PITCH * (int)sizeof(float);
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     MRS_LAUNCH(gemm_f32_few_kernel<R>, (N + FEW_COLS - 1) / FEW_COLS, FEW_THREADS, SMEM, stream, A, W, C, M, N, K);
     MRS_RETURN_LAUNCH_STATUS();

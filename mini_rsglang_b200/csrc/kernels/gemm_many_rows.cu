@@ -217,11 +217,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_many_rows_kernel(
 
 template <int ACT>
 int launch(const void* x_map, const void* w_map, void* out, int T, int N, int K, int ctas, void* stream) {
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(gemm_many_rows_kernel<ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     const int tiles = ((T + BM - 1) / BM) * ((N + BN - 1) / BN);
     MRS_LAUNCH(gemm_many_rows_kernel<ACT>, ctas < tiles ? ctas : tiles, THREADS, SMEM_BYTES, stream, *reinterpret_cast<const CUtensorMap*>(x_map),

@@ -547,10 +547,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_small_m_kernel(
 // that is asked about is launched too: its limit of shared memory is set to what a launch sets, never below.
 int resident_clusters(int ranges) {
     using S = Shape<16>;
-    static int known[17] = {};
+    static PerDevice known[17];              // clusters, or -1
     if (ranges < 2 || ranges > 16) return 0;
-    if (known[ranges] == 0) {
-        int clusters = 0;
+    int clusters = known[ranges].get();
+    if (clusters == 0) {
         const auto kernel = gemm_small_m_kernel<16, bf16, EPI_PLAIN>;
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM_BYTES) == cudaSuccess &&
             (ranges <= 8 || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
@@ -560,12 +560,13 @@ int resident_clusters(int ranges) {
             shape.id = cudaLaunchAttributeClusterDimension;
             shape.val.clusterDim.x = ranges, shape.val.clusterDim.y = 1, shape.val.clusterDim.z = 1;
             probe.attrs = &shape, probe.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &probe) != cudaSuccess || clusters < 0) clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &probe) != cudaSuccess) clusters = 0;
         }
         (void)cudaGetLastError();
-        known[ranges] = clusters > 0 ? clusters : -1;
+        if (clusters <= 0) clusters = -1;
+        known[ranges].set(clusters);
     }
-    return known[ranges] > 0 ? known[ranges] : 0;
+    return clusters > 0 ? clusters : 0;
 }
 
 // How a launch lays out its shared memory: stages of the ring, and bytes that the first CTA of a tile's cluster receives (0: the
@@ -597,13 +598,13 @@ int launch(const CUtensorMap* w_map, const CUtensorMap* x_map, void* out, float*
            int K, int splits, int ctas, cudaStream_t stream, const NormLink& link, const HeadEpilogue& heads = HeadEpilogue{}) {
     using S = Shape<MPAD>;
     const auto kernel = gemm_small_m_kernel<MPAD, OutT, EPI>;
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     const int n_tiles = (N + TILE_N - 1) / TILE_N;
     const Ranges ranges = ranges_of(splits, n_tiles);

@@ -634,11 +634,11 @@ MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float*
     if (rows > 0x7fffffff / 8) return MRS_BAD_ARGUMENT;
     const size_t share = (size_t)per_segment * (SAMPLE_SEGMENTS / blocks) * sizeof(float);
     const bool in_shared = share <= SAMPLE_SHARE_BYTES;
-    static bool configured = false;
-    if (!configured) {
+    static PerDevice configured;
+    if (!configured.get()) {
         const cudaError_t e = cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SHARE_BYTES);
         if (e != cudaSuccess) return (int)e;
-        configured = true;
+        configured.set(1);
     }
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)rows * blocks);

@@ -1472,6 +1472,7 @@ def attention_biased_mma(q, k_cache, v_cache, positions, block_table, tiles, out
 # tcgen05 attention over cached latents for prompt portions, one library per (latent, rotated) sizes
 # ------------------------------------------------------------------------------------------------
 _latent_tc_libs: dict[tuple[int, int], ctypes.CDLL] = {}
+_latent_tc_cache_maps: dict[tuple, tuple] = {}
 LATENT_TC_ROWS = 128           # query rows of a tile: 128 // heads tokens times all heads
 
 
@@ -1532,15 +1533,19 @@ def attention_latent_tc(q, cache, positions, block_table, tiles, out, heads: int
     def fail(code, what):
         raise BackendError(f"{what}: {lib.mrs_attention_latent_tc_error_string(code).decode()} (code {code})")
 
-    keep, maps = _aligned_block(512, 64)                 # two maps of the cache, two of the queries
-    code = lib.mrs_attention_latent_tc_cache_maps(cache.data_ptr(), cache.shape[0], page_size, maps)
-    if code != 0:
-        fail(code, "tensor maps of the cache")
-    code = lib.mrs_attention_latent_tc_query_maps(q.data_ptr(), tokens, heads, maps + 256)
+    key = (latent, rotated, cache.data_ptr(), tuple(cache.shape))        # all that the maps are made from
+    if key not in _latent_tc_cache_maps:
+        made, address = _aligned_block(256, 64)
+        code = lib.mrs_attention_latent_tc_cache_maps(cache.data_ptr(), cache.shape[0], page_size, address)
+        if code != 0:
+            fail(code, "tensor maps of the cache")
+        _latent_tc_cache_maps[key] = (made, address)
+    keep, query_maps = _aligned_block(256, 64)
+    code = lib.mrs_attention_latent_tc_query_maps(q.data_ptr(), tokens, heads, query_maps)
     if code != 0:
         fail(code, "tensor maps of the queries")
     launch_count += 1
-    code = lib.mrs_attention_latent_tc(maps + 256, maps, positions.data_ptr(), block_table.data_ptr(),
+    code = lib.mrs_attention_latent_tc(query_maps, _latent_tc_cache_maps[key][1], positions.data_ptr(), block_table.data_ptr(),
                                        block_table.shape[1], tiles.data_ptr(), tiles.shape[0], out.data_ptr(), _ptr(gate), _ptr(sink_logits),
                                        heads, page_size, cache.shape[0], float(scale), int(window), _stream())
     del keep                          # the maps were copied into the launch

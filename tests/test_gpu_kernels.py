@@ -1166,6 +1166,33 @@ def test_attention_latent_tc_leaves_out_rows_that_no_query_sees(heads, latent, r
             assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2]), (c, n, start)
 
 
+def test_attention_latent_tc_makes_a_caches_maps_once(monkeypatch):
+    """The tensor maps of a cache are made at its first call and kept; another cache, and the same memory as pages of another size, get
+    their own."""
+    heads, latent, rotated = 4, 64, 32
+    row = latent + rotated
+    lib = kernels.attention_latent_tc_library(latent, rotated)
+    make, made = lib.mrs_attention_latent_tc_cache_maps, []
+    monkeypatch.setattr(lib, "mrs_attention_latent_tc_cache_maps", lambda *a: made.append(a[:3]) or make(*a))
+    monkeypatch.setattr(kernels, "_latent_tc_cache_maps", {})
+    g = torch.Generator(device=DEV).manual_seed(8)
+    caches = [torch.randn(6, 1, 16, row, device=DEV, generator=g).bfloat16() for _ in range(2)]
+    caches.append(caches[0].view(3, 1, 32, row))
+    q = torch.randn(9, heads * row, device=DEV, generator=g).bfloat16()
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).to(DEV)      # noqa: E731
+    for again in range(2):
+        for cache in caches:
+            out = torch.empty(9, heads * latent, device=DEV).bfloat16()
+            kernels.attention_latent_tc(q, cache, i32(list(range(70, 79))), i32([list(range(cache.shape[0]))]), i32([(0, 0, 9, 0)]), out, heads, latent, rotated, 0.1)
+            keys = cache.view(-1, row)[:79].double()
+            scores = torch.einsum("thd,kd->thk", q.view(9, heads, row).double(), keys) * 0.1
+            scores = scores.masked_fill(torch.arange(79, device=DEV)[None, None] > torch.arange(70, 79, device=DEV)[:, None, None], -float("inf"))
+            want = torch.softmax(scores, 2) @ keys[:, :latent]
+            size = torch.softmax(scores, 2) @ keys[:, :latent].abs()
+            assert ((out.view(9, heads, latent).double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 2.0 ** -8 + 1e-6).all()
+        assert len(made) == 3
+
+
 def test_attention_latent_tc_scores_that_are_no_numbers():
     """A query that is no number gives its own (token, head) no number and no other one; rows whose scores are all -inf have no
     weights and give zeros; a score of +inf gives no number, as its softmax does."""

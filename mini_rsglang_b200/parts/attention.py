@@ -48,7 +48,7 @@ class TileLists:
 
 
 def attention_tile_lists(facts: StepFacts, group: int, wide_rows: int, kv_heads: int = 1, window: int = 0,
-                         key_block: int = 128, sms: int = 1) -> TileLists:
+                         key_block: int = 128, sms: int = 1, head_dim: int = 128) -> TileLists:
     """Cuts the step's sequences into tiles for the tensor-core kernels, on the host: sequences with few
     query rows (decoded tokens, short portions) go to the kernels for few rows in tiles of
     16 // group tokens, the others in tiles of wide_rows // group tokens, those with the most
@@ -61,8 +61,8 @@ def attention_tile_lists(facts: StepFacts, group: int, wide_rows: int, kv_heads:
     sums a second kernel merges; shorter ones into entries of one tile (68 us as 128 CTAs; a CTA
     with one tile has no partner on the tensor cores, so this pays only while SMs would idle).
     `key_block` is the kernel's block of keys and `sms` the device's multiprocessors, as the kernel's
-    library and the device state them."""
-    key = (group, wide_rows, kv_heads, window, key_block)
+    library and the device state them; `head_dim` the elements of a key, and of a value."""
+    key = (group, wide_rows, kv_heads, window, key_block, head_dim)
     if key in facts.plans:
         return facts.plans[key]
     narrow_tokens = kernels.MMA_ROWS_NARROW // group
@@ -90,7 +90,7 @@ def attention_tile_lists(facts: StepFacts, group: int, wide_rows: int, kv_heads:
     # their keys where their walks would end long after the narrow tiles.
     room = int(sms * WIDE_SHARE_BESIDE_NARROW) if narrow else sms
     spare = room // max(len(found) * kv_heads, 1) if tensor_core else 1
-    beside = shares_beside_narrow(found, lengths, facts.start_pos, narrow, kv_heads, window, sms) if tensor_core and narrow else 0
+    beside = shares_beside_narrow(found, lengths, facts.start_pos, narrow, kv_heads, window, sms, head_dim) if tensor_core and narrow else 0
     wide = []
     shared = False
     if tensor_core and tiles == 2 and spare < 2 and beside < 2 and len(found) * kv_heads <= room and not window and PAIR_FAR_TILES:
@@ -145,19 +145,22 @@ def attention_tile_lists(facts: StepFacts, group: int, wide_rows: int, kv_heads:
     return lists
 
 
-def shares_beside_narrow(found: list, lengths: list, start_pos, narrow: list, kv_heads: int, window: int, sms: int) -> int:
+def shares_beside_narrow(found: list, lengths: list, start_pos, narrow: list, kv_heads: int, window: int, sms: int, head_dim: int) -> int:
     """Shares of its keys that an entry for the kernel for wide tiles is cut into while the kernel for few rows runs beside it.
     Times in blocks of keys of a CTA's two tiles (2.3 us): a walk is its blocks, and 6 more where shares have to be merged; the
-    narrow tiles take 2.6 and one for every 15 MB of their keys and values (heads of 128), stretched where the wide CTAs leave
+    narrow tiles take 2.6 and one for every 15 MB of their keys and values, stretched where the wide CTAs leave
     them fewer than 0.6 of the SMs.  The count with the shortest time for both is taken.  Measured, steps of 4 layers, one portion
     under a budget of 512 tokens, 1, 2, 3 and 4 shares (0.6B shape: 32 CTAs a share): 27 requests at 1,100 beside a portion behind
     1,500 tokens 504, 476, 467, 468 us, behind 7,000 tokens 834, 641, 568, 551; 64 requests at 1,000, behind 512 tokens 553, 554,
     552, 556, behind 3,000 638, 587, 591, 606; 16 at 4,000, behind 1,500 528, 546, 588, 590.  1 and 2 shares (8B shape: 64 CTAs a
-    share): 27 at 1,100, behind 1,500 1,215, 1,228, behind 7,000 1,538, 1,372; 16 at 4,000, behind 3,000 1,323, 1,421."""
+    share): 27 at 1,100, behind 1,500 1,215, 1,228, behind 7,000 1,538, 1,372; 16 at 4,000, behind 3,000 1,323, 1,421.
+    The attention alone, heads of 64 and 128 (8 key/value heads, 16 and 32 query heads, 8 to 64 requests beside portions behind 512 to
+    7,000): the count that this takes is nowhere slower than one share; heads of 64 counted as 128 got fewer shares in 9 of 32 steps
+    (16 at 4,000, behind 3,000: 62.0 us with 2, 57.6 with 3; 64 at 1,000, behind 1,500: 53.7 with 1, 50.3 with 2)."""
     ctas = max(len(found) * kv_heads, 1)
     longest = max((entry[4] for entry in found), default=0)
     keys = sum(min(start_pos[i] + lengths[i], window + lengths[i]) if window else start_pos[i] + lengths[i] for i, *_ in narrow)
-    few = 2.6 + keys * kv_heads * 512 / 15e6
+    few = 2.6 + keys * kv_heads * 4 * head_dim / 15e6
     best, best_time = 1, max(longest, few)
     for shares in range(2, min(sms // ctas, longest // 4, 255) + 1):
         walk = longest / shares + 6
@@ -168,13 +171,13 @@ def shares_beside_narrow(found: list, lengths: list, start_pos, narrow: list, kv
 
 
 def plan_attention_tiles(ctx, group: int, wide_rows: int, kv_heads: int = 1, window: int = 0, key_block: int = 128,
-                         sms: int = 1):
+                         sms: int = 1, head_dim: int = 128):
     """The step's tile lists on the device: (narrow tiles, wide tiles, longest context of a narrow tile,
     whether wide tiles share their keys), None for an empty list.  The plan is kept in the context for the
     other layers of the step.  A step of single decoded tokens brings its own list; a step with fixed shapes
     finds the lists where the step function copied them (`ctx.plan_views`), at addresses that stay."""
     plans = ctx.__dict__.setdefault("_attention_plans", {})
-    key = (group, wide_rows, kv_heads, window, key_block)
+    key = (group, wide_rows, kv_heads, window, key_block, head_dim)
     if key in plans:
         return plans[key]
     narrow_tokens = kernels.MMA_ROWS_NARROW // group
@@ -188,7 +191,7 @@ def plan_attention_tiles(ctx, group: int, wide_rows: int, kv_heads: int = 1, win
     if facts is None:
         real = ctx.real_sequences or ctx.num_sequences
         facts = StepFacts(ctx.host_q_start[:real + 1], ctx.host_start_pos[:real], ctx.max_context_len)
-    lists = attention_tile_lists(facts, group, wide_rows, kv_heads, window, key_block, sms)
+    lists = attention_tile_lists(facts, group, wide_rows, kv_heads, window, key_block, sms, head_dim)
     if ctx.plan_views is not None:
         both = ctx.plan_views[key]
         plans[key] = (both[:lists.narrow_cap] if lists.narrow_cap else None, both[lists.narrow_cap:] if lists.wide_cap else None,
@@ -257,7 +260,7 @@ def tile_plan_arguments(d: int, group: int, page_size: int, nkv: int, window: in
     a wide tile and the block of keys as the kernel that will run states them."""
     sms = kernels.sm_count(device)
     if kernels.attention_prefill_tc_supported(d, group, page_size):
-        return (group, kernels.PREFILL_TC_ROWS, nkv, window, kernels.attention_prefill_tc_key_block(d), sms)
+        return (group, kernels.PREFILL_TC_ROWS, nkv, window, kernels.attention_prefill_tc_key_block(d), sms, d)
     return (group, kernels.MMA_ROWS_WIDE, nkv, window, 128, sms)
 
 

@@ -132,3 +132,15 @@ def test_a_long_walk_beside_decoded_tokens_is_cut_into_shares(decodes, context, 
     assert lists.shared == (shares > 1) and len(lists.narrow) == decodes
     assert {max(share >> 8 & 0xFF, 1) for *_, share in lists.wide} == {shares}
     assert len(lists.wide) * 8 <= 148
+
+
+@pytest.mark.parametrize("group,decodes,context,behind,heads_of_128,heads_of_64", [(2, 64, 1000, 1500, 1, 2), (2, 16, 4000, 3000, 2, 3), (4, 16, 4000, 3000, 1, 2),
+                                                                                  (2, 27, 1100, 512, 1, 1), (4, 8, 300, 7000, 2, 2)])
+def test_shares_beside_narrow_tiles_count_the_bytes_of_their_keys(group, decodes, context, behind, heads_of_128, heads_of_64):
+    """Narrow tiles of smaller heads are done sooner, so a long walk beside them is cut further; layers of other head sizes in the same
+    step have plans of their own."""
+    facts = facts_of([1] * decodes + [512 - decodes], [context] * decodes + [behind])
+    for d, shares in ((128, heads_of_128), (64, heads_of_64)):
+        lists = attention_tile_lists(facts, group, kernels.PREFILL_TC_ROWS, 8, 0, 128, 148, d)
+        assert {max(share >> 8 & 0xFF, 1) for *_, share in lists.wide} == {shares}, d
+    assert attention_tile_lists(facts, group, kernels.PREFILL_TC_ROWS, 8, 0, 128, 148) is attention_tile_lists(facts, group, kernels.PREFILL_TC_ROWS, 8, 0, 128, 148, 128)

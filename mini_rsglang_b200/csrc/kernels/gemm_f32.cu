@@ -235,13 +235,14 @@ MRS_EXPORT int mrs_gemm_f32_kernel(const float* A, const float* W, float* C, int
         // A shape's time over q tiles an SM, in microseconds at K = 1,024, is a line: measured alone at N = 1,024 to 6,144,
         // M = 17 to 2,048, q = 1 to 55 (within a fifth of it nearly everywhere).  The wide tiles win when every SM has many
         // (2,048 rows, N 4,096: 384, 418 and 457 us for the three shapes; 64 rows: 40, 30, 34; 32 rows of N = 1,024: 37, 22, 18).
+        // A grid's second dimension ends at 65,535 tiles of rows: beyond what the low tiles cover, the high ones take the product.
         const int bm[3] = {64, 32, 32}, bn[3] = {64, 64, 32}, sms = mrs_sm_count();
         const double first[3] = {45.0, 19.0, 12.0}, each[3] = {24.0, 14.3, 8.6};
         double best = 0.0;
         for (int i = 0; i < 3; ++i) {
-            const long long tiles = (long long)((M + bm[i] - 1) / bm[i]) * ((N + bn[i] - 1) / bn[i]);
+            const long long rows = ((long long)M + bm[i] - 1) / bm[i], tiles = rows * ((N + bn[i] - 1) / bn[i]);
             const double time = first[i] + each[i] * (double)((tiles + sms - 1) / sms);
-            if (i == 0 || time < best) best = time, kernel = i;
+            if (i == 0 || (time < best && rows <= 65535)) best = time, kernel = i;
         }
     }
     if (kernel == 3) return M <= 4 ? launch_few<1>(A, W, C, M, N, K, stream) : launch_few<2>(A, W, C, M, N, K, stream);

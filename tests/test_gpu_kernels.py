@@ -343,6 +343,16 @@ def test_attention_simt(dtype, nq, nkv, d, page):
     close(case.run_simt(), case.plain(), dtype, "attention_simt")
 
 
+@pytest.mark.parametrize("m", [65535 * 32, 65535 * 32 + 1, 65535 * 64])
+def test_gemm_f32_takes_as_many_rows_as_its_highest_tiles_cover(m):
+    """Few columns choose low tiles, whose grid ends at 2,097,120 rows; more rows go to the high ones (4,194,240, as before them)."""
+    x = torch.arange(m, device=DEV, dtype=torch.float32).view(m, 1) * torch.tensor([[1.0, 0.5, 0.0, 0.25]], device=DEV)
+    w = torch.tensor([[1.0, 0.0, 0.0, 0.0], [0.0, 0.0, 0.0, 2.0]], device=DEV)
+    out = torch.full((m, 2), float("nan"), device=DEV)
+    kernels.gemm_f32(x, w, out)
+    assert torch.equal(out[:, 0], x[:, 0]) and torch.equal(out[:, 1], 0.5 * x[:, 0])
+
+
 @pytest.mark.parametrize("nq,nkv,d,page,window", [(4, 2, 128, 16, 0), (16, 8, 128, 16, 0), (5, 1, 64, 8, 0), (12, 1, 96, 4, 0), (64, 1, 36, 16, 0),
                                                   (3, 3, 256, 32, 0), (4, 2, 128, 16, 700), (2, 1, 20, 4, 37)])
 def test_attention_f32_gives_a_row_the_same_bits_in_every_cut(monkeypatch, nq, nkv, d, page, window):

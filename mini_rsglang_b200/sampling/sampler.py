@@ -28,6 +28,19 @@ def uniform_from_counter(seed: int, index: int) -> float:
     return (z >> 40) / 16777216.0
 
 
+def packed_parameters(params: Sequence[SamplingParams], draw_index: Sequence[int]) -> np.ndarray:
+    """The rows' parameters as the words of one copy: all seeds (the 64-bit patterns of their values, negative ones too), then all
+    temperatures, top_k, top_p and draw indices, 32 bits each."""
+    rows = len(params)
+    packed = np.empty(6 * rows, dtype=np.int32)
+    packed[:2 * rows].view(np.uint64)[:] = np.array([int(p.seed) & _MASK64 for p in params], dtype=np.uint64)
+    packed[2 * rows:3 * rows].view(np.float32)[:] = [0.0 if p.is_greedy() else p.temperature for p in params]
+    packed[3 * rows:4 * rows] = [p.top_k or 0 for p in params]
+    packed[4 * rows:5 * rows].view(np.float32)[:] = [p.top_p for p in params]
+    packed[5 * rows:] = draw_index
+    return packed
+
+
 class Chosen:
     """Tokens that `Sampler.launch` chose: on the device (`tokens`, for a step that goes on before the host has
     seen them) and on their way to pinned host memory (`host`, complete when `arrived` has happened)."""
@@ -80,14 +93,8 @@ class Sampler:
             kernels.argmax(logits, out)
         else:
             # One copy from pinned memory carries every row's parameters: five pageable ones waited for the stream each.
-            # Seeds are 64-bit patterns of the unsigned value; then temperature, top_k, top_p and draw index, 32 bits each.
+            packed = packed_parameters(params, draw_index)
             host, copied = self._stage(rows)
-            packed = np.empty(6 * rows, dtype=np.int32)
-            packed[:2 * rows].view(np.uint64)[:] = np.array([p.seed for p in params], dtype=np.uint64)
-            packed[2 * rows:3 * rows].view(np.float32)[:] = [0.0 if p.is_greedy() else p.temperature for p in params]
-            packed[3 * rows:4 * rows] = [p.top_k or 0 for p in params]
-            packed[4 * rows:5 * rows].view(np.float32)[:] = [p.top_p for p in params]
-            packed[5 * rows:] = draw_index
             host.numpy()[:24 * rows] = packed.view(np.uint8)
             words = torch.empty(6 * rows, dtype=torch.int32, device=self.device)
             words.view(torch.uint8).copy_(host[:24 * rows], non_blocking=True)

@@ -3,11 +3,13 @@
 import copy
 import json
 
+import numpy as np
 import pytest
 from conftest import TINY_A, TINY_B
 
 from mini_rsglang_b200 import InvalidRequest, RuntimeConfig, SamplingParams
 from mini_rsglang_b200.models import ARCHITECTURES, config_from_dict, load_config, model_spec_for
+from mini_rsglang_b200.sampling.sampler import packed_parameters
 
 QWEN3_06B = dict(model_type="qwen3", architectures=["Qwen3ForCausalLM"], hidden_size=1024, intermediate_size=3072,
                  num_hidden_layers=28, num_attention_heads=16, num_key_value_heads=8, head_dim=128,
@@ -129,3 +131,17 @@ def test_sampling_params_are_checked():
                 dict(seed=-1)):
         with pytest.raises(InvalidRequest):
             SamplingParams(**bad).validate()
+
+
+def test_sampling_parameters_are_packed_word_by_word():
+    """The words that the sampler copies to the device: seeds as 64-bit patterns (also those of negative numbers, which only
+    `validate` refuses), then float32 and int32 words row by row; what has no int32 is refused."""
+    params = [SamplingParams(temperature=0.7, top_k=50, top_p=0.9, seed=2**64 - 1), SamplingParams(seed=-5), SamplingParams(temperature=1.5, top_k=1, seed=7)]
+    words = packed_parameters(params, [3, 0, 2**31 - 1])
+    assert words.dtype == np.int32 and words.shape == (18,)
+    assert words[:6].view(np.uint64).tolist() == [2**64 - 1, 2**64 - 5, 7]
+    assert words[6:9].view(np.float32).tolist() == [np.float32(0.7), 0.0, 0.0]
+    assert words[9:12].tolist() == [50, 0, 1] and words[12:15].view(np.float32).tolist() == [np.float32(0.9), 1.0, 1.0]
+    assert words[15:].tolist() == [3, 0, 2**31 - 1]
+    with pytest.raises(OverflowError):
+        packed_parameters([SamplingParams(temperature=1.0, top_k=2**31)], [0])

@@ -224,31 +224,23 @@ int launch_few(const float* A, const float* W, float* C, int M, int N, int K, vo
 
 }  // namespace
 
-// `kernel`: -1 the one that the sizes choose; else 0 to 2 the tile shapes above, 3 few rows (M <= 8, K a multiple of 4).
-MRS_EXPORT int mrs_gemm_f32_kernel(const float* A, const float* W, float* C, int M, int N, int K, int kernel, void* stream) {
+MRS_EXPORT int mrs_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return MRS_BAD_ARGUMENT;
     const bool vec = K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-    if (kernel == 3 && (M > 8 || !vec)) return MRS_BAD_ARGUMENT;
-    if (kernel < 0 && M <= 8 && vec) kernel = 3;
-    if (kernel < 0) {
-        // A shape's time over q tiles an SM, in microseconds at K = 1,024, is a line: measured alone at N = 1,024 to 6,144,
-        // M = 17 to 2,048, q = 1 to 55 (within a fifth of it nearly everywhere).  The wide tiles win when every SM has many
-        // (2,048 rows, N 4,096: 384, 418 and 457 us for the three shapes; 64 rows: 40, 30, 34; 32 rows of N = 1,024: 37, 22, 18).
-        // A grid's second dimension ends at 65,535 tiles of rows: beyond what the low tiles cover, the high ones take the product.
-        const int bm[3] = {64, 32, 32}, bn[3] = {64, 64, 32}, sms = mrs_sm_count();
-        const double first[3] = {45.0, 19.0, 12.0}, each[3] = {24.0, 14.3, 8.6};
-        double best = 0.0;
-        for (int i = 0; i < 3; ++i) {
-            const long long rows = ((long long)M + bm[i] - 1) / bm[i], tiles = rows * ((N + bn[i] - 1) / bn[i]);
-            const double time = first[i] + each[i] * (double)((tiles + sms - 1) / sms);
-            if (i == 0 || (time < best && rows <= 65535)) best = time, kernel = i;
-        }
+    if (M <= 8 && vec) return M <= 4 ? launch_few<1>(A, W, C, M, N, K, stream) : launch_few<2>(A, W, C, M, N, K, stream);
+    // A shape's time over q tiles an SM, in microseconds at K = 1,024, is a line: measured alone at N = 1,024 to 6,144,
+    // M = 17 to 2,048, q = 1 to 55 (within a fifth of it nearly everywhere).  The wide tiles win when every SM has many
+    // (2,048 rows, N 4,096: 384, 418 and 457 us for the three shapes; 64 rows: 40, 30, 34; 32 rows of N = 1,024: 37, 22, 18).
+    // A grid's second dimension ends at 65,535 tiles of rows: beyond what the low tiles cover, the high ones take the product.
+    const int bm[3] = {64, 32, 32}, bn[3] = {64, 64, 32}, sms = mrs_sm_count();
+    const double first[3] = {45.0, 19.0, 12.0}, each[3] = {24.0, 14.3, 8.6};
+    double best = 0.0;
+    int shape = 0;
+    for (int i = 0; i < 3; ++i) {
+        const long long rows = ((long long)M + bm[i] - 1) / bm[i], tiles = rows * ((N + bn[i] - 1) / bn[i]);
+        const double time = first[i] + each[i] * (double)((tiles + sms - 1) / sms);
+        if (i == 0 || (time < best && rows <= 65535)) best = time, shape = i;
     }
-    if (kernel == 3) return M <= 4 ? launch_few<1>(A, W, C, M, N, K, stream) : launch_few<2>(A, W, C, M, N, K, stream);
-    return vec ? launch_shape<true>(kernel, A, W, C, M, N, K, stream) : launch_shape<false>(kernel, A, W, C, M, N, K, stream);
-}
-
-MRS_EXPORT int mrs_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, void* stream) {
-    return mrs_gemm_f32_kernel(A, W, C, M, N, K, -1, stream);
+    return vec ? launch_shape<true>(shape, A, W, C, M, N, K, stream) : launch_shape<false>(shape, A, W, C, M, N, K, stream);
 }

@@ -1837,8 +1837,8 @@ def moe_product(x: torch.Tensor, sorted_rows: torch.Tensor, tile_expert: torch.T
 
 
 MOE_TC_BLOCK = 64              # gate rows of a block in the layout of the product for many rows; the 64 matching up rows follow
-MOE_TC_MIN_PAIRS = int(os.environ.get("MRS_MOE_TC_MIN_PAIRS", "1024"))      # the variables: for measuring other crossovers
-MOE_ROWS_MAX_PAIRS = int(os.environ.get("MRS_MOE_ROWS_MAX_PAIRS", "128"))
+MOE_TC_MIN_PAIRS = int(os.environ.get("MRS_MOE_TC_MIN_PAIRS", "1024"))      # the variable: for measuring another crossover
+MOE_ROWS_MAX_PAIRS = 512       # float32: beyond, the tiles of `moe_simt_tile()` rows
 
 
 def moe_kernel(x: torch.Tensor, pairs: int, routed: int, inner: int, tc: bool) -> str:
@@ -1847,14 +1847,20 @@ def moe_kernel(x: torch.Tensor, pairs: int, routed: int, inner: int, tc: bool) -
     are as many as the SMs (both products of 32 experts, tcgen05 against the weights straight to registers: 4 pairs an expert
     219 against 211 us at width 4,096, inner 1,536 and 86 against 78 at 2,048 and 1,024; 8 pairs 221 against 232 and 87 against
     86; 12 pairs 222 against 247 and 87 against 92); up to 32 pairs an expert the weights straight to registers; mma.sync
-    between them; else the CUDA cores, with the weights streamed once up to 4 * MOE_ROWS_MAX_PAIRS pairs.  16 tokens x 4 choices
-    of 32 experts, width 4,096, inner 1,536: both products 189 us straight to registers, 298 on the CUDA cores, 503 with
-    mma.sync from shared memory (168 us for the weights' bytes)."""
+    between them; else (float32, odd sizes) the CUDA cores, with the weights streamed once up to MOE_ROWS_MAX_PAIRS pairs.  16 tokens
+    x 4 choices of 32 experts, width 4,096, inner 1,536: both products 189 us straight to registers, 298 on the CUDA cores, 503 with
+    mma.sync from shared memory (168 us for the weights' bytes).  Other sizes, the whole of `moe_experts` with the lists, at 0.25, 1,
+    4, 8, 16, 32 pairs an expert, straight to registers against tcgen05: 8 experts of 512 x 256 13, 13, 13, 14, 18, 29 us against
+    22 to 23; 32 of 1,024 x 384 17, 18, 19, 20, 27, 44 against 29 to 36; 64 of 2,048 x 512 25, 59, 76, 90, 113, 174 against 49, 87, 104,
+    108, 109, 112; 128 of 2,048 x 768 60, 148, 208, 236, 298, 453 against 104, 198, 277, 286, 291, 300; 8 of 4,096 x 4,096 40, 107, 136,
+    165, 212, 317 against 74, 130, 149, 149, 150, 151.  What is chosen up to 32 pairs an expert is at worst 1.3 times the better
+    of the two (small experts from 24 pairs on, many experts around 8), and nowhere slower than the CUDA cores or mma.sync from shared
+    memory; beyond 32 pairs the latter is left with few small experts (8 of 512 x 256 at 64 pairs: 41 us, tcgen05 24)."""
     if tc and (pairs >= MOE_TC_MIN_PAIRS or (pairs > 8 * routed and routed * (inner // 128) >= sm_count(x.device))):
         return "tc"
     if moe_mma_supported(x, inner):
         return "few" if pairs <= 32 * routed else "mma"
-    if moe_rows_supported(x, inner) and pairs <= 4 * MOE_ROWS_MAX_PAIRS:
+    if moe_rows_supported(x, inner) and pairs <= MOE_ROWS_MAX_PAIRS:
         return "rows"
     return "simt"
 

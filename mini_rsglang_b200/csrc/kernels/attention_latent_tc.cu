@@ -337,6 +337,20 @@ __global__ void __launch_bounds__(THREADS, 1) attention_latent_kernel(
     }
 }
 
+// Tensor maps of the step's queries [tokens, heads, R + r] for copies of (128 / heads tokens, rounded down) x (heads): groups of 64
+// elements, and the last 32 (r = 32).
+int query_maps(const void* q, long long tokens, int heads, CUtensorMap* maps) {
+    if (tokens <= 0 || ((uintptr_t)q & 15)) return MRS_BAD_ARGUMENT;
+    const uint64_t strides[2] = {(uint64_t)ROW * 2, (uint64_t)heads * ROW * 2};
+    const uint64_t dims[3] = {(uint64_t)CHUNKS * 64, (uint64_t)heads, (uint64_t)tokens};
+    const uint32_t box[3] = {64, (uint32_t)heads, (uint32_t)(BM / heads)};
+    const int code = mrs_make_tensor_map_bf16(&maps[0], q, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (code != 0 || !TAIL) return code;
+    const uint64_t tail_dims[3] = {32, dims[1], dims[2]};
+    const uint32_t tail_box[3] = {32, box[1], box[2]};
+    return mrs_make_tensor_map_bf16(&maps[1], (const bf16*)q + CHUNKS * 64, 3, tail_dims, strides, tail_box, CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
 int page_shift_of(int page_size) {
     int shift = 0;
     while ((1 << shift) < page_size) ++shift;
@@ -362,24 +376,10 @@ MRS_EXPORT int mrs_attention_latent_tc_cache_maps(const void* cache, long long p
     return mrs_make_tensor_map_bf16(&maps[1], (const bf16*)cache + CHUNKS * 64, 3, tail_dims, strides, tail_box, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
-// The same of the step's queries [tokens, heads, R + r], for copies of (128 / heads tokens, rounded down) x (heads).
-MRS_EXPORT int mrs_attention_latent_tc_query_maps(const void* q, long long tokens, int heads, void* map_out) {
-    if (tokens <= 0 || heads <= 0 || heads > BM || ((uintptr_t)q & 15)) return MRS_BAD_ARGUMENT;
-    CUtensorMap* maps = reinterpret_cast<CUtensorMap*>(map_out);
-    const uint64_t strides[2] = {(uint64_t)ROW * 2, (uint64_t)heads * ROW * 2};
-    const uint64_t dims[3] = {(uint64_t)CHUNKS * 64, (uint64_t)heads, (uint64_t)tokens};
-    const uint32_t box[3] = {64, (uint32_t)heads, (uint32_t)(BM / heads)};
-    int code = mrs_make_tensor_map_bf16(&maps[0], q, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (code != 0 || !TAIL) return code;
-    const uint64_t tail_dims[3] = {32, dims[1], dims[2]};
-    const uint32_t tail_box[3] = {32, box[1], box[2]};
-    return mrs_make_tensor_map_bf16(&maps[1], (const bf16*)q + CHUNKS * 64, 3, tail_dims, strides, tail_box, CU_TENSOR_MAP_SWIZZLE_64B);
-}
-
 // Tiles of up to 128 / heads consecutive tokens of one request each: (sequence, first token, tokens, 0).  out [tokens, heads, R];
 // `gate` [tokens, heads] or null multiplies a head's result; `sinks` [heads] or null: one more term exp(sink) in the denominator.
-// `cache_pages`: the pages that the cache's maps cover.
-MRS_EXPORT int mrs_attention_latent_tc(const void* query_maps, const void* cache_maps, const int* positions, const int* block_table,
+// `cache_pages`: the pages that the cache's maps cover.  The queries' maps are made here: q is another buffer in every call.
+MRS_EXPORT int mrs_attention_latent_tc(const void* q, long long tokens, const void* cache_maps, const int* positions, const int* block_table,
                                        int table_width, const int* tiles, int num_tiles, void* out, const float* gate, const float* sinks,
                                        int heads, int page_size, long long cache_pages, float scale, int window, void* stream) {
     if (num_tiles <= 0) return 0;
@@ -393,8 +393,11 @@ MRS_EXPORT int mrs_attention_latent_tc(const void* query_maps, const void* cache
         if (e != cudaSuccess) return (int)e;
         configured.set(1);
     }
-    const CUtensorMap *q = reinterpret_cast<const CUtensorMap*>(query_maps), *k = reinterpret_cast<const CUtensorMap*>(cache_maps);
-    MRS_LAUNCH(attention_latent_kernel, num_tiles, THREADS, SMEM_BYTES, stream, q[0], q[TAIL ? 1 : 0], k[0], k[TAIL ? 1 : 0], positions, block_table,
+    CUtensorMap queries[2];
+    const int code = query_maps(q, tokens, heads, queries);
+    if (code != 0) return code;
+    const CUtensorMap* k = reinterpret_cast<const CUtensorMap*>(cache_maps);
+    MRS_LAUNCH(attention_latent_kernel, num_tiles, THREADS, SMEM_BYTES, stream, queries[0], queries[TAIL ? 1 : 0], k[0], k[TAIL ? 1 : 0], positions, block_table,
                table_width, (const Tile*)tiles, (bf16*)out, gate, sinks, heads, page_size, shift, (int)cache_pages, scale * LOG2E, window);
     MRS_RETURN_LAUNCH_STATUS();
 }

@@ -1490,11 +1490,10 @@ def attention_latent_tc_library(latent: int, rotated: int) -> ctypes.CDLL:
             raise BackendError("no CUDA device: the engine has no CPU path")
         lib = specialised_kernel_library("attention_latent_tc.cu", {"MRS_LATENT": latent, "MRS_ROTARY": rotated})
         lib.mrs_attention_latent_tc_cache_maps.argtypes = [_c_vp, ctypes.c_longlong, _c_int, _c_vp]
-        lib.mrs_attention_latent_tc_query_maps.argtypes = [_c_vp, ctypes.c_longlong, _c_int, _c_vp]
-        lib.mrs_attention_latent_tc.argtypes = [_c_vp] * 4 + [_c_int, _c_vp, _c_int, _c_vp, _c_vp, _c_vp, _c_int, _c_int, ctypes.c_longlong, _c_float, _c_int,
+        lib.mrs_attention_latent_tc.argtypes = [_c_vp, ctypes.c_longlong] + [_c_vp] * 3 + [_c_int, _c_vp, _c_int, _c_vp, _c_vp, _c_vp, _c_int, _c_int, ctypes.c_longlong, _c_float, _c_int,
                                                               _c_vp]
         lib.mrs_attention_latent_tc_take_error.argtypes = [ctypes.POINTER(ctypes.c_uint)]
-        for name in ("cache_maps", "query_maps", "take_error", "rows"):
+        for name in ("cache_maps", "take_error", "rows"):
             getattr(lib, f"mrs_attention_latent_tc_{name}").restype = _c_int
         lib.mrs_attention_latent_tc.restype = _c_int
         lib.mrs_attention_latent_tc_error_string.argtypes = [_c_int]
@@ -1540,15 +1539,10 @@ def attention_latent_tc(q, cache, positions, block_table, tiles, out, heads: int
         if code != 0:
             fail(code, "tensor maps of the cache")
         _latent_tc_cache_maps[key] = (made, address)
-    keep, query_maps = _aligned_block(256, 64)
-    code = lib.mrs_attention_latent_tc_query_maps(q.data_ptr(), tokens, heads, query_maps)
-    if code != 0:
-        fail(code, "tensor maps of the queries")
     launch_count += 1
-    code = lib.mrs_attention_latent_tc(query_maps, _latent_tc_cache_maps[key][1], positions.data_ptr(), block_table.data_ptr(),
+    code = lib.mrs_attention_latent_tc(q.data_ptr(), tokens, _latent_tc_cache_maps[key][1], positions.data_ptr(), block_table.data_ptr(),
                                        block_table.shape[1], tiles.data_ptr(), tiles.shape[0], out.data_ptr(), _ptr(gate), _ptr(sink_logits),
                                        heads, page_size, cache.shape[0], float(scale), int(window), _stream())
-    del keep                          # the maps were copied into the launch
     if code != 0:
         fail(code, "attention_latent_tc")
 

@@ -18,9 +18,10 @@
 // fills zeros, and the others' rows before the window and behind the last key are cleared once the scores were made.  (A row that
 // one token of a tile sees reaches the tile's other tokens when it is not finite.)
 // Two warps issue because a commit holds its issuer some 400 clocks and a block's MMAs run 1,300: 18 of 45 clocks for the
-// scores (N 64), 4 of 128 for the values (N 256), 82% of the tensor cores' rate.  Four stages and four score buffers let scores run
-// ahead of softmax, which is as long.  A prompt of 2,048 tokens, 16 heads, R 256, r 32, a window of 1,024: 50 us
-// (mma.sync in tiles of 64 rows 197).
+// scores (N 64), 4 of 128 for the values (N 256); at the full rate they would run 1,090.  Four stages and four score buffers let scores
+// run ahead of softmax, which with its trips to tensor memory sets the pace: a block takes some 3,300 clocks (tensor pipe 33% of an
+// SM's active clocks).  A prompt of 2,048 tokens, 16 heads, R 256, r 32, a window of 1,024: 50 us (mma.sync in tiles of 64 rows
+// 197), 256 tiles on 148 SMs.
 // Every wait is bounded (tma.cuh).
 #include "tcgen05.cuh"
 

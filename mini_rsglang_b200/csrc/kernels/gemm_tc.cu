@@ -22,7 +22,7 @@
 // previous kernel's end, x, the MMAs, the ranges' meeting, the store.  Ranges that meet in a cluster,
 // and rings no longer than a CTA's range (two kernels' CTAs then share an SM, and the next one's
 // weights come in under this one): q/k/v 9.1 -> 7.9 us, o and down 7.8 -> 6.5, gate/up 8.5 -> 7.5
-// alone; a step of one token through 4 layers and the head 209 -> 187 to 193 us (three boxes), of 12 tokens
+// alone; a step of one token through 4 layers and the head 209 -> 187 to 193 us (three machines), of 12 tokens
 // 258 -> 223, a decode step of 8 requests at the 8B shape 629 -> 616 us.     (reference: cuBLAS in 32-row blocks, crates/kernels/src/lib.rs:241-322)
 #include "tcgen05.cuh"
 

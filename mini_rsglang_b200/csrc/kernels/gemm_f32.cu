@@ -1,225 +1,370 @@
-// True float32 matrix product C[M,N] = A[M,K] . W[N,K]^T with float32 FMA on the CUDA cores: no tensor cores, no TF32.  It
-// carries every projection of the 32-bit path.  In every kernel here an output element is one chain of multiply-adds over
-// K in ascending order, so its bits depend on K alone: not on M, not on the kernel that the sizes chose, and a token's result
-// does not change with what else is in the batch.            (reference: cuBLAS, kernels/src/lib.rs:298-321)
+// float32 matrix product C[M,N] = A[M,K] . W[N,K]^T on the tcgen05 tensor cores, without giving up a bit of the inputs: every
+// projection of the 32-bit path.
 //
-//   tiles      outer products of 8 x 4 or 4 x 4 outputs a thread, both matrices through a ring of cp.async stages.  Bound by the
-//              multiply-add pipe and by shared memory.  Plain fmaf, not fma.rn.f32x2: with three operands of 64 bits the
-//              packed form stops at half the rate (a loop over registers: 68 TFLOP/s plain, 37 packed; the product of 2,048
-//              rows, N 4,096, K 1,024 517 us packed, 394 plain).
-//   few rows   (M <= 8) the weights streamed once, a lane a column and some rows.  Bound by the weights' bytes and, for
-//              short rows of few columns, by the chain of K multiply-adds.
+// A float32 is the sum of three bfloat16 (8 + 8 + 8 bits of its significand), so a product of two is nine products of bfloat16, each
+// exact in float32.  Six of them are computed; the other three are below 2^-26 of the product together.  The MMAs add 32
+// elements of K at a time into a fresh accumulator in tensor memory, small products first, and from there on a sum is ordinary
+// float32 addition in registers: 32-element sums into one of four ranges of K, the four ranges in order.  An element's bits depend
+// on K alone: not on M, not on the tile or the cut that the sizes chose, and a token's result does not change with what else is in the
+// batch.  A result that is no number or infinite, or below 2^-60 where a part of a factor may lie under bfloat16's range, is computed
+// again in float64 from the inputs (`exact_dot`), so infinities and NaN are those of the sum of the products.
 //
-// Alone, before (one shape of 64 x 64 tiles, transposed element by element, two barriers every 16 elements of K) and now:
-// N 4,096, K 1,024: 1 row 161 -> 15 us, 32 rows 161 -> 21, 128 rows 157 -> 38, 777 rows 320 -> 169, 2,048 rows 587 -> 385
-// (45 TFLOP/s); N 1,024, K 2,048: 8 rows 297 -> 19, 777 rows 314 -> 120; N = K = 4,096: 8 rows 647 -> 49, 512 rows 877 -> 422.
-#include "common.cuh"
+// What bounds it: the workers' instructions (a float32 into three bfloat16 is some thirty instructions for four elements, and the
+// sums), then shared memory (both matrices pass through it; parts of W lie in tensor memory, which took a step of 96 tokens from 0.80 to
+// 0.70 us).  One turn of writers instead of two that overlap: 24 against 19 us for 8 rows in one CTA a tile.  Tiles of 128 tokens
+// spill registers (90 against 63 us for 777 rows, N 4,096, K 1,024).
+// Alone, before (multiply-adds on the CUDA cores) and now: N 4,096, K 1,024: 1 row 15 -> 11 us, 64 rows 35 -> 12, 128 rows 38 -> 18, 777
+// rows 168 -> 63; N 1,024, K 2,048: 8 rows 18.5 -> 12.8, 777 rows 121 -> 34; N 6,144, K 1,024, 777 rows 263 -> 93.  Error against 64
+// bits (relative, normal inputs): K = 1,024 5.7e-7 -> 0.9e-7, K = 3,072 1.0e-6 -> 1.2e-7.
+//             (reference: cuBLAS, kernels/src/lib.rs:298-321)
+#include <cooperative_groups.h>
+
+#include <cfloat>
+
+#include "tcgen05.cuh"
 
 namespace {
+namespace cg = cooperative_groups;
 
-// PIECE bytes from global to shared memory, zeros where `live` is false
+constexpr int BM = 128;              // weight rows of a tile: the M of the MMA, a lane of tensor memory each
+constexpr int BK = 32;               // elements of K of a step: 64 bytes of bfloat16, one swizzled row
+constexpr int RANGES = 4;            // of K, added in order
+constexpr int WORKERS = 512, TURNS = 2, WRITERS = WORKERS / TURNS, THREADS = WORKERS + 32 * TURNS;
+constexpr int PARTS = 3;             // bfloat16 of a float32
+
+// Of a step: a weight row's parts in tensor memory (A of the MMA), the tokens' in shared memory (B); STAGES of both, two
+// accumulators, and a ring of float32 pieces on their way.
+template <int BN>
+struct Tile {
+    static constexpr int W_MINE = BM * BK / 4 / WRITERS, A_PIECES = BN * BK / 4, A_MINE = (A_PIECES + WRITERS - 1) / WRITERS;    // sixteen bytes each
+    static constexpr int W_BYTES = BM * BK * 4, RAW_BYTES = W_BYTES + A_PIECES * 16;
+    static constexpr int PART_BYTES = BN * BK * 2, STAGE_BYTES = PARTS * PART_BYTES;
+    static constexpr int STAGES = BN == 96 ? 3 : 4, DEPTH = BN >= 64 ? 2 : 4;                         // DEPTH: of each turn's steps
+    static constexpr int COLUMNS = BN / 4;                                                            // of a thread's row
+    static constexpr uint32_t W_COLUMNS = PARTS * BK / 2, TMEM = 2 * BN + STAGES * W_COLUMNS <= 256 ? 256 : 512;
+    static constexpr int SUM_BYTES = BM * BN * 4;                                                     // a range's sums
+    static constexpr size_t SMEM = 1024 + STAGES * (size_t)STAGE_BYTES + TURNS * (size_t)DEPTH * RAW_BYTES + 2 * STAGES * sizeof(uint64_t) + 16;
+    static_assert(SMEM <= 232448 && 2 * SUM_BYTES <= STAGES * STAGE_BYTES + TURNS * DEPTH * RAW_BYTES, "shared memory of an SM");
+    static_assert(2 * BN + STAGES * W_COLUMNS <= TMEM, "tensor memory of an SM");
+};
+
 template <int PIECE>
-__device__ __forceinline__ void copy_piece(float* to, const float* from, bool live) {
-    const uint32_t at = (uint32_t)__cvta_generic_to_shared(to);
-    if (PIECE == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(at), "l"(from), "r"(live ? 16 : 0));
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(at), "l"(from), "r"(live ? 4 : 0));
+__device__ __forceinline__ void copy_piece(uint32_t to, const float* from, bool live) {
+    if (PIECE == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to), "l"(from), "r"(live ? 16 : 0));
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(to), "l"(from), "r"(live ? 4 : 0));
 }
 
-// Rows of A and W lie in shared memory as they lie in memory, BK elements a row, with four floats between rows, so that the
-// sixteen bytes that 8 neighbouring rows' readers take fall on 32 banks once.  A warp is 4 x 8 threads; a thread has the rows
-// lane / 8 + 4 i and the columns lane % 8 + 8 j of its warp's part and reads four elements of K of each at a time.
+// Rows of 64 bytes in groups of 8, sixteen-byte pieces xor-ed with half the row's number: the 64-byte swizzle.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t address) {
+    return (uint64_t)((address & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
+}
+
+__device__ __forceinline__ void tmem_load_4_async(uint32_t address, float* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(address) : "memory");
+}
+__device__ __forceinline__ void tmem_load_8_async(uint32_t address, float* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(address) : "memory");
+}
+// x += y, two floats of a register pair at a time
+__device__ __forceinline__ void add_pair(float& x0, float& x1, float y0, float y1) {
+    asm("{\n .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %3};\n add.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}" : "+f"(x0), "+f"(x1) : "f"(y0), "f"(y1));
+}
+template <int C>
+__device__ __forceinline__ void add_columns(uint32_t address, float (&sum)[C]) {
+    constexpr int STEP = C % 16 == 0 ? 16 : C < 8 ? C : 8;
+#pragma unroll
+    for (int c = 0; c < C; c += STEP) {
+        float v[STEP];
+        if constexpr (STEP == 16) tmem_load_16_async(address + c, v);
+        else if constexpr (STEP == 8) tmem_load_8_async(address + c, v);
+        else tmem_load_4_async(address + c, v);
+        tmem_load_wait();
+#pragma unroll
+        for (int e = 0; e < STEP; e += 2) add_pair(sum[c + e], sum[c + e + 1], v[e], v[e + 1]);
+    }
+}
+
+// 16 lanes x 8 columns: a thread has two columns, 2 (lane % 4) and the next, of lanes lane / 4 and 8 further.
+__device__ __forceinline__ void tmem_store_16x8(uint32_t address, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1, %2, %3, %4};" ::"r"(address), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// Two floats as three pairs of bfloat16; what a rounding leaves is exact in float32.  Beyond bfloat16's range the parts are no numbers.
+__device__ __forceinline__ uint32_t take_part(float& x, float& y) {
+    const __nv_bfloat162 pair = __floats2bfloat162_rn(x, y);
+    const uint32_t bits = *reinterpret_cast<const uint32_t*>(&pair);
+    add_pair(x, y, -__uint_as_float(bits << 16), -__uint_as_float(bits & 0xFFFF0000u));
+    return bits;
+}
+
+// The whole warp: a . w over K in float64.
+__device__ __noinline__ float exact_dot(const float* __restrict__ a, const float* __restrict__ w, int K) {
+    double sum = 0.0;
+    for (int k = threadIdx.x & 31; k < K; k += 32) sum = fma((double)a[k], (double)w[k], sum);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return (float)sum;
+}
+
+// Stores the warp's 32 weight rows' results for one token; those that the parts cannot be trusted with are computed again.
+__device__ __forceinline__ void store_column(float v, const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int m,
+                                             int n, int M, int N, int K) {
+    if (m >= M) return;                                      // the same for the whole warp
+    const float size = fabsf(v);
+    unsigned odd = __ballot_sync(0xffffffffu, n < N && !(size <= FLT_MAX && size >= 0x1p-60f) && v != 0.0f);
+    while (odd) {
+        const int lane = __ffs(odd) - 1;
+        odd &= odd - 1;
+        const float again = exact_dot(A + (size_t)m * K, W + (size_t)__shfl_sync(0xffffffffu, n, lane) * K, K);
+        if ((int)(threadIdx.x & 31) == lane) v = again;
+    }
+    if (n < N) C[(size_t)m * N + n] = v;
+}
+
+// A CTA has a tile of 128 weight rows x BN tokens, or (a cluster of 2 or 4) some of the tile's ranges of K.  Sixteen warps copy the
+// float32 rows into shared memory (cp.async; a thread reads back only what it copied itself), write their parts as bfloat16 tiles
+// and add finished accumulators to their sums; two more warps issue the MMAs of every other step.
 // VEC: sixteen-byte copies (K a multiple of 4, both matrices on 16-byte boundaries), else four-byte ones.
-template <int BM, int BN, int TM, int TN, int BK, int STAGES, int MIN_CTAS, bool VEC>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), MIN_CTAS) gemm_f32_tiles_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                                                                                        float* __restrict__ C, int M, int N, int K) {
-    constexpr int THREADS = (BM / TM) * (BN / TN), WARPS_N = BN / (8 * TN), PITCH = BK + 4, STAGE = (BM + BN) * PITCH;
-    constexpr int PIECE = VEC ? 4 : 1, PIECES = BK / PIECE;
-    static_assert((BM + BN) * PIECES % THREADS == 0, "whole copies");
-    extern __shared__ __align__(16) float ring[];
+template <int BN, bool VEC>
+__global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M,
+                                                              int N, int K, int m_tiles, int cut) {
+    using T = Tile<BN>;
+    constexpr int STAGES = T::STAGES;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    unsigned char* raw = smem + STAGES * T::STAGE_BYTES;
+    uint64_t* full = reinterpret_cast<uint64_t*>(raw + TURNS * T::DEPTH * T::RAW_BYTES);       // a stage's parts are written
+    uint64_t* done = full + STAGES;                                                    // a stage's MMAs have finished
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + STAGES);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tile = blockIdx.x / cut, rank = blockIdx.x % cut;
+    const int m0 = tile % m_tiles * BN, n0 = tile / m_tiles * BM;
+    const int steps = (K + BK - 1) / BK, range = (steps + RANGES - 1) / RANGES, ranges = RANGES / cut;
+    const int first = min(rank * ranges * range, steps), count = min((rank + 1) * ranges * range, steps) - first;
+
+    if (tid == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full[s], WORKERS / 32);
+            mbar_init(&done[s], 1);
+        }
+        mbar_fence_init();
+    }
+    if (warp == WORKERS / 32) {
+        tmem_alloc(tmem_slot, T::TMEM);
+        tmem_relinquish_alloc_permit();
+    }
+    tcgen05_fence_before_sync();
+    __syncthreads();
+    tcgen05_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
     pdl_wait();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int tm = (warp / WARPS_N) * 4 * TM + (lane >> 3), tn = (warp % WARPS_N) * 8 * TN + (lane & 7);
-    const int steps = (K + BK - 1) / BK;
-    auto issue = [&](int step) {
-        if (step < steps) {
-            float* stage = ring + (step % STAGES) * STAGE;
+
+    const int row = (warp & 3) * 32 + lane, column0 = (warp >> 2) * T::COLUMNS;        // of a worker's sums
+    if (warp >= WORKERS / 32) {
+        const bool leader = elect_one();
+        constexpr uint32_t idesc = umma_idesc_bf16_f32(BM, BN);
+        for (int i = warp - WORKERS / 32; i < count; i += TURNS) {
+            const int s = i % STAGES;
+            mbar_wait(&full[s], i / STAGES & 1);
+            tcgen05_fence_after_sync();
+            const uint32_t stage = smem_u32(smem + s * T::STAGE_BYTES), parts = tmem_base + 2 * BN + s * T::W_COLUMNS, d = tmem_base + (i & 1) * BN;
+            if (leader) {
+                // (part of W, part of A): products of 2^-16, then 2^-8, then the leading parts
+                constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
 #pragma unroll
-            for (int i = 0; i < (BM + BN) * PIECES / THREADS; ++i) {
-                const int idx = tid + i * THREADS, row = idx / PIECES, c = idx % PIECES * PIECE, k = step * BK + c;
-                // rows beyond the last repeat it and are not stored
-                const float* from = row < BM ? A + (size_t)min(m0 + row, M - 1) * K : W + (size_t)min(n0 + row - BM, N - 1) * K;
-                copy_piece<4 * PIECE>(stage + row * PITCH + c, from + (k < K ? k : 0), k < K);
+                for (int j = 0; j < 6; ++j) {
+                    const uint32_t w = parts + order[j][0] * (BK / 2);
+                    const uint64_t a = smem_desc_sw64(stage + order[j][1] * T::PART_BYTES);
+                    umma_bf16_a_tmem(d, w, a, idesc, j > 0);
+                    umma_bf16_a_tmem(d, w + 8, a + 2, idesc, true);
+                }
+                umma_commit(&done[s]);
             }
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-    };
-    float acc[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
-#pragma unroll 1
-    for (int s = 0; s < STAGES - 1; ++s) issue(s);
-#pragma unroll 1
-    for (int step = 0; step < steps; ++step) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
-        __syncthreads();                                     // the stage is there, and the one before it has been read
-        issue(step + STAGES - 1);
-        const float* a_s = ring + (step % STAGES) * STAGE + tm * PITCH;
-        const float* w_s = ring + (step % STAGES) * STAGE + (BM + tn) * PITCH;
-#pragma unroll
-        for (int kk = 0; kk < BK; kk += 4) {
-            float w[TN][4];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) *reinterpret_cast<float4*>(w[j]) = *reinterpret_cast<const float4*>(w_s + 8 * j * PITCH + kk);
-#pragma unroll
-            for (int i = 0; i < TM; ++i) {
-                float a[4];
-                *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(a_s + 4 * i * PITCH + kk);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[u], w[j][u], acc[i][j]);
-            }
+            __syncwarp();
         }
     }
-    asm volatile("cp.async.wait_group 0;\n" ::);
+    float now[T::COLUMNS], before[T::COLUMNS];               // the running range, the ranges before it (one CTA a tile: their sum)
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int m = m0 + tm + 4 * i;
-        if (m >= M) continue;
+    for (int c = 0; c < T::COLUMNS; ++c) now[c] = before[c] = 0.0f;
+    if (warp < WORKERS / 32) {
+        // A step's writers: of W, sixteen bytes of rows lane / 4 + 8 j of the warp's lanes of tensor memory, half of the step's K a
+        // warp; of A, sixteen bytes of rows line + 32 j.
+        const int turn = tid / WRITERS, writer = tid % WRITERS, half = writer / (WRITERS / 2), line = writer >> 3;
+        const int w_line = (warp & 3) * 32 + (lane >> 2), w_k = half * 16 + (lane & 3) * 4, a_k = (writer & 7) * 4;
+        const uint32_t to_w = tmem_base + 2 * BN + ((uint32_t)((warp & 3) * 32) << 16) + half * 8;
+        const uint32_t to_a = smem_u32(smem) + line * 64 + (((a_k >> 3) ^ ((line >> 1) & 3)) << 4) + (a_k & 4) * 2;
+        raw += turn * (T::DEPTH * T::RAW_BYTES) + writer * 16;
+        const float* w_tile = W + (size_t)n0 * K;
+        const float* a_tile = A + (size_t)m0 * K;
+        const int w_last = N - 1 - n0, a_last = M - 1 - m0;  // rows beyond the last repeat it and are not stored
+        int issued = turn, issue_slot = 0;                   // the next step to ask for
+        auto copy = [&](uint32_t to, const float* row, int k) {
+            if (VEC) {
+                copy_piece<16>(to, row + (k < K ? k : 0), k < K);
+            } else {
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int n = n0 + tn + 8 * j;
-            if (n < N) C[(size_t)m * N + n] = acc[i][j];
-        }
-    }
-}
-
-// Up to 8 rows: a block has 16 columns over the whole of K (two warps of 8 columns, four lanes a column with R rows each), W
-// and A come through a ring of stages of 128 elements of K.  K a multiple of 4, A and W on 16-byte boundaries.
-constexpr int FEW_COLS = 16, FEW_K = 128, FEW_PITCH = FEW_K + 4, FEW_STAGES = 6, FEW_THREADS = 64;
-
-template <int R>
-__global__ void __launch_bounds__(FEW_THREADS) gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                                                                  float* __restrict__ C, int M, int N, int K) {
-    constexpr int ROWS = 4 * R, STAGE = (FEW_COLS + ROWS) * FEW_PITCH;
-    extern __shared__ __align__(16) float ring[];
-    pdl_launch_dependents();
-    pdl_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n0 = blockIdx.x * FEW_COLS, steps = (K + FEW_K - 1) / FEW_K;
-    auto issue = [&](int step) {
-        if (step < steps) {
-            float* stage = ring + (step % FEW_STAGES) * STAGE;
-            const int k0 = step * FEW_K, live = min(FEW_K, K - k0) / 4;      // sixteen bytes a copy
-            if (lane < live) {
-                for (int r = warp; r < FEW_COLS + ROWS; r += FEW_THREADS / 32) {
-                    // a column or row beyond the last repeats it and is not stored
-                    const float* from = r < FEW_COLS ? W + (size_t)min(n0 + r, N - 1) * K : A + (size_t)min(r - FEW_COLS, M - 1) * K;
-                    copy_piece<16>(stage + r * FEW_PITCH + 4 * lane, from + k0 + 4 * lane, true);
+                for (int e = 0; e < 4; ++e) copy_piece<4>(to + 4 * e, row + (k + e < K ? k + e : 0), k + e < K);
+            }
+        };
+        auto issue = [&]() {
+            if (issued < count) {
+                const int k0 = (first + issued) * BK;
+                const uint32_t to = smem_u32(raw) + issue_slot * T::RAW_BYTES;
+#pragma unroll
+                for (int j = 0; j < T::W_MINE; ++j) copy(to + j * WRITERS * 16, w_tile + (size_t)min(w_line + 8 * j, w_last) * K, k0 + w_k);
+#pragma unroll
+                for (int j = 0; j < T::A_MINE; ++j)
+                    if (T::A_PIECES % WRITERS == 0 || writer + j * WRITERS < T::A_PIECES)
+                        copy(to + T::W_BYTES + j * WRITERS * 16, a_tile + (size_t)min(line + WRITERS / 8 * j, a_last) * K, k0 + a_k);
+            }
+            asm volatile("cp.async.commit_group;\n" ::);
+            issued += TURNS;
+            issue_slot = issue_slot + 1 == T::DEPTH ? 0 : issue_slot + 1;
+        };
+        for (int i = 0; i < T::DEPTH - 1; ++i) issue();
+        bool kept = false;
+        int stage = 0, slot = 0, left = range;               // stage of step i, slot of this turn's next step, steps to a range's end
+        int done_stage = 0;                                  // of step i - 2
+        uint32_t parity = 0;
+#pragma unroll 1
+        for (int i = 0; i < count + 2; ++i) {
+            if (i < count && i % TURNS == turn) {            // the stage's last step, i - STAGES, is over: waited for below
+                issue();
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(T::DEPTH - 1) : "memory");
+                const unsigned char* from = raw + slot * T::RAW_BYTES;
+                const uint32_t w = to_w + stage * T::W_COLUMNS, a = to_a + stage * T::STAGE_BYTES;
+#pragma unroll
+                for (int j = 0; j < T::W_MINE; j += 2) {     // 16 lanes
+                    float4 x = *reinterpret_cast<const float4*>(from + j * WRITERS * 16), y = *reinterpret_cast<const float4*>(from + (j + 1) * WRITERS * 16);
+#pragma unroll
+                    for (int part = 0; part < PARTS; ++part) {
+                        const uint32_t x0 = take_part(x.x, x.y), x1 = take_part(x.z, x.w), y0 = take_part(y.x, y.y), y1 = take_part(y.z, y.w);
+                        tmem_store_16x8(w + ((uint32_t)(8 * j) << 16) + part * (BK / 2), x0, x1, y0, y1);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < T::A_MINE; ++j)
+                    if (T::A_PIECES % WRITERS == 0 || writer + j * WRITERS < T::A_PIECES) {
+                        float4 x = *reinterpret_cast<const float4*>(from + T::W_BYTES + j * WRITERS * 16);
+#pragma unroll
+                        for (int part = 0; part < PARTS; ++part) {
+                            const uint32_t low = take_part(x.x, x.y), high = take_part(x.z, x.w);
+                            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a + part * T::PART_BYTES + j * (WRITERS / 8 * BK * 2)), "r"(low), "r"(high));
+                        }
+                    }
+                fence_async_shared();
+                tmem_store_wait();
+                slot = slot + 1 == T::DEPTH ? 0 : slot + 1;
+            }
+            if (i >= 2) {                                    // step i - 2 is over: frees its stage and its accumulator
+                mbar_wait(&done[done_stage], parity);
+                __syncwarp();
+                tcgen05_fence_after_sync();
+                add_columns(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (i & 1) * BN + column0, now);
+                if (++done_stage == STAGES) {
+                    done_stage = 0;
+                    parity ^= 1;
+                }
+                if (--left == 0 || i - 1 == count) {         // a range's end
+                    left = range;
+                    if (cut == 1 || (cut == 2 && !kept)) {
+                        kept = true;
+#pragma unroll
+                        for (int c = 0; c < T::COLUMNS; ++c) {
+                            before[c] += now[c];
+                            now[c] = 0.0f;
+                        }
+                    }
                 }
             }
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-    };
-    for (int s = 0; s < FEW_STAGES - 1; ++s) issue(s);
-    const int col = warp * 8 + (lane & 7), row = lane >> 3;                  // rows row, row + 4, ...
-    float acc[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) acc[i] = 0.0f;
-    for (int step = 0; step < steps; ++step) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(FEW_STAGES - 2));
-        __syncthreads();                                                     // the stage is there, and the one before it read
-        issue(step + FEW_STAGES - 1);
-        const float* stage = ring + (step % FEW_STAGES) * STAGE;
-        const float* w = stage + col * FEW_PITCH;
-        const float* a = stage + (FEW_COLS + row) * FEW_PITCH;
-        const int live = min(FEW_K, K - step * FEW_K);
-        // the chain of multiply-adds is short of work to hide a read behind: the next 16 elements are read ahead of it
-        float4 wv[2][4], av[2][R][4];
-        auto read = [&](int buffer, int k) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                wv[buffer][u] = *reinterpret_cast<const float4*>(w + k + 4 * u);
-#pragma unroll
-                for (int i = 0; i < R; ++i) av[buffer][i][u] = *reinterpret_cast<const float4*>(a + 4 * i * FEW_PITCH + k + 4 * u);
+            if (i < count) {
+                // all warps arrive: the step's MMAs write an accumulator that each of them has read its columns of
+                tcgen05_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[stage]);
             }
-        };
-        auto add = [&](float4 x, const float4 (&y)[R][4], int u) {
-#pragma unroll
-            for (int i = 0; i < R; ++i) acc[i] = fmaf(y[i][u].x, x.x, acc[i]);
-#pragma unroll
-            for (int i = 0; i < R; ++i) acc[i] = fmaf(y[i][u].y, x.y, acc[i]);
-#pragma unroll
-            for (int i = 0; i < R; ++i) acc[i] = fmaf(y[i][u].z, x.z, acc[i]);
-#pragma unroll
-            for (int i = 0; i < R; ++i) acc[i] = fmaf(y[i][u].w, x.w, acc[i]);
-        };
-        if (live == FEW_K) {
-            read(0, 0);
-#pragma unroll
-            for (int k = 0; k < FEW_K; k += 16) {
-                const int buffer = (k / 16) & 1;
-                if (k + 16 < FEW_K) read(buffer ^ 1, k + 16);
-#pragma unroll
-                for (int u = 0; u < 4; ++u) add(wv[buffer][u], av[buffer], u);
-            }
-        } else {
-            for (int k = 0; k < live; k += 4) {
-                wv[0][0] = *reinterpret_cast<const float4*>(w + k);
-#pragma unroll
-                for (int i = 0; i < R; ++i) av[0][i][0] = *reinterpret_cast<const float4*>(a + 4 * i * FEW_PITCH + k);
-                add(wv[0][0], av[0], 0);
-            }
+            if (++stage == STAGES) stage = 0;
         }
     }
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    if (n0 + col >= N) return;
+    if (cut == 1) {
+        if (warp < WORKERS / 32) {
 #pragma unroll
-    for (int i = 0; i < R; ++i)
-        if (row + 4 * i < M) C[(size_t)(row + 4 * i) * N + n0 + col] = acc[i];
+            for (int c = 0; c < T::COLUMNS; ++c) store_column(before[c], A, W, C, m0 + column0 + c, n0 + row, M, N, K);
+        }
+    } else {
+        // every CTA leaves its ranges' sums in its shared memory and adds up a slice of the columns
+        cg::cluster_group cluster = cg::this_cluster();
+        __syncthreads();
+        float* sums = reinterpret_cast<float*>(smem);
+        if (warp < WORKERS / 32) {
+#pragma unroll
+            for (int c = 0; c < T::COLUMNS; ++c) {
+                const int at = (column0 + c) * BM + row;
+                sums[at] = cut == 2 ? before[c] : now[c];
+                if (cut == 2) sums[BM * BN + at] = now[c];
+            }
+        }
+        cluster.sync();
+        if (warp < WORKERS / 32) {
+            const int slice = BN / cut;
+            for (int c = rank * slice + (warp >> 2); c < (rank + 1) * slice; c += WORKERS / BM) {
+                float v = 0.0f;
+#pragma unroll
+                for (int r = 0; r < RANGES; ++r) v += cluster.map_shared_rank(sums, r / ranges)[r % ranges * (BM * BN) + c * BM + row];
+                store_column(v, A, W, C, m0 + c, n0 + row, M, N, K);
+            }
+        }
+        cluster.sync();                                      // no CTA leaves while another reads its sums
+    }
+    tcgen05_fence_before_sync();
+    __syncthreads();
+    if (warp == WORKERS / 32) {
+        tcgen05_fence_after_sync();
+        tmem_dealloc(tmem_base, T::TMEM);
+    }
 }
 
-template <int BM, int BN, int TM, int TN, int BK, int STAGES, int MIN_CTAS, bool VEC>
-int launch_tiles(const float* A, const float* W, float* C, int M, int N, int K, void* stream) {
-    constexpr int SMEM = STAGES * (BM + BN) * (BK + 4) * (int)sizeof(float);
+template <int BN, bool VEC>
+int launch(const float* A, const float* W, float* C, int M, int N, int K, int cut, void* stream) {
     static PerDevice configured;
-    auto kernel = gemm_f32_tiles_kernel<BM, BN, TM, TN, BK, STAGES, MIN_CTAS, VEC>;
+    auto kernel = gemm_f32_kernel<BN, VEC>;
     if (!configured.get()) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<BN>::SMEM);
         if (e != cudaSuccess) return (int)e;
         configured.set(1);
     }
-    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    if (grid.y > 65535) return MRS_BAD_ARGUMENT;
-    MRS_LAUNCH(kernel, grid, (BM / TM) * (BN / TN), SMEM, stream, A, W, C, M, N, K);
-    MRS_RETURN_LAUNCH_STATUS();
+    const long long m_tiles = ((long long)M + BN - 1) / BN, ctas = m_tiles * (((long long)N + BM - 1) / BM) * cut;
+    if (ctas > 0x7fffffffll) return MRS_BAD_ARGUMENT;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((unsigned)ctas);
+    config.blockDim = dim3(THREADS);
+    config.dynamicSmemBytes = Tile<BN>::SMEM;
+    config.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attributes[2];
+    static const bool plain = getenv("MRS_PLAIN_LAUNCH") != nullptr;
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = cut;
+    attributes[0].val.clusterDim.y = 1;
+    attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = plain ? 1 : 2;
+    const cudaError_t e = cudaLaunchKernelEx(&config, kernel, A, W, C, M, N, K, (int)m_tiles, cut);
+    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
 template <bool VEC>
-int launch_shape(int shape, const float* A, const float* W, float* C, int M, int N, int K, void* stream) {
-    switch (shape) {
-        case 0: return launch_tiles<64, 64, 8, 4, 16, 4, 4, VEC>(A, W, C, M, N, K, stream);
-        case 1: return launch_tiles<32, 64, 4, 4, 32, 4, 4, VEC>(A, W, C, M, N, K, stream);
-        case 2: return launch_tiles<32, 32, 4, 4, 32, 6, 4, VEC>(A, W, C, M, N, K, stream);
+int launch_tile(int bn, const float* A, const float* W, float* C, int M, int N, int K, int cut, void* stream) {
+    switch (bn) {
+        case 16: return launch<16, VEC>(A, W, C, M, N, K, cut, stream);
+        case 32: return launch<32, VEC>(A, W, C, M, N, K, cut, stream);
+        case 64: return launch<64, VEC>(A, W, C, M, N, K, cut, stream);
+        default: return launch<96, VEC>(A, W, C, M, N, K, cut, stream);
     }
-    return MRS_BAD_ARGUMENT;
-}
-
-template <int R>
-int launch_few(const float* A, const float* W, float* C, int M, int N, int K, void* stream) {
-    constexpr int SMEM = FEW_STAGES * (FEW_COLS + 4 * R) * FEW_PITCH * (int)sizeof(float);
-    static PerDevice configured;
-    if (!configured.get()) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured.set(1);
-    }
-    MRS_LAUNCH(gemm_f32_few_kernel<R>, (N + FEW_COLS - 1) / FEW_COLS, FEW_THREADS, SMEM, stream, A, W, C, M, N, K);
-    MRS_RETURN_LAUNCH_STATUS();
 }
 
 }  // namespace
@@ -228,19 +373,25 @@ MRS_EXPORT int mrs_gemm_f32(const float* A, const float* W, float* C, int M, int
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return MRS_BAD_ARGUMENT;
     const bool vec = K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-    if (M <= 8 && vec) return M <= 4 ? launch_few<1>(A, W, C, M, N, K, stream) : launch_few<2>(A, W, C, M, N, K, stream);
-    // A shape's time over q tiles an SM, in microseconds at K = 1,024, is a line: measured alone at N = 1,024 to 6,144,
-    // M = 17 to 2,048, q = 1 to 55 (within a fifth of it nearly everywhere).  The wide tiles win when every SM has many
-    // (2,048 rows, N 4,096: 384, 418 and 457 us for the three shapes; 64 rows: 40, 30, 34; 32 rows of N = 1,024: 37, 22, 18).
-    // A grid's second dimension ends at 65,535 tiles of rows: beyond what the low tiles cover, the high ones take the product.
-    const int bm[3] = {64, 32, 32}, bn[3] = {64, 64, 32}, sms = mrs_sm_count();
-    const double first[3] = {45.0, 19.0, 12.0}, each[3] = {24.0, 14.3, 8.6};
+    // A round of CTAs takes a line over a CTA's steps, in microseconds, measured alone at N = 1,024 to 6,144, K = 1,024 to 3,072 and
+    // M = 1 to 777 (within a tenth nearly everywhere): 8 rows of N 4,096, K 1,024 18.7, 13.1 and 11.0 us with 1, 2 and 4 CTAs a tile; 777
+    // rows 63 us with tiles of 96 tokens in two rounds, 73 with 64 in three.  Clusters of 4 do not come onto every SM.
+    constexpr int widths[4] = {16, 32, 64, 96};
+    constexpr double fixed[4] = {6.0, 6.5, 8.0, 9.3}, each[4] = {0.43, 0.45, 0.57, 0.70};
+    const int sms = mrs_sm_count(), range = ((K + BK - 1) / BK + RANGES - 1) / RANGES;
     double best = 0.0;
-    int shape = 0;
-    for (int i = 0; i < 3; ++i) {
-        const long long rows = ((long long)M + bm[i] - 1) / bm[i], tiles = rows * ((N + bn[i] - 1) / bn[i]);
-        const double time = first[i] + each[i] * (double)((tiles + sms - 1) / sms);
-        if (i == 0 || (time < best && rows <= 65535)) best = time, shape = i;
+    int bn = 0, cut = 1;
+    for (int i = 0; i < 4; ++i) {
+        const long long tiles = ((long long)N + BM - 1) / BM * (((long long)M + widths[i] - 1) / widths[i]);
+        for (int c = 1; c <= RANGES; c *= 2) {
+            const long long held = c == 4 ? sms * 7 / 8 / 4 * 4 : sms / c * c, rounds = held ? (tiles * c + held - 1) / held : tiles * c;
+            const double time = (double)rounds * (fixed[i] + each[i] * (RANGES / c) * range);
+            if (bn == 0 || time < best) best = time, bn = widths[i], cut = c;
+        }
     }
-    return vec ? launch_shape<true>(shape, A, W, C, M, N, K, stream) : launch_shape<false>(shape, A, W, C, M, N, K, stream);
+    return vec ? launch_tile<true>(bn, A, W, C, M, N, K, cut, stream) : launch_tile<false>(bn, A, W, C, M, N, K, cut, stream);
 }
+
+MRS_EXPORT int mrs_gemm_f32_take_error(unsigned int* word) { return mrs_take_error_word(word); }
+// Mirrors the error word into a word of pinned host memory from now on.
+MRS_EXPORT int mrs_gemm_f32_mirror_errors(unsigned int* host_word) { return mrs_set_error_mirror(host_word); }

@@ -53,7 +53,10 @@ def library() -> ctypes.CDLL:
             fn.restype = _c_int
         lib.mrs_error_string.argtypes = [_c_int]
         lib.mrs_error_string.restype = ctypes.c_char_p
+        lib.mrs_gemm_f32_take_error.argtypes = [ctypes.POINTER(ctypes.c_uint)]
+        lib.mrs_gemm_f32_take_error.restype = _c_int
         _lib = lib
+        _register_error_word("gemm_f32", lib, "mrs_gemm_f32")
     return _lib
 
 

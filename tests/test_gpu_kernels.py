@@ -2,6 +2,7 @@
 at sizes other than the engine's tiny configurations (widths and vocabularies that are no power
 of two, head sizes in steps of 16, odd numbers of heads and groups)."""
 
+import math
 import os
 import subprocess
 import sys
@@ -149,6 +150,47 @@ def test_gemm_f32_sizes_keep_a_rows_bits(m, n, k):
     other = torch.empty_like(out)
     kernels.gemm_f32(shifted, w, other)
     assert torch.equal(out, other)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 130, 1024), (17, 127, 3072), (95, 129, 2048), (97, 128, 1000), (260, 300, 4100)])
+def test_gemm_f32_keeps_every_bit_of_its_inputs(m, n, k):
+    """Both sides of the tiles' edges, short and long ranges of K, one CTA and clusters a tile.  A product of two float32 loses at most
+    2^-26 of itself, 32 are added by the tensor cores, the rest is k / 32 + 4 additions: within 2^-23 of the sum of the products'
+    sizes for the first and, a rounding each, (k / 32 + 4) 2^-24 for the others; and closer than a chain of k multiply-adds in
+    float32 comes."""
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    x, w = torch.randn(m, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    out = torch.empty(m, n, device=DEV)
+    kernels.gemm_f32(x, w, out)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert ((out.double() - want).abs() <= size * 2.0 ** -23 + want.abs().max() * (k / 32 + 4) * 2.0 ** -24).all()
+    chain = torch.zeros(m, n, device=DEV, dtype=torch.float64)
+    for i in range(k):                                       # a multiply-add: exact in 64 bits, then rounded
+        chain = (chain + x[:, i, None].double() * w[:, i].double()).float().double()
+    assert (out.double() - want).norm() <= (chain - want).norm()
+
+
+@pytest.mark.parametrize("m", [1, 20, 100])
+def test_gemm_f32_of_values_at_the_ends_of_the_range(m):
+    """Infinities, NaN, values that bfloat16 rounds to infinity and products far below one: what the sum of the products is."""
+    g = torch.Generator(device=DEV).manual_seed(m)
+    n, k = 140, 300
+    x, w = torch.randn(m, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    w[3] *= 1e-30                                            # small results, their factors' parts partly below bfloat16's range
+    w[5, 7], w[6, 8], w[7, 9] = math.inf, math.nan, 0.0
+    x[m // 2, 9], x[m // 2, 11] = math.inf, 3.4e38           # infinity times 0 in column 7
+    w[:, 11] *= 1e-3
+    w[11] = 0.0
+    x[m - 1] *= 1e-9
+    out = torch.empty(m, n, device=DEV)
+    kernels.gemm_f32(x, w, out)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert torch.equal(out.isnan(), want.isnan())
+    infinite = want.float().isinf()
+    assert torch.equal(out[infinite], want.float()[infinite])
+    finite = want.float().isfinite()
+    assert ((out.double() - want).abs() <= size * k * 2.0 ** -24)[finite].all() and out[finite].isfinite().all()
+    assert (out[m - 1, 3].double() - want[m - 1, 3]).abs() <= 2.0 ** -23 * size[m - 1, 3] or not want[m - 1, 3].isfinite()
 
 
 def plain_qk(qkv, positions, q_w, k_w, eps, theta, nq, nkv, d):

@@ -12,20 +12,30 @@
 // the chunks' results (maximum, sum, weighted values) are joined in ascending order by the same arithmetic whether one block
 // walked them all or each had a block of its own (few rows with long contexts; a second kernel then joins them).
 //
-// Bound by the multiply-add pipe and shared memory for prompts, by the cache's bytes for decoded tokens.  Alone, 16 query and
-// 8 key/value heads of 128, one warp a (token, head) before and now: a prompt of 777 tokens 2,661 -> 190 us, of 2,000 16,388 -> 719
-// (23 TFLOP/s), 512 tokens behind 1,536 8,094 -> 366; one token behind 4,000 2,120 -> 105, 8 tokens behind 2,000 1,723 -> 130,
-// 64 tokens behind 256 325 -> 127.
+// Bound by the multiply-add pipe and shared memory for prompts; for decoded tokens by a tile's chain of page numbers, keys, scores,
+// weights and values.  Up to 8 rows take steps of two blocks: a warp a row and a block of scores, a column a thread, keys of two
+// steps and values of one ahead, page numbers three.  Chunks of 256 keys: of 512, 400 tokens walk 13 blocks in a row on a third of the
+// SMs (attention layer of the 0.6B shape 199 against 167 us; 20 tokens behind 980 126 against 78); of 128, the joining outweighs it (decoded
+// tokens of 4 requests at 3,000 98 against 92, 880 tokens behind 1,420 863 against 687 us).
+// Kernel alone, 16 query and 8 key/value heads of 128, before (a page's number looked up in front of every copy, one warp a row) and
+// now: one token behind 4,000 105 -> 18 + 5 us, 30 requests at 400 99 -> 38 + 3, a prompt of 777 tokens 168 -> 146 + 8.
 #include "common.cuh"
 
 #include <type_traits>
 
 namespace {
 
-constexpr int ROWS = 64, KEYS = 32, CHUNK = 512, THREADS = 256, FEW_ROWS = 8;
+constexpr int ROWS = 64, KEYS = 32, CHUNK = 256, THREADS = 256, FEW_ROWS = 8;
 constexpr int P_PITCH = KEYS + 4;
 
-template <int D> constexpr int smem_floats() { return ROWS * (D + 4) + KEYS * (D + 4) + KEYS * D + ROWS * P_PITCH; }
+constexpr int FEW_KEYS = 2 * KEYS, FEW_PITCH = FEW_KEYS + 4, AHEAD = 4;
+
+// shared memory of the walks over many and over few rows, each with the running sums of the chunks that !SPLIT keeps
+template <int D, bool SPLIT> constexpr int smem_floats() {
+    const int many = ROWS * (D + 4) + KEYS * (D + 4) + KEYS * D + ROWS * P_PITCH + (SPLIT ? 0 : ROWS * D);
+    const int few = FEW_ROWS * (D + 4) + 2 * FEW_KEYS * (D + 4) + FEW_KEYS * D + FEW_ROWS * FEW_PITCH + (SPLIT ? 0 : FEW_ROWS * D);
+    return many > few ? many : few;
+}
 
 __device__ __forceinline__ void copy16(float* to, const float* from, bool live) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from), "r"(live ? 16 : 0));
@@ -55,8 +65,8 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
     float* k_s = q_s + ROWS * PITCH;                     // [KEYS][PITCH]
     float* v_s = k_s + KEYS * PITCH;                     // [KEYS][D]
     float* p_s = v_s + KEYS * D;                         // [ROWS][P_PITCH]
-    float* total_s = p_s + ROWS * P_PITCH;               // !SPLIT: [4 * COLS][THREADS], a thread's own
     __shared__ float keep_s[ROWS], take_s[ROWS];
+    __shared__ long long place_s[AHEAD * FEW_KEYS];       // where cached rows begin, of the steps (few rows) or blocks that come next; -1: not seen
     __shared__ int found[2], warp_count[THREADS / 32];
     pdl_launch_dependents();
     pdl_wait();
@@ -116,21 +126,31 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
             if (c < d) x = *reinterpret_cast<const float4*>(A.q + ((size_t)(t0 + r / group) * A.nq + g * group + r % group) * d + c);
             *reinterpret_cast<float4*>(q_s + r * PITCH + c) = x;
         }
-        // keys (or values) of the block that begins at key `at`, zeros outside begin .. end
-        auto fetch = [&](const float* __restrict__ cache, float* to, int pitch, int at) {
-            if (at < end) {
-                for (int i = tid; i < KEYS * (D / 4); i += THREADS) {
-                    const int j = i / (D / 4), c = i % (D / 4) * 4, p = at + j;
-                    const bool live = p >= begin && p < end && c < d;
-                    const float* from = cache;
-                    if (live) from += (((size_t)pages[p / A.page_size] * A.nkv + g) * A.page_size + p % A.page_size) * d + c;
-                    copy16(to + j * pitch + c, from, live);
-                }
+        // where the row of key p begins in the cache.  The page's number comes from memory: it is asked for a step before the
+        // copies want it (a lookup in front of every copy was half the time of a block)
+        auto place_of = [&](int p) -> long long {
+            if (p < begin || p >= end) return -1;
+            return (((long long)pages[p / A.page_size] * A.nkv + g) * A.page_size + p % A.page_size) * d;
+        };
+        // rows to shared memory, zeros for those that are not seen
+        auto fetch = [&](auto count, const float* __restrict__ cache, float* to, int pitch, const long long* places) {
+            constexpr int MINE = decltype(count)::value * (D / 4) / THREADS;
+            long long place[MINE];
+#pragma unroll
+            for (int i = 0; i < MINE; ++i) place[i] = places[(tid + i * THREADS) / (D / 4)];
+#pragma unroll
+            for (int i = 0; i < MINE; ++i) {
+                const int j = (tid + i * THREADS) / (D / 4), c = (tid + i * THREADS) % (D / 4) * 4;
+                const bool live = place[i] >= 0 && c < d;
+                copy16(to + j * pitch + c, cache + (live ? place[i] + c : 0), live);
             }
             copies_commit();
         };
+        constexpr std::integral_constant<int, KEYS> block_rows;
+        constexpr std::integral_constant<int, FEW_KEYS> step_rows;
         const bool few = rows <= FEW_ROWS;
-        // scores: a warp has 16 rows x 16 keys, lanes 4 x 8; few rows: a warp a row, a lane a key
+        float* total_s = few ? smem + FEW_ROWS * PITCH + 2 * FEW_KEYS * PITCH + FEW_KEYS * D + FEW_ROWS * FEW_PITCH : p_s + ROWS * P_PITCH;      // !SPLIT: [4 * COLS][THREADS], few rows [FEW_OWN][THREADS]: a thread's own
+        // scores: a warp has 16 rows x 16 keys, lanes 4 x 8; few rows: a warp a row and a block, a lane a key
         const int s_row = (warp >> 1) * 16 + (lane >> 3), s_key = (warp & 1) * 16 + (lane & 7);
         // values: a thread has rows o_row .. o_row + 3 and COLS columns in pieces of 4, 64 apart; few rows: a column of every
         // FEW_STEP-th row
@@ -144,7 +164,7 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
                 o[i][c] = 0.0f;
-                if (!SPLIT) total_s[(i * COLS + c) * THREADS + tid] = 0.0f;
+                if (!SPLIT && (!few || i * COLS + c < FEW_OWN)) total_s[(i * COLS + c) * THREADS + tid] = 0.0f;
             }
         // a row's maximum and sum: four threads a row, eight keys of a block each
         const int m_row = tid >> 2, m_key = (tid & 3) * 8;
@@ -152,151 +172,216 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
         const int m_pos = m_row < rows ? pos0 + m_row / group : -1;      // rows beyond the last see nothing
         const int m_first = A.window > 0 ? max(0, m_pos + 1 - A.window) : 0;
 
+        // the chunk joins those before it
+        auto join_chunk = [&]() {
+            __syncthreads();                             // keep_s has been read
+            if ((tid & 3) == 0) {
+                const float next = fmaxf(m_all, m), keep = m_all == next ? 1.0f : ratio(m_all, next), take = ratio(m, next);
+                l_all = join(l_all, keep, l, take);
+                m_all = next;
+                keep_s[m_row] = keep;
+                take_s[m_row] = take;
+            }
+            m = -CUDART_INF_F, l = 0.0f;
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 4 * COLS; ++i) {
+                if (few && i >= FEW_OWN) continue;
+                const int r = few ? min(f_row + i * FEW_STEP, ROWS - 1) : o_row + i / COLS;
+                float& total = total_s[i * THREADS + tid];
+                total = join(total, keep_s[r], o[i / COLS][i % COLS], take_s[r]);
+                o[i / COLS][i % COLS] = 0.0f;
+            }
+        };
+        // a thread's eight scores of a block that begins at key `at`: masked, the row's maximum, exponentials in their place and their
+        // sum; returns what the sums before are multiplied with.  The four threads of a row lie in one warp and come here together.
+        auto weigh = [&](float* p, int at) {
+            float x[8], top = -CUDART_INF_F;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int key = at + m_key + u;
+                x[u] = key <= m_pos && key >= m_first ? p[u] * A.scale : -CUDART_INF_F;
+                top = fmaxf(top, x[u]);
+            }
+            const unsigned quad = 0xfu << (lane & 28);
+            top = fmaxf(top, __shfl_xor_sync(quad, top, 1));
+            top = fmaxf(top, __shfl_xor_sync(quad, top, 2));
+            const float next = fmaxf(m, top), alpha = m == next ? 1.0f : ratio(m, next);
+            float sum = 0.0f;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float e = ratio(x[u], next);
+                p[u] = e;
+                sum += e;
+            }
+            sum += __shfl_xor_sync(quad, sum, 1);
+            sum += __shfl_xor_sync(quad, sum, 2);
+            l = l * alpha + sum;
+            m = next;
+            return alpha;
+        };
+        // where some row does not see all of the block's keys, weights of zero are skipped: a value that a row does not see never
+        // reaches it, not even one that is no number
+        auto some_unseen = [&](int at) { return at + KEYS > pos0 + 1 || (A.window > 0 && at < end_key - A.window); };
+
         int at = begin / KEYS * KEYS;
-        fetch(A.k, k_s, PITCH, at);
-        fetch(A.v, v_s, D, at);
-        for (; at < end; at += KEYS) {
-            copies_wait<1>();
-            __syncthreads();                             // the keys are there (and q)
-            if (few) {
-                if (warp < rows) {
+        if (few) {
+            // Steps of up to two blocks of keys (they end at multiples of FEW_KEYS).  The keys of the next two steps and the values
+            // of the next are on their way while one is worked on.
+            float* fk_s = smem + FEW_ROWS * PITCH;       // [2][FEW_KEYS][PITCH], behind q
+            float* fv_s = fk_s + 2 * FEW_KEYS * PITCH;   // [FEW_KEYS][D]
+            float* fp_s = fv_s + FEW_KEYS * D;           // [FEW_ROWS][FEW_PITCH]
+            auto keys_of = [&](int from) { return from < end ? (from % FEW_KEYS ? KEYS : FEW_KEYS) : 0; };
+            auto after = [&](int from) { return from + (from % FEW_KEYS ? KEYS : FEW_KEYS); };
+            const int second = after(at), third = after(second);
+            if (tid < 3 * FEW_KEYS) place_s[tid] = place_of((tid < FEW_KEYS ? at : tid < 2 * FEW_KEYS ? second : third) + tid % FEW_KEYS);
+            __syncthreads();
+            int coming = after(third);                   // the step whose places come next, AHEAD - 1 ahead of the running one
+            fetch(step_rows, A.k, fk_s, PITCH, place_s);
+            fetch(step_rows, A.v, fv_s, D, place_s);
+            fetch(step_rows, A.k, fk_s + FEW_KEYS * PITCH, PITCH, place_s + FEW_KEYS);
+            for (int step = 0; at < end; ++step) {
+                const int blocks = keys_of(at) / KEYS;
+                const long long later = tid < FEW_KEYS ? place_of(coming + tid) : -1;
+                copies_wait<2>();
+                __syncthreads();                         // the step's keys are there (and q)
+                const float* k_now = fk_s + (step & 1) * FEW_KEYS * PITCH;
+                for (int task = warp; task < rows * blocks; task += THREADS / 32) {
+                    const int r = task % rows, b = task / rows;
                     float s = 0.0f;
-#pragma unroll 8
+#pragma unroll 16
                     for (int e = 0; e < D; e += 4) {
-                        const float4 x = *reinterpret_cast<const float4*>(q_s + warp * PITCH + e), y = *reinterpret_cast<const float4*>(k_s + lane * PITCH + e);
+                        const float4 x = *reinterpret_cast<const float4*>(q_s + r * PITCH + e);
+                        const float4 y = *reinterpret_cast<const float4*>(k_now + (b * KEYS + lane) * PITCH + e);
                         s = fmaf(x.x, y.x, s), s = fmaf(x.y, y.y, s), s = fmaf(x.z, y.z, s), s = fmaf(x.w, y.w, s);
                     }
-                    p_s[warp * P_PITCH + lane] = s;
+                    fp_s[r * FEW_PITCH + b * KEYS + lane] = s;
                 }
-            } else if ((warp >> 1) * 16 < rows) {
-                float s[4][2] = {};
+                __syncthreads();                         // the scores are there, the keys have been read
+                fetch(step_rows, A.k, fk_s + (step & 1) * FEW_KEYS * PITCH, PITCH, place_s + (step + 2) % AHEAD * FEW_KEYS);
+                if (m_row < rows)
+                    for (int b = 0; b < blocks; ++b) {
+                        const float alpha = weigh(fp_s + m_row * FEW_PITCH + b * KEYS + m_key, at + b * KEYS);
+                        if ((tid & 3) == 0) keep_s[b * FEW_ROWS + m_row] = alpha;
+                    }
+                if (tid < FEW_KEYS) place_s[(step + AHEAD - 1) % AHEAD * FEW_KEYS + tid] = later;
+                coming = after(coming);
+                copies_wait<1>();
+                __syncthreads();                         // the weights and the values are there
+                // rows beyond the last add what nothing reads
+                auto values = [&](auto own, auto skip, int b) {
+                    constexpr int OWN = decltype(own)::value;
+                    float f[OWN];
+#pragma unroll
+                    for (int i = 0; i < OWN; ++i) f[i] = o_few[i] * keep_s[b * FEW_ROWS + f_row + i * FEW_STEP];
+                    const float* p = fp_s + f_row * FEW_PITCH + b * KEYS;
 #pragma unroll 4
-                for (int e = 0; e < D; e += 4) {
-                    float4 y[2];
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) y[j] = *reinterpret_cast<const float4*>(k_s + (s_key + 8 * j) * PITCH + e);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float4 x = *reinterpret_cast<const float4*>(q_s + (s_row + 4 * i) * PITCH + e);
-#pragma unroll
-                        for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.x, y[j].x, s[i][j]);
-#pragma unroll
-                        for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.y, y[j].y, s[i][j]);
-#pragma unroll
-                        for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.z, y[j].z, s[i][j]);
-#pragma unroll
-                        for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.w, y[j].w, s[i][j]);
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) p_s[(s_row + 4 * i) * P_PITCH + s_key + 8 * j] = s[i][j];
-            }
-            __syncthreads();                             // the scores are there, the keys have been read
-            fetch(A.k, k_s, PITCH, at + KEYS);
-            if (m_row < rows || !few) {
-                float* p = p_s + m_row * P_PITCH + m_key;
-                float x[8], top = -CUDART_INF_F;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int key = at + m_key + u;
-                    x[u] = key <= m_pos && key >= m_first ? p[u] * A.scale : -CUDART_INF_F;
-                    top = fmaxf(top, x[u]);
-                }
-                // the four threads of a row lie in one warp and take this branch together
-                const unsigned quad = 0xfu << (lane & 28);
-                top = fmaxf(top, __shfl_xor_sync(quad, top, 1));
-                top = fmaxf(top, __shfl_xor_sync(quad, top, 2));
-                const float next = fmaxf(m, top), alpha = m == next ? 1.0f : ratio(m, next);
-                float sum = 0.0f;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const float e = ratio(x[u], next);
-                    p[u] = e;
-                    sum += e;
-                }
-                sum += __shfl_xor_sync(quad, sum, 1);
-                sum += __shfl_xor_sync(quad, sum, 2);
-                l = l * alpha + sum;
-                m = next;
-                if ((tid & 3) == 0) keep_s[m_row] = alpha;
-            }
-            copies_wait<1>();
-            __syncthreads();                             // the weights and the values are there
-            // where some row does not see all of the block's keys, weights of zero are skipped: a value that a row does not
-            // see never reaches it, not even one that is no number
-            const bool masked = at + KEYS > pos0 + 1 || (A.window > 0 && at < end_key - A.window);
-            if (few) {
-                const int live = min(KEYS, end - at);
-                float f[FEW_OWN];
-#pragma unroll
-                for (int i = 0; i < FEW_OWN; ++i) f[i] = f_row + i * FEW_STEP < rows ? o_few[i] * keep_s[f_row + i * FEW_STEP] : 0.0f;
-                for (int j = 0; j < live; ++j) {
-                    const float y = v_s[j * D + f_col];
-#pragma unroll
-                    for (int i = 0; i < FEW_OWN; ++i) {
-                        const int r = f_row + i * FEW_STEP;
-                        if (r >= rows) continue;
-                        const float w = p_s[r * P_PITCH + j];
-                        if (!masked || w != 0.0f) f[i] = fmaf(w, y, f[i]);
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < FEW_OWN; ++i) o_few[i] = f[i];
-            } else if (o_row < rows) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float alpha = keep_s[o_row + i];
-#pragma unroll
-                    for (int c = 0; c < COLS; ++c) o[i][c] *= alpha;
-                }
-                auto keys = [&](auto skip) {
-#pragma unroll 2
                     for (int j = 0; j < KEYS; j += 4) {
-                        float w[4][4];
+                        float y[4], w[OWN][4];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(p_s + (o_row + i) * P_PITCH + j);
+                        for (int u = 0; u < 4; ++u) y[u] = fv_s[(b * KEYS + j + u) * D + f_col];
+#pragma unroll
+                        for (int i = 0; i < OWN; ++i) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(p + i * FEW_STEP * FEW_PITCH + j);
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
 #pragma unroll
-                            for (int c = 0; c < COLS; c += 4) {
-                                float y[4];
-                                *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(v_s + (j + u) * D + o_col + 16 * c);
-#pragma unroll
-                                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                                    for (int b = 0; b < 4; ++b)
-                                        if (!decltype(skip)::value || w[i][u] != 0.0f) o[i][c + b] = fmaf(w[i][u], y[b], o[i][c + b]);
-                            }
+                            for (int i = 0; i < OWN; ++i)
+                                if (!decltype(skip)::value || w[i][u] != 0.0f) f[i] = fmaf(w[i][u], y[u], f[i]);
                     }
-                };
-                if (masked) keys(std::true_type{});
-                else keys(std::false_type{});
-            }
-            if (!SPLIT && (at + KEYS >= end || (at + KEYS) % CHUNK == 0)) {
-                // the chunk joins those before it
-                __syncthreads();                         // keep_s has been read
-                if ((tid & 3) == 0) {
-                    const float next = fmaxf(m_all, m), keep = m_all == next ? 1.0f : ratio(m_all, next), take = ratio(m, next);
-                    l_all = join(l_all, keep, l, take);
-                    m_all = next;
-                    keep_s[m_row] = keep;
-                    take_s[m_row] = take;
-                }
-                m = -CUDART_INF_F, l = 0.0f;
-                __syncthreads();
 #pragma unroll
-                for (int i = 0; i < 4 * COLS; ++i) {
-                    if (few && i >= FEW_OWN) continue;
-                    const int r = few ? min(f_row + i * FEW_STEP, ROWS - 1) : o_row + i / COLS;
-                    float& total = total_s[i * THREADS + tid];
-                    total = join(total, keep_s[r], o[i / COLS][i % COLS], take_s[r]);
-                    o[i / COLS][i % COLS] = 0.0f;
+                    for (int i = 0; i < OWN; ++i) o_few[i] = f[i];
+                };
+                for (int b = 0; b < blocks; ++b) {
+                    const bool masked = some_unseen(at + b * KEYS);
+                    if (rows <= FEW_STEP) masked ? values(std::integral_constant<int, 1>{}, std::true_type{}, b) : values(std::integral_constant<int, 1>{}, std::false_type{}, b);
+                    else masked ? values(std::integral_constant<int, FEW_OWN>{}, std::true_type{}, b) : values(std::integral_constant<int, FEW_OWN>{}, std::false_type{}, b);
                 }
+                at = after(at);
+                if (!SPLIT && (at >= end || at % CHUNK == 0)) join_chunk();
+                __syncthreads();                         // values, weights and factors have been read
+                fetch(step_rows, A.v, fv_s, D, place_s + (step + 1) % AHEAD * FEW_KEYS);
             }
-            __syncthreads();                             // values, weights and factors have been read
-            fetch(A.v, v_s, D, at + KEYS);
+        } else {
+            // A block's keys and values are asked for while the block before it is worked on, their places one block earlier.
+            if (tid < 2 * KEYS) place_s[tid] = place_of(at + tid);
+            __syncthreads();
+            fetch(block_rows, A.k, k_s, PITCH, place_s);
+            fetch(block_rows, A.v, v_s, D, place_s);
+            for (int block = 0; at < end; ++block, at += KEYS) {
+                const long long later = tid < KEYS ? place_of(at + 2 * KEYS + tid) : -1;
+                const long long* next_places = place_s + ((block + 1) & 1) * KEYS;
+                const bool more = at + KEYS < end;
+                copies_wait<1>();
+                __syncthreads();                         // the keys are there (and q)
+                if ((warp >> 1) * 16 < rows) {
+                    float s[4][2] = {};
+#pragma unroll 4
+                    for (int e = 0; e < D; e += 4) {
+                        float4 y[2];
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) y[j] = *reinterpret_cast<const float4*>(k_s + (s_key + 8 * j) * PITCH + e);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 x = *reinterpret_cast<const float4*>(q_s + (s_row + 4 * i) * PITCH + e);
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.x, y[j].x, s[i][j]);
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.y, y[j].y, s[i][j]);
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.z, y[j].z, s[i][j]);
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) s[i][j] = fmaf(x.w, y[j].w, s[i][j]);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) p_s[(s_row + 4 * i) * P_PITCH + s_key + 8 * j] = s[i][j];
+                }
+                __syncthreads();                         // the scores are there, the keys have been read
+                if (more) fetch(block_rows, A.k, k_s, PITCH, next_places);
+                else copies_commit();
+                const float alpha = weigh(p_s + m_row * P_PITCH + m_key, at);
+                if ((tid & 3) == 0) keep_s[m_row] = alpha;
+                copies_wait<1>();
+                __syncthreads();                         // the weights and the values are there
+                const bool masked = some_unseen(at);
+                if (o_row < rows) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float alpha = keep_s[o_row + i];
+#pragma unroll
+                        for (int c = 0; c < COLS; ++c) o[i][c] *= alpha;
+                    }
+                    auto keys = [&](auto skip) {
+#pragma unroll 2
+                        for (int j = 0; j < KEYS; j += 4) {
+                            float w[4][4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(p_s + (o_row + i) * P_PITCH + j);
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                                for (int c = 0; c < COLS; c += 4) {
+                                    float y[4];
+                                    *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(v_s + (j + u) * D + o_col + 16 * c);
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                                        for (int b = 0; b < 4; ++b)
+                                            if (!decltype(skip)::value || w[i][u] != 0.0f) o[i][c + b] = fmaf(w[i][u], y[b], o[i][c + b]);
+                                }
+                        }
+                    };
+                    if (masked) keys(std::true_type{});
+                    else keys(std::false_type{});
+                }
+                if (!SPLIT && (at + KEYS >= end || (at + KEYS) % CHUNK == 0)) join_chunk();
+                if (tid < KEYS) place_s[(block & 1) * KEYS + tid] = later;
+                __syncthreads();                         // values, weights and factors have been read
+                if (more) fetch(block_rows, A.v, v_s, D, next_places);
+                else copies_commit();
+            }
         }
         copies_wait<0>();
         auto row_of = [&](int r) { return (size_t)(t0 + r / group) * A.nq + g * group + r % group; };
@@ -360,14 +445,25 @@ __global__ void attention_f32_join_kernel(const Args A) {
     const int first = min((A.window > 0 ? max(0, pos + 1 - A.window) : 0) / CHUNK, A.chunks - 1), last = min(pos / CHUNK, A.chunks - 1);
     const float* ml = A.part_ml + 2 * row * A.chunks;
     float m_all = -CUDART_INF_F, l_all = 0.0f, total[8] = {};
-    for (int c = first; c <= last; ++c) {
-        const float m = ml[2 * c], next = fmaxf(m_all, m), keep = m_all == next ? 1.0f : ratio(m_all, next), take = ratio(m, next);
-        l_all = join(l_all, keep, ml[2 * c + 1], take);
-        m_all = next;
-        const float* o = A.part_o + (row * A.chunks + c) * A.d;
+    constexpr int BATCH = 4;                             // chunks whose parts are loaded together
+    for (int c0 = first; c0 <= last; c0 += BATCH) {
+        float m[BATCH], l[BATCH], o[BATCH][8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (lane + 32 * i < A.d) total[i] = join(total[i], keep, o[lane + 32 * i], take);
+        for (int b = 0; b < BATCH; ++b) {
+            const int c = min(c0 + b, last);
+            m[b] = ml[2 * c], l[b] = ml[2 * c + 1];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[b][i] = lane + 32 * i < A.d ? A.part_o[(row * A.chunks + c) * A.d + lane + 32 * i] : 0.0f;
+        }
+#pragma unroll
+        for (int b = 0; b < BATCH; ++b) {
+            if (c0 + b > last) break;
+            const float next = fmaxf(m_all, m[b]), keep = m_all == next ? 1.0f : ratio(m_all, next), take = ratio(m[b], next);
+            l_all = join(l_all, keep, l[b], take);
+            m_all = next;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) total[i] = join(total[i], keep, o[b][i], take);
+        }
     }
     const float inv = 1.0f / l_all;
 #pragma unroll
@@ -377,7 +473,7 @@ __global__ void attention_f32_join_kernel(const Args A) {
 
 template <int D, bool SPLIT>
 int launch(const Args& A, int tiles, void* stream) {
-    constexpr int SMEM = (smem_floats<D>() + (SPLIT ? 0 : THREADS * D / 4)) * (int)sizeof(float);
+    constexpr int SMEM = smem_floats<D, SPLIT>() * (int)sizeof(float);
     static PerDevice configured;
     if (!configured.get()) {
         const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<D, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);

@@ -244,7 +244,7 @@ def silu_mul(gate_up: torch.Tensor, out: torch.Tensor, block: int = 0) -> None:
                                   _stream()), "silu_mul")
 
 
-ATTENTION_F32_PARTS_BYTES = 64 << 20       # scratch up to which the chunks of a row's keys get blocks of their own
+ATTENTION_F32_PARTS_BYTES = 128 << 20      # scratch up to which the chunks of a row's keys get blocks of their own
 
 
 def attention_simt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, positions: torch.Tensor,

@@ -424,6 +424,18 @@ def test_attention_f32_gives_a_row_the_same_bits_in_every_cut(monkeypatch, nq, n
             assert torch.equal(out[row - rows.start], got[row]), (row, rows)
 
 
+@pytest.mark.parametrize("nq,nkv,d,page,window", [(2, 1, 128, 16, 0), (8, 1, 64, 4, 0), (3, 3, 256, 1, 0), (6, 2, 40, 16, 90), (1, 1, 128, 64, 33)])
+def test_attention_f32_single_tokens_at_the_edges_of_steps(monkeypatch, nq, nkv, d, page, window):
+    """One to eight rows a tile: contexts around a block of 32 keys, a step of 64 and a chunk of 256, windows that begin inside
+    them; chunks in blocks of their own and in one walk give the same bits, and those of the rows inside a prompt."""
+    spans = [(p, 1) for p in (0, 30, 31, 32, 62, 63, 64, 95, 96, 254, 255, 256, 287, 320, 511, 512, 700)]
+    case = PagedCase(torch.float32, nq, nkv, d, page, spans, seed=d + window, window=window)
+    got = case.run_simt()
+    close(got, case.plain(), torch.float32, "attention_f32")
+    monkeypatch.setattr(kernels, "ATTENTION_F32_PARTS_BYTES", 0)
+    assert torch.equal(got, case.run_simt())
+
+
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_attention_window_edges(window):
     for dtype in DTYPES:

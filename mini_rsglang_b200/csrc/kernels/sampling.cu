@@ -120,12 +120,14 @@ MRS_EXPORT int mrs_argmax(const float* logits, int* out, int rows, int vocab, vo
 // ------------------------------------------------------------------------------------------------
 // Sampling.  A row belongs to a thread-block cluster (1, 4 or 8 CTAs): every CTA brings its share of the row into shared
 // memory once, and everything after that (largest logit, the two thresholds, the draw) reads it there; the CTAs meet
-// through distributed shared memory.  What bounds it is the chain of those meetings: a row is read once (608 KB at
-// 151,936 logits), a threshold takes three digits of 11, 11 and 10 bits with two cluster barriers each.  One CTA a row,
-// which read the row from L2 some fifteen times with 8-bit digits, took 1,626 us for 24 rows of 151,936 logits (top-k and
-// top-p rows among them); a cluster with weights added as floats and one warp that walked the drawn segment took 87 us.  With weights
-// as whole numbers, all warps at the segment and counts only in the digits that need them, 24 rows with top-k and top-p take 68 us,
-// with top-p alone 69, top-k alone 35, temperature alone 23, greedy 8 (one row: 47, 48, 25, 17, 6).
+// through distributed shared memory.  A threshold that at most SAMPLE_LIST candidates decide takes one histogram of the cluster and
+// a sort in every CTA; others (more equals at the edge, temperatures that crowd a row into one bin, rows read from memory) take three
+// digits of 11, 11 and 10 bits with two meetings each.  What bounds it is the chain: of some 60,000 clocks of a row with top-p the
+// largest logit takes 8,000, the weights' histogram 14,000 (an exponential and two or three additions in shared memory an element), its
+// meetings and scan 9,000, the candidates 12,000, the draw 15,000.
+// Rows of 151,936 logits, three digits always and now: 24 with top-p 69 -> 50 us, top-k and top-p 68 -> 36, top-k 35 -> 34, temperature
+// alone 23 -> 24; one row 48 -> 31, 47 -> 27, 25 -> 23, 17 -> 16; 24 of 32,768 with top-p 47 -> 27.  (One CTA a row, which read it
+// from L2 some fifteen times with 8-bit digits, took 1,626 us for 24 rows.)
 //
 // The weights of the kept set are summed in 32 segments of a row, in id order, whatever the cluster's size: a row's token
 // does not depend on how many CTAs shared it.
@@ -167,7 +169,9 @@ struct SampleShared {
     int bad;
     // This CTA's histogram.  By count it is `high`; by weight it is the three parts, which give their place (`high` and `mid`) to the
     // words of a float64 when the walk is over; the last digit, of half as many bins, also counts, in the upper half of `high`.
-    unsigned high[SAMPLE_BINS], mid[SAMPLE_BINS], low[SAMPLE_BINS];
+    alignas(16) unsigned high[SAMPLE_BINS];
+    alignas(16) unsigned mid[SAMPLE_BINS];
+    alignas(16) unsigned low[SAMPLE_BINS];
     unsigned slice_count[SAMPLE_BINS / 4];           // this CTA's slice of the bins, summed over the cluster
     double slice_weight[SAMPLE_BINS / 4];
     int seg_ties[SAMPLE_SEGMENTS];                   // this CTA's segments
@@ -179,6 +183,10 @@ struct SampleShared {
     double above_weight;
     int all_ties[SAMPLE_SEGMENTS];
     float all_weight[SAMPLE_SEGMENTS];
+    float temperature, top_p;                        // of the row
+    int top_k, draw_index;
+    unsigned long long seed;
+    unsigned listed;                                 // of this CTA's candidates (in `high`); read by the whole cluster
 };
 
 // What the digit search knows: keys that match `prefix` under `mask` hold the edge, `above` of them (by count or weight)
@@ -349,13 +357,149 @@ __device__ void sample_digit(cg::cluster_group& cluster, SampleShared& s, unsign
     // the histogram is written again after the next barrier of the cluster's first kind: every CTA has read its slices by then
 }
 
+// Candidates of a threshold.  Elements are binned by how many 64ths of a (natural) logarithm their weight lies below the largest: a
+// function that never rises with the key, and that spreads a row over some hundred bins where the keys' first 11 bits (sign, exponent
+// and two bits) crowd it into some ten.  What the edge's bin holds (by count: all bins down to it) is then few enough to be sorted in
+// every CTA, which finds the threshold without another meeting of the cluster.
+#define SAMPLE_LIST 1024
+__device__ __forceinline__ float log_steps(float v, float top, float inv_t) { return (top - v) * inv_t * 64.0f; }
+__device__ __forceinline__ unsigned log_bin(float v, float top, float inv_t) { return (unsigned)fminf(log_steps(v, top, inv_t), (float)(SAMPLE_BINS - 1)); }
+
+// f(index, value) for this CTA's elements, in shared memory on a 16-byte boundary, four at a time
+template <typename F>
+__device__ __forceinline__ void each_shared(const float* x, int length, F f) {
+#pragma unroll 2
+    for (int i = threadIdx.x; i < length / 4; i += SAMPLE_CTA_THREADS) {
+        const float4 v = reinterpret_cast<const float4*>(x)[i];
+        f(4 * i, v.x), f(4 * i + 1, v.y), f(4 * i + 2, v.z), f(4 * i + 3, v.w);
+    }
+    const int i = (length & ~3) + threadIdx.x;
+    if (i < length) f(i, x[i]);
+}
+
+// Gathers the keys for which `wanted(v)` holds from all CTAs and sorts them, largest first, into candidates(s): their count, or -1 if
+// they are more than SAMPLE_LIST.  Every CTA gets the same.  The CTA's own go through s.high, all of them through s.mid.
+__device__ __forceinline__ unsigned* candidates(SampleShared& s) { return s.mid + SAMPLE_LIST; }
+template <typename Wanted>
+__device__ int sample_candidates(cg::cluster_group& cluster, SampleShared& s, unsigned blocks, const float* x, int length, Wanted wanted) {
+    if (threadIdx.x == 0) s.listed = 0u;
+    __syncthreads();
+    each_shared(x, length, [&](int, float v) {
+        if (!wanted(v)) return;
+        const unsigned at = atomicAdd(&s.listed, 1u);
+        if (at < SAMPLE_LIST) s.high[at] = ordered_key(v);
+    });
+    if (blocks > 1) cluster.sync();
+    else __syncthreads();
+    constexpr int TEAM = SAMPLE_CTA_THREADS / SAMPLE_MAX_BLOCKS;          // threads that bring a CTA's
+    const unsigned team = threadIdx.x / TEAM;
+    unsigned n = 0u, from = 0u, count = 0u;
+#pragma unroll
+    for (unsigned r = 0; r < SAMPLE_MAX_BLOCKS; ++r) {
+        const unsigned c = r < blocks ? *cluster.map_shared_rank(&s.listed, r) : 0u;
+        if (r < team) from += c;
+        if (r == team) count = c;
+        n += c;
+    }
+    if (n > SAMPLE_LIST) return -1;
+    if (count > 0u) {
+        const unsigned* list = cluster.map_shared_rank(s.high, team);
+        for (unsigned i = threadIdx.x % TEAM; i < count; i += TEAM) s.mid[from + i] = list[i];
+    }
+    if (threadIdx.x < (n + 3u) / 4u * 4u - n) s.mid[n + threadIdx.x] = 0u;      // no finite float's key
+    __syncthreads();
+    // a key's place: how many are larger, or equal and before it; of keys before those of its warp, how many are larger than key - 1
+    for (unsigned i = threadIdx.x; i < n; i += SAMPLE_CTA_THREADS) {
+        const unsigned key = s.mid[i], base = i & ~31u;
+        unsigned place = 0u;
+        auto larger = [&](unsigned from, unsigned to, unsigned than) {
+#pragma unroll 4
+            for (unsigned j = from; j < to; j += 4) {
+                const uint4 k = *reinterpret_cast<const uint4*>(s.mid + j);
+                place += (unsigned)(k.x > than) + (unsigned)(k.y > than) + (unsigned)(k.z > than) + (unsigned)(k.w > than);
+            }
+        };
+        larger(0u, base, key - 1u);
+        for (unsigned j = base; j < min(base + 32u, n); ++j) place += (unsigned)(s.mid[j] > key || (s.mid[j] == key && j < i));
+        larger(base + 32u, n, key);
+        candidates(s)[place] = key;
+    }
+    __syncthreads();
+    return (int)n;
+}
+
+// The first of `n` sorted candidates at which their running weight reaches `goal` (where rounding left the sum a hair short: the last
+// that has a weight).  key, the weight of the candidates above it and the count of its equals (among all `listed`).
+struct Reached {
+    unsigned key;
+    int equals;
+    double above;
+};
+__device__ __forceinline__ unsigned long long fixed_units(float w) {
+    const Fixed f = fixed_weight(w);
+    return ((unsigned long long)f.high << 32) + ((unsigned long long)f.mid << 16) + f.low;
+}
+// Running sums of the candidates' weights in units of 2^-48 (whole numbers), in place of what `sums` held; their total.
+template <typename Weight>
+__device__ unsigned long long sample_running(SampleShared& s, int n, Weight weight_of_key, unsigned long long* sums) {
+    constexpr int OWN = SAMPLE_LIST / SAMPLE_CTA_THREADS;
+    unsigned long long* warps = reinterpret_cast<unsigned long long*>(s.warp_weight);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long own[OWN], run = 0ull;
+#pragma unroll
+    for (int j = 0; j < OWN; ++j) {
+        const int i = threadIdx.x * OWN + j;
+        run += i < n ? fixed_units(weight_of_key(candidates(s)[i])) : 0ull;
+        own[j] = run;
+    }
+    unsigned long long before = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long up = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += up;
+    }
+    if (lane == 31) warps[warp] = before;
+    before -= run;
+    __syncthreads();
+    unsigned long long total = 0ull;
+    for (int i = 0; i < SAMPLE_CTA_WARPS; ++i) {
+        if (i < warp) before += warps[i];
+        total += warps[i];
+    }
+#pragma unroll
+    for (int j = 0; j < OWN; ++j) sums[threadIdx.x * OWN + j] = before + own[j];
+    if (threadIdx.x == 0) s.first = 0x7fffffff, s.lowest = -1;
+    __syncthreads();
+    return total;
+}
+__device__ Reached sample_reached(SampleShared& s, int n, int listed, const unsigned long long* sums, double goal) {
+    constexpr double UNIT = 1.0 / 281474976710656.0;
+    for (int i = threadIdx.x; i < n; i += SAMPLE_CTA_THREADS) {
+        const unsigned long long below = i > 0 ? sums[i - 1] : 0ull;
+        if (sums[i] == below) continue;
+        atomicMax(&s.lowest, i);
+        if ((double)sums[i] * UNIT >= goal && !(i > 0 && (double)below * UNIT >= goal)) atomicMin(&s.first, i);
+    }
+    __syncthreads();
+    const int place = s.first != 0x7fffffff ? s.first : max(s.lowest, 0);
+    const unsigned* list = candidates(s);
+    const unsigned key = list[place];
+    int above = 0, equals = 0;
+    for (int base = 0; base < listed; base += SAMPLE_CTA_THREADS) {
+        const int i = base + threadIdx.x;
+        above += __syncthreads_count(i < listed && list[i] > key);
+        equals += __syncthreads_count(i < listed && list[i] == key);
+    }
+    return Reached{key, equals, above > 0 ? (double)sums[above - 1] * UNIT : 0.0};
+}
+
 // IN_SHARED: the CTA's share of the row lies in shared memory (and gives its place to the weights of the kept set);
 // otherwise a row is too long for that and is read from memory each time.
 template <bool IN_SHARED>
 __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     const float* __restrict__ logits, int vocab, int per_segment, const float* __restrict__ temperature,
     const int* __restrict__ top_k, const float* __restrict__ top_p, const unsigned long long* __restrict__ seed,
-    const int* __restrict__ draw_index, int* __restrict__ out) {
+    const int* __restrict__ draw_index, int* __restrict__ out, int* __restrict__ copy) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float share[];
@@ -368,10 +512,15 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     const int begin = min(vocab, (int)rank * own_segments * per_segment);
     const int length = min(vocab, begin + own_segments * per_segment) - begin;      // of this CTA's share
     const float* row = logits + (size_t)r * vocab + begin;
-    const float temp = temperature[r];
-    const int k_raw = top_k[r];
-    const float p_raw = top_p[r];
-
+    // one thread asks for the parameters, beside the logits: they may lie in the host's memory, where every access goes its own way
+    if (threadIdx.x == SAMPLE_CTA_THREADS - 1) {
+        s.temperature = temperature[r], s.top_k = top_k[r], s.top_p = top_p[r];
+        s.seed = seed[r], s.draw_index = draw_index[r];
+    }
+    auto answer = [&](int token) {
+        out[r] = token;
+        if (copy) copy[r] = token;
+    };
     // Largest logit (also the greedy answer) and a check that the row is finite.
     int bad = 0;
     Best mine = {-CUDART_INF_F, 0x7fffffff};
@@ -382,7 +531,7 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     int vectors = 0;
     if (((uintptr_t)row & 15) == 0) {
         vectors = length / 4;
-#pragma unroll 4
+#pragma unroll 5
         for (int i = threadIdx.x; i < vectors; i += SAMPLE_CTA_THREADS) {
             const float4 v = reinterpret_cast<const float4*>(row)[i];
             if (IN_SHARED) reinterpret_cast<float4*>(share)[i] = v;
@@ -407,10 +556,12 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
         top = better(top, *cluster.map_shared_rank(&s.best, q));
         bad |= *cluster.map_shared_rank(&s.bad, q);
     }
+    const float temp = s.temperature, p_raw = s.top_p;
+    const int k_raw = s.top_k;
     // the same in every CTA of the cluster: they leave together, and none while another still reads its shared memory
     const float inv_t = 1.0f / temp;                 // beyond a float's range: as temperature 0
     if (bad || temp == 0.0f || k_raw == 1 || isinf(inv_t)) {
-        if (rank == 0 && threadIdx.x == 0) out[r] = bad ? -1 : top.id;
+        if (rank == 0 && threadIdx.x == 0) answer(bad ? -1 : top.id);
         if (blocks > 1) cluster.sync();
         return;
     }
@@ -421,7 +572,74 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     // Kept are the keys from cut.low on; of those equal to it, where there are more than `quota`, the first ids.
     Cut cut = {0u, 0x7fffffff};
     int ties = 0;                                    // elements of the row whose key is cut.low, where some of them may be left out
-    if (k_raw > 0 && k_raw < vocab) {
+    const bool by_count = k_raw > 0 && k_raw < vocab;
+    // how many equals of weight `one` it takes from `above` to `target`; a weight of nothing: all of them
+    auto equals_to = [](double target, double above, double one) {
+        const double missing = (target - above) / one;
+        return missing < 2147483647.0 ? max(1, (int)ceil(missing)) : 0x7fffffff;
+    };
+    bool found = false;                              // both thresholds, from candidates
+    if (IN_SHARED && (by_count ? k_raw <= SAMPLE_LIST : p_raw < 1.0f)) {
+        Edge e = {0u, 0u, 0u, 0u, 0.0, 0.0};
+        auto each = [&](int, auto add) {
+            each_shared(x, length, [&](int, float v) { add((SAMPLE_BINS - 1 - log_bin(v, top.value, inv_t)) << 21, [&] { return weight_of(v); }); });
+        };
+        unsigned long long* sums = reinterpret_cast<unsigned long long*>(s.low);
+        static_assert(sizeof(s.low) >= SAMPLE_LIST * sizeof(*sums), "running sums of the candidates");
+        auto weight_of_key = [&](unsigned key) { return weight_of(key_value(key)); };
+        if (by_count) {
+            sample_digit<false, 11>(cluster, s, rank, blocks, 21, e, each, 1, 0.0f, (unsigned)k_raw, false, 0u, 0.0);
+            const unsigned edge = SAMPLE_BINS - 1 - (e.prefix >> 21);
+            const float end = (float)(edge + 1u);
+            const int n = edge + 1u < SAMPLE_BINS && e.above_count + e.count <= SAMPLE_LIST        // the last bin's end is open
+                ? sample_candidates(cluster, s, blocks, x, length, [&](float v) { return log_steps(v, top.value, inv_t) < end; }) : -1;
+            if (n >= 0) {
+                found = true;
+                const unsigned* list = candidates(s);
+                cut.low = list[k_raw - 1];
+                int above = 0;
+                for (int base = 0; base < n; base += SAMPLE_CTA_THREADS) {
+                    const int i = base + threadIdx.x;
+                    above += __syncthreads_count(i < n && list[i] > cut.low);
+                    ties += __syncthreads_count(i < n && list[i] == cut.low);
+                }
+                cut.quota = k_raw - above;
+                if (p_raw < 1.0f) {
+                    const double total = (double)sample_running(s, k_raw, weight_of_key, sums) * (1.0 / 281474976710656.0);
+                    const double target = (double)(p_raw * (float)total);
+                    const Reached at = sample_reached(s, k_raw, n, sums, target);
+                    const int need = equals_to(target, at.above, (double)fixed_units(weight_of_key(at.key)) * (1.0 / 281474976710656.0));
+                    if (at.key == cut.low) {
+                        cut.quota = min(cut.quota, need);
+                    } else {
+                        cut.low = at.key;
+                        cut.quota = need;
+                        ties = at.equals;
+                    }
+                }
+            }
+        } else {
+            sample_digit<true, 11>(cluster, s, rank, blocks, 21, e, each, 1, p_raw, 0u, false, 0u, 0.0);
+            const unsigned edge = SAMPLE_BINS - 1 - (e.prefix >> 21);
+            const float start = (float)edge, end = (float)(edge + 1u);
+            const int n = edge + 1u < SAMPLE_BINS
+                ? sample_candidates(cluster, s, blocks, x, length,
+                                    [&](float v) { const float at = log_steps(v, top.value, inv_t); return at >= start && at < end; }) : -1;
+            if (n >= 0) {
+                found = true;
+                sample_running(s, n, weight_of_key, sums);
+                const Reached at = sample_reached(s, n, n, sums, e.target - e.above_weight);
+                cut.low = at.key;
+                cut.quota = equals_to(e.target, e.above_weight + at.above, (double)fixed_units(weight_of_key(at.key)) * (1.0 / 281474976710656.0));
+                ties = at.equals;
+            }
+        }
+        if (!found) {                                // the digits' histograms take the lists' place: no CTA reads them any more
+            if (blocks > 1) cluster.sync();
+            else __syncthreads();
+        }
+    }
+    if (!found && by_count) {
         Edge e = {0u, 0u, 0u, 0u, 0.0, 0.0};
         auto each = [&](int, auto add) {
 #pragma unroll 4
@@ -440,7 +658,7 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     }
 
     // ---- top_p: the key at which the running weight reaches top_p times the top_k set's weight ---
-    if (p_raw < 1.0f) {
+    if (!found && p_raw < 1.0f) {
         Edge e = {0u, 0u, 0u, 0u, 0.0, 0.0};
         auto counted = [&](float w) {                // a weight as the histograms count it
             const Fixed f = fixed_weight(w);
@@ -463,8 +681,7 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
         sample_digit<true, 11>(cluster, s, rank, blocks, 10, e, each, pieces, p_raw, 0u, some, low, low_weight);
         sample_digit<true, 10>(cluster, s, rank, blocks, 0, e, each, pieces, p_raw, 0u, some, low, low_weight);
         const double one = counted(weight_of(key_value(e.prefix)));
-        const double missing = (e.target - e.above_weight) / one;
-        const int need = missing < 2147483647.0 ? max(1, (int)ceil(missing)) : 0x7fffffff;        // a weight of nothing: all its equals
+        const int need = equals_to(e.target, e.above_weight, one);
         if (some && e.prefix == cut.low) {
             cut.quota = min(cut.quota, need);
         } else {
@@ -520,11 +737,7 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
             for (int g = warp; g < own_segments; g += SAMPLE_CTA_WARPS)
                 walk(g, [&](int i, bool live, float w) { if (live) share[i] = w; });
         } else {
-#pragma unroll 4
-            for (int i = threadIdx.x; i < length; i += SAMPLE_CTA_THREADS) {
-                const float v = share[i];
-                share[i] = ordered_key(v) >= cut.low ? weight_of(v) : SAMPLE_NOT_KEPT;
-            }
+            each_shared(share, length, [&](int i, float v) { share[i] = ordered_key(v) >= cut.low ? weight_of(v) : SAMPLE_NOT_KEPT; });
         }
         __syncthreads();
     }
@@ -549,20 +762,26 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     else __syncthreads();
 
     // ---- inverse CDF over the kept set in id order ------------------------------------------------
-    float retained = 0.0f;
-    for (int g = 0; g < SAMPLE_SEGMENTS; ++g) retained += s.all_weight[g];
-    const float u = uniform_from_counter(seed[r], (unsigned long long)draw_index[r]) * retained;
-    float run = 0.0f;
+    float of_segment[SAMPLE_SEGMENTS], retained = 0.0f;
+#pragma unroll
+    for (int g = 0; g < SAMPLE_SEGMENTS; ++g) of_segment[g] = s.all_weight[g];
+#pragma unroll
+    for (int g = 0; g < SAMPLE_SEGMENTS; ++g) retained += of_segment[g];
+    const float u = uniform_from_counter(s.seed, (unsigned long long)s.draw_index) * retained;
+    float run = 0.0f, before_last = 0.0f;
     int chosen = -1, last = 0;
+#pragma unroll
     for (int g = 0; g < SAMPLE_SEGMENTS; ++g) {
-        if (s.all_weight[g] <= 0.0f) continue;
+        if (chosen >= 0 || of_segment[g] <= 0.0f) continue;
+        const float with = run + of_segment[g];
         last = g;
-        if (run + s.all_weight[g] > u) { chosen = g; break; }
-        run += s.all_weight[g];
+        before_last = with - of_segment[g];
+        if (with > u) chosen = g;
+        else run = with;
     }
     if (chosen < 0) {
         chosen = last;
-        run -= s.all_weight[last];
+        run = before_last;
     }
     if (chosen / own_segments != (int)rank) return;
     chosen %= own_segments;
@@ -606,7 +825,7 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
         const int g = group >= 0 ? group : last_group, i = from + 32 * g + lane;
         const float w = i < to ? share[i] : SAMPLE_NOT_KEPT, cum = scan(w);
         const unsigned hit = __ballot_sync(0xffffffffu, w >= 0.0f && run + cum > u), kept = __ballot_sync(0xffffffffu, w >= 0.0f);
-        if (lane == 0) out[r] = begin + from + 32 * g + (group >= 0 ? __ffs(hit) - 1 : 31 - __clz(kept));
+        if (lane == 0) answer(begin + from + 32 * g + (group >= 0 ? __ffs(hit) - 1 : 31 - __clz(kept)));
     } else {
         if (warp != 0) return;
         int picked = -1, last_kept = -1;
@@ -617,15 +836,16 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
             if (kept) last_kept = begin + i - lane + (31 - __clz(kept));
             run += __shfl_sync(0xffffffffu, cum, 31);
         });
-        if (lane == 0) out[r] = picked >= 0 ? picked : last_kept;
+        if (lane == 0) answer(picked >= 0 ? picked : last_kept);
     }
 }
 
 // temperature, top_k (<= 0: off), top_p, seed and draw_index are per row.
-// out[r] = the token, or -1 when the row holds a NaN or an infinity.
+// out[r] = the token, or -1 when the row holds a NaN or an infinity; the same to copy[r], where that is not null.  The parameters and
+// `copy` may lie in pinned host memory: a row's are read beside its logits, which hides the way.
 MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float* temperature, const int* top_k,
                           const float* top_p, const unsigned long long* seed, const int* draw_index, int* out,
-                          void* stream) {
+                          int* copy, void* stream) {
     if (rows <= 0) return 0;
     if (vocab <= 0) return MRS_BAD_ARGUMENT;
     const int per_segment = (int)((((long long)vocab + SAMPLE_SEGMENTS - 1) / SAMPLE_SEGMENTS + 31) & ~31LL);
@@ -653,8 +873,8 @@ MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float*
     static const bool plain = getenv("MRS_PLAIN_LAUNCH") != nullptr;
     config.attrs = attributes;
     config.numAttrs = plain ? 1 : 2;
-    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out)
-                                    : cudaLaunchKernelEx(&config, sample_kernel<false>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out);
+    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out, copy)
+                                    : cudaLaunchKernelEx(&config, sample_kernel<false>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out, copy);
     if (e != cudaSuccess) return (int)e;
     MRS_RETURN_LAUNCH_STATUS();
 }

@@ -1015,6 +1015,46 @@ def test_sampler_rows_that_several_ctas_share(vocab):
     assert sampler.sample(logits.to(DEV), params, list(range(21))) == got          # whole numbers and fixed orders: the same bits
 
 
+@pytest.mark.parametrize("vocab", [4000, 20000, 70000])
+@pytest.mark.parametrize("bunch", [1, 1000, 1023, 1024, 1025, 3000])
+def test_sampler_candidates_up_to_their_limit(vocab, bunch):
+    """Thresholds inside a bunch of `bunch` logits that lie within a 64th of a logarithm (half of them equal): as many candidates as
+    are sorted at once, and more; temperatures that put every logit into one bin, or nearly all behind the last."""
+    g = torch.Generator().manual_seed(vocab + bunch)
+    row = torch.randn(vocab, generator=g) * 2 - 9.0
+    at = torch.randperm(vocab, generator=g)
+    row[at[:20]] = 8.0 - 0.1 * torch.arange(20)
+    row[at[20:20 + bunch]] = 4.0001 + 0.01 * torch.rand(bunch, generator=g)
+    row[at[20:20 + bunch // 2]] = 4.005
+    settings = [SamplingParams(temperature=1.0, top_k=20 + k, seed=k) for k in {1, bunch // 3, bunch - 1, bunch} if k > 0]
+    settings += [SamplingParams(temperature=1.0, top_k=min(20 + bunch, 1000), top_p=p, seed=3) for p in (0.5, 0.97, 0.999)]
+    settings += [SamplingParams(temperature=1.0, top_p=p, seed=5) for p in (0.4, 0.93, 0.999)]
+    settings += [SamplingParams(temperature=t, top_k=k, top_p=0.9, seed=7) for t in (1e-3, 300.0) for k in (None, 3, 40)]
+    params = [p for p in settings for _ in range(3)]
+    got = Sampler(torch.device(DEV)).sample(row.expand(len(params), vocab).contiguous().to(DEV), params, list(range(len(params))))
+    wrong = sum(not drawn(row.double(), p, i, token, 1e-5) for i, (p, token) in enumerate(zip(params, got)))
+    assert wrong <= 1, wrong
+
+
+def test_sampler_launches_that_are_outstanding():
+    """Launches behind one another, with more rows each and on streams of their own, before any is read; a sampler that goes while its
+    last launch is under way."""
+    logits = torch.randn(400, 9000, device=DEV) * 2
+    sampler, held = Sampler(torch.device(DEV)), []
+    params = [SamplingParams(temperature=1.0, top_k=1 + i % 40, seed=i) for i in range(400)]
+    torch.cuda.synchronize()
+    for n in (3, 100, 400):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            held.append((n, sampler.launch(logits[:n].contiguous(), params[:n], list(range(n)))))
+    got = [sampler.read(chosen) for _, chosen in held]
+    last = sampler.launch(logits, params, list(range(400)))
+    del sampler
+    want = Sampler(torch.device(DEV)).sample(logits, params, list(range(400)))
+    assert all(tokens == want[:n] and chosen.tokens.tolist() == tokens for (n, chosen), tokens in zip(held, got))
+    assert last.host.tolist() == want
+
+
 def drawn(row, p, index, token, tolerance) -> bool:
     """Whether `token` is the draw restated in float64: the support by a stable sort, then the inverse CDF in id order.  A token that is
     not has to be one that float32 sums may give instead: u within `tolerance` of the kept weight of that token's own interval, and the

@@ -12,6 +12,8 @@
 // request's tokens do not depend on what else is in the batch.
 #include "common.cuh"
 #include <cooperative_groups.h>
+
+#include <cstring>
 namespace cg = cooperative_groups;
 
 #define ARGMAX_THREADS 1024
@@ -183,9 +185,6 @@ struct SampleShared {
     double above_weight;
     int all_ties[SAMPLE_SEGMENTS];
     float all_weight[SAMPLE_SEGMENTS];
-    float temperature, top_p;                        // of the row
-    int top_k, draw_index;
-    unsigned long long seed;
     unsigned listed;                                 // of this CTA's candidates (in `high`); read by the whole cluster
 };
 
@@ -493,13 +492,30 @@ __device__ Reached sample_reached(SampleShared& s, int n, int listed, const unsi
     return Reached{key, equals, above > 0 ? (double)sums[above - 1] * UNIT : 0.0};
 }
 
+// The rows' parameters: arrays on the device, or (what the host has just made) up to ROWS of them in the launch itself: reading them
+// from pinned memory takes a row 10 us (24 rows 57 instead of 45), a copy to the device a launch.
+struct SampleArrays {
+    const float* temperature;
+    const int* top_k;
+    const float* top_p;
+    const unsigned long long* seed;
+    const int* draw_index;
+};
+template <int ROWS>
+struct SampleWords {
+    unsigned long long seed[ROWS];
+    float temperature[ROWS];
+    int top_k[ROWS];
+    float top_p[ROWS];
+    int draw_index[ROWS];
+};
+
 // IN_SHARED: the CTA's share of the row lies in shared memory (and gives its place to the weights of the kept set);
 // otherwise a row is too long for that and is read from memory each time.
-template <bool IN_SHARED>
+template <bool IN_SHARED, typename Params>
 __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
-    const float* __restrict__ logits, int vocab, int per_segment, const float* __restrict__ temperature,
-    const int* __restrict__ top_k, const float* __restrict__ top_p, const unsigned long long* __restrict__ seed,
-    const int* __restrict__ draw_index, int* __restrict__ out, int* __restrict__ copy) {
+    const float* __restrict__ logits, int vocab, int per_segment, const __grid_constant__ Params params, int* __restrict__ out,
+    int* __restrict__ copy) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float share[];
@@ -512,11 +528,9 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     const int begin = min(vocab, (int)rank * own_segments * per_segment);
     const int length = min(vocab, begin + own_segments * per_segment) - begin;      // of this CTA's share
     const float* row = logits + (size_t)r * vocab + begin;
-    // one thread asks for the parameters, beside the logits: they may lie in the host's memory, where every access goes its own way
-    if (threadIdx.x == SAMPLE_CTA_THREADS - 1) {
-        s.temperature = temperature[r], s.top_k = top_k[r], s.top_p = top_p[r];
-        s.seed = seed[r], s.draw_index = draw_index[r];
-    }
+    const float temp = params.temperature[r], p_raw = params.top_p[r];
+    const int k_raw = params.top_k[r];
+
     auto answer = [&](int token) {
         out[r] = token;
         if (copy) copy[r] = token;
@@ -556,8 +570,6 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
         top = better(top, *cluster.map_shared_rank(&s.best, q));
         bad |= *cluster.map_shared_rank(&s.bad, q);
     }
-    const float temp = s.temperature, p_raw = s.top_p;
-    const int k_raw = s.top_k;
     // the same in every CTA of the cluster: they leave together, and none while another still reads its shared memory
     const float inv_t = 1.0f / temp;                 // beyond a float's range: as temperature 0
     if (bad || temp == 0.0f || k_raw == 1 || isinf(inv_t)) {
@@ -767,7 +779,7 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     for (int g = 0; g < SAMPLE_SEGMENTS; ++g) of_segment[g] = s.all_weight[g];
 #pragma unroll
     for (int g = 0; g < SAMPLE_SEGMENTS; ++g) retained += of_segment[g];
-    const float u = uniform_from_counter(s.seed, (unsigned long long)s.draw_index) * retained;
+    const float u = uniform_from_counter(params.seed[r], (unsigned long long)params.draw_index[r]) * retained;
     float run = 0.0f, before_last = 0.0f;
     int chosen = -1, last = 0;
 #pragma unroll
@@ -840,23 +852,16 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     }
 }
 
-// temperature, top_k (<= 0: off), top_p, seed and draw_index are per row.
-// out[r] = the token, or -1 when the row holds a NaN or an infinity; the same to copy[r], where that is not null.  The parameters and
-// `copy` may lie in pinned host memory: a row's are read beside its logits, which hides the way.
-MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float* temperature, const int* top_k,
-                          const float* top_p, const unsigned long long* seed, const int* draw_index, int* out,
-                          int* copy, void* stream) {
-    if (rows <= 0) return 0;
-    if (vocab <= 0) return MRS_BAD_ARGUMENT;
+template <typename Params>
+static int launch_sample(const float* logits, int rows, int vocab, const Params& params, int* out, int* copy, void* stream) {
     const int per_segment = (int)((((long long)vocab + SAMPLE_SEGMENTS - 1) / SAMPLE_SEGMENTS + 31) & ~31LL);
     // short rows gain nothing from more CTAs: their meetings cost more than the walks
     const int blocks = vocab >= 65536 ? 8 : (vocab >= 8192 ? 4 : 1);
-    if (rows > 0x7fffffff / 8) return MRS_BAD_ARGUMENT;
     const size_t share = (size_t)per_segment * (SAMPLE_SEGMENTS / blocks) * sizeof(float);
     const bool in_shared = share <= SAMPLE_SHARE_BYTES;
     static PerDevice configured;
     if (!configured.get()) {
-        const cudaError_t e = cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SHARE_BYTES);
+        const cudaError_t e = cudaFuncSetAttribute(sample_kernel<true, Params>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SHARE_BYTES);
         if (e != cudaSuccess) return (int)e;
         configured.set(1);
     }
@@ -873,8 +878,46 @@ MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float*
     static const bool plain = getenv("MRS_PLAIN_LAUNCH") != nullptr;
     config.attrs = attributes;
     config.numAttrs = plain ? 1 : 2;
-    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out, copy)
-                                    : cudaLaunchKernelEx(&config, sample_kernel<false>, logits, vocab, per_segment, temperature, top_k, top_p, seed, draw_index, out, copy);
+    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true, Params>, logits, vocab, per_segment, params, out, copy)
+                                    : cudaLaunchKernelEx(&config, sample_kernel<false, Params>, logits, vocab, per_segment, params, out, copy);
     if (e != cudaSuccess) return (int)e;
     MRS_RETURN_LAUNCH_STATUS();
+}
+
+// temperature, top_k (<= 0: off), top_p, seed and draw_index are per row.
+// out[r] = the token, or -1 when the row holds a NaN or an infinity.
+MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float* temperature, const int* top_k,
+                          const float* top_p, const unsigned long long* seed, const int* draw_index, int* out,
+                          void* stream) {
+    if (rows <= 0) return 0;
+    if (vocab <= 0 || rows > 0x7fffffff / 8) return MRS_BAD_ARGUMENT;
+    return launch_sample(logits, rows, vocab, SampleArrays{temperature, top_k, top_p, seed, draw_index}, out, nullptr, stream);
+}
+
+template <int ROWS>
+static int launch_sample_words(const float* logits, int first, int count, int rows, int vocab, const unsigned char* words, int* out, int* copy,
+                               void* stream) {
+    SampleWords<ROWS> w = {};
+    const size_t n = (size_t)rows, bytes = 4 * (size_t)count;
+    memcpy(w.seed, words + 8 * (size_t)first, 2 * bytes);
+    memcpy(w.temperature, words + 8 * n + 4 * (size_t)first, bytes);
+    memcpy(w.top_k, words + 12 * n + 4 * (size_t)first, bytes);
+    memcpy(w.top_p, words + 16 * n + 4 * (size_t)first, bytes);
+    memcpy(w.draw_index, words + 20 * n + 4 * (size_t)first, bytes);
+    return launch_sample(logits + (size_t)first * vocab, count, vocab, w, out + first, copy + first, stream);
+}
+
+// The same with the parameters in the host's memory, read before this returns: all rows' seeds, then their temperatures, top_k, top_p
+// and draw indices.  copy[r] = out[r], in pinned memory: complete when the stream has come here.
+MRS_EXPORT int mrs_sample_words(const float* logits, int rows, int vocab, const unsigned char* words, int* out, int* copy, void* stream) {
+    if (rows <= 0) return 0;
+    if (vocab <= 0 || rows > 0x7fffffff / 8 || !words || !copy) return MRS_BAD_ARGUMENT;
+    constexpr int FEW = 32, MANY = 160;                      // 4 KB of arguments
+    for (int first = 0; first < rows; first += MANY) {
+        const int count = rows - first < MANY ? rows - first : MANY;
+        const int code = count <= FEW ? launch_sample_words<FEW>(logits, first, count, rows, vocab, words, out, copy, stream)
+                                      : launch_sample_words<MANY>(logits, first, count, rows, vocab, words, out, copy, stream);
+        if (code != 0) return code;
+    }
+    return 0;
 }

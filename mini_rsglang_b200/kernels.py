@@ -33,7 +33,8 @@ _SIGNATURES = {
     "mrs_attention_f32_chunk": [],
     "mrs_gemm_f32": [_c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_vp],
     "mrs_argmax": [_c_vp, _c_vp, _c_int, _c_int, _c_vp],
-    "mrs_sample": [_c_vp, _c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp],
+    "mrs_sample": [_c_vp, _c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp],
+    "mrs_sample_words": [_c_vp, _c_int, _c_int, ctypes.c_char_p, _c_vp, _c_vp, _c_vp],
 }
 
 _lib = None
@@ -316,18 +317,19 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
     _need(draw_index, torch.int32, "draw_index", (rows,))
     _need(out, torch.int32, "sample out", (rows,))
     _check(library().mrs_sample(logits.data_ptr(), rows, vocab, temperature.data_ptr(), top_k.data_ptr(),
-                                top_p.data_ptr(), seed.data_ptr(), draw_index.data_ptr(), out.data_ptr(), None,
+                                top_p.data_ptr(), seed.data_ptr(), draw_index.data_ptr(), out.data_ptr(),
                                 _stream()), "sample")
 
 
-def sample_staged(logits: torch.Tensor, words: int, out: torch.Tensor, copy: int) -> None:
-    """`sample` with the rows' parameters as the words of `sampling.packed_parameters` at address `words` and the tokens also
-    written to address `copy`, both in pinned host memory that stays as it is until the kernel has ended."""
+def sample_words(logits: torch.Tensor, words: bytes, out: torch.Tensor, copy: int) -> None:
+    """`sample` with the rows' parameters as the words of `sampling.packed_parameters`, which travel with the launch, and the
+    tokens also written to address `copy` in pinned host memory, which stays until the kernel has ended."""
     rows, vocab = logits.shape
     _need(logits, torch.float32, "logits")
     _need(out, torch.int32, "sample out", (rows,))
-    _check(library().mrs_sample(logits.data_ptr(), rows, vocab, words + 8 * rows, words + 12 * rows, words + 16 * rows, words,
-                                words + 20 * rows, out.data_ptr(), copy, _stream()), "sample")
+    if len(words) != 24 * rows:
+        raise InvalidRequest(f"sample: {len(words)} bytes of parameters for {rows} rows")
+    _check(library().mrs_sample_words(logits.data_ptr(), rows, vocab, words, out.data_ptr(), copy, _stream()), "sample")
 
 
 # ------------------------------------------------------------------------------------------------

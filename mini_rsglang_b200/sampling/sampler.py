@@ -36,13 +36,12 @@ def _words(rows: int) -> struct.Struct:
     return struct.Struct(f"={rows}Q{rows}f{rows}i{rows}f{rows}i")
 
 
-def _pack_into(buffer, params: Sequence[SamplingParams], draw_index: Sequence[int]) -> None:
-    """Writes the words of `packed_parameters` into a writable buffer of bytes (a third of the time that arrays of numpy take for
-    some ten rows)."""
+def packed_bytes(params: Sequence[SamplingParams], draw_index: Sequence[int]) -> bytes:
+    """The bytes of `packed_parameters` (in a third of the time that numpy's arrays take for some ten rows)."""
     temperatures = [0.0 if p.is_greedy() else p.temperature for p in params]
     try:
-        _words(len(params)).pack_into(buffer, 0, *[int(p.seed) & _MASK64 for p in params], *temperatures, *[p.top_k or 0 for p in params],
-                                      *[p.top_p for p in params], *draw_index)
+        return _words(len(params)).pack(*[int(p.seed) & _MASK64 for p in params], *temperatures, *[p.top_k or 0 for p in params],
+                                        *[p.top_p for p in params], *draw_index)
     except (struct.error, OverflowError):
         # what a word of this kind does not hold: a float beyond float32 is infinite, an integer beyond 32 bits is refused
         rows = len(params)
@@ -52,15 +51,13 @@ def _pack_into(buffer, params: Sequence[SamplingParams], draw_index: Sequence[in
         packed[3 * rows:4 * rows] = [p.top_k or 0 for p in params]
         packed[4 * rows:5 * rows].view(np.float32)[:] = [p.top_p for p in params]
         packed[5 * rows:] = draw_index
-        buffer[:24 * rows] = packed.tobytes()
+        return packed.tobytes()
 
 
 def packed_parameters(params: Sequence[SamplingParams], draw_index: Sequence[int]) -> np.ndarray:
     """The rows' parameters as the words that the kernel reads: all seeds (the 64-bit patterns of their values, negative ones too),
     then all temperatures, top_k, top_p and draw indices, 32 bits each."""
-    buffer = bytearray(24 * len(params))
-    _pack_into(buffer, params, draw_index)
-    return np.frombuffer(buffer, dtype=np.int32)
+    return np.frombuffer(packed_bytes(params, draw_index), dtype=np.int32)
 
 
 class Chosen:
@@ -72,13 +69,10 @@ class Chosen:
 
 
 class _Turn:
-    """Pinned host memory of one launch: the rows' parameters and their tokens, which the kernel reads and writes there itself.  It is
-    used again, or given back, only behind `last`: the allocator of pinned memory does not know of a kernel's accesses."""
+    """Pinned host memory that one launch's kernel writes its tokens to.  It is used again, or given back, only behind `last`: the
+    allocator of pinned memory does not know of a kernel's accesses."""
 
     def __init__(self, rows: int):
-        self.rows = rows
-        self.words = torch.empty(24 * rows, dtype=torch.uint8, pin_memory=True)
-        self.bytes = memoryview(self.words.numpy())
         self.tokens = torch.empty(rows, dtype=torch.int32, pin_memory=True)
         self.last: torch.cuda.Event | None = None
 
@@ -107,7 +101,7 @@ class Sampler:
         turn = self._turns[self._at]
         if turn is not None:
             turn.wait()
-        if turn is None or turn.rows < rows:
+        if turn is None or turn.tokens.numel() < rows:
             turn = self._turns[self._at] = _Turn(max(256, 2 * rows))
         return turn
 
@@ -137,10 +131,9 @@ class Sampler:
             kernels.argmax(logits, out)
             host.copy_(out, non_blocking=True)
         else:
-            # The kernel reads the rows' parameters from pinned memory and writes the tokens there too: a copy each way is a launch on
-            # the host and a wait on the device (with arrays and copies a launch took the host 75 us for 24 rows, the kernel 68).
-            _pack_into(turn.bytes, params, draw_index)
-            kernels.sample_staged(logits, turn.words.data_ptr(), out, host.data_ptr())
+            # The parameters travel with the launch and the kernel writes the tokens to pinned memory: a copy each way is a launch on the
+            # host and a wait on the device (with numpy's arrays and copies a launch took the host 75 us for 24 rows, the kernel 68).
+            kernels.sample_words(logits, packed_bytes(params, draw_index), out, host.data_ptr())
         arrived.record()
         turn.last = arrived
         return Chosen(out, host, arrived)

@@ -14,7 +14,6 @@
 //   channel_fold       keeps a key channel from two thin products, folded into k and q so that the recurrence itself meets none
 //   narrow_columns     a range of float32 columns as rows of the engine's dtype
 #include "common.cuh"
-#include "pairs.cuh"
 
 namespace {
 
@@ -129,11 +128,13 @@ __global__ void memory_gates_kernel(const float* __restrict__ raw, int raw_strid
 }
 
 // ---------------------------------------------------------------------------------------------
-// The recurrence.  A thread keeps SCAN_ROWS rows x 4 neighbouring columns of S in registers, two rows to a 64-bit register
-// pair, so that one instruction (fma.rn.f32x2, two independent float32 multiply-adds) serves two rows; the PARTS lanes that
-// share four columns cover the d rows, so what a thread reads of k and q from shared memory serves four columns, and a
-// token's read-out is a reduction that hands its columns out while it sums (2 + 1 + 1 ... shuffles).  The tokens' k, q and v
-// come through two stages of shared memory, filled by cp.async a batch ahead.
+// The recurrence.  A thread keeps SCAN_ROWS rows x 4 neighbouring columns of S in registers; the PARTS lanes that share four
+// columns cover the d rows, so what a thread reads of k and q from shared memory serves four columns, and two tokens' read-outs
+// are a reduction that hands their eight columns out while it sums.  The tokens' k, q and v come through two stages of shared
+// memory, filled by cp.async a batch ahead.  Bound by the float32 multiply-adds and the registers they read: 2,000 tokens of 16 heads
+// of 128 x 256 take 87 us (states alone) and 144 us (with read-outs), a multiply-add every 1.6 clocks a scheduler.  With two rows to a
+// register pair (fma.rn.f32x2, half the instructions but four clocks each with three operands of 64 bits) and a token's reduction by
+// itself 91 and 157 us, 5 sequences of 300 tokens 332 against 312 us for the layer.
 //
 // The decay costs no instruction an element: with P the product of the keeps since S was last rescaled, the registers hold
 // S / P, a token adds (take / P) k v^T and its read-out is P (S / P)^T q.  A batch's prefix products are made by one warp a
@@ -280,7 +281,6 @@ __global__ void __launch_bounds__(256, 2) linear_scan_kernel(const ScanArgs A) {
     __shared__ __align__(16) float4 facts[2][SCAN_BATCH];    // of a token: take / p, p, keep, take; p the batch's product of keeps so far
     constexpr int GROUPS = 32 / PARTS;                       // groups of four columns a warp covers
     constexpr int VECTOR = PARTS * SCAN_PITCH;               // floats of a k (or q) in shared memory
-    constexpr int PAIRS = SCAN_ROWS / 2;
     constexpr bool PRODUCTS = CHANNEL && MODE == SCAN_LOCAL;
     __shared__ float products[PRODUCTS ? PARTS * SCAN_ROWS : 1];     // of the chunk's keeps, a channel each; one warp's alone
     pdl_launch_dependents();
@@ -311,11 +311,24 @@ __global__ void __launch_bounds__(256, 2) linear_scan_kernel(const ScanArgs A) {
     const bool zero = MODE == SCAN_LOCAL || (MODE == SCAN_WHOLE && A.positions[seq_first] == 0);
 
     const int q_at = head * A.d, v_at = head * A.e + slice * A.cols, live_cols = min(A.cols, A.e - slice * A.cols);
+    // where a lane's copies come from and go to: of a token's row and in a token's place
+    const float *k_from = A.k + q_at + 4 * lane, *v_from = A.v + v_at + 4 * lane;
+    const long long q_behind_k = A.q - A.k;
+    const int where = (4 * lane / SCAN_ROWS) * SCAN_PITCH + 4 * lane % SCAN_ROWS;
+    const bool small_rows = A.vec_qk && A.d <= 128 && A.vec_v && live_cols <= 128, has_qk = 4 * lane < A.d, has_v = 4 * lane < live_cols;
     auto issue = [&](int t0, int n, int buffer) {
         float* base = stage + buffer * stage_floats;
         for (int j = warp; j < n; j += warps) {              // a warp copies a token
             float* to = base + j * token_floats;
             const size_t row = (size_t)(t0 + j) * A.stride;
+            if (small_rows) {
+                if (has_qk) {
+                    scan_copy16(to + where, k_from + row);
+                    if (MODE != SCAN_LOCAL) scan_copy16(to + VECTOR + where, k_from + row + q_behind_k);
+                }
+                if (has_v) scan_copy16(to + 2 * VECTOR + 4 * lane, v_from + row);
+                continue;
+            }
             if (A.vec_qk) {
                 for (int i = 4 * lane; i < A.d; i += 128) {
                     const int where = (i / SCAN_ROWS) * SCAN_PITCH + i % SCAN_ROWS;
@@ -346,9 +359,9 @@ __global__ void __launch_bounds__(256, 2) linear_scan_kernel(const ScanArgs A) {
         }
         asm volatile("cp.async.commit_group;\n" ::);
     };
-    // rows of the batch that begins at row t
-    auto rows_at = [&](int t) { return min(CHANNEL ? A.batch - t % A.batch : A.batch, last - t); };
-    auto direct_at = [&](int t) { return CHANNEL && A.direct[(size_t)(t / A.batch) * A.heads + head] != 0; };
+    // batches begin at multiples of A.batch (CHANNEL; a power of two), so only the first may be a part of one
+    const int first_rows = min(CHANNEL ? A.batch - (first & (A.batch - 1)) : A.batch, last - first);
+    const int* direct_from = CHANNEL ? A.direct + (size_t)(first / A.batch) * A.heads + head : nullptr;
     const float fixed = A.decay ? A.decay[head] : 1.0f;
     auto read_facts = [&](int t0, int n) {                   // keep and take of token t0 + lane, warp 0
         if (A.decay || lane >= n) return make_float2(lane < n ? fixed : 1.0f, 1.0f);
@@ -364,40 +377,43 @@ __global__ void __launch_bounds__(256, 2) linear_scan_kernel(const ScanArgs A) {
         }
         if (lane < A.batch) facts[buffer][lane] = make_float4(raw.y / p, p, raw.x, raw.y);
     };
-    issue(first, rows_at(first), 0);
-    if (!CHANNEL && warp == 0) write_facts(read_facts(first, rows_at(first)), 0);
-    bool direct = direct_at(first);
+    issue(first, first_rows, 0);
+    if (!CHANNEL && warp == 0) write_facts(read_facts(first, first_rows), 0);
+    bool direct = CHANNEL && *direct_from != 0;
 
-    pair s[4][PAIRS];                                        // a column's rows two by two
+    float s[SCAN_ROWS][4];
 #pragma unroll
-    for (int i = 0; i < PAIRS; ++i) {
-        float x[4][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
+    for (int i = 0; i < SCAN_ROWS; ++i) {
+        const int row = row0 + i;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int row = row0 + 2 * i + u;
-            if (zero || row >= A.d) continue;
-            const float* from = mine + (size_t)row * A.e + col;
-            if (A.vec_state) {
-                if (col < A.e) {
-                    const float4 f = *reinterpret_cast<const float4*>(from);
-                    x[0][u] = f.x, x[1][u] = f.y, x[2][u] = f.z, x[3][u] = f.w;
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (col + c < A.e) x[c][u] = from[c];
+        for (int c = 0; c < 4; ++c) s[i][c] = 0.0f;
+        if (zero || row >= A.d) continue;
+        const float* from = mine + (size_t)row * A.e + col;
+        if (A.vec_state) {
+            if (col < A.e) {
+                const float4 f = *reinterpret_cast<const float4*>(from);
+                s[i][0] = f.x, s[i][1] = f.y, s[i][2] = f.z, s[i][3] = f.w;
             }
-            if (is_norm) x[0][u] = norm_mine[row];
-        }
+        } else {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) s[c][i] = make_pair(x[c][0], x[c][1]);
+            for (int c = 0; c < 4; ++c)
+                if (col + c < A.e) s[i][c] = from[c];
+        }
+        if (is_norm) s[i][0] = norm_mine[row];
     }
     auto rescale = [&](float by) {
-        const pair f = make_pair(by, by);
 #pragma unroll
-        for (int i = 0; i < PAIRS; ++i) {
+        for (int i = 0; i < SCAN_ROWS; ++i)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) s[c][i] = mul2(s[c][i], f);
+            for (int c = 0; c < 4; ++c) s[i][c] *= by;
+    };
+    // S's rows multiplied by a channel's keeps each, in shared memory
+    auto keep_rows = [&](const float* keep) {
+#pragma unroll
+        for (int i = 0; i < SCAN_ROWS; i += 4) {
+            const float4 f = *reinterpret_cast<const float4*>(keep + i);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) s[i][c] *= f.x, s[i + 1][c] *= f.y, s[i + 2][c] *= f.z, s[i + 3][c] *= f.w;
         }
     };
     // one token: `weight` multiplies what is added, `factor` what is read
@@ -405,30 +421,37 @@ __global__ void __launch_bounds__(256, 2) linear_scan_kernel(const ScanArgs A) {
     if (is_norm) to = A.norm_out + (size_t)first * A.heads + head;
     const size_t out_step = is_norm ? A.heads : (size_t)A.heads * A.e;
     const int live = is_norm ? 1 : A.e - col;                // columns of these four that are there
-    auto walk = [&](const float* token, float weight, float factor) {
+    // what a token adds, and this thread's rows' part of its read-out (even and odd rows are summed side by side)
+    auto take_in = [&](const float* token, float weight, float (&z)[4]) {
         float4 vv = *reinterpret_cast<const float4*>(token + 2 * VECTOR + place);
         if (is_norm) vv.x = 1.0f;                            // the columns behind e are zero
-        const pair tv[4] = {make_pair(vv.x * weight, vv.x * weight), make_pair(vv.y * weight, vv.y * weight),
-                            make_pair(vv.z * weight, vv.z * weight), make_pair(vv.w * weight, vv.w * weight)};
-        pair y[4];
+        const float tv[4] = {vv.x * weight, vv.y * weight, vv.z * weight, vv.w * weight};
+        float y[4][2];
         const float* kp = token + part * SCAN_PITCH;
 #pragma unroll
-        for (int i = 0; i < PAIRS; i += 2) {
-            const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(kp + 2 * i);
-            ulonglong2 qq = make_ulonglong2(0ull, 0ull);
-            if (MODE != SCAN_LOCAL) qq = *reinterpret_cast<const ulonglong2*>(kp + VECTOR + 2 * i);
+        for (int i = 0; i < SCAN_ROWS; i += 4) {
+            float kk[4], qq[4];
+            *reinterpret_cast<float4*>(kk) = *reinterpret_cast<const float4*>(kp + i);
+            if (MODE != SCAN_LOCAL) *reinterpret_cast<float4*>(qq) = *reinterpret_cast<const float4*>(kp + VECTOR + i);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                s[c][i] = fma2(kk.x, tv[c], s[c][i]);
-                s[c][i + 1] = fma2(kk.y, tv[c], s[c][i + 1]);
-                if (MODE != SCAN_LOCAL) {
-                    y[c] = i == 0 ? mul2(s[c][i], qq.x) : fma2(s[c][i], qq.x, y[c]);
-                    y[c] = fma2(s[c][i + 1], qq.y, y[c]);
-                }
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s[i + u][c] = fmaf(kk[u], tv[c], s[i + u][c]);
+            if (MODE != SCAN_LOCAL) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) y[c][u & 1] = i + u < 2 ? s[i + u][c] * qq[u] : fmaf(s[i + u][c], qq[u], y[c][u & 1]);
             }
         }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) z[c] = MODE != SCAN_LOCAL ? y[c][0] + y[c][1] : 0.0f;
+    };
+    // one token: `weight` multiplies what is added, `factor` what is read
+    auto walk = [&](const float* token, float weight, float factor) {
+        float z[4];
+        take_in(token, weight, z);
         if (MODE == SCAN_LOCAL) return;
-        const float z[4] = {both(y[0]), both(y[1]), both(y[2]), both(y[3])};
         if (PARTS == 1) {
             if (A.vec_out && !is_norm) {
                 if (live > 0) *reinterpret_cast<float4*>(to) = make_float4(z[0] * factor, z[1] * factor, z[2] * factor, z[3] * factor);
@@ -456,17 +479,63 @@ __global__ void __launch_bounds__(256, 2) linear_scan_kernel(const ScanArgs A) {
         for (int o = 4 * GROUPS; o < 32; o <<= 1) one += __shfl_xor_sync(0xffffffffu, one, o);
         if (part < 4 && at + (second ? 1 : 0) < live) to[at + (second ? 1 : 0)] = one * factor;
     };
+    // Two tokens: their eight columns' sums are handed out while they are added up, so that the third exchange is one number too and
+    // (with 8 parts) every lane stores one.  The sums are those of `walk`.
+    auto walk_two = [&](const float* token, float2 weight, float2 factor) {
+        float z[2][4];
+        take_in(token, weight.x, z[0]);
+        take_in(token + token_floats, weight.y, z[1]);
+        if (MODE == SCAN_LOCAL) return;
+        const bool upper = part & 1, second = part & 2, later = part & 4;
+        float h[2][2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float mine_z = upper ? z[j][2 + u] : z[j][u];
+                h[j][u] = mine_z + __shfl_xor_sync(0xffffffffu, upper ? z[j][u] : z[j][2 + u], GROUPS);
+            }
+        float one[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float mine_h = second ? h[j][1] : h[j][0];
+            one[j] = mine_h + __shfl_xor_sync(0xffffffffu, second ? h[j][0] : h[j][1], 2 * GROUPS);
+        }
+        const float mine_one = later ? one[1] : one[0];
+        float sum = mine_one + __shfl_xor_sync(0xffffffffu, later ? one[0] : one[1], 4 * GROUPS);
+#pragma unroll
+        for (int o = 8 * GROUPS; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        const int at = (upper ? 2 : 0) + (second ? 1 : 0);
+        if (part < 8 && at < live) to[(later ? out_step : 0) + at] = sum * (later ? factor.y : factor.x);
+    };
+    // the tokens of a batch; facts of token j: (weight, factor)
+    auto walk_batch = [&](const float* token, int n, auto fact) {
+        int j = 0;
+        if (PARTS >= 8 || MODE == SCAN_LOCAL) {
+#pragma unroll 1
+            for (; j + 1 < n; j += 2, token += 2 * token_floats) {
+                const float2 f0 = fact(j), f1 = fact(j + 1);
+                walk_two(token, make_float2(f0.x, f1.x), make_float2(f0.y, f1.y));
+                to += 2 * out_step;
+            }
+        }
+#pragma unroll 1
+        for (; j < n; ++j, token += token_floats) {
+            const float2 f = fact(j);
+            walk(token, f.x, f.y);
+            to += out_step;
+        }
+    };
 
     float P = 1.0f, product = 1.0f;
-    for (int t0 = first, b = 0; t0 < last; ++b) {
-        const int n = rows_at(t0), t1 = t0 + n;
+    for (int t0 = first, n = first_rows, b = 0; t0 < last; ++b) {
+        const int t1 = t0 + n, n1 = min(A.batch, last - t1);
         float2 next = make_float2(1.0f, 1.0f);
         bool next_direct = false;
         if (t1 < last) {
-            const int n1 = rows_at(t1);
             issue(t1, n1, (b + 1) & 1);
             if (!CHANNEL && warp == 0) next = read_facts(t1, n1);
-            next_direct = direct_at(t1);
+            if (CHANNEL) next_direct = *(direct_from += A.heads) != 0;
             asm volatile("cp.async.wait_group 1;\n" ::);
         } else {
             asm volatile("cp.async.wait_group 0;\n" ::);
@@ -490,31 +559,20 @@ __global__ void __launch_bounds__(256, 2) linear_scan_kernel(const ScanArgs A) {
                 for (int j = 0; j < n; ++j, token += token_floats) {
                     const float* keep = A.keeps + (size_t)(t0 + j) * A.heads * A.d + q_at;
 #pragma unroll
-                    for (int i = 0; i < PAIRS; ++i) {
-                        const int row = row0 + 2 * i;
-                        const pair f = make_pair(row < A.d ? keep[row] : 0.0f, row + 1 < A.d ? keep[row + 1] : 0.0f);
+                    for (int i = 0; i < SCAN_ROWS; ++i) {
+                        const float f = row0 + i < A.d ? keep[row0 + i] : 0.0f;
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) s[c][i] = mul2(s[c][i], f);
+                        for (int c = 0; c < 4; ++c) s[i][c] *= f;
                     }
                     walk(token, 1.0f, 1.0f);
                     to += out_step;
                 }
             } else if (!idle) {
-                const float* keep = token + A.batch * token_floats + part * SCAN_PITCH;
-#pragma unroll 1
-                for (int j = 0; j < n; ++j, token += token_floats) {
-                    walk(token, 1.0f, 1.0f);
-                    to += out_step;
-                }
-#pragma unroll
-                for (int i = 0; i < PAIRS; i += 2) {
-                    const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(keep + 2 * i);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) s[c][i] = mul2(s[c][i], f.x), s[c][i + 1] = mul2(s[c][i + 1], f.y);
-                }
+                walk_batch(token, n, [](int) { return make_float2(1.0f, 1.0f); });
+                keep_rows(token + A.batch * token_floats + part * SCAN_PITCH);
             }
             direct = next_direct;
-            t0 = t1;
+            t0 = t1, n = n1;
             __syncthreads();                                 // the stage is copied into again two batches on
             continue;
         }
@@ -535,16 +593,14 @@ __global__ void __launch_bounds__(256, 2) linear_scan_kernel(const ScanArgs A) {
             }
         } else {
             const float inverse = 1.0f / P;
-#pragma unroll 1
-            for (int j = 0; j < n; ++j, token += token_floats) {
+            walk_batch(token, n, [&](int j) {
                 const float2 f = *reinterpret_cast<const float2*>(&fact[j]);
-                walk(token, f.x * inverse, f.y * P);
-                to += out_step;
-            }
+                return make_float2(f.x * inverse, f.y * P);
+            });
         }
         if (end >= SCAN_LEAST) P *= end;
         if (warp == 0 && t1 < last) write_facts(next, (b + 1) & 1);
-        t0 = t1;
+        t0 = t1, n = n1;
         __syncthreads();                                     // the stage is copied into again two batches on
     }
     if (MODE == SCAN_LOCAL && !CHANNEL && threadIdx.x == 0 && slice == 0) A.chunk_decay[chunk_at] = product;
@@ -553,24 +609,18 @@ __global__ void __launch_bounds__(256, 2) linear_scan_kernel(const ScanArgs A) {
     if (MODE == SCAN_LOCAL || (MODE == SCAN_WHOLE && A.write_state)) {
         rescale(P);
 #pragma unroll
-        for (int i = 0; i < PAIRS; ++i) {
-            const float2 x[4] = {split(s[0][i]), split(s[1][i]), split(s[2][i]), split(s[3][i])};
+        for (int i = 0; i < SCAN_ROWS; ++i) {
+            const int row = row0 + i;
+            if (row >= A.d) continue;
+            float* to = mine + (size_t)row * A.e + col;
+            if (A.vec_state) {
+                if (col < A.e) *reinterpret_cast<float4*>(to) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+            } else {
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int row = row0 + 2 * i + u;
-                if (row >= A.d) continue;
-                const float4 f = u ? make_float4(x[0].y, x[1].y, x[2].y, x[3].y) : make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
-                float* to = mine + (size_t)row * A.e + col;
-                if (A.vec_state) {
-                    if (col < A.e) *reinterpret_cast<float4*>(to) = f;
-                } else {
-                    if (col < A.e) to[0] = f.x;
-                    if (col + 1 < A.e) to[1] = f.y;
-                    if (col + 2 < A.e) to[2] = f.z;
-                    if (col + 3 < A.e) to[3] = f.w;
-                }
-                if (is_norm) norm_mine[row] = f.x;
+                for (int c = 0; c < 4; ++c)
+                    if (col + c < A.e) to[c] = s[i][c];
             }
+            if (is_norm) norm_mine[row] = s[i][0];
         }
     }
 }

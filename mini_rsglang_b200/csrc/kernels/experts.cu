@@ -87,38 +87,75 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int stride, c
     if (has_shared && lane == 0) shared_gate[t] = 1.0f / (1.0f + expf(-z[all]));
 }
 
-// One block.  Dynamic shared memory: 3 * routed ints (count, first row, filled).
-__global__ void moe_align_kernel(const int* __restrict__ chosen, int pairs, int routed, int tile, int* __restrict__ sorted_rows,
-                                 int* __restrict__ tile_expert, int capacity) {
+// One block.  Dynamic shared memory: 3 * routed ints (count, first row, filled).  Bound by its chain: the choices' loads, the counts, the
+// scan over the experts, the stores.  Up to ALIGN_OWN choices a thread are loaded together and stay in registers with the places that
+// the counting gave them; 7,108 choices among 32 experts take 6.5 us (12 with two
+// passes over the choices and one thread that added up the experts).
+constexpr int ALIGN_OWN = 8;
+__global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__ chosen, int pairs, int routed, int tile, int* __restrict__ sorted_rows,
+                                                         int* __restrict__ tile_expert, int capacity) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ int align_smem[];
     int* count = align_smem;
     int* first = count + routed;
     int* filled = first + routed;
+    const bool few = pairs <= ALIGN_OWN * (int)blockDim.x;
+    int own[ALIGN_OWN], place[ALIGN_OWN];
+#pragma unroll
+    for (int j = 0; j < ALIGN_OWN; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        own[j] = few && i < pairs ? chosen[i] : -1;
+    }
     for (int e = threadIdx.x; e < routed; e += blockDim.x) count[e] = 0, filled[e] = 0;
-    for (int i = threadIdx.x; i < capacity; i += blockDim.x) sorted_rows[i] = -1;
+    if (((uintptr_t)sorted_rows & 15) == 0) {
+        for (int i = threadIdx.x; i < capacity / 4; i += blockDim.x) reinterpret_cast<int4*>(sorted_rows)[i] = make_int4(-1, -1, -1, -1);
+        for (int i = capacity / 4 * 4 + threadIdx.x; i < capacity; i += blockDim.x) sorted_rows[i] = -1;
+    } else {
+        for (int i = threadIdx.x; i < capacity; i += blockDim.x) sorted_rows[i] = -1;
+    }
     for (int i = threadIdx.x; i < capacity / tile; i += blockDim.x) tile_expert[i] = -1;
     __syncthreads();
-    for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-        const int e = chosen[i];
-        if (e >= 0 && e < routed) atomicAdd(&count[e], 1);
+    if (few) {
+#pragma unroll
+        for (int j = 0; j < ALIGN_OWN; ++j) {
+            if (own[j] >= routed) own[j] = -1;
+            place[j] = own[j] >= 0 ? atomicAdd(&count[own[j]], 1) : 0;
+        }
+    } else {
+        for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+            const int e = chosen[i];
+            if (e >= 0 && e < routed) atomicAdd(&count[e], 1);
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         int at = 0;
-        for (int e = 0; e < routed; ++e) {
-            first[e] = at;
-            at += (count[e] + tile - 1) / tile * tile;
+        for (int base = 0; base < routed; base += 32) {
+            const int e = base + threadIdx.x, rows = e < routed ? (count[e] + tile - 1) / tile * tile : 0;
+            int upto = rows;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, upto, o);
+                if ((int)threadIdx.x >= o) upto += up;
+            }
+            if (e < routed) first[e] = at + upto - rows;
+            at += __shfl_sync(0xffffffffu, upto, 31);
         }
-        tile_expert[capacity / tile] = at / tile;
+        if (threadIdx.x == 0) tile_expert[capacity / tile] = at / tile;
     }
     __syncthreads();
     for (int e = threadIdx.x; e < routed; e += blockDim.x)
         for (int i = first[e] / tile; i < (first[e] + count[e] + tile - 1) / tile; ++i) tile_expert[i] = e;
-    for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-        const int e = chosen[i];
-        if (e >= 0 && e < routed) sorted_rows[first[e] + atomicAdd(&filled[e], 1)] = i;
+    if (few) {
+#pragma unroll
+        for (int j = 0; j < ALIGN_OWN; ++j)
+            if (own[j] >= 0) sorted_rows[first[own[j]] + place[j]] = threadIdx.x + j * blockDim.x;
+    } else {
+        for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+            const int e = chosen[i];
+            if (e >= 0 && e < routed) sorted_rows[first[e] + atomicAdd(&filled[e], 1)] = i;
+        }
     }
 }
 
@@ -301,11 +338,13 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS) moe_product_rows_kernel(const
     }
 }
 
-// One block a listed row: sixteen bytes a thread and step.
-__global__ void moe_gather_rows_kernel(const bf16* __restrict__ x, const int* __restrict__ sorted_rows, bf16* __restrict__ out, int k, int top) {
+// One block a listed row: sixteen bytes a thread and step.  `fill`: places without a pair become zeros; else they keep what was there.
+__global__ void moe_gather_rows_kernel(const bf16* __restrict__ x, const int* __restrict__ sorted_rows, bf16* __restrict__ out, int k, int top,
+                                       int fill) {
     pdl_launch_dependents();
     pdl_wait();
     const int pair = sorted_rows[blockIdx.x];
+    if (pair < 0 && !fill) return;
     const uint4* src = pair >= 0 ? reinterpret_cast<const uint4*>(x + (size_t)(pair / top) * k) : nullptr;
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * k);
     for (int i = threadIdx.x; i < k / 8; i += blockDim.x) dst[i] = src ? src[i] : make_uint4(0u, 0u, 0u, 0u);
@@ -504,11 +543,11 @@ MRS_EXPORT int mrs_moe_product_rows(int is_bf16, int gated, const void* x, const
     MRS_RETURN_LAUNCH_STATUS();
 }
 
-// out [capacity, k] = the input rows x[pair / top] of the listed pairs, zeros for -1; bfloat16, k a multiple of 8.
-MRS_EXPORT int mrs_moe_gather_rows(const void* x, const int* sorted_rows, void* out, int capacity, int k, int top, void* stream) {
+// out [capacity, k] = the input rows x[pair / top] of the listed pairs, zeros for -1 (`fill`); bfloat16, k a multiple of 8.
+MRS_EXPORT int mrs_moe_gather_rows(const void* x, const int* sorted_rows, void* out, int capacity, int k, int top, int fill, void* stream) {
     if (capacity <= 0) return 0;
     if (k <= 0 || k % 8 || top <= 0 || (((uintptr_t)x | (uintptr_t)out) & 15)) return MRS_BAD_ARGUMENT;
-    MRS_LAUNCH(moe_gather_rows_kernel, capacity, 128, 0, stream, (const bf16*)x, sorted_rows, (bf16*)out, k, top);
+    MRS_LAUNCH(moe_gather_rows_kernel, capacity, 128, 0, stream, (const bf16*)x, sorted_rows, (bf16*)out, k, top, fill);
     MRS_RETURN_LAUNCH_STATUS();
 }
 

@@ -3,12 +3,16 @@
 // (mrs_moe_gather_rows in experts.cu), so that a tile of 128 rows, all of one expert, comes in by bulk tensor copies;
 // the experts' weights are one matrix [experts * rows an expert, K], and a tile's weight rows start at its expert's
 // first row.  As in gemm_many_rows.cu a CTA computes a tile of 128 rows x 256 weight rows into one of two
-// accumulators in tensor memory while four warps turn the other, finished one into values:
+// accumulators in tensor memory while eight warps turn the other, finished one into values:
 //   warp 0   fetches 128 x 64 row tiles and 256 x 64 weight tiles (TMA, 128-byte swizzle) into a ring of stages;
 //   warp 1   one thread issues tcgen05.mma (M 128, N 256, K 16) on the stages;
-//   warps 2-5 a thread a row: the row's 256 sums from tensor memory;
+//   warps 2-9 two threads a row, 128 of its sums from tensor memory each;
 //             gated: a weight tile holds two blocks of 64 gate and 64 up rows, out[row] = silu(gate) * up;
 //             plain: out[pair of the row] = the sums (the rows go back to their (token, choice) pairs).
+// Bound by the weights' bytes, then by the MMAs.  With one thread a row and a full division a sum the epilogue took a tile 18,000 clocks,
+// longer than its MMAs (16,400 at K = 2,048); two threads and the fast division take 5,300.  32 experts, 1,777 tokens x 4, width 2,048,
+// inner 1,024: gated product 84 -> 67 us, down product 41 (unchanged); 200 tokens, width 4,096, inner 1,536: 156 -> 136 and 72 -> 70.  Two tiles of rows a
+// CTA (weights fetched once for 256 rows) leave some SMs 6 tiles where others have 2 and no accumulator free meanwhile: 107 us.
 // Only the tiles that the lists use are walked: their count stands behind the tiles' experts.  CTAs are
 // persistent; tiles that share a weight tile are taken by neighbouring CTAs at the same time.  Every wait is bounded
 // (tma.cuh).
@@ -17,10 +21,26 @@
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16, STAGES = 4, THREADS = 192;
+constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16, STAGES = 4, EPILOGUE = 2, THREADS = 64 + EPILOGUE * 128;      // groups of four warps that share a tile's columns
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int TMEM_COLUMNS = 2 * BN;
 constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * sizeof(uint64_t) + 16;
+
+// How L2 keeps a tile of weights: to go first where the tiles of rows that share it, which run side by side, are done with it before
+// it would go; the gathered rows, which come once for every 256 weight rows, then stay.  All SMs' tiles of weights are 148 * 512 K bytes
+// at a time, and as long as these about fit L2 that is so: K = 2,048 78 -> 68 us (DRAM reads 407 -> 310 MB, of 268 MB of weights), 500 rows
+// 55 -> 47; K = 1,536 111 -> 103 and 84 -> 77 us; K = 4,096 163 -> 160 us at 700 rows, but 214 -> 237 at 1,777, where tiles drift apart.
+constexpr int STREAMED_K = 2048;
+__device__ __forceinline__ uint64_t weights_policy(bool first_to_go) {
+    uint64_t policy;
+    if (first_to_go) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+    return policy;
+}
+__device__ __forceinline__ void tma_load_2d_hint(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, uint64_t policy) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "l"(policy) : "memory");
+}
 
 // x_map: the gathered rows [capacity, K]; w_map: the weights [experts * N, K]; N: weight rows an expert.
 // tile_expert [capacity / 128 + 1]: the expert of every tile of rows, then the number of tiles in use.
@@ -50,7 +70,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4);
+            mbar_init(&acc_empty[b], 4 * EPILOGUE);
         }
         mbar_fence_init();
     }
@@ -70,6 +90,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
 
     if (warp == 0) {
         const bool leader = elect_one();
+        const uint64_t streamed = weights_policy(K <= STREAMED_K);
         if (leader) {
             tma_prefetch_descriptor(&x_map);
             tma_prefetch_descriptor(&w_map);
@@ -87,7 +108,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
                 if (leader) {
                     mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
                     tma_load_2d(stage, &x_map, &full[s], kb * BK, m0);
-                    tma_load_2d(stage + A_BYTES, &w_map, &full[s], kb * BK, n0);
+                    tma_load_2d_hint(stage + A_BYTES, &w_map, &full[s], kb * BK, n0, streamed);
                 }
                 __syncwarp();
             }
@@ -125,22 +146,22 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
             __syncwarp();
         }
     } else {
-        const int quarter = warp & 3;
+        const int quarter = warp & 3, group = (warp - 2) >> 2;
         const int row = quarter * 32 + lane;                 // row within the tile
         int round = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++round) {
             const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
             const int buffer = round & 1;
+            const int pair = sorted_rows[m0 + row];
             mbar_wait(&acc_full[buffer], (round >> 1) & 1);
             __syncwarp();
             tcgen05_fence_after_sync();
             const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * BN;
-            const int pair = sorted_rows[m0 + row];
             if (GATED) {
                 const int half_n = N >> 1;
                 bf16* dst = out + (size_t)(m0 + row) * half_n + (n0 >> 1);
-#pragma unroll
-                for (int block = 0; block < BN / 128; ++block) {          // 64 gate columns, then their 64 up columns
+                {
+                    const int block = group;                  // 64 gate columns, then their 64 up columns
 #pragma unroll
                     for (int c = 0; c < 64; c += 32) {
                         float g[32], u[32];
@@ -155,7 +176,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
                                 for (int p = 0; p < 4; ++p) {
                                     const float g0 = __bfloat162float(__float2bfloat16_rn(g[e + 2 * p])), g1 = __bfloat162float(__float2bfloat16_rn(g[e + 2 * p + 1]));
                                     const float u0 = __bfloat162float(__float2bfloat16_rn(u[e + 2 * p])), u1 = __bfloat162float(__float2bfloat16_rn(u[e + 2 * p + 1]));
-                                    __nv_bfloat162 two = __floats2bfloat162_rn(g0 / (1.0f + __expf(-g0)) * u0, g1 / (1.0f + __expf(-g1)) * u1);
+                                    __nv_bfloat162 two = __floats2bfloat162_rn(__fdividef(g0, 1.0f + __expf(-g0)) * u0, __fdividef(g1, 1.0f + __expf(-g1)) * u1);
                                     w[p] = *reinterpret_cast<uint32_t*>(&two);
                                 }
                                 *reinterpret_cast<uint4*>(dst + block * 64 + c + e) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -166,7 +187,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
             } else {
                 bf16* dst = out + (size_t)(pair < 0 ? 0 : (ACT >= 0 ? m0 + row : pair)) * N + n0;
 #pragma unroll 2
-                for (int c = 0; c < BN; c += 32) {
+                for (int c = group * (BN / EPILOGUE); c < (group + 1) * (BN / EPILOGUE); c += 32) {
                     float v[32];
                     tmem_load_32_async(acc + c, v);
                     tmem_load_wait();

@@ -894,11 +894,10 @@ def gemm_tc_qkv_heads(x: torch.Tensor, weight: torch.Tensor, q_out: torch.Tensor
 _many_rows_lib = None
 _many_rows_maps: dict[tuple, tuple] = {}
 # Measured against the library's product followed by `silu_mul` (8B shape, K 4096, N 24576): 290 against 299 us at
-# 2,048 rows, 418 against 429 us at 3,072, 550 against 646 us at 4,096; below 2,048 rows the library's pair is ahead
-# (1,536: 221 against 217 us; 512: 90 against 83 us: the 128 x 256 tiles fill the SMs' last round badly).  At other
-# shapes the order differs (prefill of 2,048 tokens: 14B shape, K 5120, N 34816: 58.2 ms with this kernel against
-# 57.7 ms; 0.6B shape, K 1024, N 6144: 4.9 against 4.4 ms), so from GEMM_GATED_ROWS_MIN rows on the two are timed
-# once per (N, K, thousand of rows) on the first such product and the faster one is kept (`gemm_gated_rows_wins`).
+# 2,048 rows, 418 against 429 us at 3,072, 550 against 646 us at 4,096.  At other shapes the order differs (prefill of 2,048 tokens: 14B
+# shape, K 5120, N 34816: 58.2 ms with this kernel against 57.7 ms), so from GEMM_GATED_ROWS_MIN rows on the two are timed
+# once per (N, K, thousand of rows) on the first such product and the faster one is kept (`gemm_gated_rows_wins`); below, the count
+# of the tiles says it (`gemm_gated_rows_fills`).
 GEMM_GATED_ROWS_MIN = int(os.environ.get("MRS_GEMM_GATED_ROWS_MIN", "2048"))      # the variable: for measuring other crossovers
 GEMM_GATED_MEASURE = "MRS_GEMM_GATED_ROWS_MIN" not in os.environ                  # False: the kernel from that many rows on
 _gated_rows_choice: dict[tuple, bool] = {}
@@ -1580,7 +1579,7 @@ _EXPERT_SIGNATURES = {
     "mrs_moe_product_simt": [_c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_vp],
     "mrs_moe_product_rows": [_c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_vp],
     "mrs_moe_product_few": [_c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_vp],
-    "mrs_moe_gather_rows": [_c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_vp],
+    "mrs_moe_gather_rows": [_c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_vp],
     "mrs_moe_gather_scaled_rows": [_c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_vp],
     "mrs_moe_product_mma": [_c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_vp],
     "mrs_moe_combine": [_c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_int, _c_int, _c_vp],
@@ -1952,12 +1951,13 @@ def moe_product_tc(x_rows: torch.Tensor, sorted_rows: torch.Tensor, tile_expert:
         raise BackendError(f"moe_product_tc: {lib.mrs_moe_tc_error_string(code).decode()} (code {code})")
 
 
-def moe_gather_rows(x: torch.Tensor, sorted_rows: torch.Tensor, out: torch.Tensor, top: int) -> None:
-    """out[place] = x[pair / top] for every listed pair, zeros where a run is filled up (bfloat16, rows of a multiple of 8)."""
+def moe_gather_rows(x: torch.Tensor, sorted_rows: torch.Tensor, out: torch.Tensor, top: int, fill: bool = True) -> None:
+    """out[place] = x[pair / top] for every listed pair, zeros where a run is filled up (bfloat16, rows of a multiple of 8); without
+    `fill` those places are left as they are (the tcgen05 product keeps no sums of theirs)."""
     _need(x, torch.bfloat16, "expert input")
     _need(out, torch.bfloat16, "gathered rows", (sorted_rows.shape[0], x.shape[1]))
     _check(expert_library().mrs_moe_gather_rows(x.data_ptr(), sorted_rows.data_ptr(), out.data_ptr(), out.shape[0], x.shape[1], top,
-                                                _stream()), "moe_gather_rows")
+                                                int(fill), _stream()), "moe_gather_rows")
 
 
 def moe_gather_scaled_rows(x: torch.Tensor, sorted_rows: torch.Tensor, weights: torch.Tensor, out: torch.Tensor, top: int) -> None:
@@ -1990,7 +1990,7 @@ def moe_plain_experts(h: torch.Tensor, chosen: torch.Tensor, weights: torch.Tens
     if weights is not None:
         moe_gather_scaled_rows(h, sorted_rows, weights, rows, top)
     elif h.dtype is torch.bfloat16 and h.shape[1] % 8 == 0:
-        moe_gather_rows(h, sorted_rows, rows, top)
+        moe_gather_rows(h, sorted_rows, rows, top, fill=kernel != "tc")
     else:
         moe_gather_scaled_rows(h, sorted_rows, torch.ones((tokens, top), dtype=torch.float32, device=h.device), rows, top)
     act = torch.empty((capacity, inner), dtype=h.dtype, device=h.device)
@@ -2030,7 +2030,7 @@ def moe_experts(h: torch.Tensor, chosen: torch.Tensor, gate_up: torch.Tensor, do
         if not moe_tc_supported(h, gate_up, down, block):
             raise InvalidRequest("the experts' product for many rows needs bfloat16, blocks of 64 gate and up rows and sizes of a multiple of 8")
         rows = torch.empty((capacity, h.shape[1]), dtype=h.dtype, device=h.device)
-        moe_gather_rows(h, sorted_rows, rows, top)
+        moe_gather_rows(h, sorted_rows, rows, top, fill=False)
         moe_product_tc(rows, sorted_rows, tile_expert, gate_up, act, gated=True)
         moe_product_tc(act, sorted_rows, tile_expert, down, y, gated=False)
         return

@@ -944,6 +944,26 @@ def test_argmax_takes_the_smaller_id_on_a_tie():
     assert out.tolist() == want
 
 
+@pytest.mark.parametrize("tokens,top,routed,tile", [(1, 1, 1, 32), (5, 3, 33, 32), (2047, 4, 32, 128), (2048, 4, 200, 128), (2049, 4, 7, 128), (7001, 6, 64, 128)])
+def test_expert_lists_hold_every_pair_once(tokens, top, routed, tile):
+    """On both sides of the choices that one block's threads keep in registers, experts beyond a warp's, choices without weights
+    (numbers from `routed` on): every pair of a routed expert once, in tiles of its expert, the others nowhere."""
+    g = torch.Generator().manual_seed(tokens)
+    chosen = torch.randint(0, routed + 2, (tokens, top), generator=g, dtype=torch.int32)
+    capacity = kernels.moe_capacity(tokens * top, routed, tile)
+    rows = torch.full((capacity,), 77, dtype=torch.int32, device=DEV)
+    experts = torch.full((capacity // tile + 1,), 77, dtype=torch.int32, device=DEV)
+    kernels.moe_align(chosen.to(DEV), routed, tile, rows, experts)
+    rows, experts, flat = rows.cpu(), experts.cpu(), chosen.flatten()
+    assert sorted(rows[rows >= 0].tolist()) == (flat < routed).nonzero().flatten().tolist()
+    used = sum(-(-int((flat == e).sum()) // tile) for e in range(routed))
+    assert int(experts[-1]) == used and (experts[used:-1] == -1).all() and (rows[used * tile:] == -1).all()
+    for i in range(used):
+        listed = rows[i * tile:(i + 1) * tile]
+        assert (flat[listed[listed >= 0].long()] == experts[i]).all() and (listed >= 0).any()
+    assert experts[:used].tolist() == sorted(experts[:used].tolist())
+
+
 @pytest.mark.parametrize("vocab", [16384, 70001, 151936])
 def test_argmax_of_long_rows_shared_by_a_cluster(vocab):
     """Rows long enough to be shared by the blocks of a cluster: ties across shares, the last id,

@@ -5,14 +5,15 @@
 //
 // The library's product for these sizes runs near the tensor cores' peak, but it leaves its result in
 // memory, which a second kernel reads again (2,048 tokens: 150 MB and 34 us a layer).  Here a CTA computes a
-// tile of 128 tokens x 256 weight rows into one of two accumulators in tensor memory, and four warps turn a
+// tile of 128 tokens x 256 weight rows into one of two accumulators in tensor memory, and eight warps turn a
 // finished accumulator into the final values and store them while the next tile's MMAs run:
 //   warp 0   fetches 128 x 64 token tiles and 256 x 64 weight tiles with bulk tensor copies (TMA,
 //            128-byte swizzle) into a ring of stages;
 //   warp 1   one thread issues tcgen05.mma (M 128, N 256, K 16) on the stages;
-//   warps 2-5 a thread a token: the row's 256 sums from tensor memory.  A tile holds two blocks of 64 gate
+//   warps 2-9 two threads a token, 128 of its sums from tensor memory each.  A tile holds two blocks of 64 gate
 //            and 64 up rows (the weights are stored so), so a thread has both factors of its outputs; the plain
-//            product applies its activation to every sum.
+//            product applies its activation to every sum.  (One thread a token and full divisions: some 18,000 clocks a tile, longer
+//            than the MMAs of K = 2,048; N 6,144, K 1,024: 18.5 -> 14 us at 512 rows, 33 -> 24 at 2,000.)
 // CTAs are persistent; the tiles that share a weight tile are taken by neighbouring CTAs at the same
 // time, so the weights come from HBM once.  Every wait is bounded (tma.cuh).
 //   (reference: cuBLAS and a kernel of its own, crates/models/src/qwen3.rs:255-261; ops.cu:91-94)
@@ -25,7 +26,8 @@ constexpr int BN = 256;              // weight rows of a tile: two blocks of 64 
 constexpr int BK = 64;               // one 128-byte swizzled row of bfloat16
 constexpr int UMMA_K = 16;
 constexpr int STAGES = 4;
-constexpr int THREADS = 192;
+constexpr int EPILOGUE = 2;          // groups of four warps that share a tile's columns
+constexpr int THREADS = 64 + EPILOGUE * 128;
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int TMEM_COLUMNS = 2 * BN;
 constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + (2 * STAGES + 4) * sizeof(uint64_t) + 16;
@@ -40,7 +42,7 @@ __device__ __forceinline__ float activate(float z, int kind) {
 }
 
 // 0.5 z (1 + tanh(u)) = z / (1 + exp(-2 u)) with u = sqrt(2 / pi) (z + 0.044715 z^3)
-__device__ __forceinline__ float gelu_tanh_gate(float z) { return z / (1.0f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z))); }
+__device__ __forceinline__ float gelu_tanh_gate(float z) { return __fdividef(z, 1.0f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z))); }
 
 // ACT < 0: the gated product (-1: silu(gate) * up, -2: relu(gate) * up, -3: gelu with tanh); 0 to 4: the plain product with gelu (error
 // function), gelu (tanh), silu, relu or the square of relu on every sum.
@@ -67,7 +69,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_many_rows_kernel(
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4);
+            mbar_init(&acc_empty[b], 4 * EPILOGUE);
         }
         mbar_fence_init();
     }
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_many_rows_kernel(
             __syncwarp();
         }
     } else {
-        const int quarter = warp & 3;
+        const int quarter = warp & 3, group = (warp - 2) >> 2;
         const int row = quarter * 32 + lane;                 // token within the tile
         const int half_n = N >> 1;
         int round = 0;
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_many_rows_kernel(
             if constexpr (ACT >= 0) {
                 bf16* dst = out + (size_t)token * N + n0;
 #pragma unroll 2
-                for (int c = 0; c < BN; c += 32) {
+                for (int c = group * (BN / EPILOGUE); c < (group + 1) * (BN / EPILOGUE); c += 32) {
                     float v[32];
                     tmem_load_32_async(acc + c, v);
                     tmem_load_wait();
@@ -173,8 +175,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_many_rows_kernel(
                 }
             } else {
             bf16* dst = out + (size_t)token * half_n + (n0 >> 1);
-#pragma unroll
-            for (int block = 0; block < BN / 128; ++block) {          // 64 gate columns, then their 64 up columns
+            {
+                const int block = group;                              // 64 gate columns, then their 64 up columns
 #pragma unroll
                 for (int c = 0; c < 64; c += 32) {
                     float g[32], u[32];
@@ -192,8 +194,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_many_rows_kernel(
                                     ? __floats2bfloat162_rn(fmaxf(g0, 0.0f) * u[e + 2 * p], fmaxf(g1, 0.0f) * u[e + 2 * p + 1])
                                     : ACT == -3
                                     ? __floats2bfloat162_rn(gelu_tanh_gate(g0) * u[e + 2 * p], gelu_tanh_gate(g1) * u[e + 2 * p + 1])
-                                    : __floats2bfloat162_rn(g0 / (1.0f + __expf(-g0)) * u[e + 2 * p],
-                                                            g1 / (1.0f + __expf(-g1)) * u[e + 2 * p + 1]);
+                                    : __floats2bfloat162_rn(__fdividef(g0, 1.0f + __expf(-g0)) * u[e + 2 * p],
+                                                            __fdividef(g1, 1.0f + __expf(-g1)) * u[e + 2 * p + 1]);
                                 w[p] = *reinterpret_cast<uint32_t*>(&pair);
                             }
                             *reinterpret_cast<uint4*>(dst + block * 64 + c + e) = make_uint4(w[0], w[1], w[2], w[3]);

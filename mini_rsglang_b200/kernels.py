@@ -7,6 +7,7 @@ or without the compiled library, they raise `BackendError`."""
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 
@@ -901,6 +902,33 @@ _many_rows_maps: dict[tuple, tuple] = {}
 GEMM_GATED_ROWS_MIN = int(os.environ.get("MRS_GEMM_GATED_ROWS_MIN", "2048"))      # the variable: for measuring other crossovers
 GEMM_GATED_MEASURE = "MRS_GEMM_GATED_ROWS_MIN" not in os.environ                  # False: the kernel from that many rows on
 _gated_rows_choice: dict[tuple, bool] = {}
+
+
+def gemm_gated_rows_fills(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether the tcgen05 gate/up product takes fewer than GEMM_GATED_ROWS_MIN rows, by how well its tiles of 128 x 256 fill the SMs'
+    rounds with rows that are there.  On the device, with the library's product and `silu_mul` behind it:
+      one round            from 0.56 of the SMs on: N 6,144, K 1,024, 448 to 768 rows 11.3 to 11.5 against 11.7 to 14.1 us, 400 rows (0.51) 11.2
+                           against 11.0, 64 rows 9.8 against 7.7; N 16,384, K 2,048, 256 rows 18.8 against 20.5, 128 (0.43) 18.2 against 16.9
+      K > 2,048, one round up to 128 rows: the weights' bytes are the time, the activation's kernel comes on top (N 24,576, K 4,096, 17 to 128
+                           rows 38 to 40 against 38 to 42; N 34,816, K 5,120 58 to 61 against 64 to 71)
+      K > 2,048, more      the library's tiles are the better ones but where two rounds are full (N 24,576, K 4,096, 384 rows 65 against 76;
+                           350 rows 64 against 60, 512 85 against 79, 1,024 156 against 149)
+      K <= 2,048, more     from 0.72 on: N 16,384, K 2,048, 448 rows 29.8 against 31.0, 1,300 68 against 71, 400 rows (0.68) 29.1 against 27.2
+    Products smaller than the least measured one (N 4,096, K 1,024) stay with the library."""
+    rows = x.shape[0]
+    return 0 < rows < GEMM_GATED_ROWS_MIN and _rows_fill(rows, *weight.shape, sm_count(x.device)) and gemm_gated_rows_supported(x, weight)
+
+
+@functools.lru_cache(maxsize=4096)
+def _rows_fill(rows: int, n: int, k: int, sms: int) -> bool:
+    """`gemm_gated_rows_fills`, of the sizes."""
+    if n < 4096 or k < 1024:
+        return False
+    columns = -(-n // 256)
+    rounds, filled = -(-(-(-rows // 128) * columns) // sms), rows * columns / (128 * sms)
+    if rounds == 1:
+        return filled >= 0.56 or (k > 2048 and rows <= 128 and columns >= 0.6 * sms)
+    return filled >= (0.72 if k <= 2048 else 0.95 if rounds == 2 else math.inf) * rounds
 
 
 def gemm_gated_rows_wins(x: torch.Tensor, weight: torch.Tensor, gate: str = "silu") -> bool:

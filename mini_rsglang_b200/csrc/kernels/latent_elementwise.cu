@@ -229,7 +229,7 @@ __global__ void latent_prepare_kernel(const float* __restrict__ proj, int proj_w
 // The same with four neighbouring columns a thread and step: all sizes (and half of `rotary`, where element i turns with i + rotary / 2)
 // multiples of 4, rows of proj and of T on 16-byte boundaries, up to PREPARE_QUADS * 1,024 columns.  A token's loads are under way
 // together, ahead of the cosines and the norm.  2,048 tokens of 1,840 columns: 15.3 us an element a thread (two divisions and a dependent
-// load each), MEASURED_PREPARE here (23 MB).
+// load each), 13.1 us here (23 MB).
 constexpr int PREPARE_THREADS = 256, PREPARE_QUADS = 4;
 template <typename T>
 __global__ void __launch_bounds__(PREPARE_THREADS) latent_prepare_vec_kernel(

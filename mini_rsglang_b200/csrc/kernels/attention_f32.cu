@@ -12,14 +12,14 @@
 // the chunks' results (maximum, sum, weighted values) are joined in ascending order by the same arithmetic whether one block
 // walked them all or each had a block of its own (few rows with long contexts; a second kernel then joins them).
 //
-// Bound by the multiply-add pipe and shared memory for prompts; for decoded tokens by a tile's chain of page numbers, keys, scores,
-// weights and values.  Up to 8 rows take steps of two blocks: a warp a row and a block of scores, a column a thread, keys of two
-// steps and values of one ahead, page numbers three.  Chunks of 256 keys: of 512, 400 tokens walk 13 blocks in a row on a third of the
-// SMs (attention layer of the 0.6B shape 199 against 167 us; 20 tokens behind 980 126 against 78); of 128, the joining outweighs it (decoded
-// tokens of 4 requests at 3,000 98 against 92, 880 tokens behind 1,420 863 against 687 us).
-// Kernel alone, 16 query and 8 key/value heads of 128, before (a page's number looked up in front of every copy, one warp a row) and
-// now: one token behind 4,000 105 -> 18 + 5 us, 30 requests at 400 99 -> 38 + 3, a prompt of 777 tokens 168 -> 146 + 8.
-#include "common.cuh"
+// Heads of 128 elements run on the tensor cores (below).  The other sizes: bound by the multiply-add pipe and shared memory for prompts;
+// for decoded tokens by a tile's chain of page numbers, keys, scores, weights and values.  Up to 8 rows take steps of two blocks: a warp
+// a row and a block of scores, a column a thread, keys of two steps and values of one ahead, page numbers three.  Chunks of 256 keys: of
+// 512, 400 tokens walk 13 blocks in a row on a third of the SMs (attention layer with 16 heads of 128 on this kernel 199 against
+// 167 us; 20 tokens behind 980 126 against 78); of 128, the joining outweighs it (decoded tokens of 4 requests at 3,000 98 against 92, 880
+// tokens behind 1,420 863 against 687 us).
+#include "parts3.cuh"
+#include "tcgen05.cuh"
 
 #include <type_traits>
 
@@ -56,6 +56,50 @@ struct Args {
     float scale;
 };
 
+// The first token of the step's `tile`-th tile from the end (late tiles walk the most keys: they start first), its tokens in found[1];
+// -1: there are fewer tiles.  The whole block; what it used of shared memory before has been read.
+template <int BLOCK>
+__device__ int find_tile(const Args& A, int tile, int* found, int* warp_count) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto begins = [&](int t) {
+        if (t >= A.tokens) return true;
+        const int pos = A.positions[t];
+        return t == 0 || pos % A.tile_tokens == 0 || A.seq_of_token[t] != A.seq_of_token[t - 1] || pos != A.positions[t - 1] + 1;
+    };
+    __syncthreads();
+    if (tid == 0) found[0] = -1;
+    __syncthreads();
+    int before = 0;
+    for (int base = (A.tokens - 1) / BLOCK * BLOCK; base >= 0; base -= BLOCK) {
+        const int t = base + tid;
+        const bool first = t < A.tokens && begins(t);
+        const int here = __syncthreads_count(first);
+        if (before + here > tile) {
+            const int wanted = here - 1 - (tile - before);               // from the front of these
+            const unsigned mask = __ballot_sync(0xffffffffu, first);
+            if (lane == 0) warp_count[warp] = __popc(mask);
+            __syncthreads();
+            int ahead = 0;
+            for (int w = 0; w < warp; ++w) ahead += warp_count[w];
+            if (first && ahead + __popc(mask & ((1u << lane) - 1u)) == wanted) found[0] = t;
+            break;
+        }
+        before += here;
+    }
+    __syncthreads();
+    const int t0 = found[0];
+    if (t0 < 0) return -1;
+    if (tid < 32) {                                          // tokens of the tile
+        int count = A.tile_tokens;
+        for (int i = 1 + lane; i < A.tile_tokens; i += 32)
+            if (begins(t0 + i)) { count = i; break; }
+        count = __reduce_min_sync(0xffffffffu, count);
+        if (lane == 0) found[1] = count;
+    }
+    __syncthreads();
+    return t0;
+}
+
 // SPLIT: a block takes one chunk (blockIdx.z) of its tiles' keys and leaves its parts in part_o and part_ml; otherwise all of them.
 template <int D, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kernel(const Args A) {
@@ -72,44 +116,9 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
     pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = blockIdx.y, group = A.nq / A.nkv, d = A.d;
-    auto begins = [&](int t) {
-        if (t >= A.tokens) return true;
-        const int pos = A.positions[t];
-        return t == 0 || pos % A.tile_tokens == 0 || A.seq_of_token[t] != A.seq_of_token[t - 1] || pos != A.positions[t - 1] + 1;
-    };
     for (int tile = blockIdx.x;; tile += gridDim.x) {
-        // ---- the tile-th of the step's tiles from the end (late tiles walk the most keys: they start first) ------------------
-        __syncthreads();                                 // what the tile before used has been read
-        if (tid == 0) found[0] = -1;
-        __syncthreads();
-        int before = 0;
-        for (int base = (A.tokens - 1) / THREADS * THREADS; base >= 0; base -= THREADS) {
-            const int t = base + tid;
-            const bool first = t < A.tokens && begins(t);
-            const int here = __syncthreads_count(first);
-            if (before + here > tile) {
-                const int wanted = here - 1 - (tile - before);           // from the front of these
-                const unsigned mask = __ballot_sync(0xffffffffu, first);
-                if (lane == 0) warp_count[warp] = __popc(mask);
-                __syncthreads();
-                int ahead = 0;
-                for (int w = 0; w < warp; ++w) ahead += warp_count[w];
-                if (first && ahead + __popc(mask & ((1u << lane) - 1u)) == wanted) found[0] = t;
-                break;
-            }
-            before += here;
-        }
-        __syncthreads();
-        const int t0 = found[0];
+        const int t0 = find_tile<THREADS>(A, tile, found, warp_count);
         if (t0 < 0) return;
-        if (tid < 32) {                                  // tokens of the tile
-            int count = A.tile_tokens;
-            for (int i = 1 + lane; i < A.tile_tokens; i += 32)
-                if (begins(t0 + i)) { count = i; break; }
-            count = __reduce_min_sync(0xffffffffu, count);
-            if (lane == 0) found[1] = count;
-        }
-        __syncthreads();
         const int tokens = found[1], rows = tokens * group;
         const int pos0 = A.positions[t0], end_key = pos0 + tokens;
         int begin = A.window > 0 ? max(0, pos0 + 1 - A.window) : 0, end = end_key;       // keys that some row sees
@@ -434,6 +443,408 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Heads of 128 elements on the tcgen05 tensor cores, with every bit of the inputs: a float32 is three bfloat16 (parts3.cuh), a product
+// of two is six products of parts (the other three are below 2^-26 of it).  A block takes a tile of up to 128 rows and walks their keys
+// in blocks of 64:
+//   warps 0-7   two threads a row, 32 scores and 64 columns each: scores from tensor memory, maximum, exponentials, the weights' parts
+//               back into tensor memory; a block's weighted values (a fresh accumulator) are added to the row's in registers, in
+//               float32.  Between a block's scores and its softmax they write the next block's keys as bfloat16 tiles, so that its MMAs
+//               run under the softmax
+//   warps 8-10  the values' tiles (rows come by cp.async a block ahead, page numbers four)
+//   warp 11     issues the MMAs: scores = q parts (tensor memory) . keys, values = weights (tensor memory) . values
+// A row's result has the same bits however its request is cut: blocks of keys begin at multiples of 64, chunks at multiples of CHUNK, and
+// what a tile holds beside a row touches neither its scores nor its sums.  Values that bfloat16 has no parts for (infinite, NaN, beyond
+// its largest number) are zeros in the tiles and added by the rows that see them; a score that is no number or infinite is
+// computed again from its row and key, so that what a row does not see never reaches it.
+//
+// What bounds it: the parts' instructions and the chain of a block (some 7,000 clocks, of which the MMAs run 3,000), a CTA an SM.  Kernel
+// alone, 16 query and 8 key/value heads of 128, on the CUDA cores and here: a prompt of 777 tokens 146 -> 65 us, 880 tokens behind
+// 1,420 497 -> 205.  Decoded tokens pay for 128 rows: one behind 4,000 18 -> 25, 4 requests at 3,000 41 -> 77, 30 at 400 38 -> 75 (105, 112 and
+// 99 before either); they take this kernel for the bits' sake.  Error of the layer against 64 bits: 1.26e-6 -> 1.24e-6 (777 tokens).
+// Tried: all conversions in the copying warps (100 us at 777 tokens), masks and exponentials with a branch an element (softmax 10,700
+// clocks a block, 2,000 now).
+// ------------------------------------------------------------------------------------------------
+constexpr int TC_D = 128, TC_ROWS = 128, TC_KEYS = 64, TC_ROW_WARPS = 8, TC_COPY_WARPS = 3, TC_THREADS = (TC_ROW_WARPS + TC_COPY_WARPS + 1) * 32;
+constexpr int TC_PART = TC_KEYS * TC_D * 2, TC_RAW = TC_KEYS * TC_D * 4;         // bytes of a block's part, of its float32 rows
+constexpr int TC_S = 0, TC_O = TC_KEYS, TC_Q = TC_O + TC_D, TC_P = TC_Q + 3 * TC_D / 2, TC_TMEM = 512;      // columns of tensor memory
+constexpr size_t TC_SMEM = 1024 + 6 * (size_t)TC_PART + 2 * (size_t)TC_RAW + TC_KEYS * TC_ROWS * 4;
+static_assert(TC_P + 3 * TC_KEYS / 2 <= TC_TMEM, "tensor memory");
+static_assert(CHUNK % TC_KEYS == 0, "whole blocks a chunk");
+constexpr int TC_PLACES = 8, TC_AHEAD = 4;                               // blocks whose places are held; how far ahead they are looked up
+constexpr float BF16_MOST = 3.38953139e38f;
+
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// four floats as two words of each part; true where a part is not finite
+__device__ __forceinline__ bool split4(float4 v, uint2 (&parts)[3]) {
+#pragma unroll
+    for (int p = 0; p < 3; ++p) parts[p].x = take_part(v.x, v.y), parts[p].y = take_part(v.z, v.w);
+    const float left = (v.x + v.y) + (v.z + v.w);
+    return left != left;
+}
+
+// a row and a key that the parts cannot be trusted with
+__device__ __noinline__ float whole_score(const float* q, const float* k) {
+    float s = 0.0f;
+    for (int e = 0; e < TC_D; ++e) s = fmaf(q[e], k[e], s);
+    return s;
+}
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const Args A) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    unsigned char *k_parts = smem, *v_parts = smem + 3 * TC_PART, *k_raw = smem + 6 * TC_PART, *v_raw = k_raw + TC_RAW;
+    float* weights = reinterpret_cast<float*>(v_raw + TC_RAW);           // [TC_KEYS][TC_ROWS], read where values have no parts
+    // v_full: two in turn, so that the rows too may wait for it (what the copying warps left for them is then there)
+    __shared__ uint64_t k_full, s_full, p_full, v_full[2], o_full;
+    __shared__ uint32_t tmem_slot;
+    __shared__ long long place_s[TC_PLACES][TC_KEYS];                    // where cached rows begin; -1: not seen
+    __shared__ float met[2][2][TC_ROWS];
+    __shared__ unsigned odd_values[2][TC_KEYS / 32];                     // keys whose values have no parts
+    __shared__ int found[2], warp_count[TC_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int ISSUER = TC_ROW_WARPS + TC_COPY_WARPS;
+    if (tid == 0) {
+        mbar_init(&k_full, TC_ROW_WARPS);
+        for (int b = 0; b < 2; ++b) mbar_init(&v_full[b], TC_COPY_WARPS);
+        mbar_init(&s_full, 1);
+        mbar_init(&p_full, TC_ROW_WARPS);
+        mbar_init(&o_full, 1);
+        mbar_fence_init();
+    }
+    if (warp == ISSUER) {
+        tmem_alloc(&tmem_slot, TC_TMEM);
+        tmem_relinquish_alloc_permit();
+    }
+    tcgen05_fence_before_sync();
+    __syncthreads();
+    tcgen05_fence_after_sync();
+    const uint32_t tmem = tmem_slot, lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int g = blockIdx.y, group = A.nq / A.nkv;
+    int it = 0;                                                          // blocks of keys so far, over all tiles
+    for (int tile = blockIdx.x;; tile += gridDim.x) {
+        const int t0 = find_tile<TC_THREADS>(A, tile, found, warp_count);
+        if (t0 < 0) break;
+        const int tokens = found[1], rows = tokens * group;
+        const int pos0 = A.positions[t0], end_key = pos0 + tokens;
+        int begin = A.window > 0 ? max(0, pos0 + 1 - A.window) : 0, end = end_key;
+        if (SPLIT) {
+            begin = max(begin, (int)blockIdx.z * CHUNK);                 // keys beyond the last chunk that was planned go with it
+            if ((int)blockIdx.z + 1 < A.chunks) end = min(end, ((int)blockIdx.z + 1) * CHUNK);
+            if (begin >= end) continue;
+        }
+        const int at0 = begin / TC_KEYS * TC_KEYS, blocks = (end - at0 + TC_KEYS - 1) / TC_KEYS;
+        const int* pages = A.table + (size_t)A.seq_of_token[t0] * A.table_width;
+        auto place_of = [&](int p) -> long long {
+            if (p < begin || p >= end) return -1;
+            return (((long long)pages[p / A.page_size] * A.nkv + g) * A.page_size + p % A.page_size) * TC_D;
+        };
+        if (tid < TC_AHEAD * TC_KEYS) place_s[(it + tid / TC_KEYS) % TC_PLACES][tid % TC_KEYS] = place_of(at0 + tid);
+        __syncthreads();
+        // rows `mine`, mine + COUNT, ... of a block: a lane four of a row's elements, which it fetches and converts itself
+        auto fetch = [&](auto count, const float* cache, unsigned char* raw, int mine, int i, bool wanted) {
+            constexpr int COUNT = decltype(count)::value;
+            if (wanted) {
+#pragma unroll 4
+                for (int row = mine; row < TC_KEYS; row += COUNT) {
+                    const long long place = place_s[i % TC_PLACES][row];
+                    copy16(reinterpret_cast<float*>(raw) + row * TC_D + 4 * lane, cache + (place >= 0 ? place + 4 * lane : 0), place >= 0);
+                }
+            }
+            copies_commit();
+        };
+        const uint32_t part_at = (lane >> 4) * (TC_PART / 2) + (lane & 1) * 8, piece = (lane & 15) >> 1;
+        auto put = [&](unsigned char* to, int row, float4 v) {
+            uint2 parts[3];
+            const bool odd = split4(v, parts);
+            to += part_at + row * 128 + ((piece ^ (row & 7)) << 4);
+#pragma unroll
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(to + p * TC_PART) = parts[p];
+            return odd;
+        };
+        auto raw_of = [&](const unsigned char* raw, int row) { return *reinterpret_cast<const float4*>(raw + row * TC_D * 4 + 16 * lane); };
+        // some read together; whether one of them has no parts
+        auto convert = [&](auto count, unsigned char* to, const unsigned char* raw, int mine) {
+            constexpr int COUNT = decltype(count)::value, TOGETHER = 4;
+            bool odd = false;
+#pragma unroll 1
+            for (int first = mine; first < TC_KEYS; first += TOGETHER * COUNT) {
+                float4 v[TOGETHER];
+#pragma unroll
+                for (int r = 0; r < TOGETHER; ++r) v[r] = raw_of(raw, min(first + r * COUNT, TC_KEYS - 1));
+#pragma unroll
+                for (int r = 0; r < TOGETHER; ++r)
+                    if (first + r * COUNT < TC_KEYS) odd |= put(to, first + r * COUNT, v[r]);
+            }
+            return odd;
+        };
+        constexpr std::integral_constant<int, TC_ROW_WARPS> by_rows;
+        constexpr std::integral_constant<int, TC_COPY_WARPS> by_copies;
+        if (warp == ISSUER) {
+            const bool leader = elect_one();
+            constexpr uint32_t s_desc = umma_idesc_bf16_f32(TC_ROWS, TC_KEYS), o_desc = umma_idesc_bf16_f32(TC_ROWS, TC_D, true);
+            constexpr int order[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};      // (part of A, part of B): small products first
+            auto scores = [&](int i) {
+                mbar_wait(&k_full, i & 1);
+                tcgen05_fence_after_sync();
+                if (leader) {
+#pragma unroll 1
+                    for (int j = 0; j < 6; ++j) {
+                        const uint32_t a = tmem + TC_Q + order[j][0] * (TC_D / 2), b = smem_u32(k_parts) + order[j][1] * TC_PART;
+#pragma unroll
+                        for (int k = 0; k < TC_D / 16; ++k)              // two groups of 64 columns
+                            umma_bf16_a_tmem(tmem + TC_S, a + 8 * k, umma_smem_desc_sw128(b + (k / 4) * (TC_PART / 2)) + 2 * (k % 4), s_desc, j > 0 || k > 0);
+                    }
+                    umma_commit(&s_full);
+                }
+                __syncwarp();
+            };
+            scores(it);
+            for (int n = 0; n < blocks; ++n) {
+                if (n + 1 < blocks) scores(it + n + 1);
+                mbar_wait(&p_full, (it + n) & 1);
+                mbar_wait(&v_full[(it + n) & 1], (it + n) >> 1 & 1);
+                tcgen05_fence_after_sync();
+                if (leader) {
+#pragma unroll 1
+                    for (int j = 0; j < 6; ++j) {
+                        const uint32_t a = tmem + TC_P + order[j][0] * (TC_KEYS / 2), b = smem_u32(v_parts) + order[j][1] * TC_PART;
+#pragma unroll
+                        for (int k = 0; k < TC_KEYS / 16; ++k)
+                            umma_bf16_a_tmem(tmem + TC_O, a + 8 * k, umma_smem_desc_sw128_mn(b + k * 16 * 128, TC_PART / 2), o_desc, j > 0 || k > 0);
+                    }
+                    umma_commit(&o_full);
+                }
+                __syncwarp();
+            }
+        } else if (warp >= TC_ROW_WARPS) {
+            const int mine = warp - TC_ROW_WARPS, ct = tid - TC_ROW_WARPS * 32;
+            fetch(by_copies, A.v, v_raw, mine, it, true);
+            for (int n = 0; n < blocks; ++n) {
+                const int i = it + n;
+                const long long later = ct < TC_KEYS ? place_of(at0 + (n + TC_AHEAD) * TC_KEYS + ct) : -1;
+                copies_wait<0>();
+                if (i > 0) mbar_wait(&o_full, (i - 1) & 1);              // the values' parts have been read, and the odd values two blocks before
+                if (ct < TC_KEYS / 32) odd_values[i & 1][ct] = 0u;
+                if (ct < TC_KEYS) place_s[(i + TC_AHEAD) % TC_PLACES][ct] = later;
+                bar_sync(1, TC_COPY_WARPS * 32);
+                if (convert(by_copies, v_parts, v_raw, mine)) {
+#pragma unroll 1
+                    for (int row = mine; row < TC_KEYS; row += TC_COPY_WARPS) {
+                        float4 v = raw_of(v_raw, row);
+                        if (!put(v_parts, row, v)) continue;
+                        if (!(fabsf(v.x) < BF16_MOST)) v.x = 0.0f;
+                        if (!(fabsf(v.y) < BF16_MOST)) v.y = 0.0f;
+                        if (!(fabsf(v.z) < BF16_MOST)) v.z = 0.0f;
+                        if (!(fabsf(v.w) < BF16_MOST)) v.w = 0.0f;
+                        put(v_parts, row, v);
+                        atomicOr(&odd_values[i & 1][row / 32], 1u << (row % 32));
+                    }
+                }
+                fence_async_shared();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&v_full[i & 1]);
+                fetch(by_copies, A.v, v_raw, mine, i + 1, n + 1 < blocks);
+            }
+            copies_wait<0>();
+        } else {
+            const int row = (warp & 3) * 32 + lane, half = warp >> 2, pair_bar = 2 + (warp & 3);
+            const bool live = row < rows;
+            const size_t row_at = (size_t)(t0 + (live ? row / group : 0)) * A.nq + g * group + (live ? row % group : 0);
+            const float* q = A.q + row_at * TC_D;
+            fetch(by_rows, A.k, k_raw, warp, it, true);
+#pragma unroll 1
+            for (int c = 0; c < 64; c += 32) {
+                uint32_t words[3][16];
+#pragma unroll
+                for (int e = 0; e < 32; e += 4) {
+                    uint2 parts[3];
+                    split4(live ? *reinterpret_cast<const float4*>(q + half * 64 + c + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f), parts);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) words[p][e / 2] = parts[p].x, words[p][e / 2 + 1] = parts[p].y;
+                }
+#pragma unroll
+                for (int p = 0; p < 3; ++p) tmem_store_16_words(lanes + TC_Q + p * (TC_D / 2) + half * 32 + c / 2, words[p]);
+            }
+            tmem_store_wait();
+            // block i's keys as parts: q is there, and the scores of the block before have been read
+            auto keys_ready = [&](int i, bool more) {
+                copies_wait<0>();
+                convert(by_rows, k_parts, k_raw, warp);
+                fence_async_shared();
+                tcgen05_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&k_full);
+                fetch(by_rows, A.k, k_raw, warp, i + 1, more);
+            };
+            keys_ready(it, blocks > 1);
+            const int my_pos = live ? pos0 + row / group : -1, my_first = A.window > 0 ? max(0, my_pos + 1 - A.window) : 0;
+            float o[64];
+#pragma unroll
+            for (int c = 0; c < 64; ++c) o[c] = 0.0f;
+            float m = -CUDART_INF_F, l = 0.0f, m_all = -CUDART_INF_F, l_all = 0.0f;
+            bool joined = false;
+            // block i's weighted values join the row's
+            auto take_values = [&](int i) {
+                mbar_wait(&v_full[i & 1], i >> 1 & 1);
+                mbar_wait(&o_full, i & 1);
+                __syncwarp();
+                tcgen05_fence_after_sync();
+#pragma unroll
+                for (int c = 0; c < 64; c += 16) {
+                    float v[16];
+                    tmem_load_16_async(lanes + TC_O + half * 64 + c, v);
+                    tmem_load_wait();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) o[c + e] += v[e];
+                }
+                if (odd_values[i & 1][0] | odd_values[i & 1][1]) {
+                    bar_sync(pair_bar, 64);                              // the other half's weights are there
+#pragma unroll 1
+                    for (int k = 0; k < TC_KEYS; ++k) {
+                        if (!(odd_values[i & 1][k / 32] >> (k % 32) & 1u)) continue;
+                        const float w = weights[k * TC_ROWS + row];
+                        const long long place = place_s[i % TC_PLACES][k];
+                        if (w == 0.0f || place < 0) continue;
+#pragma unroll
+                        for (int c = 0; c < 64; ++c) {
+                            const float v = A.v[place + half * 64 + c];
+                            if (!(fabsf(v) < BF16_MOST)) o[c] = fmaf(w, v, o[c]);
+                        }
+                    }
+                    bar_sync(pair_bar, 64);
+                }
+            };
+            auto whole_sum = [&]() {                                     // both halves' sums; `met` is free: every exchange was read
+                bar_sync(pair_bar, 64);
+                met[0][half][row] = l;
+                bar_sync(pair_bar, 64);
+                return met[0][0][row] + met[0][1][row];
+            };
+            float* out = A.out + row_at * TC_D + half * 64;
+            auto join_chunk = [&]() {                                    // !SPLIT: the chunk joins those before it, which lie in `out`
+                const float sum = whole_sum();
+                const float next = fmaxf(m_all, m), keep = m_all == next ? 1.0f : ratio(m_all, next), take = ratio(m, next);
+                l_all = join(l_all, keep, sum, take);
+                m_all = next;
+                if (live) {
+#pragma unroll
+                    for (int c = 0; c < 64; c += 4) {
+                        float4 total = joined ? *reinterpret_cast<const float4*>(out + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        total = make_float4(join(total.x, keep, o[c], take), join(total.y, keep, o[c + 1], take), join(total.z, keep, o[c + 2], take),
+                                            join(total.w, keep, o[c + 3], take));
+                        *reinterpret_cast<float4*>(out + c) = total;
+                    }
+                }
+                joined = true;
+                m = -CUDART_INF_F, l = 0.0f;
+#pragma unroll
+                for (int c = 0; c < 64; ++c) o[c] = 0.0f;
+            };
+            bool pending = false;                                        // a block's values are still to come
+#pragma unroll 1
+            for (int n = 0; n < blocks; ++n) {
+                const int i = it + n, at = at0 + n * TC_KEYS;
+                if (!SPLIT && n > 0 && at % CHUNK == 0) {
+                    take_values(i - 1);
+                    join_chunk();
+                    pending = false;
+                }
+                float x[32], top = -CUDART_INF_F;
+                mbar_wait(&s_full, i & 1);
+                __syncwarp();
+                tcgen05_fence_after_sync();
+                tmem_load_32(lanes + TC_S + half * 32, x);
+                if (n + 1 < blocks) keys_ready(i + 1, n + 2 < blocks);
+                bool odd = false;
+#pragma unroll
+                for (int u = 0; u < 32; ++u) odd |= !(fabsf(x[u]) <= 3.402823466e38f);
+                if (__any_sync(0xffffffffu, odd)) {                      // parts beyond bfloat16's range: the rows and the keys themselves
+#pragma unroll
+                    for (int u = 0; u < 32; ++u) {
+                        const int key = at + half * 32 + u;
+                        if (key <= my_pos && key >= my_first && !(fabsf(x[u]) <= 3.402823466e38f)) x[u] = whole_score(q, A.k + place_s[i % TC_PLACES][half * 32 + u]);
+                    }
+                }
+                if (at + TC_KEYS > pos0 + 1 || (A.window > 0 && at < end_key - A.window)) {       // some row does not see all of the block
+                    const int last = my_pos - (at + half * 32), first = my_first - (at + half * 32);
+#pragma unroll
+                    for (int u = 0; u < 32; ++u) x[u] = u <= last && u >= first ? x[u] * A.scale : -CUDART_INF_F;
+                } else if (live) {
+#pragma unroll
+                    for (int u = 0; u < 32; ++u) x[u] *= A.scale;
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 32; ++u) x[u] = -CUDART_INF_F;
+                }
+#pragma unroll
+                for (int u = 0; u < 32; ++u) top = fmaxf(top, x[u]);
+                met[i & 1][half][row] = top;
+                bar_sync(pair_bar, 64);
+                top = fmaxf(top, met[i & 1][half ^ 1][row]);
+                const float next = fmaxf(m, top), alpha = m == next ? 1.0f : ratio(m, next);
+                float sum = 0.0f;
+                const float from = next == -CUDART_INF_F ? 0.0f : next;  // nothing seen yet: zeros
+#pragma unroll
+                for (int u = 0; u < 32; ++u) x[u] = expf(x[u] - from);
+#pragma unroll
+                for (int u = 0; u < 32; ++u) sum += x[u];
+                l = l * alpha + sum;
+                m = next;
+                if (pending) take_values(i - 1);
+#pragma unroll
+                for (int c = 0; c < 64; ++c) o[c] *= alpha;
+#pragma unroll
+                for (int u = 0; u < 32; ++u) weights[(half * 32 + u) * TC_ROWS + row] = x[u];
+                uint32_t words[16];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+#pragma unroll
+                    for (int u = 0; u < 32; u += 2) words[u / 2] = take_part(x[u], x[u + 1]);
+                    tmem_store_16_words(lanes + TC_P + p * (TC_KEYS / 2) + half * 16, words);
+                }
+                tmem_store_wait();
+                tcgen05_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&p_full);
+                pending = true;
+            }
+            copies_wait<0>();
+            take_values(it + blocks - 1);
+            if (SPLIT) {
+                const float sum = whole_sum();
+                if (live) {
+                    const size_t place = row_at * A.chunks + blockIdx.z;
+                    if (half == 0) A.part_ml[2 * place] = m, A.part_ml[2 * place + 1] = sum;
+#pragma unroll
+                    for (int c = 0; c < 64; c += 4)
+                        *reinterpret_cast<float4*>(A.part_o + place * TC_D + half * 64 + c) = make_float4(o[c], o[c + 1], o[c + 2], o[c + 3]);
+                }
+            } else {
+                join_chunk();
+                const float inv = 1.0f / l_all;
+                if (live) {
+#pragma unroll
+                    for (int c = 0; c < 64; c += 4) {
+                        const float4 total = *reinterpret_cast<const float4*>(out + c);
+                        *reinterpret_cast<float4*>(out + c) = make_float4(total.x * inv, total.y * inv, total.z * inv, total.w * inv);
+                    }
+                }
+            }
+        }
+        it += blocks;
+    }
+    tcgen05_fence_before_sync();
+    __syncthreads();
+    if (warp == ISSUER) {
+        tcgen05_fence_after_sync();
+        tmem_dealloc(tmem, TC_TMEM);
+    }
+}
+
 // Joins a row's chunks in ascending order: a warp a (token, head).
 __global__ void attention_f32_join_kernel(const Args A) {
     pdl_launch_dependents();
@@ -484,7 +895,23 @@ int launch(const Args& A, int tiles, void* stream) {
     MRS_RETURN_LAUNCH_STATUS();
 }
 
+template <bool SPLIT>
+int launch_tc(const Args& A, int tiles, void* stream) {
+    static PerDevice configured;
+    if (!configured.get()) {
+        const cudaError_t e = cudaFuncSetAttribute(attention_f32_tc_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured.set(1);
+    }
+    MRS_LAUNCH(attention_f32_tc_kernel<SPLIT>, dim3(tiles, A.nkv, SPLIT ? A.chunks : 1), TC_THREADS, TC_SMEM, stream, A);
+    MRS_RETURN_LAUNCH_STATUS();
+}
+
 }  // namespace
+
+MRS_EXPORT int mrs_attention_f32_take_error(unsigned int* word) { return mrs_take_error_word(word); }
+// Mirrors the error word into a word of pinned host memory from now on.
+MRS_EXPORT int mrs_attention_f32_mirror_errors(unsigned int* host_word) { return mrs_set_error_mirror(host_word); }
 
 MRS_EXPORT int mrs_attention_f32_chunk() { return CHUNK; }
 
@@ -500,13 +927,15 @@ MRS_EXPORT int mrs_attention_f32(const float* q, const float* k_cache, const flo
     Args A = {};
     A.q = q, A.k = k_cache, A.v = v_cache, A.positions = positions, A.seq_of_token = seq_of_token, A.table = block_table, A.out = out;
     A.tokens = tokens, A.nq = nq, A.nkv = nkv, A.d = d, A.page_size = page_size, A.table_width = table_width, A.window = window, A.scale = scale;
-    A.tile_tokens = ROWS / (nq / nkv);
+    const bool tc = d == TC_D;
+    A.tile_tokens = (tc ? TC_ROWS : ROWS) / (nq / nkv);
     A.chunks = parts ? chunks : 1;
     A.part_o = parts, A.part_ml = parts ? parts + (size_t)tokens * nq * chunks * d : nullptr;
     // a request's rows make at most two tiles that are not whole; rows that lie otherwise make more, and blocks take several
     const long long most = (long long)tokens / A.tile_tokens + 2LL * sequences + 1;
     const int tiles = (int)(most < tokens ? most : tokens);
-    const int code = d <= 64 ? (parts ? launch<64, true>(A, tiles, stream) : launch<64, false>(A, tiles, stream))
+    const int code = tc ? (parts ? launch_tc<true>(A, tiles, stream) : launch_tc<false>(A, tiles, stream))
+                   : d <= 64 ? (parts ? launch<64, true>(A, tiles, stream) : launch<64, false>(A, tiles, stream))
                    : d <= 128 ? (parts ? launch<128, true>(A, tiles, stream) : launch<128, false>(A, tiles, stream))
                               : (parts ? launch<256, true>(A, tiles, stream) : launch<256, false>(A, tiles, stream));
     if (code != 0 || !parts) return code;

@@ -21,6 +21,7 @@
 
 #include <cfloat>
 
+#include "parts3.cuh"
 #include "tcgen05.cuh"
 
 namespace {
@@ -66,10 +67,6 @@ __device__ __forceinline__ void tmem_load_8_async(uint32_t address, float* v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(address) : "memory");
 }
-// x += y, two floats of a register pair at a time
-__device__ __forceinline__ void add_pair(float& x0, float& x1, float y0, float y1) {
-    asm("{\n .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %3};\n add.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}" : "+f"(x0), "+f"(x1) : "f"(y0), "f"(y1));
-}
 template <int C>
 __device__ __forceinline__ void add_columns(uint32_t address, float (&sum)[C]) {
     constexpr int STEP = C % 16 == 0 ? 16 : C < 8 ? C : 8;
@@ -88,14 +85,6 @@ __device__ __forceinline__ void add_columns(uint32_t address, float (&sum)[C]) {
 // 16 lanes x 8 columns: a thread has two columns, 2 (lane % 4) and the next, of lanes lane / 4 and 8 further.
 __device__ __forceinline__ void tmem_store_16x8(uint32_t address, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1, %2, %3, %4};" ::"r"(address), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
-// Two floats as three pairs of bfloat16; what a rounding leaves is exact in float32.  Beyond bfloat16's range the parts are no numbers.
-__device__ __forceinline__ uint32_t take_part(float& x, float& y) {
-    const __nv_bfloat162 pair = __floats2bfloat162_rn(x, y);
-    const uint32_t bits = *reinterpret_cast<const uint32_t*>(&pair);
-    add_pair(x, y, -__uint_as_float(bits << 16), -__uint_as_float(bits & 0xFFFF0000u));
-    return bits;
 }
 
 // The whole warp: a . w over K in float64.

@@ -58,7 +58,10 @@ def library() -> ctypes.CDLL:
         lib.mrs_gemm_f32_take_error.argtypes = [ctypes.POINTER(ctypes.c_uint)]
         lib.mrs_gemm_f32_take_error.restype = _c_int
         _lib = lib
+        lib.mrs_attention_f32_take_error.argtypes = [ctypes.POINTER(ctypes.c_uint)]
+        lib.mrs_attention_f32_take_error.restype = _c_int
         _register_error_word("gemm_f32", lib, "mrs_gemm_f32")
+        _register_error_word("attention_f32", lib, "mrs_attention_f32")
     return _lib
 
 

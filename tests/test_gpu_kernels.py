@@ -1362,3 +1362,62 @@ def test_attention_f32_keeps_what_is_no_number_in_its_row():
         assert torch.isnan(got[token, head]).all()
         got[token, head] = clean[token, head]
     assert torch.equal(got, clean)
+
+
+@pytest.mark.parametrize("whole", [False, True])
+@pytest.mark.parametrize("window", [0, 300])
+def test_attention_f32_on_tensor_cores_of_values_without_parts(monkeypatch, window, whole):
+    """Heads of 128: queries, keys and values that bfloat16 has no parts for (infinite, NaN, beyond its largest number), chunks in
+    blocks of their own and in one walk.  What sees such a value has it in that column alone, what does not has the same bits as
+    without it; a score of such a key is the score of its elements."""
+    if whole:
+        monkeypatch.setattr(kernels, "ATTENTION_F32_PARTS_BYTES", 0)
+    nq, nkv, d, page = 4, 2, 128, 16
+    spans = [(0, 200), (700, 3), (400, 70)]
+    case = PagedCase(torch.float32, nq, nkv, d, page, spans, seed=11, window=window)
+    clean = case.run_simt().view(-1, nq, d)
+    position, seq = case.positions, case.seq
+
+    def sees(request, key):
+        return (seq == request) & (position >= key) & ((position < key + window) if window else True)
+
+    # a query that is no number: its own (token, head) alone
+    kept = case.q.clone()
+    case.q.view(-1, nq, d)[201, 2, 7] = math.nan
+    got = case.run_simt().view(-1, nq, d)
+    assert got[201, 2].isnan().all()
+    got[201, 2] = clean[201, 2]
+    assert torch.equal(got, clean)
+    case.q = kept
+    # values: of request 0 key 150 (head 1), request 1 key 690 (head 0), request 2 keys 410 and 411
+    marks = ((0, 150, 1, 9, math.inf), (1, 690, 0, 3, math.nan), (2, 410, 1, 100, -math.inf), (2, 411, 0, 64, 3.4e38))
+    kept = case.vc.clone()
+    for request, key, head, column, value in marks:
+        case.vc[case.table[request, key // page], head, key % page, column] = value
+    got = case.run_simt().view(-1, nq, d)
+    expected = clean.clone()
+    for request, key, head, column, value in marks:
+        rows, heads = sees(request, key).nonzero().flatten().tolist(), (2 * head, 2 * head + 1)
+        assert rows
+        for row in rows:
+            for h in heads:
+                x = float(got[row, h, column])
+                if math.isnan(value):
+                    assert math.isnan(x)
+                elif math.isinf(value):
+                    assert x == value
+                else:                                        # a weight times the value: from the row's weights in 64 bits
+                    keys = torch.arange(max(0, int(position[row]) + 1 - window) if window else 0, int(position[row]) + 1)
+                    score = case.ks[request][keys, head].double() @ case.q.view(-1, nq, d)[row, h].double() * d ** -0.5
+                    want = float(torch.softmax(score, 0)[keys.tolist().index(key)]) * value
+                    assert abs(x - want) <= 1e-4 * abs(want)
+                got[row, h, column] = expected[row, h, column]
+    assert torch.equal(got, expected)
+    case.vc = kept
+    # keys: an element beyond bfloat16's range met by a tiny query, and -inf, whose weight is nothing
+    q = case.q.view(-1, nq, d)
+    q[:, :, 5] = 1e-38
+    for request, key, value in ((0, 60, 3.4e38), (1, 650, -3.4e38), (2, 420, -math.inf)):
+        case.kc[case.table[request, key // page], 0, key % page, 5] = value
+        case.ks[request][key, 0, 5] = value
+    close(case.run_simt(), case.plain(), torch.float32, "attention_f32")

@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
 
 // ------------------------------------------------------------------------------------------------
 // Heads of 128 elements on the tcgen05 tensor cores, with every bit of the inputs: a float32 is three bfloat16 (parts3.cuh), a product
-// of two is six products of parts (the other three are below 2^-26 of it).  A block takes a tile of up to 128 rows and walks their keys
+// of two is six products of parts (the other three are some 2^-26 of it).  A block takes a tile of up to 128 rows and walks their keys
 // in blocks of 64:
 //   warps 0-7   two threads a row, 32 scores and 64 columns each: scores from tensor memory, maximum, exponentials, the weights' parts
 //               back into tensor memory; a block's weighted values (a fresh accumulator) are added to the row's in registers, in
@@ -456,7 +456,8 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
 // A row's result has the same bits however its request is cut: blocks of keys begin at multiples of 64, chunks at multiples of CHUNK, and
 // what a tile holds beside a row touches neither its scores nor its sums.  Values that bfloat16 has no parts for (infinite, NaN, beyond
 // its largest number) are zeros in the tiles and added by the rows that see them; a score that is no number or infinite is
-// computed again from its row and key, so that what a row does not see never reaches it.
+// computed again from its row and key, so that what a row does not see never reaches it. (Below 2^-110 a value's last part lies
+// under bfloat16's range: such values keep fewer bits of their own, 2^-134 off at most.)
 //
 // What bounds it: the parts' instructions and the chain of a block (some 7,000 clocks, of which the MMAs run 3,000), a CTA an SM.  Kernel
 // alone, 16 query and 8 key/value heads of 128, on the CUDA cores and here: a prompt of 777 tokens 146 -> 65 us, 880 tokens behind
@@ -477,8 +478,10 @@ constexpr float BF16_MOST = 3.38953139e38f;
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 // four floats as two words of each part; true where a part is not finite
 __device__ __forceinline__ bool split4(float4 v, uint2 (&parts)[3]) {
+    uint32_t low[3], high[3];
+    three_parts(v.x, v.y, low), three_parts(v.z, v.w, high);
 #pragma unroll
-    for (int p = 0; p < 3; ++p) parts[p].x = take_part(v.x, v.y), parts[p].y = take_part(v.z, v.w);
+    for (int p = 0; p < 3; ++p) parts[p] = make_uint2(low[p], high[p]);
     const float left = (v.x + v.y) + (v.z + v.w);
     return left != left;
 }
@@ -799,13 +802,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
                 for (int c = 0; c < 64; ++c) o[c] *= alpha;
 #pragma unroll
                 for (int u = 0; u < 32; ++u) weights[(half * 32 + u) * TC_ROWS + row] = x[u];
-                uint32_t words[16];
+                uint32_t words[3][16];
 #pragma unroll
-                for (int p = 0; p < 3; ++p) {
+                for (int u = 0; u < 32; u += 2) {
+                    uint32_t parts[3];
+                    three_parts(x[u], x[u + 1], parts);
 #pragma unroll
-                    for (int u = 0; u < 32; u += 2) words[u / 2] = take_part(x[u], x[u + 1]);
-                    tmem_store_16_words(lanes + TC_P + p * (TC_KEYS / 2) + half * 16, words);
+                    for (int p = 0; p < 3; ++p) words[p][u / 2] = parts[p];
                 }
+#pragma unroll
+                for (int p = 0; p < 3; ++p) tmem_store_16_words(lanes + TC_P + p * (TC_KEYS / 2) + half * 16, words[p]);
                 tmem_store_wait();
                 tcgen05_fence_before_sync();
                 __syncwarp();

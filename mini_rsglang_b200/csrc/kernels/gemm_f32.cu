@@ -2,19 +2,19 @@
 // projection of the 32-bit path.
 //
 // A float32 is the sum of three bfloat16 (8 + 8 + 8 bits of its significand), so a product of two is nine products of bfloat16, each
-// exact in float32.  Six of them are computed; the other three are below 2^-26 of the product together.  The MMAs add 32
+// exact in float32.  Six of them are computed; the other three are some 2^-26 of the product.  The MMAs add 32
 // elements of K at a time into a fresh accumulator in tensor memory, small products first, and from there on a sum is ordinary
 // float32 addition in registers: 32-element sums into one of four ranges of K, the four ranges in order.  An element's bits depend
 // on K alone: not on M, not on the tile or the cut that the sizes chose, and a token's result does not change with what else is in the
 // batch.  A result that is no number or infinite, or below 2^-60 where a part of a factor may lie under bfloat16's range, is computed
 // again in float64 from the inputs (`exact_dot`), so infinities and NaN are those of the sum of the products.
 //
-// What bounds it: the workers' instructions (a float32 into three bfloat16 is some thirty instructions for four elements, and the
+// What bounds it: the workers' instructions (a float32 into three bfloat16 is some twenty-five instructions for four elements, and the
 // sums), then shared memory (both matrices pass through it; parts of W lie in tensor memory, which took a step of 96 tokens from 0.80 to
 // 0.70 us).  One turn of writers instead of two that overlap: 24 against 19 us for 8 rows in one CTA a tile.  Tiles of 128 tokens
 // spill registers (90 against 63 us for 777 rows, N 4,096, K 1,024).
-// Alone, before (multiply-adds on the CUDA cores) and now: N 4,096, K 1,024: 1 row 15 -> 11 us, 64 rows 35 -> 12, 128 rows 38 -> 18, 777
-// rows 168 -> 63; N 1,024, K 2,048: 8 rows 18.5 -> 12.8, 777 rows 121 -> 34; N 6,144, K 1,024, 777 rows 263 -> 93.  Error against 64
+// Alone, before (multiply-adds on the CUDA cores) and now: N 4,096, K 1,024: 1 row 15 -> 10.5 us, 64 rows 35 -> 11.5, 128 rows 38 -> 18, 777
+// rows 168 -> 61; N 1,024, K 2,048: 8 rows 18.5 -> 12.3, 777 rows 121 -> 33; N 6,144, K 1,024, 777 rows 263 -> 90.  Error against 64
 // bits (relative, normal inputs): K = 1,024 5.7e-7 -> 0.9e-7, K = 3,072 1.0e-6 -> 1.2e-7.
 //             (reference: cuBLAS, kernels/src/lib.rs:298-321)
 #include <cooperative_groups.h>
@@ -228,21 +228,21 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __res
 #pragma unroll
                 for (int j = 0; j < T::W_MINE; j += 2) {     // 16 lanes
                     float4 x = *reinterpret_cast<const float4*>(from + j * WRITERS * 16), y = *reinterpret_cast<const float4*>(from + (j + 1) * WRITERS * 16);
+                    uint32_t x0[PARTS], x1[PARTS], y0[PARTS], y1[PARTS];
+                    three_parts(x.x, x.y, x0), three_parts(x.z, x.w, x1), three_parts(y.x, y.y, y0), three_parts(y.z, y.w, y1);
 #pragma unroll
-                    for (int part = 0; part < PARTS; ++part) {
-                        const uint32_t x0 = take_part(x.x, x.y), x1 = take_part(x.z, x.w), y0 = take_part(y.x, y.y), y1 = take_part(y.z, y.w);
-                        tmem_store_16x8(w + ((uint32_t)(8 * j) << 16) + part * (BK / 2), x0, x1, y0, y1);
-                    }
+                    for (int part = 0; part < PARTS; ++part)
+                        tmem_store_16x8(w + ((uint32_t)(8 * j) << 16) + part * (BK / 2), x0[part], x1[part], y0[part], y1[part]);
                 }
 #pragma unroll
                 for (int j = 0; j < T::A_MINE; ++j)
                     if (T::A_PIECES % WRITERS == 0 || writer + j * WRITERS < T::A_PIECES) {
                         float4 x = *reinterpret_cast<const float4*>(from + T::W_BYTES + j * WRITERS * 16);
+                        uint32_t low[PARTS], high[PARTS];
+                        three_parts(x.x, x.y, low), three_parts(x.z, x.w, high);
 #pragma unroll
-                        for (int part = 0; part < PARTS; ++part) {
-                            const uint32_t low = take_part(x.x, x.y), high = take_part(x.z, x.w);
-                            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a + part * T::PART_BYTES + j * (WRITERS / 8 * BK * 2)), "r"(low), "r"(high));
-                        }
+                        for (int part = 0; part < PARTS; ++part)
+                            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a + part * T::PART_BYTES + j * (WRITERS / 8 * BK * 2)), "r"(low[part]), "r"(high[part]));
                     }
                 fence_async_shared();
                 tmem_store_wait();

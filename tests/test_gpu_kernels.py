@@ -155,7 +155,7 @@ def test_gemm_f32_sizes_keep_a_rows_bits(m, n, k):
 @pytest.mark.parametrize("m,n,k", [(1, 130, 1024), (17, 127, 3072), (95, 129, 2048), (97, 128, 1000), (260, 300, 4100)])
 def test_gemm_f32_keeps_every_bit_of_its_inputs(m, n, k):
     """Both sides of the tiles' edges, short and long ranges of K, one CTA and clusters a tile.  A product of two float32 loses at most
-    2^-26 of itself, 32 are added by the tensor cores, the rest is k / 32 + 4 additions: within 2^-23 of the sum of the products'
+    2^-24 of itself (parts of 2^-9 and 2^-16 twice), 32 are added by the tensor cores, the rest is k / 32 + 4 additions: within 2^-23 of the sum of the products'
     sizes for the first and, a rounding each, (k / 32 + 4) 2^-24 for the others; and closer than a chain of k multiply-adds in
     float32 comes."""
     g = torch.Generator(device=DEV).manual_seed(m + n + k)

@@ -455,9 +455,9 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
 //   warp 11     issues the MMAs: scores = q parts (tensor memory) . keys, values = weights (tensor memory) . values
 // A row's result has the same bits however its request is cut: blocks of keys begin at multiples of 64, chunks at multiples of CHUNK, and
 // what a tile holds beside a row touches neither its scores nor its sums.  Values that bfloat16 has no parts for (infinite, NaN, beyond
-// its largest number) are zeros in the tiles and added by the rows that see them; a score that is no number or infinite is
-// computed again from its row and key, so that what a row does not see never reaches it. (Below 2^-110 a value's last part lies
-// under bfloat16's range: such values keep fewer bits of their own, 2^-134 off at most.)
+// its largest number, so small that the last part lies under its range) are zeros in the tiles and added by the rows that see them; a
+// score that is no number or infinite is computed again from its row and key, so that what a row does not see never reaches it.  (Queries
+// and keys of less than 2^-110 are 2^-134 off at most, which a score shows only beside a factor of 2^100.)
 //
 // What bounds it: the parts' instructions and the chain of a block (some 7,000 clocks, of which the MMAs run 3,000), a CTA an SM.  Kernel
 // alone, 16 query and 8 key/value heads of 128, on the CUDA cores and here: a prompt of 777 tokens 146 -> 65 us, 880 tokens behind
@@ -473,17 +473,18 @@ constexpr size_t TC_SMEM = 1024 + 6 * (size_t)TC_PART + 2 * (size_t)TC_RAW + TC_
 static_assert(TC_P + 3 * TC_KEYS / 2 <= TC_TMEM, "tensor memory");
 static_assert(CHUNK % TC_KEYS == 0, "whole blocks a chunk");
 constexpr int TC_PLACES = 8, TC_AHEAD = 4;                               // blocks whose places are held; how far ahead they are looked up
-constexpr float BF16_MOST = 3.38953139e38f;
+constexpr float BF16_MOST = 3.38953139e38f, BF16_LEAST = 0x1p-96f;
+__device__ __forceinline__ bool has_parts(float v) { return fabsf(v) < BF16_MOST && !(fabsf(v) < BF16_LEAST && v != 0.0f); }
 
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-// four floats as two words of each part; true where a part is not finite
+// four floats as two words of each part; true where the parts are not the floats: what the third one should be has bits below it (a NaN,
+// which arithmetic makes of what is infinite, has all of them)
 __device__ __forceinline__ bool split4(float4 v, uint2 (&parts)[3]) {
     uint32_t low[3], high[3];
     three_parts(v.x, v.y, low), three_parts(v.z, v.w, high);
 #pragma unroll
     for (int p = 0; p < 3; ++p) parts[p] = make_uint2(low[p], high[p]);
-    const float left = (v.x + v.y) + (v.z + v.w);
-    return left != left;
+    return (__float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w)) & 0xFFFF;
 }
 
 // a row and a key that the parts cannot be trusted with
@@ -634,17 +635,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
                 if (ct < TC_KEYS / 32) odd_values[i & 1][ct] = 0u;
                 if (ct < TC_KEYS) place_s[(i + TC_AHEAD) % TC_PLACES][ct] = later;
                 bar_sync(1, TC_COPY_WARPS * 32);
-                if (convert(by_copies, v_parts, v_raw, mine)) {
+                if (__any_sync(0xffffffffu, convert(by_copies, v_parts, v_raw, mine))) {
 #pragma unroll 1
                     for (int row = mine; row < TC_KEYS; row += TC_COPY_WARPS) {
                         float4 v = raw_of(v_raw, row);
-                        if (!put(v_parts, row, v)) continue;
-                        if (!(fabsf(v.x) < BF16_MOST)) v.x = 0.0f;
-                        if (!(fabsf(v.y) < BF16_MOST)) v.y = 0.0f;
-                        if (!(fabsf(v.z) < BF16_MOST)) v.z = 0.0f;
-                        if (!(fabsf(v.w) < BF16_MOST)) v.w = 0.0f;
+                        if (!__any_sync(0xffffffffu, put(v_parts, row, v))) continue;      // a row's lanes agree: its readers ask each value
+                        if (!has_parts(v.x)) v.x = 0.0f;
+                        if (!has_parts(v.y)) v.y = 0.0f;
+                        if (!has_parts(v.z)) v.z = 0.0f;
+                        if (!has_parts(v.w)) v.w = 0.0f;
                         put(v_parts, row, v);
-                        atomicOr(&odd_values[i & 1][row / 32], 1u << (row % 32));
+                        if (lane == 0) atomicOr(&odd_values[i & 1][row / 32], 1u << (row % 32));
                     }
                 }
                 fence_async_shared();
@@ -715,7 +716,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
 #pragma unroll
                         for (int c = 0; c < 64; ++c) {
                             const float v = A.v[place + half * 64 + c];
-                            if (!(fabsf(v) < BF16_MOST)) o[c] = fmaf(w, v, o[c]);
+                            if (!has_parts(v)) o[c] = fmaf(w, v, o[c]);
                         }
                     }
                     bar_sync(pair_bar, 64);

@@ -1364,6 +1364,19 @@ def test_attention_f32_keeps_what_is_no_number_in_its_row():
     assert torch.equal(got, clean)
 
 
+@pytest.mark.parametrize("exponent", [-90, -105, -113, -122, -126, 100])
+def test_attention_f32_on_tensor_cores_of_small_and_large_values(exponent):
+    """Heads of 128: values of one power of two keep every bit, also where the last bfloat16 part would lie under that type's range.  The
+    error is that of the values before the scaling, beside half a unit of the smallest float32 a key."""
+    spans = [(0, 130), (300, 5)]
+    case = PagedCase(torch.float32, 4, 2, 128, 16, spans, seed=12)
+    want = case.plain()
+    error = (case.run_simt().cpu().double() - want).abs().max().item()
+    case.vc = torch.ldexp(case.vc, torch.tensor(exponent))
+    got = case.run_simt().cpu().double()
+    assert (got - want * 2.0 ** exponent).abs().max().item() <= 2 * error * 2.0 ** exponent + 305 * 2.0 ** -150 * 4
+
+
 @pytest.mark.parametrize("whole", [False, True])
 @pytest.mark.parametrize("window", [0, 300])
 def test_attention_f32_on_tensor_cores_of_values_without_parts(monkeypatch, window, whole):

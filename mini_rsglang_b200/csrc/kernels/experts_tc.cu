@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
                                 for (int p = 0; p < 4; ++p) {
                                     const float g0 = __bfloat162float(__float2bfloat16_rn(g[e + 2 * p])), g1 = __bfloat162float(__float2bfloat16_rn(g[e + 2 * p + 1]));
                                     const float u0 = __bfloat162float(__float2bfloat16_rn(u[e + 2 * p])), u1 = __bfloat162float(__float2bfloat16_rn(u[e + 2 * p + 1]));
-                                    __nv_bfloat162 two = __floats2bfloat162_rn(__fdividef(g0, 1.0f + __expf(-g0)) * u0, __fdividef(g1, 1.0f + __expf(-g1)) * u1);
+                                    __nv_bfloat162 two = __floats2bfloat162_rn(by_reciprocal(g0, 1.0f + __expf(-g0)) * u0, by_reciprocal(g1, 1.0f + __expf(-g1)) * u1);
                                     w[p] = *reinterpret_cast<uint32_t*>(&two);
                                 }
                                 *reinterpret_cast<uint4*>(dst + block * 64 + c + e) = make_uint4(w[0], w[1], w[2], w[3]);

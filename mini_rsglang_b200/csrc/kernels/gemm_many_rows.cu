@@ -18,6 +18,7 @@
 // time, so the weights come from HBM once.  Every wait is bounded (tma.cuh).
 //   (reference: cuBLAS and a kernel of its own, crates/models/src/qwen3.rs:255-261; ops.cu:91-94)
 #include "tcgen05.cuh"
+#include "activations.cuh"
 
 namespace {
 
@@ -42,7 +43,7 @@ __device__ __forceinline__ float activate(float z, int kind) {
 }
 
 // 0.5 z (1 + tanh(u)) = z / (1 + exp(-2 u)) with u = sqrt(2 / pi) (z + 0.044715 z^3)
-__device__ __forceinline__ float gelu_tanh_gate(float z) { return __fdividef(z, 1.0f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z))); }
+__device__ __forceinline__ float gelu_tanh_gate(float z) { return by_reciprocal(z, 1.0f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z))); }
 
 // ACT < 0: the gated product (-1: silu(gate) * up, -2: relu(gate) * up, -3: gelu with tanh); 0 to 4: the plain product with gelu (error
 // function), gelu (tanh), silu, relu or the square of relu on every sum.
@@ -194,8 +195,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_many_rows_kernel(
                                     ? __floats2bfloat162_rn(fmaxf(g0, 0.0f) * u[e + 2 * p], fmaxf(g1, 0.0f) * u[e + 2 * p + 1])
                                     : ACT == -3
                                     ? __floats2bfloat162_rn(gelu_tanh_gate(g0) * u[e + 2 * p], gelu_tanh_gate(g1) * u[e + 2 * p + 1])
-                                    : __floats2bfloat162_rn(__fdividef(g0, 1.0f + __expf(-g0)) * u[e + 2 * p],
-                                                            __fdividef(g1, 1.0f + __expf(-g1)) * u[e + 2 * p + 1]);
+                                    : __floats2bfloat162_rn(by_reciprocal(g0, 1.0f + __expf(-g0)) * u[e + 2 * p],
+                                                            by_reciprocal(g1, 1.0f + __expf(-g1)) * u[e + 2 * p + 1]);
                                 w[p] = *reinterpret_cast<uint32_t*>(&pair);
                             }
                             *reinterpret_cast<uint4*>(dst + block * 64 + c + e) = make_uint4(w[0], w[1], w[2], w[3]);

@@ -228,8 +228,8 @@ __global__ void latent_prepare_kernel(const float* __restrict__ proj, int proj_w
 
 // The same with four neighbouring columns a thread and step: all sizes (and half of `rotary`, where element i turns with i + rotary / 2)
 // multiples of 4, rows of proj and of T on 16-byte boundaries, up to PREPARE_QUADS * 1,024 columns.  A token's loads are under way
-// together, ahead of the cosines and the norm.  2,048 tokens of 1,840 columns: 15.3 us an element a thread (two divisions and a dependent
-// load each), 13.1 us here (23 MB).
+// together, ahead of the cosines and the norm; every output has the bits that the kernel above gives it.  2,048 tokens of 1,840 columns,
+// from a cold L2: 18.2 us an element a thread (two divisions and a dependent load each), 14.4 us here (23 MB).
 constexpr int PREPARE_THREADS = 256, PREPARE_QUADS = 4;
 template <typename T>
 __global__ void __launch_bounds__(PREPARE_THREADS) latent_prepare_vec_kernel(
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(PREPARE_THREADS) latent_prepare_vec_kernel(
     T* __restrict__ cache, float* __restrict__ gate, int tokens, LatentSizes z) {
     pdl_launch_dependents();
     pdl_wait();
-    extern __shared__ float turn[];
+    extern __shared__ __align__(16) float turn[];
     __shared__ float scratch[33];
     const int t = blockIdx.x, half = z.rotary / 2, per_head = z.plain + z.rotated, key_width = z.latent + z.rotated;
     const int q_columns = z.heads * per_head, key_columns = z.has_latent ? key_width : 0;
@@ -270,10 +270,10 @@ __global__ void __launch_bounds__(PREPARE_THREADS) latent_prepare_vec_kernel(
     }
     float scale = 0.0f;
     if (z.has_latent) {
+        // the squares in the order of the kernel above: a cached row has the same bits from either
+        const float* low = row + q_columns;
         float sum = 0.0f;
-#pragma unroll
-        for (int j = 0; j < PREPARE_QUADS; ++j)
-            if (head[j] == z.heads && at[j] < 0) sum += own[j].x * own[j].x + own[j].y * own[j].y + own[j].z * own[j].z + own[j].w * own[j].w;
+        for (int i = threadIdx.x; i < z.latent; i += blockDim.x) sum += low[i] * low[i];
         scale = rsqrtf(block_sum(sum, scratch) / (float)z.latent + eps);
     }
     __syncthreads();                                         // the cosines are there
@@ -295,10 +295,9 @@ __global__ void __launch_bounds__(PREPARE_THREADS) latent_prepare_vec_kernel(
             } else {
                 const bool lower = at[j] < half;
                 const int p = lower ? at[j] : at[j] - half;
-                const float4 o = other[j];
-                const float sign = lower ? -1.0f : 1.0f;
-                x = make_float4(x.x * turn[p] + sign * (o.x * turn[half + p]), x.y * turn[p + 1] + sign * (o.y * turn[half + p + 1]),
-                                x.z * turn[p + 2] + sign * (o.z * turn[half + p + 2]), x.w * turn[p + 3] + sign * (o.w * turn[half + p + 3]));
+                const float4 o = other[j], c = *reinterpret_cast<const float4*>(turn + p), s = *reinterpret_cast<const float4*>(turn + half + p);
+                x = lower ? make_float4(x.x * c.x - o.x * s.x, x.y * c.y - o.y * s.y, x.z * c.z - o.z * s.z, x.w * c.w - o.w * s.w)
+                          : make_float4(x.x * c.x + o.x * s.x, x.y * c.y + o.y * s.y, x.z * c.z + o.z * s.z, x.w * c.w + o.w * s.w);
             }
         }
         if (!key) {

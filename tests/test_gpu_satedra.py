@@ -254,6 +254,36 @@ def test_latent_rows_rotation_and_gates(H, d, r, R, rotary, scaling, keeps, gate
             assert (flat == 7.0).all()
 
 
+@pytest.mark.parametrize("pairing", ["split_half", "interleaved"])
+@pytest.mark.parametrize("H,d,r,R,rotary,gated,keeps", [(16, 64, 32, 256, 32, True, True), (4, 12, 16, 516, 8, True, True), (3, 8, 24, 1028, 24, False, True),
+                                                        (256, 4, 8, 12, 8, True, False), (2, 8, 4, 40, 0, False, True)])
+def test_latent_prepare_gives_the_same_bits_wherever_its_rows_lie(H, d, r, R, rotary, gated, keeps, pairing):
+    """Rows of proj on 16-byte boundaries are read four columns at a time, others one: every output has the same bits.  Sizes around a block of 256 squares and more, one
+    quarter that turns, none, as many columns as four a thread can take."""
+    from mini_rsglang_b200 import kernels
+
+    tokens, page, pool = 67, 16, 6
+    gen = torch.Generator().manual_seed(R + r)
+    width = H * (d + r) + (R + r if keeps else 0) + (H if gated else 0)
+    assert width % 4 == 0
+    proj = torch.randn(tokens, width, generator=gen).to(DEV)
+    shifted = torch.cat([torch.zeros(1, device=DEV), proj.flatten()])[1:].view(tokens, width)
+    positions = torch.randint(0, 9000, (tokens,), generator=gen, dtype=torch.int32).to(DEV)
+    slots = torch.randperm(pool * page, generator=gen)[:tokens].to(torch.int32).to(DEV)
+    f, w = P.yarn_frequencies(rotary, 10000.0, None)[0].float().to(DEV) if rotary else None, (torch.rand(R, generator=gen) + 0.5).to(DEV)
+    for dtype in (torch.float32, torch.bfloat16):
+        got = []
+        for rows in (proj, shifted):
+            q_plain, q_rows = torch.empty(H, tokens, d, dtype=dtype, device=DEV), torch.zeros(tokens, H, R + r, dtype=dtype, device=DEV)
+            cache = torch.zeros(pool, 1, page, R + r, dtype=dtype, device=DEV)
+            gate = torch.zeros(tokens, H, device=DEV)
+            kernels.latent_prepare(rows, w if keeps else None, 1e-5, f, 1.1, positions, slots if keeps else None, q_plain, q_rows,
+                                   cache if keeps else None, gate if gated else None, H, d, r, R, rotary, keeps, pairing=pairing)
+            got.append((q_plain, q_rows, cache, gate))
+        for name, one, other in zip(("q_plain", "q_rows", "cache", "gate"), *got):
+            assert torch.equal(one, other), (name, dtype)
+
+
 def plain_latent_attention(q_rows, rows, gate, R, scale, window):
     """Attention in the latent space: scores against whole rows, sums over the rows' first R elements."""
     T_, H, _ = q_rows.shape

@@ -2,14 +2,6 @@
 // tanh, 2 silu, 3 relu, 4 the square of relu.  Exact float32 forms.
 #pragma once
 
-// x / y of a y from 1 on by the reciprocal unit, for results that are rounded to bfloat16 (over 4 M gates of up to +-1, 16 and 89 their
-// largest and mean error against 64 bits are those of the division to seven digits).  `__fdividef` is 0 from y = 2^126 on, this is not.
-__device__ __forceinline__ float by_reciprocal(float x, float y) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
-    return x * r;
-}
-
 __device__ __forceinline__ float mrs_activate(float z, int kind) {
     if (kind == 0) return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
     if (kind == 1) return 0.5f * z * (1.0f + tanhf(0.79788456080286536f * (z + 0.044715f * z * z * z)));

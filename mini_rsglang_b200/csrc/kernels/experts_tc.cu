@@ -9,10 +9,10 @@
 //   warps 2-9 two threads a row, 128 of its sums from tensor memory each;
 //             gated: a weight tile holds two blocks of 64 gate and 64 up rows, out[row] = silu(gate) * up;
 //             plain: out[pair of the row] = the sums (the rows go back to their (token, choice) pairs).
-// Bound by the weights' bytes, then by the MMAs.  With one thread a row and a full division a sum the epilogue took a tile 18,000 clocks,
-// longer than its MMAs (16,400 at K = 2,048); two threads and the fast division take 5,300.  32 experts, 1,777 tokens x 4, width 2,048,
-// inner 1,024: gated product 84 -> 67 us, down product 41 (unchanged); 200 tokens, width 4,096, inner 1,536: 156 -> 136 and 72 -> 70.  Two tiles of rows a
-// CTA (weights fetched once for 256 rows) leave some SMs 6 tiles where others have 2 and no accumulator free meanwhile: 107 us.
+// Bound by the weights' bytes, then by the MMAs.  With one thread a row the epilogue took a tile 18,000 clocks, longer than its MMAs
+// (16,400 at K = 2,048); two take half of that.  With that, the weights' policy below and no rows fetched for places without a pair, from a
+// cold L2: 32 experts, 1,777 tokens x 4, width 2,048, inner 1,024: gated product 88.9 -> 76.2 us, down product 49.2 -> 45.5; 200 tokens,
+// width 4,096, inner 1,536: 161 -> 157 and 84.8 -> 74.9.  Two tiles of rows a CTA (weights fetched once for 256 rows) leave some SMs 6 tiles where others have 2 and no accumulator free meanwhile: 107 us.
 // Only the tiles that the lists use are walked: their count stands behind the tiles' experts.  CTAs are
 // persistent; tiles that share a weight tile are taken by neighbouring CTAs at the same time.  Every wait is bounded
 // (tma.cuh).
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_product_tc_kernel(
                                 for (int p = 0; p < 4; ++p) {
                                     const float g0 = __bfloat162float(__float2bfloat16_rn(g[e + 2 * p])), g1 = __bfloat162float(__float2bfloat16_rn(g[e + 2 * p + 1]));
                                     const float u0 = __bfloat162float(__float2bfloat16_rn(u[e + 2 * p])), u1 = __bfloat162float(__float2bfloat16_rn(u[e + 2 * p + 1]));
-                                    __nv_bfloat162 two = __floats2bfloat162_rn(by_reciprocal(g0, 1.0f + __expf(-g0)) * u0, by_reciprocal(g1, 1.0f + __expf(-g1)) * u1);
+                                    __nv_bfloat162 two = __floats2bfloat162_rn(g0 / (1.0f + __expf(-g0)) * u0, g1 / (1.0f + __expf(-g1)) * u1);
                                     w[p] = *reinterpret_cast<uint32_t*>(&two);
                                 }
                                 *reinterpret_cast<uint4*>(dst + block * 64 + c + e) = make_uint4(w[0], w[1], w[2], w[3]);

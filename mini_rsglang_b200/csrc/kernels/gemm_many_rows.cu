@@ -12,13 +12,14 @@
 //   warp 1   one thread issues tcgen05.mma (M 128, N 256, K 16) on the stages;
 //   warps 2-9 two threads a token, 128 of its sums from tensor memory each.  A tile holds two blocks of 64 gate
 //            and 64 up rows (the weights are stored so), so a thread has both factors of its outputs; the plain
-//            product applies its activation to every sum.  (One thread a token and full divisions: some 18,000 clocks a tile, longer
-//            than the MMAs of K = 2,048; N 6,144, K 1,024: 18.5 -> 14 us at 512 rows, 33 -> 24 at 2,000.)
+//            product applies its activation to every sum.  (One thread a token: some 18,000 clocks a tile, longer than the MMAs of
+//            K = 2,048.  From a cold L2, N 6,144, K 1,024: 18.3 -> 14.9 us at 512 rows, 35.5 -> 28.4 at 2,000.  The divisions are
+//            full ones, 1.5 us of these and of N 24,576, K 4,096, 92 us at 512 rows: the reciprocal unit rounds 4 results in a
+//            million the other way, and the products for few rows divide too.)
 // CTAs are persistent; the tiles that share a weight tile are taken by neighbouring CTAs at the same
 // time, so the weights come from HBM once.  Every wait is bounded (tma.cuh).
 //   (reference: cuBLAS and a kernel of its own, crates/models/src/qwen3.rs:255-261; ops.cu:91-94)
 #include "tcgen05.cuh"
-#include "activations.cuh"
 
 namespace {
 
@@ -43,7 +44,7 @@ __device__ __forceinline__ float activate(float z, int kind) {
 }
 
 // 0.5 z (1 + tanh(u)) = z / (1 + exp(-2 u)) with u = sqrt(2 / pi) (z + 0.044715 z^3)
-__device__ __forceinline__ float gelu_tanh_gate(float z) { return by_reciprocal(z, 1.0f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z))); }
+__device__ __forceinline__ float gelu_tanh_gate(float z) { return z / (1.0f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z))); }
 
 // ACT < 0: the gated product (-1: silu(gate) * up, -2: relu(gate) * up, -3: gelu with tanh); 0 to 4: the plain product with gelu (error
 // function), gelu (tanh), silu, relu or the square of relu on every sum.
@@ -195,8 +196,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_many_rows_kernel(
                                     ? __floats2bfloat162_rn(fmaxf(g0, 0.0f) * u[e + 2 * p], fmaxf(g1, 0.0f) * u[e + 2 * p + 1])
                                     : ACT == -3
                                     ? __floats2bfloat162_rn(gelu_tanh_gate(g0) * u[e + 2 * p], gelu_tanh_gate(g1) * u[e + 2 * p + 1])
-                                    : __floats2bfloat162_rn(by_reciprocal(g0, 1.0f + __expf(-g0)) * u[e + 2 * p],
-                                                            by_reciprocal(g1, 1.0f + __expf(-g1)) * u[e + 2 * p + 1]);
+                                    : __floats2bfloat162_rn(g0 / (1.0f + __expf(-g0)) * u[e + 2 * p],
+                                                            g1 / (1.0f + __expf(-g1)) * u[e + 2 * p + 1]);
                                 w[p] = *reinterpret_cast<uint32_t*>(&pair);
                             }
                             *reinterpret_cast<uint4*>(dst + block * 64 + c + e) = make_uint4(w[0], w[1], w[2], w[3]);

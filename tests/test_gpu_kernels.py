@@ -678,6 +678,34 @@ def test_gemm_gated_rows(t, inner, k):
     assert not kernels.gemm_gated_rows_supported(x.to(DEV), mixed.to(DEV)[:64])          # half a block of gate rows
 
 
+@pytest.mark.parametrize("gate", ["silu", "gelu_tanh"])
+def test_gated_products_give_an_activation_the_same_bits_for_few_and_many_rows(gate):
+    """Rows with a single 1 make every sum a weight itself, 8 million pairs of a gate and an up value over all gates that count and
+    some whose exponential overflows: the products for many rows (dense and of one expert) divide as the product for few rows does."""
+    g = torch.Generator().manual_seed(5)
+    rows, inner = 1024, 8192
+    scale = torch.cat([torch.full((inner - 1024,), 1.0), torch.full((1024,), 30.0)])
+    gates = (torch.randn(inner, rows, generator=g) * scale[:, None]).bfloat16()
+    ups = torch.randn(inner, rows, generator=g).bfloat16()
+    mixed = torch.stack([gates.view(-1, 64, rows), ups.view(-1, 64, rows)], dim=1).reshape(2 * inner, rows).to(DEV).contiguous()
+    x = torch.eye(rows, dtype=torch.bfloat16, device=DEV)
+    few = torch.empty(rows, inner, dtype=torch.bfloat16, device=DEV)
+    for first in range(0, rows, 128):
+        kernels.gemm_tc(x[first:first + 128], mixed, few[first:first + 128], gated=True, gate=gate)
+    z = gates.double().t()
+    want = z * ups.double().t() * (torch.sigmoid(z) if gate == "silu" else 0.5 * (1 + torch.tanh(math.sqrt(2 / math.pi) * (z + 0.044715 * z ** 3))))
+    close(few, want, torch.bfloat16, "gated gemm_tc")
+    many = torch.empty(rows, inner, dtype=torch.bfloat16, device=DEV)
+    kernels.gemm_gated_rows(x, mixed, many, gate)
+    assert torch.equal(many, few)
+    if gate == "silu":
+        listed = torch.arange(rows, dtype=torch.int32, device=DEV)
+        tile_expert = torch.tensor([0] * (rows // 128) + [rows // 128], dtype=torch.int32, device=DEV)
+        many.zero_()
+        kernels.moe_product_tc(x, listed, tile_expert, mixed.view(1, 2 * inner, rows), many, gated=True)
+        assert torch.equal(many, few)
+
+
 @pytest.mark.parametrize("m,nq,nkv,k,page", [(1, 2, 1, 64, 8), (8, 32, 8, 4096, 16), (19, 3, 3, 520, 4), (32, 8, 2, 1024, 32)])
 def test_gemm_tc_qkv_heads(m, nq, nkv, k, page):
     """The fused q/k/v projection with head norms, rotation and cache write in its epilogue, against the

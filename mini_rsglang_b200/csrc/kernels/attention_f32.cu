@@ -722,15 +722,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
                     bar_sync(pair_bar, 64);
                 }
             };
-            auto whole_sum = [&]() {                                     // both halves' sums; `met` is free: every exchange was read
+            // both halves' sums, behind block i: through that block's place in `met`, which is written again only behind the barrier of
+            // the block after it (the other place is written ahead of that barrier, when the other half may not have read these yet)
+            auto whole_sum = [&](int i) {
+                bar_sync(pair_bar, 64);                                  // block i's maxima have been read
+                met[i & 1][half][row] = l;
                 bar_sync(pair_bar, 64);
-                met[0][half][row] = l;
-                bar_sync(pair_bar, 64);
-                return met[0][0][row] + met[0][1][row];
+                return met[i & 1][0][row] + met[i & 1][1][row];
             };
             float* out = A.out + row_at * TC_D + half * 64;
-            auto join_chunk = [&]() {                                    // !SPLIT: the chunk joins those before it, which lie in `out`
-                const float sum = whole_sum();
+            auto join_chunk = [&](int i) {                               // !SPLIT: the chunk that ends with block i joins those before it, which lie in `out`
+                const float sum = whole_sum(i);
                 const float next = fmaxf(m_all, m), keep = m_all == next ? 1.0f : ratio(m_all, next), take = ratio(m, next);
                 l_all = join(l_all, keep, sum, take);
                 m_all = next;
@@ -754,7 +756,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
                 const int i = it + n, at = at0 + n * TC_KEYS;
                 if (!SPLIT && n > 0 && at % CHUNK == 0) {
                     take_values(i - 1);
-                    join_chunk();
+                    join_chunk(i - 1);
                     pending = false;
                 }
                 float x[32], top = -CUDART_INF_F;
@@ -822,7 +824,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
             copies_wait<0>();
             take_values(it + blocks - 1);
             if (SPLIT) {
-                const float sum = whole_sum();
+                const float sum = whole_sum(it + blocks - 1);
                 if (live) {
                     const size_t place = row_at * A.chunks + blockIdx.z;
                     if (half == 0) A.part_ml[2 * place] = m, A.part_ml[2 * place + 1] = sum;
@@ -831,7 +833,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
                         *reinterpret_cast<float4*>(A.part_o + place * TC_D + half * 64 + c) = make_float4(o[c], o[c + 1], o[c + 2], o[c + 3]);
                 }
             } else {
-                join_chunk();
+                join_chunk(it + blocks - 1);
                 const float inv = 1.0f / l_all;
                 if (live) {
 #pragma unroll

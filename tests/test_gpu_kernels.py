@@ -424,6 +424,17 @@ def test_attention_f32_gives_a_row_the_same_bits_in_every_cut(monkeypatch, nq, n
             assert torch.equal(out[row - rows.start], got[row]), (row, rows)
 
 
+@pytest.mark.parametrize("window", [0, 900])
+def test_attention_f32_joins_chunks_the_same_way_every_time(monkeypatch, window):
+    """Heads of 128, walks over up to 16 chunks: at a chunk's end the two threads of a row exchange their sums through memory that also
+    carries the blocks' maxima.  Tiles that begin with an even and an odd block, run after run: the bits of chunks in blocks of their own."""
+    case = PagedCase(torch.float32, 8, 2, 128, 16, [(0, 1100), (2900, 75), (4000, 1), (190, 700)], seed=window, window=window)
+    want = case.run_simt()
+    monkeypatch.setattr(kernels, "ATTENTION_F32_PARTS_BYTES", 0)
+    for _ in range(20):
+        assert torch.equal(case.run_simt(), want)
+
+
 @pytest.mark.parametrize("nq,nkv,d,page,window", [(2, 1, 128, 16, 0), (8, 1, 64, 4, 0), (3, 3, 256, 1, 0), (6, 2, 40, 16, 90), (1, 1, 128, 64, 33)])
 def test_attention_f32_single_tokens_at_the_edges_of_steps(monkeypatch, nq, nkv, d, page, window):
     """One to eight rows a tile: contexts around a block of 32 keys, a step of 64 and a chunk of 256, windows that begin inside

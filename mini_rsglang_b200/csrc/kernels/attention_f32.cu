@@ -484,7 +484,7 @@ __device__ __forceinline__ bool split4(float4 v, uint2 (&parts)[3]) {
     three_parts(v.x, v.y, low), three_parts(v.z, v.w, high);
 #pragma unroll
     for (int p = 0; p < 3; ++p) parts[p] = make_uint2(low[p], high[p]);
-    return (__float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w)) & 0xFFFF;
+    return left_bits(v) & LOST_BITS;
 }
 
 // a row and a key that the parts cannot be trusted with

@@ -6,8 +6,11 @@
 // elements of K at a time into a fresh accumulator in tensor memory, small products first, and from there on a sum is ordinary
 // float32 addition in registers: 32-element sums into one of four ranges of K, the four ranges in order.  An element's bits depend
 // on K alone: not on M, not on the tile or the cut that the sizes chose, and a token's result does not change with what else is in the
-// batch.  A result that is no number or infinite, or below 2^-60 where a part of a factor may lie under bfloat16's range, is computed
-// again in float64 from the inputs (`exact_dot`), so infinities and NaN are those of the sum of the products.
+// batch.  Results that the parts cannot be trusted with are computed again in float64 from the inputs: those that are no number or
+// infinite, so that infinities and NaN are those of the sum of the products; those below 2^-60, whose smallest products may lie under
+// float32's range (`store_column`); and those of rows with an element below some 2^-110, which has bits under bfloat16's range (2^-133),
+// where the result is below 2^-60 or the other row has an element from 2^24 on (`mend_lost`).  Elsewhere K such bits are less than
+// K 2^-48 of the result.  Looking for them takes 0.4 to 0.8 us of a call of up to 128 rows (K = 1,024 to 3,072), none that shows of 777.
 //
 // What bounds it: the workers' instructions (a float32 into three bfloat16 is some twenty-five instructions for four elements, and the
 // sums), then shared memory (both matrices pass through it; parts of W lie in tensor memory, which took a step of 96 tokens from 0.80 to
@@ -96,12 +99,54 @@ __device__ __noinline__ float exact_dot(const float* __restrict__ a, const float
     return (float)sum;
 }
 
-// Stores the warp's 32 weight rows' results for one token; those that the parts cannot be trusted with are computed again.
-__device__ __forceinline__ void store_column(float v, const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int m,
-                                             int n, int M, int N, int K) {
+// What a row's elements say of its results: some have bits under bfloat16's range; some are large enough for the other row's such bits
+// to show.  The whole warp.
+constexpr unsigned LOST = 1, LARGE = 2;
+constexpr float LEAST = 0x1p-60f;
+__device__ __noinline__ unsigned row_facts(const float* __restrict__ row, int K) {
+    uint32_t rest = 0;
+    float top = 0.0f;
+    for (int k = threadIdx.x & 31; k < K; k += 32) {
+        float x = row[k], none = 0.0f;
+        uint32_t parts[PARTS];
+        top = fmaxf(top, fabsf(x));
+        three_parts(x, none, parts);
+        rest |= __float_as_uint(x);
+    }
+    return (__any_sync(0xffffffffu, rest & LOST_BITS) ? LOST : 0) | (__any_sync(0xffffffffu, top >= 0x1p24f) ? LARGE : 0);
+}
+
+// The tile's results of LOST rows, once they are stored: 128 weight rows from n0 on, `tokens` tokens from m0 on.  The facts are read from the
+// rows themselves over the whole of K, so that a result depends on its own two rows alone.  The whole block; `facts`: BM + tokens.
+__device__ __noinline__ void mend_lost(unsigned char* facts, const float* __restrict__ A, const float* __restrict__ W, float* C, int m0, int n0,
+                                       int tokens, int M, int N, int K) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    tokens = min(tokens, M - m0);
+    for (int r = warp; r < BM + tokens; r += THREADS / 32) {
+        const unsigned f = r >= BM ? row_facts(A + (size_t)(m0 + r - BM) * K, K) : n0 + r < N ? row_facts(W + (size_t)(n0 + r) * K, K) : 0;
+        if (lane == 0) facts[r] = (unsigned char)f;
+    }
+    __syncthreads();                                         // the facts are there, and the results
+    for (int task = warp; task < tokens * (BM / 32); task += THREADS / 32) {
+        const int row = task % (BM / 32) * 32 + lane, n = n0 + row, m = m0 + task / (BM / 32);
+        const unsigned w = facts[row], a = facts[BM + m - m0];
+        const bool lost = (w | a) & LOST, shows = ((w & LARGE) && (a & LOST)) || ((w & LOST) && (a & LARGE));
+        unsigned odd = __ballot_sync(0xffffffffu, n < N && lost && (shows || fabsf(C[(size_t)m * N + n]) < LEAST));
+        while (odd) {
+            const int of = __ffs(odd) - 1;
+            odd &= odd - 1;
+            const float v = exact_dot(A + (size_t)m * K, W + (size_t)__shfl_sync(0xffffffffu, n, of) * K, K);
+            if (lane == of) C[(size_t)m * N + n] = v;
+        }
+    }
+}
+
+// Stores the warp's 32 weight rows' results for one token; those that are no number, infinite or too small are computed again.
+__device__ __forceinline__ void store_column(float v, const float* __restrict__ A, const float* __restrict__ W, float* C, int m, int n, int M, int N,
+                                             int K) {
     if (m >= M) return;                                      // the same for the whole warp
     const float size = fabsf(v);
-    unsigned odd = __ballot_sync(0xffffffffu, n < N && !(size <= FLT_MAX && size >= 0x1p-60f) && v != 0.0f);
+    unsigned odd = __ballot_sync(0xffffffffu, n < N && !(size <= FLT_MAX && size >= LEAST) && v != 0.0f);
     while (odd) {
         const int lane = __ffs(odd) - 1;
         odd &= odd - 1;
@@ -116,7 +161,7 @@ __device__ __forceinline__ void store_column(float v, const float* __restrict__ 
 // and add finished accumulators to their sums; two more warps issue the MMAs of every other step.
 // VEC: sixteen-byte copies (K a multiple of 4, both matrices on 16-byte boundaries), else four-byte ones.
 template <int BN, bool VEC>
-__global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M,
+__global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* C, int M,
                                                               int N, int K, int m_tiles, int cut) {
     using T = Tile<BN>;
     constexpr int STAGES = T::STAGES;
@@ -126,6 +171,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __res
     uint64_t* full = reinterpret_cast<uint64_t*>(raw + TURNS * T::DEPTH * T::RAW_BYTES);       // a stage's parts are written
     uint64_t* done = full + STAGES;                                                    // a stage's MMAs have finished
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + STAGES);
+
+    __shared__ unsigned char facts[BM + BN];                                           // of the tile's weight rows, then of its tokens
+    __shared__ int met_lost;                                                           // read by the cluster
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tile = blockIdx.x / cut, rank = blockIdx.x % cut;
@@ -175,6 +223,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __res
             __syncwarp();
         }
     }
+    uint32_t rest = 0;                                       // what three parts leave of this thread's elements: LOST_BITS of it
     float now[T::COLUMNS], before[T::COLUMNS];               // the running range, the ranges before it (one CTA a tile: their sum)
 #pragma unroll
     for (int c = 0; c < T::COLUMNS; ++c) now[c] = before[c] = 0.0f;
@@ -230,6 +279,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __res
                     float4 x = *reinterpret_cast<const float4*>(from + j * WRITERS * 16), y = *reinterpret_cast<const float4*>(from + (j + 1) * WRITERS * 16);
                     uint32_t x0[PARTS], x1[PARTS], y0[PARTS], y1[PARTS];
                     three_parts(x.x, x.y, x0), three_parts(x.z, x.w, x1), three_parts(y.x, y.y, y0), three_parts(y.z, y.w, y1);
+                    rest |= left_bits(x) | left_bits(y);
 #pragma unroll
                     for (int part = 0; part < PARTS; ++part)
                         tmem_store_16x8(w + ((uint32_t)(8 * j) << 16) + part * (BK / 2), x0[part], x1[part], y0[part], y1[part]);
@@ -240,6 +290,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __res
                         float4 x = *reinterpret_cast<const float4*>(from + T::W_BYTES + j * WRITERS * 16);
                         uint32_t low[PARTS], high[PARTS];
                         three_parts(x.x, x.y, low), three_parts(x.z, x.w, high);
+                        rest |= left_bits(x);
 #pragma unroll
                         for (int part = 0; part < PARTS; ++part)
                             asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a + part * T::PART_BYTES + j * (WRITERS / 8 * BK * 2)), "r"(low[part]), "r"(high[part]));
@@ -278,6 +329,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __res
             if (++stage == STAGES) stage = 0;
         }
     }
+    int some = __syncthreads_or(rest & LOST_BITS), mine = 0, of_mine = BN;     // some thread met LOST bits; this CTA's tokens
     if (cut == 1) {
         if (warp < WORKERS / 32) {
 #pragma unroll
@@ -286,7 +338,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __res
     } else {
         // every CTA leaves its ranges' sums in its shared memory and adds up a slice of the columns
         cg::cluster_group cluster = cg::this_cluster();
-        __syncthreads();
+        if (tid == 0) met_lost = some;
         float* sums = reinterpret_cast<float*>(smem);
         if (warp < WORKERS / 32) {
 #pragma unroll
@@ -297,9 +349,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __res
             }
         }
         cluster.sync();
+        of_mine = BN / cut, mine = rank * of_mine;
+        some = 0;
+#pragma unroll
+        for (int r = 0; r < RANGES; ++r) some |= *cluster.map_shared_rank(&met_lost, r % cut);      // wanted only behind the columns
         if (warp < WORKERS / 32) {
-            const int slice = BN / cut;
-            for (int c = rank * slice + (warp >> 2); c < (rank + 1) * slice; c += WORKERS / BM) {
+            for (int c = mine + (warp >> 2); c < mine + of_mine; c += WORKERS / BM) {
                 float v = 0.0f;
 #pragma unroll
                 for (int r = 0; r < RANGES; ++r) v += cluster.map_shared_rank(sums, r / ranges)[r % ranges * (BM * BN) + c * BM + row];
@@ -308,6 +363,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_kernel(const float* __res
         }
         cluster.sync();                                      // no CTA leaves while another reads its sums
     }
+    if (some && m0 + mine < M) mend_lost(facts, A, W, C, m0 + mine, n0, of_mine, M, N, K);
     tcgen05_fence_before_sync();
     __syncthreads();
     if (warp == WORKERS / 32) {

@@ -24,3 +24,7 @@ __device__ __forceinline__ void three_parts(float& x, float& y, uint32_t (&parts
     less_part(x, y, parts[1]);
     parts[2] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
 }
+// Bits of a float32 that three parts leave: in what is left in place of the float (three_parts), the lower half is 0 unless bits of it lie
+// under bfloat16's range (2^-133), or unless it is no number.
+constexpr uint32_t LOST_BITS = 0xFFFF;
+__device__ __forceinline__ uint32_t left_bits(float4 v) { return __float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w); }

@@ -193,6 +193,37 @@ def test_gemm_f32_of_values_at_the_ends_of_the_range(m):
     assert (out[m - 1, 3].double() - want[m - 1, 3]).abs() <= 2.0 ** -23 * size[m - 1, 3] or not want[m - 1, 3].isfinite()
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 140, 1024), (7, 4096, 300), (20, 140, 3072), (100, 500, 301), (97, 4100, 1024)])
+def test_gemm_f32_of_factors_with_bits_under_the_parts_range(m, n, k):
+    """Elements below 2^-110, whose last bits bfloat16 has no room for, and subnormal ones, beside factors that bring their products
+    back to ordinary numbers or up to 1: one CTA and clusters a tile, whole rows and single elements.  A result is the sum of the products
+    to a rounding each of k / 32 + 8 additions; what shares a tile with such rows keeps its bits."""
+    g = torch.Generator(device=DEV).manual_seed(m + n)
+    x, w = torch.randn(m, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+    plain = torch.empty(m, n, device=DEV)
+    kernels.gemm_f32(x, w, plain)
+    whole, single = sorted({0, m // 2}), sorted({m // 3, m - 1} - {0, m // 2})
+    for row in whole:
+        x[row] = torch.ldexp(x[row], torch.tensor(-120 if row == 0 else -136, device=DEV))       # from 2^-126 on down: subnormal
+    for row in single:
+        x[row, k // 2] = 1.2345678e-38
+    w[3] = torch.ldexp(w[3], torch.tensor(70, device=DEV))
+    w[5] = torch.ldexp(w[5], torch.tensor(120, device=DEV))
+    w[7] = 0.0
+    w[7, k // 2] = 1e30                                      # 1.2e-38 times 1e30 alone
+    w[n - 1] = torch.ldexp(w[n - 1], torch.tensor(-125, device=DEV))
+    out = torch.empty(m, n, device=DEV)
+    kernels.gemm_f32(x, w, out)
+    torch.cuda.synchronize()
+    kernels.check_device_errors()
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert ((out.double() - want).abs() <= size * (k / 32 + 8) * 2.0 ** -24 + 2.0 ** -149).all()
+    odd = torch.zeros(n, dtype=torch.bool, device=DEV)
+    odd[[3, 5, 7, n - 1]] = True
+    rows = [r for r in range(m) if r not in whole + single]
+    assert torch.equal(out[rows][:, ~odd], plain[rows][:, ~odd])
+
+
 def plain_qk(qkv, positions, q_w, k_w, eps, theta, nq, nkv, d):
     """q and k after head norm and rotation, v untouched, from the plain implementation's parts."""
     ar = P.Arith(None)

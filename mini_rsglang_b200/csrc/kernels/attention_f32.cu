@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
 
 // ------------------------------------------------------------------------------------------------
 // Heads of 128 elements on the tcgen05 tensor cores, with every bit of the inputs: a float32 is three bfloat16 (parts3.cuh), a product
-// of two is six products of parts (the other three are some 2^-26 of it).  A block takes a tile of up to 128 rows and walks their keys
+// of two is six products of parts (the other three are at most 2^-24 of it).  A block takes a tile of up to 128 rows and walks their keys
 // in blocks of 64:
 //   warps 0-7   two threads a row, 32 scores and 64 columns each: scores from tensor memory, maximum, exponentials, the weights' parts
 //               back into tensor memory; a block's weighted values (a fresh accumulator) are added to the row's in registers, in

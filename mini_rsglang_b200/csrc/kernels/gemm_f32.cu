@@ -2,7 +2,7 @@
 // projection of the 32-bit path.
 //
 // A float32 is the sum of three bfloat16 (8 + 8 + 8 bits of its significand), so a product of two is nine products of bfloat16, each
-// exact in float32.  Six of them are computed; the other three are some 2^-26 of the product.  The MMAs add 32
+// exact in float32.  Six of them are computed; the other three are at most 2^-24 of the product.  The MMAs add 32
 // elements of K at a time into a fresh accumulator in tensor memory, small products first, and from there on a sum is ordinary
 // float32 addition in registers: 32-element sums into one of four ranges of K, the four ranges in order.  An element's bits depend
 // on K alone: not on M, not on the tile or the cut that the sizes chose, and a token's result does not change with what else is in the
@@ -16,9 +16,9 @@
 // sums), then shared memory (both matrices pass through it; parts of W lie in tensor memory, which took a step of 96 tokens from 0.80 to
 // 0.70 us).  One turn of writers instead of two that overlap: 24 against 19 us for 8 rows in one CTA a tile.  Tiles of 128 tokens
 // spill registers (90 against 63 us for 777 rows, N 4,096, K 1,024).
-// Alone, before (multiply-adds on the CUDA cores) and now: N 4,096, K 1,024: 1 row 15 -> 10.5 us, 64 rows 35 -> 11.5, 128 rows 38 -> 18, 777
-// rows 168 -> 61; N 1,024, K 2,048: 8 rows 18.5 -> 12.3, 777 rows 121 -> 33; N 6,144, K 1,024, 777 rows 263 -> 90.  Error against 64
-// bits (relative, normal inputs): K = 1,024 5.7e-7 -> 0.9e-7, K = 3,072 1.0e-6 -> 1.2e-7.
+// The kernel from a cold L2, before (multiply-adds on the CUDA cores) and now: N 4,096, K 1,024: 1 row 12.0 -> 12.3 us, 8 rows 12.3 -> 12.6, 64
+// rows 23 -> 13.8, 128 rows 38 -> 19, 777 rows 171 -> 67; N 1,024, K 2,048: 8 rows 18.4 -> 14.3, 777 rows 101 -> 36; N 6,144, K 1,024, 777
+// rows 267 -> 97.  Error against 64 bits (relative, normal inputs): K = 1,024 5.7e-7 -> 0.9e-7, K = 3,072 1.0e-6 -> 1.2e-7.
 //             (reference: cuBLAS, kernels/src/lib.rs:298-321)
 #include <cooperative_groups.h>
 

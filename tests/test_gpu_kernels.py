@@ -155,7 +155,7 @@ def test_gemm_f32_sizes_keep_a_rows_bits(m, n, k):
 @pytest.mark.parametrize("m,n,k", [(1, 130, 1024), (17, 127, 3072), (95, 129, 2048), (97, 128, 1000), (260, 300, 4100)])
 def test_gemm_f32_keeps_every_bit_of_its_inputs(m, n, k):
     """Both sides of the tiles' edges, short and long ranges of K, one CTA and clusters a tile.  A product of two float32 loses at most
-    2^-24 of itself (parts of 2^-9 and 2^-16 twice), 32 are added by the tensor cores, the rest is k / 32 + 4 additions: within 2^-23 of the sum of the products'
+    2^-24 of itself (parts of 2^-8 and 2^-17 twice), 32 are added by the tensor cores, the rest is k / 32 + 4 additions: within 2^-23 of the sum of the products'
     sizes for the first and, a rounding each, (k / 32 + 4) 2^-24 for the others; and closer than a chain of k multiply-adds in
     float32 comes."""
     g = torch.Generator(device=DEV).manual_seed(m + n + k)
@@ -222,6 +222,19 @@ def test_gemm_f32_of_factors_with_bits_under_the_parts_range(m, n, k):
     odd[[3, 5, 7, n - 1]] = True
     rows = [r for r in range(m) if r not in whole + single]
     assert torch.equal(out[rows][:, ~odd], plain[rows][:, ~odd])
+
+
+@pytest.mark.parametrize("k", [1, 3, 32, 1024])
+def test_gemm_f32_of_factors_whose_parts_are_largest(k):
+    """Factors just below 1 + 2^-8, whose second part is 2^-8 and whose third would be 2^-16 if the second were cut off: a product loses at most
+    2^-24 of itself and is rounded once, few of them are added by few roundings; on average they come within half of that."""
+    g = torch.Generator(device=DEV).manual_seed(k)
+    x, w = (1 + 2.0 ** -8 - torch.randint(1, 200, (rows, k), generator=g, device=DEV) * 2.0 ** -23 for rows in (64, 256))
+    out = torch.empty(64, 256, device=DEV)
+    kernels.gemm_f32(x, w, out)
+    want = x.double() @ w.double().T
+    error = (out.double() - want).abs() / want
+    assert error.max() <= 2.0 ** -24 + (1 + k / 32 + 4 * (k > 1)) * 2.0 ** -24 and error.mean() <= 2.0 ** -24 * (1 + (k > 32))
 
 
 def plain_qk(qkv, positions, q_w, k_w, eps, theta, nq, nkv, d):

@@ -454,10 +454,11 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
 //   warps 8-10  the values' tiles (rows come by cp.async a block ahead, page numbers four)
 //   warp 11     issues the MMAs: scores = q parts (tensor memory) . keys, values = weights (tensor memory) . values
 // A row's result has the same bits however its request is cut: blocks of keys begin at multiples of 64, chunks at multiples of CHUNK, and
-// what a tile holds beside a row touches neither its scores nor its sums.  Values that bfloat16 has no parts for (infinite, NaN, beyond
-// its largest number, so small that the last part lies under its range) are zeros in the tiles and added by the rows that see them; a
-// score that is no number or infinite is computed again from its row and key, so that what a row does not see never reaches it.  (Queries
-// and keys of less than 2^-110 are 2^-134 off at most, which a score shows only beside a factor of 2^100.)
+// what a tile holds beside a row touches neither its scores nor its sums.  Values that the parts cannot be trusted with (infinite, NaN, from
+// 2^64 on, beside which a weight's bits under bfloat16's range would show, or so small that their own last part lies under it) are zeros in
+// the tiles and added by the rows that see them.  A score that is no number or infinite is computed again from its row and key, so that
+// what a row does not see never reaches it, and so is one of a row with bits under bfloat16's range (2^-133) and one with an element
+// from 2^64 on.  (Elsewhere such bits are 2^-62 of a score at most; of weights, 2^-134, they show in sums below 2^-110.)
 //
 // What bounds it: the parts' instructions and the chain of a block (some 7,000 clocks, of which the MMAs run 3,000), a CTA an SM.  Kernel
 // alone, 16 query and 8 key/value heads of 128, on the CUDA cores and here: a prompt of 777 tokens 146 -> 65 us, 880 tokens behind
@@ -473,18 +474,26 @@ constexpr size_t TC_SMEM = 1024 + 6 * (size_t)TC_PART + 2 * (size_t)TC_RAW + TC_
 static_assert(TC_P + 3 * TC_KEYS / 2 <= TC_TMEM, "tensor memory");
 static_assert(CHUNK % TC_KEYS == 0, "whole blocks a chunk");
 constexpr int TC_PLACES = 8, TC_AHEAD = 4;                               // blocks whose places are held; how far ahead they are looked up
-constexpr float BF16_MOST = 3.38953139e38f, BF16_LEAST = 0x1p-96f;
-__device__ __forceinline__ bool has_parts(float v) { return fabsf(v) < BF16_MOST && !(fabsf(v) < BF16_LEAST && v != 0.0f); }
+constexpr float LARGE = 0x1p64f, SMALL = 0x1p-96f;
+__device__ __forceinline__ bool has_parts(float v) { return fabsf(v) < LARGE && !(fabsf(v) < SMALL && v != 0.0f); }
 
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-// four floats as two words of each part; true where the parts are not the floats: what the third one should be has bits below it (a NaN,
-// which arithmetic makes of what is infinite, has all of them)
-__device__ __forceinline__ bool split4(float4 v, uint2 (&parts)[3]) {
+// What was met among floats that became parts: bits that three parts leave (of a NaN, which arithmetic makes of what is infinite, all of
+// them), and the largest size.
+struct Met {
+    uint32_t rest = 0;
+    __nv_bfloat162 top = __floats2bfloat162_rn(0.0f, 0.0f);
+    __device__ __forceinline__ bool lost() const { return rest & LOST_BITS; }
+    __device__ __forceinline__ bool large() const { return fmaxf(__low2float(top), __high2float(top)) >= LARGE; }
+};
+// four floats as two words of each part
+__device__ __forceinline__ void split4(float4 v, uint2 (&parts)[3], Met& met) {
     uint32_t low[3], high[3];
     three_parts(v.x, v.y, low), three_parts(v.z, v.w, high);
 #pragma unroll
     for (int p = 0; p < 3; ++p) parts[p] = make_uint2(low[p], high[p]);
-    return left_bits(v) & LOST_BITS;
+    met.rest |= left_bits(v);
+    met.top = __hmax2(met.top, __hmax2(__habs2(*reinterpret_cast<const __nv_bfloat162*>(&low[0])), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&high[0]))));
 }
 
 // a row and a key that the parts cannot be trusted with
@@ -506,6 +515,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
     __shared__ long long place_s[TC_PLACES][TC_KEYS];                    // where cached rows begin; -1: not seen
     __shared__ float met[2][2][TC_ROWS];
     __shared__ unsigned odd_values[2][TC_KEYS / 32];                     // keys whose values have no parts
+    // rows that met something: of the queries LOST and LARGE_ONE by halves; of a block's keys, by the warp that wrote them, a bit a key that
+    // lost bits and, eight bits further, one a key with a large element
+    __shared__ unsigned char q_facts[2][TC_ROWS];
+    __shared__ __align__(16) unsigned short key_facts[2][TC_ROW_WARPS];
+    constexpr unsigned LOST = 1, LARGE_ONE = 2;
     __shared__ int found[2], warp_count[TC_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int ISSUER = TC_ROW_WARPS + TC_COPY_WARPS;
@@ -561,19 +575,18 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
             copies_commit();
         };
         const uint32_t part_at = (lane >> 4) * (TC_PART / 2) + (lane & 1) * 8, piece = (lane & 15) >> 1;
-        auto put = [&](unsigned char* to, int row, float4 v) {
+        auto put = [&](unsigned char* to, int row, float4 v, Met& met) {
             uint2 parts[3];
-            const bool odd = split4(v, parts);
+            split4(v, parts, met);
             to += part_at + row * 128 + ((piece ^ (row & 7)) << 4);
 #pragma unroll
             for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(to + p * TC_PART) = parts[p];
-            return odd;
         };
         auto raw_of = [&](const unsigned char* raw, int row) { return *reinterpret_cast<const float4*>(raw + row * TC_D * 4 + 16 * lane); };
-        // some read together; whether one of them has no parts
+        // some read together; what was met
         auto convert = [&](auto count, unsigned char* to, const unsigned char* raw, int mine) {
             constexpr int COUNT = decltype(count)::value, TOGETHER = 4;
-            bool odd = false;
+            Met met;
 #pragma unroll 1
             for (int first = mine; first < TC_KEYS; first += TOGETHER * COUNT) {
                 float4 v[TOGETHER];
@@ -581,9 +594,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
                 for (int r = 0; r < TOGETHER; ++r) v[r] = raw_of(raw, min(first + r * COUNT, TC_KEYS - 1));
 #pragma unroll
                 for (int r = 0; r < TOGETHER; ++r)
-                    if (first + r * COUNT < TC_KEYS) odd |= put(to, first + r * COUNT, v[r]);
+                    if (first + r * COUNT < TC_KEYS) put(to, first + r * COUNT, v[r], met);
             }
-            return odd;
+            return met;
         };
         constexpr std::integral_constant<int, TC_ROW_WARPS> by_rows;
         constexpr std::integral_constant<int, TC_COPY_WARPS> by_copies;
@@ -635,16 +648,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
                 if (ct < TC_KEYS / 32) odd_values[i & 1][ct] = 0u;
                 if (ct < TC_KEYS) place_s[(i + TC_AHEAD) % TC_PLACES][ct] = later;
                 bar_sync(1, TC_COPY_WARPS * 32);
-                if (__any_sync(0xffffffffu, convert(by_copies, v_parts, v_raw, mine))) {
+                const Met all = convert(by_copies, v_parts, v_raw, mine);
+                if (__any_sync(0xffffffffu, all.lost() || all.large())) {
 #pragma unroll 1
                     for (int row = mine; row < TC_KEYS; row += TC_COPY_WARPS) {
                         float4 v = raw_of(v_raw, row);
-                        if (!__any_sync(0xffffffffu, put(v_parts, row, v))) continue;      // a row's lanes agree: its readers ask each value
+                        Met met;
+                        put(v_parts, row, v, met);
+                        if (!__any_sync(0xffffffffu, met.lost() || met.large())) continue;      // a row's lanes agree: its readers ask each value
                         if (!has_parts(v.x)) v.x = 0.0f;
                         if (!has_parts(v.y)) v.y = 0.0f;
                         if (!has_parts(v.z)) v.z = 0.0f;
                         if (!has_parts(v.w)) v.w = 0.0f;
-                        put(v_parts, row, v);
+                        put(v_parts, row, v, met);
                         if (lane == 0) atomicOr(&odd_values[i & 1][row / 32], 1u << (row % 32));
                     }
                 }
@@ -660,13 +676,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
             const size_t row_at = (size_t)(t0 + (live ? row / group : 0)) * A.nq + g * group + (live ? row % group : 0);
             const float* q = A.q + row_at * TC_D;
             fetch(by_rows, A.k, k_raw, warp, it, true);
+            Met of_q;
 #pragma unroll 1
             for (int c = 0; c < 64; c += 32) {
                 uint32_t words[3][16];
 #pragma unroll
                 for (int e = 0; e < 32; e += 4) {
                     uint2 parts[3];
-                    split4(live ? *reinterpret_cast<const float4*>(q + half * 64 + c + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f), parts);
+                    split4(live ? *reinterpret_cast<const float4*>(q + half * 64 + c + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f), parts, of_q);
 #pragma unroll
                     for (int p = 0; p < 3; ++p) words[p][e / 2] = parts[p].x, words[p][e / 2 + 1] = parts[p].y;
                 }
@@ -674,10 +691,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
                 for (int p = 0; p < 3; ++p) tmem_store_16_words(lanes + TC_Q + p * (TC_D / 2) + half * 32 + c / 2, words[p]);
             }
             tmem_store_wait();
+            q_facts[half][row] = (of_q.lost() ? LOST : 0) | (of_q.large() ? LARGE_ONE : 0);
             // block i's keys as parts: q is there, and the scores of the block before have been read
             auto keys_ready = [&](int i, bool more) {
                 copies_wait<0>();
-                convert(by_rows, k_parts, k_raw, warp);
+                const Met all = convert(by_rows, k_parts, k_raw, warp);
+                unsigned met_keys = 0;
+                if (__any_sync(0xffffffffu, all.lost() || all.large())) {
+#pragma unroll 1
+                    for (int b = 0; b < TC_KEYS / TC_ROW_WARPS; ++b) {
+                        Met met;
+                        uint2 parts[3];
+                        split4(raw_of(k_raw, warp + b * TC_ROW_WARPS), parts, met);
+                        met_keys |= (__any_sync(0xffffffffu, met.lost()) ? 1u : 0u) << b | (__any_sync(0xffffffffu, met.large()) ? 256u : 0u) << b;
+                    }
+                }
+                if (lane == 0) key_facts[i & 1][warp] = (unsigned short)met_keys;
                 fence_async_shared();
                 tcgen05_fence_before_sync();
                 __syncwarp();
@@ -764,15 +793,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) attention_f32_tc_kernel(const A
                 __syncwarp();
                 tcgen05_fence_after_sync();
                 tmem_load_32(lanes + TC_S + half * 32, x);
+                const uint4 met_keys = *reinterpret_cast<const uint4*>(key_facts[i & 1]);      // block i + 2's come when all warps are here
                 if (n + 1 < blocks) keys_ready(i + 1, n + 2 < blocks);
-                bool odd = false;
+                bool odd = met_keys.x | met_keys.y | met_keys.z | met_keys.w;
 #pragma unroll
                 for (int u = 0; u < 32; ++u) odd |= !(fabsf(x[u]) <= 3.402823466e38f);
-                if (__any_sync(0xffffffffu, odd)) {                      // parts beyond bfloat16's range: the rows and the keys themselves
+                if (__any_sync(0xffffffffu, odd)) {                      // parts that cannot be trusted: the rows and the keys themselves
+                    const unsigned f = q_facts[0][row] | q_facts[1][row], words[4] = {met_keys.x, met_keys.y, met_keys.z, met_keys.w};
 #pragma unroll
                     for (int u = 0; u < 32; ++u) {
                         const int key = at + half * 32 + u;
-                        if (key <= my_pos && key >= my_first && !(fabsf(x[u]) <= 3.402823466e38f)) x[u] = whole_score(q, A.k + place_s[i % TC_PLACES][half * 32 + u]);
+                        const unsigned of_key = words[u % 8 / 2] >> (u % 2 * 16 + half * 4 + u / 8);      // written by warp u % 8, its row half * 4 + u / 8
+                        const bool shows = ((of_key & 1u) && (f & LARGE_ONE)) || ((of_key & 256u) && (f & LOST));
+                        if (key <= my_pos && key >= my_first && (shows || !(fabsf(x[u]) <= 3.402823466e38f)))
+                            x[u] = whole_score(q, A.k + place_s[i % TC_PLACES][half * 32 + u]);
                     }
                 }
                 if (at + TC_KEYS > pos0 + 1 || (A.window > 0 && at < end_key - A.window)) {       // some row does not see all of the block

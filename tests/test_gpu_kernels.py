@@ -1460,6 +1460,61 @@ def test_attention_f32_on_tensor_cores_of_small_and_large_values(exponent):
     assert (got - want * 2.0 ** exponent).abs().max().item() <= 2 * error * 2.0 ** exponent + 305 * 2.0 ** -150 * 4
 
 
+@pytest.mark.parametrize("small,large", [(1.2345678e-38, 2e38), (1.3e-40, 3e38), (1.7e-36, 1e37)])
+def test_attention_f32_on_tensor_cores_of_factors_with_bits_under_the_parts_range(small, large):
+    """Heads of 128: an element of the queries whose last bits bfloat16 has no room for beside large ones of the keys, and the other way
+    round; scores of ordinary size come of it.  Rows and keys without such elements keep their bits."""
+    nq, nkv, d = 4, 2, 128
+    case = PagedCase(torch.float32, nq, nkv, d, 16, [(0, 150), (290, 4)], seed=21)
+    clean = case.run_simt().view(-1, nq, d)
+    g = torch.Generator().manual_seed(3)
+    q, kept = case.q.view(-1, nq, d), case.q.clone()
+
+    def set_key(request, key, head, column, value):
+        case.kc[case.table[request, key // 16], head, key % 16, column] = value
+        case.ks[request][key, head, column] = value
+
+    # queries of heads 0 and 1 (key head 0) small in column 5, every third key large there
+    q[:, :2, 5] = small * (1 + torch.rand(q.shape[0], 2, generator=g))
+    for request, length in ((0, 150), (1, 294)):
+        for key in range(0, length, 3):
+            set_key(request, key, 0, 5, large * (0.5 + 0.5 * float(torch.rand((), generator=g))) * (-1) ** key)
+    got = case.run_simt()
+    close(got, case.plain(), torch.float32, "small queries, large keys")
+    assert torch.equal(got.view(-1, nq, d)[:, 2:], clean[:, 2:])
+    # the other way round: every third key small, the others nothing there
+    case.q.copy_(kept)
+    q[:, :2, 5] = large * (0.5 + 0.5 * torch.rand(q.shape[0], 2, generator=g))
+    for request, length in ((0, 150), (1, 294)):
+        for key in range(length):
+            set_key(request, key, 0, 5, small * (1 + float(torch.rand((), generator=g))) if key % 3 == 0 else 0.0)
+    got = case.run_simt()
+    close(got, case.plain(), torch.float32, "large queries, small keys")
+    assert torch.equal(got.view(-1, nq, d)[:, 2:], clean[:, 2:])
+
+
+def test_attention_f32_on_tensor_cores_of_a_small_weight_and_a_large_value():
+    """Heads of 128: one key's weight is exp(-86), whose last bits bfloat16 has no room for, and its value brings their product to 1."""
+    nq, nkv, d = 4, 2, 128
+    case = PagedCase(torch.float32, nq, nkv, d, 16, [(0, 90), (400, 2)], seed=22)
+    case.q.zero_()
+    case.q.view(-1, nq, d)[:, :, 7] = 10.0
+    case.kc[:, :, :, 7] = 0.0
+    case.vc[:, :, :, 9] = 0.0
+    for request in range(2):
+        case.ks[request][:, :, 7] = 0.0
+        case.vs[request][:, :, 9] = 0.0
+        for key in (3, 70):
+            case.kc[case.table[request, key // 16], :, key % 16, 7] = -8.6 * d ** 0.5
+            case.ks[request][key, :, 7] = -8.6 * d ** 0.5
+            case.vc[case.table[request, key // 16], :, key % 16, 9] = 3e37
+            case.vs[request][key, :, 9] = 3e37
+    got, want = case.run_simt(), case.plain()
+    close(got, want, torch.float32, "small weights")
+    got, want = (x.double().cpu().view(-1, nq, d)[:, :, 9] for x in (got, want))
+    assert (want[3:] > 1e-3).all() and ((got - want).abs() <= 2e-5 * want.abs()).all()
+
+
 @pytest.mark.parametrize("whole", [False, True])
 @pytest.mark.parametrize("window", [0, 300])
 def test_attention_f32_on_tensor_cores_of_values_without_parts(monkeypatch, window, whole):

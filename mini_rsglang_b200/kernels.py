@@ -7,7 +7,6 @@ or without the compiled library, they raise `BackendError`."""
 from __future__ import annotations
 
 import ctypes
-import functools
 import math
 import os
 
@@ -897,41 +896,17 @@ def gemm_tc_qkv_heads(x: torch.Tensor, weight: torch.Tensor, q_out: torch.Tensor
 # ------------------------------------------------------------------------------------------------
 _many_rows_lib = None
 _many_rows_maps: dict[tuple, tuple] = {}
-# Measured against the library's product followed by `silu_mul` (8B shape, K 4096, N 24576): 290 against 299 us at
-# 2,048 rows, 418 against 429 us at 3,072, 550 against 646 us at 4,096.  At other shapes the order differs (prefill of 2,048 tokens: 14B
-# shape, K 5120, N 34816: 58.2 ms with this kernel against 57.7 ms), so from GEMM_GATED_ROWS_MIN rows on the two are timed
-# once per (N, K, thousand of rows) on the first such product and the faster one is kept (`gemm_gated_rows_wins`); below, the count
-# of the tiles says it (`gemm_gated_rows_fills`).
+# Measured against the library's product followed by `silu_mul` (8B shape, K 4096, N 24576): 278 against 292 us at
+# 2,048 rows, 550 against 646 us at 4,096.  Below 2,048 rows the library's pair stays: of eight shapes (N 6,144 to 34,816,
+# K 1,024 to 5,120) and 128 to 1,920 rows its time was 0.74 to 1.30 of this kernel's, and which is ahead follows the
+# library's choice of tiles (N 24,576: 79 against 92 us at 512 rows, 82 against 71 at 384; N 8,192, K 2,048: 19 against 22
+# at 512, 42 against 35 at 1,152; N 12,288: 34 against 36 at 768, in two full rounds) and no count of rounds that was tried.
+# From GEMM_GATED_ROWS_MIN rows on the order differs too (14B shape, K 5120, N 34816, prefill of 2,048 tokens: 58.2 ms with
+# this kernel against 57.7 ms), so the two are timed once per (N, K, thousand of rows) on the first such product and the
+# faster one is kept (`gemm_gated_rows_wins`): where they are about as fast, a step's bits follow that timing.
 GEMM_GATED_ROWS_MIN = int(os.environ.get("MRS_GEMM_GATED_ROWS_MIN", "2048"))      # the variable: for measuring other crossovers
 GEMM_GATED_MEASURE = "MRS_GEMM_GATED_ROWS_MIN" not in os.environ                  # False: the kernel from that many rows on
 _gated_rows_choice: dict[tuple, bool] = {}
-
-
-def gemm_gated_rows_fills(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    """Whether the tcgen05 gate/up product takes fewer than GEMM_GATED_ROWS_MIN rows, by how well its tiles of 128 x 256 fill the SMs'
-    rounds with rows that are there.  On the device, with the library's product and `silu_mul` behind it:
-      one round            from 0.56 of the SMs on: N 6,144, K 1,024, 448 to 768 rows 11.3 to 11.5 against 11.7 to 14.1 us, 400 rows (0.51) 11.2
-                           against 11.0, 64 rows 9.8 against 7.7; N 16,384, K 2,048, 256 rows 18.8 against 20.5, 128 (0.43) 18.2 against 16.9
-      K > 2,048, one round up to 128 rows: the weights' bytes are the time, the activation's kernel comes on top (N 24,576, K 4,096, 17 to 128
-                           rows 38 to 40 against 38 to 42; N 34,816, K 5,120 58 to 61 against 64 to 71)
-      K > 2,048, more      the library's tiles are the better ones but where two rounds are full (N 24,576, K 4,096, 384 rows 65 against 76;
-                           350 rows 64 against 60, 512 85 against 79, 1,024 156 against 149)
-      K <= 2,048, more     from 0.72 on: N 16,384, K 2,048, 448 rows 29.8 against 31.0, 1,300 68 against 71, 400 rows (0.68) 29.1 against 27.2
-    Products smaller than the least measured one (N 4,096, K 1,024) stay with the library."""
-    rows = x.shape[0]
-    return 0 < rows < GEMM_GATED_ROWS_MIN and _rows_fill(rows, *weight.shape, sm_count(x.device)) and gemm_gated_rows_supported(x, weight)
-
-
-@functools.lru_cache(maxsize=4096)
-def _rows_fill(rows: int, n: int, k: int, sms: int) -> bool:
-    """`gemm_gated_rows_fills`, of the sizes."""
-    if n < 4096 or k < 1024:
-        return False
-    columns = -(-n // 256)
-    rounds, filled = -(-(-(-rows // 128) * columns) // sms), rows * columns / (128 * sms)
-    if rounds == 1:
-        return filled >= 0.56 or (k > 2048 and rows <= 128 and columns >= 0.6 * sms)
-    return filled >= (0.72 if k <= 2048 else 0.95 if rounds == 2 else math.inf) * rounds
 
 
 def gemm_gated_rows_wins(x: torch.Tensor, weight: torch.Tensor, gate: str = "silu") -> bool:

@@ -58,8 +58,7 @@ class SwiGLU(FeedForward):
                 kernels.gemm_tc(h, self.gate_up, act, gated=True)
         else:
             h = plain(h)
-            if self.block == 64 and not observing(ctx) and (kernels.gemm_gated_rows_fills(h, self.gate_up)
-                                                            or kernels.gemm_gated_rows_wins(h, self.gate_up)):
+            if self.block == 64 and not observing(ctx) and kernels.gemm_gated_rows_wins(h, self.gate_up):
                 kernels.gemm_gated_rows(h, self.gate_up, act)      # many rows: the tcgen05 product with the activation in it
             else:
                 kernels.silu_mul(linear(h, self.gate_up), act, self.block)
@@ -183,7 +182,7 @@ class GatedMLP(FeedForward):
         if self.block and self.activation in kernels.GEMM_TC_GATES and few_rows(h, self.gate_up) and not observing(ctx):
             kernels.gemm_tc(h, self.gate_up, act, gated=True, gate=self.activation)          # few rows: the product's tiles hold both halves
         elif self.block and self.activation in kernels.GATE_ACTIVATIONS and not observing(ctx) \
-                and (kernels.gemm_gated_rows_fills(h, self.gate_up) or kernels.gemm_gated_rows_wins(h, self.gate_up, self.activation)):
+                and kernels.gemm_gated_rows_wins(h, self.gate_up, self.activation):
             kernels.gemm_gated_rows(h, self.gate_up, act, self.activation)
         else:
             kernels.gated_activation(linear(h, self.gate_up), act, self.activation, self.block)

@@ -144,11 +144,3 @@ def test_shares_beside_narrow_tiles_count_the_bytes_of_their_keys(group, decodes
         lists = attention_tile_lists(facts, group, kernels.PREFILL_TC_ROWS, 8, 0, 128, 148, d)
         assert {max(share >> 8 & 0xFF, 1) for *_, share in lists.wide} == {shares}, d
     assert attention_tile_lists(facts, group, kernels.PREFILL_TC_ROWS, 8, 0, 128, 148) is attention_tile_lists(facts, group, kernels.PREFILL_TC_ROWS, 8, 0, 128, 148, 128)
-
-
-@pytest.mark.parametrize("n,k,chosen", [(6144, 1024, {448, 512, 768, 1300}), (16384, 2048, {192, 256, 448, 512, 768, 1024, 1300}),
-                                        (24576, 4096, {17, 64, 128, 384}), (34816, 5120, {17, 64, 128}), (2048, 1024, set()), (6144, 512, set())])
-def test_the_gate_up_product_takes_rows_that_fill_its_rounds(n, k, chosen):
-    """Which row counts the product with the activation in it takes on 148 SMs: those it was measured ahead at."""
-    rows = (17, 64, 128, 192, 256, 350, 384, 448, 512, 768, 1024, 1300)
-    assert {m for m in rows if kernels._rows_fill(m, n, k, 148)} == chosen & set(rows)

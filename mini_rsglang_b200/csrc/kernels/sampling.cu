@@ -492,15 +492,8 @@ __device__ Reached sample_reached(SampleShared& s, int n, int listed, const unsi
     return Reached{key, equals, above > 0 ? (double)sums[above - 1] * UNIT : 0.0};
 }
 
-// The rows' parameters: arrays on the device, or (what the host has just made) up to ROWS of them in the launch itself: reading them
-// from pinned memory takes a row 10 us (24 rows 57 instead of 45), a copy to the device a launch.
-struct SampleArrays {
-    const float* temperature;
-    const int* top_k;
-    const float* top_p;
-    const unsigned long long* seed;
-    const int* draw_index;
-};
+// The parameters of up to ROWS rows, in the launch itself: reading them from pinned memory takes a row 10 us (24 rows 57 instead of
+// 45), a copy to the device a launch.
 template <int ROWS>
 struct SampleWords {
     unsigned long long seed[ROWS];
@@ -512,9 +505,9 @@ struct SampleWords {
 
 // IN_SHARED: the CTA's share of the row lies in shared memory (and gives its place to the weights of the kept set);
 // otherwise a row is too long for that and is read from memory each time.
-template <bool IN_SHARED, typename Params>
+template <bool IN_SHARED, int ROWS>
 __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
-    const float* __restrict__ logits, int vocab, int per_segment, const __grid_constant__ Params params, int* __restrict__ out,
+    const float* __restrict__ logits, int vocab, int per_segment, const __grid_constant__ SampleWords<ROWS> params, int* __restrict__ out,
     int* __restrict__ copy) {
     pdl_launch_dependents();
     pdl_wait();
@@ -533,7 +526,7 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
 
     auto answer = [&](int token) {
         out[r] = token;
-        if (copy) copy[r] = token;
+        copy[r] = token;
     };
     // Largest logit (also the greedy answer) and a check that the row is finite.
     int bad = 0;
@@ -852,8 +845,8 @@ __global__ void __launch_bounds__(SAMPLE_CTA_THREADS, 2) sample_kernel(
     }
 }
 
-template <typename Params>
-static int launch_sample(const float* logits, int rows, int vocab, const Params& params, int* out, int* copy, void* stream) {
+template <int ROWS>
+static int launch_sample(const float* logits, int rows, int vocab, const SampleWords<ROWS>& params, int* out, int* copy, void* stream) {
     const int per_segment = (int)((((long long)vocab + SAMPLE_SEGMENTS - 1) / SAMPLE_SEGMENTS + 31) & ~31LL);
     // short rows gain nothing from more CTAs: their meetings cost more than the walks
     const int blocks = vocab >= 65536 ? 8 : (vocab >= 8192 ? 4 : 1);
@@ -861,7 +854,7 @@ static int launch_sample(const float* logits, int rows, int vocab, const Params&
     const bool in_shared = share <= SAMPLE_SHARE_BYTES;
     static PerDevice configured;
     if (!configured.get()) {
-        const cudaError_t e = cudaFuncSetAttribute(sample_kernel<true, Params>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SHARE_BYTES);
+        const cudaError_t e = cudaFuncSetAttribute(sample_kernel<true, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SHARE_BYTES);
         if (e != cudaSuccess) return (int)e;
         configured.set(1);
     }
@@ -878,20 +871,10 @@ static int launch_sample(const float* logits, int rows, int vocab, const Params&
     static const bool plain = getenv("MRS_PLAIN_LAUNCH") != nullptr;
     config.attrs = attributes;
     config.numAttrs = plain ? 1 : 2;
-    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true, Params>, logits, vocab, per_segment, params, out, copy)
-                                    : cudaLaunchKernelEx(&config, sample_kernel<false, Params>, logits, vocab, per_segment, params, out, copy);
+    const cudaError_t e = in_shared ? cudaLaunchKernelEx(&config, sample_kernel<true, ROWS>, logits, vocab, per_segment, params, out, copy)
+                                    : cudaLaunchKernelEx(&config, sample_kernel<false, ROWS>, logits, vocab, per_segment, params, out, copy);
     if (e != cudaSuccess) return (int)e;
     MRS_RETURN_LAUNCH_STATUS();
-}
-
-// temperature, top_k (<= 0: off), top_p, seed and draw_index are per row.
-// out[r] = the token, or -1 when the row holds a NaN or an infinity.
-MRS_EXPORT int mrs_sample(const float* logits, int rows, int vocab, const float* temperature, const int* top_k,
-                          const float* top_p, const unsigned long long* seed, const int* draw_index, int* out,
-                          void* stream) {
-    if (rows <= 0) return 0;
-    if (vocab <= 0 || rows > 0x7fffffff / 8) return MRS_BAD_ARGUMENT;
-    return launch_sample(logits, rows, vocab, SampleArrays{temperature, top_k, top_p, seed, draw_index}, out, nullptr, stream);
 }
 
 template <int ROWS>
@@ -907,8 +890,9 @@ static int launch_sample_words(const float* logits, int first, int count, int ro
     return launch_sample(logits + (size_t)first * vocab, count, vocab, w, out + first, copy + first, stream);
 }
 
-// The same with the parameters in the host's memory, read before this returns: all rows' seeds, then their temperatures, top_k, top_p
-// and draw indices.  copy[r] = out[r], in pinned memory: complete when the stream has come here.
+// `words`, in the host's memory and read before this returns: all rows' seeds, then their temperatures, top_k (<= 0: off), top_p and draw
+// indices.  out[r] = the token, or -1 when the row holds a NaN or an infinity; copy[r] = out[r], in pinned memory: complete when the
+// stream has come here.
 MRS_EXPORT int mrs_sample_words(const float* logits, int rows, int vocab, const unsigned char* words, int* out, int* copy, void* stream) {
     if (rows <= 0) return 0;
     if (vocab <= 0 || rows > 0x7fffffff / 8 || !words || !copy) return MRS_BAD_ARGUMENT;

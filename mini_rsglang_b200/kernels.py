@@ -33,7 +33,6 @@ _SIGNATURES = {
     "mrs_attention_f32_chunk": [],
     "mrs_gemm_f32": [_c_vp, _c_vp, _c_vp, _c_int, _c_int, _c_int, _c_vp],
     "mrs_argmax": [_c_vp, _c_vp, _c_int, _c_int, _c_vp],
-    "mrs_sample": [_c_vp, _c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp],
     "mrs_sample_words": [_c_vp, _c_int, _c_int, ctypes.c_char_p, _c_vp, _c_vp, _c_vp],
 }
 
@@ -309,24 +308,10 @@ def argmax(logits: torch.Tensor, out: torch.Tensor) -> None:
     _check(library().mrs_argmax(logits.data_ptr(), out.data_ptr(), rows, vocab, _stream()), "argmax")
 
 
-def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor,
-           seed: torch.Tensor, draw_index: torch.Tensor, out: torch.Tensor) -> None:
-    rows, vocab = logits.shape
-    _need(logits, torch.float32, "logits")
-    _need(temperature, torch.float32, "temperature", (rows,))
-    _need(top_k, torch.int32, "top_k", (rows,))
-    _need(top_p, torch.float32, "top_p", (rows,))
-    _need(seed, torch.int64, "seed", (rows,))
-    _need(draw_index, torch.int32, "draw_index", (rows,))
-    _need(out, torch.int32, "sample out", (rows,))
-    _check(library().mrs_sample(logits.data_ptr(), rows, vocab, temperature.data_ptr(), top_k.data_ptr(),
-                                top_p.data_ptr(), seed.data_ptr(), draw_index.data_ptr(), out.data_ptr(),
-                                _stream()), "sample")
-
-
 def sample_words(logits: torch.Tensor, words: bytes, out: torch.Tensor, copy: int) -> None:
-    """`sample` with the rows' parameters as the words of `sampling.packed_parameters`, which travel with the launch, and the
-    tokens also written to address `copy` in pinned host memory, which stays until the kernel has ended."""
+    """A token a row by temperature, top_k and top_p (argmax for a temperature of 0, -1 for a row that is not finite): the rows' parameters
+    are the words of `sampling.packed_parameters` and travel with the launch; the tokens go to `out` and to address `copy` in
+    pinned host memory, which stays until the kernel has ended."""
     rows, vocab = logits.shape
     _need(logits, torch.float32, "logits")
     _need(out, torch.int32, "sample out", (rows,))

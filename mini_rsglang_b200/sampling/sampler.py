@@ -86,6 +86,7 @@ class Sampler:
         self.device = device
         self._turns: list[_Turn | None] = [None] * 3         # two results may be outstanding
         self._at = 0
+        self._recorded: list[_Turn] = []                     # of launches in graphs, which write again at every replay
 
     def __del__(self):
         for turn in getattr(self, "_turns", ()):
@@ -97,6 +98,9 @@ class Sampler:
 
     def _turn(self, rows: int) -> _Turn:
         """Pinned memory for `rows` rows that no launch uses any more."""
+        if torch.cuda.is_current_stream_capturing():         # an event of a graph cannot be waited for
+            self._recorded.append(_Turn(rows))
+            return self._recorded[-1]
         self._at = (self._at + 1) % 3
         turn = self._turns[self._at]
         if turn is not None:
@@ -127,13 +131,16 @@ class Sampler:
         turn = self._turn(rows)
         host = turn.tokens[:rows]
         arrived = torch.cuda.Event()
-        if all(p.is_greedy() for p in params):
-            kernels.argmax(logits, out)
-            host.copy_(out, non_blocking=True)
-        else:
-            # The parameters travel with the launch and the kernel writes the tokens to pinned memory: a copy each way is a launch on the
-            # host and a wait on the device (with numpy's arrays and copies a launch took the host 75 us for 24 rows, the kernel 68).
-            kernels.sample_words(logits, packed_bytes(params, draw_index), out, host.data_ptr())
-        arrived.record()
-        turn.last = arrived
+        try:
+            if all(p.is_greedy() for p in params):
+                kernels.argmax(logits, out)
+                host.copy_(out, non_blocking=True)
+            else:
+                # The parameters travel with the launch and the kernel writes the tokens to pinned memory: a copy each way is a launch on the
+                # host and a wait on the device (with numpy's arrays and copies a launch took the host 75 us for 24 rows, the kernel 68).
+                kernels.sample_words(logits, packed_bytes(params, draw_index), out, host.data_ptr())
+        finally:                                             # many rows are several launches: one may fail behind others
+            arrived.record()
+            if turn in self._turns:
+                turn.last = arrived
         return Chosen(out, host, arrived)

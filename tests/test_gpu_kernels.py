@@ -1158,6 +1158,27 @@ def test_sampler_launches_that_are_outstanding():
     assert last.host.tolist() == want
 
 
+@pytest.mark.parametrize("greedy", [False, True])
+def test_sampler_launches_in_a_graph(greedy):
+    """More launches recorded in one graph than a sampler has buffers in turn, behind and before ordinary ones; every replay chooses from
+    the logits that are there then."""
+    params = [SamplingParams(temperature=0.0 if greedy else 0.9, top_k=None if greedy else 30, seed=i) for i in range(7)]
+    logits, sampler = torch.randn(7, 5000, device=DEV), Sampler(torch.device(DEV))
+    for _ in range(4):
+        sampler.sample(logits, params, [0] * 7)
+    graph, held = torch.cuda.CUDAGraph(), []
+    with torch.cuda.graph(graph):
+        for n in range(5):
+            held.append(sampler.launch(logits, params, [n] * 7))
+    for _ in range(2):
+        logits.normal_()
+        graph.replay()
+        torch.cuda.synchronize()
+        for n, chosen in enumerate(held):
+            want = sampler.sample(logits, params, [n] * 7)
+            assert chosen.tokens.tolist() == want and chosen.host.tolist() == want
+
+
 def drawn(row, p, index, token, tolerance) -> bool:
     """Whether `token` is the draw restated in float64: the support by a stable sort, then the inverse CDF in id order.  A token that is
     not has to be one that float32 sums may give instead: u within `tolerance` of the kept weight of that token's own interval, and the

@@ -14,10 +14,10 @@
 //
 // Heads of 128 elements run on the tensor cores (below).  The other sizes: bound by the multiply-add pipe and shared memory for prompts;
 // for decoded tokens by a tile's chain of page numbers, keys, scores, weights and values.  Up to 8 rows take steps of two blocks: a warp
-// a row and a block of scores, a column a thread, keys of two steps and values of one ahead, page numbers three.  Chunks of 256 keys: of
-// 512, 400 tokens walk 13 blocks in a row on a third of the SMs (attention layer with 16 heads of 128 on this kernel 199 against
-// 167 us; 20 tokens behind 980 126 against 78); of 128, the joining outweighs it (decoded tokens of 4 requests at 3,000 98 against 92, 880
-// tokens behind 1,420 863 against 687 us).
+// a row and a block of scores, a column a thread, keys of two steps and values of one ahead, page numbers three.  Chunks of 256 keys, with
+// the joining, from a cold L2, 16 query and 8 key/value heads of 64 and of 256: of 512, 400 tokens walk 13 blocks in a row on a third of
+// the SMs (52 and 139 us against 50 and 105), 20 tokens behind 980 take 49 and 113 against 29 and 64; of 128, the joining outweighs it
+// (880 tokens behind 1,420 361 and 1,319 against 322 and 1,153).
 #include "parts3.cuh"
 #include "tcgen05.cuh"
 
@@ -460,10 +460,11 @@ __global__ void __launch_bounds__(THREADS, D <= 128 ? 2 : 1) attention_f32_kerne
 // what a row does not see never reaches it, and so is one of a row with bits under bfloat16's range (2^-133) and one with an element
 // from 2^64 on.  (Elsewhere such bits are 2^-62 of a score at most; of weights, 2^-134, they show in sums below 2^-110.)
 //
-// What bounds it: the parts' instructions and the chain of a block (some 7,000 clocks, of which the MMAs run 3,000), a CTA an SM.  Kernel
-// alone, 16 query and 8 key/value heads of 128, on the CUDA cores and here: a prompt of 777 tokens 146 -> 65 us, 880 tokens behind
-// 1,420 497 -> 205.  Decoded tokens pay for 128 rows: one behind 4,000 18 -> 25, 4 requests at 3,000 41 -> 77, 30 at 400 38 -> 75 (105, 112 and
-// 99 before either); they take this kernel for the bits' sake.  Error of the layer against 64 bits: 1.26e-6 -> 1.24e-6 (777 tokens).
+// What bounds it: the parts' instructions and the chain of a block (some 7,000 clocks, of which the MMAs run 3,000), a CTA an SM.  With the
+// joining, from a cold L2, 16 query and 8 key/value heads of 128, on the CUDA cores (the kernel above) and here: a prompt of 777 tokens
+// 159 -> 76 us, 880 tokens behind 1,420 514 -> 229, 20 behind 980 41 -> 31.  Decoded tokens pay for 128 rows: one behind 4,000 24 -> 32, 4
+// requests at 3,000 47 -> 81, 30 at 400 46 -> 92; they take this kernel for the bits' sake.  Error of the layer against 64 bits:
+// 1.26e-6 -> 1.24e-6 (777 tokens).
 // Tried: all conversions in the copying warps (100 us at 777 tokens), masks and exponentials with a branch an element (softmax 10,700
 // clocks a block, 2,000 now).
 // ------------------------------------------------------------------------------------------------

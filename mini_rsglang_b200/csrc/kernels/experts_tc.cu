@@ -12,7 +12,8 @@
 // Bound by the weights' bytes, then by the MMAs.  With one thread a row the epilogue took a tile 18,000 clocks, longer than its MMAs
 // (16,400 at K = 2,048); two take half of that.  With that, the weights' policy below and no rows fetched for places without a pair, from a
 // cold L2: 32 experts, 1,777 tokens x 4, width 2,048, inner 1,024: gated product 88.9 -> 76.2 us, down product 49.2 -> 45.5; 200 tokens,
-// width 4,096, inner 1,536: 161 -> 157 and 84.8 -> 74.9.  Two tiles of rows a CTA (weights fetched once for 256 rows) leave some SMs 6 tiles where others have 2 and no accumulator free meanwhile: 107 us.
+// width 4,096, inner 1,536: 161 -> 157 and 84.8 -> 74.9.  Two tiles of rows a CTA (weights fetched once for 256 rows) leave some SMs 6
+// tiles where others have 2 and no accumulator free meanwhile: 107 us for the gated product of 1,777 tokens.
 // Only the tiles that the lists use are walked: their count stands behind the tiles' experts.  CTAs are
 // persistent; tiles that share a weight tile are taken by neighbouring CTAs at the same time.  Every wait is bounded
 // (tma.cuh).
@@ -28,8 +29,10 @@ constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + (2 * STAGES 
 
 // How L2 keeps a tile of weights: to go first where the tiles of rows that share it, which run side by side, are done with it before
 // it would go; the gathered rows, which come once for every 256 weight rows, then stay.  All SMs' tiles of weights are 148 * 512 K bytes
-// at a time, and as long as these about fit L2 that is so: K = 2,048 78 -> 68 us (DRAM reads 407 -> 310 MB, of 268 MB of weights), 500 rows
-// 55 -> 47; K = 1,536 111 -> 103 and 84 -> 77 us; K = 4,096 163 -> 160 us at 700 rows, but 214 -> 237 at 1,777, where tiles drift apart.
+// at a time, and as long as these about fit L2 that is so: times without and with it, from a cold L2, 32 experts, 4 choices a token, are
+// 1.01 to 1.17 over K = 512 to 2,048 and 200 to 4,096 tokens (K = 2,048, 1,777 tokens 85.6 and 76.2 us, DRAM reads 407 and 310 MB, of
+// 268 MB of weights), 0.96 to 1.09 at 8,192 tokens.  Beyond, it holds for fewer and fewer tokens: K = 2,560 1.02 at 4,096 and 0.95
+// at 8,192, K = 3,072 1.10 at 1,777 and 0.88 at 4,096, K = 4,096 1.02 and 0.84: tiles drift apart.
 constexpr int STREAMED_K = 2048;
 __device__ __forceinline__ uint64_t weights_policy(bool first_to_go) {
     uint64_t policy;

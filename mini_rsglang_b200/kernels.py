@@ -253,9 +253,9 @@ ATTENTION_F32_PARTS_BYTES = 128 << 20      # scratch up to which the chunks of a
 def attention_simt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, positions: torch.Tensor,
                    seq_of_token: torch.Tensor, block_table: torch.Tensor, out: torch.Tensor, nq: int, nkv: int,
                    d: int, window: int = 0, scale: float | None = None, longest: int = 0) -> None:
-    """Causal paged attention on the CUDA cores; any sizes; float32 or bfloat16.  float32 with heads of a multiple of 4
-    elements and up to 64 query heads a key/value head takes tiles of rows (`attention_f32.cu`), the rest one warp a (token,
-    head).  `longest`: keys of the longest row as far as the host knows (0: the block table's width); with few rows and long
+    """Causal paged attention for any sizes; float32 or bfloat16.  float32 with heads of a multiple of 4 elements and up to 64
+    query heads a key/value head takes tiles of rows (`attention_f32.cu`: heads of 128 on the tensor cores with every bit of
+    the inputs, others on the CUDA cores), the rest one warp a (token, head) on the CUDA cores.  `longest`: keys of the longest row as far as the host knows (0: the block table's width); with few rows and long
     contexts the keys are then shared among blocks in chunks, and a second kernel joins them."""
     global launch_count
     tokens = q.shape[0]
@@ -273,8 +273,9 @@ def attention_simt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
     lib = library()
     if q.dtype is torch.float32 and d % 4 == 0 and d <= 256 and nkv > 0 and nq % nkv == 0 and nq // nkv <= 64 and \
             not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) & 15:
-        # A prompt of 777 rows of 16 heads walks at most two chunks: 26 tiles x 8 heads are 1.4 rounds of SMs, with blocks a
-        # chunk 2.1 shorter ones.  Many rows have blocks enough, and their parts would cost more than they bring.
+        # A prompt of 777 tokens, 16 heads on 8 key/value heads of 128: 13 tiles x 8 heads are 104 blocks, the last of which walk
+        # all keys; with blocks a chunk 224 shorter ones.  Many rows have blocks enough, and their parts would cost more than
+        # they bring.
         chunks = -(-(longest or block_table.shape[1] * page_size) // int(lib.mrs_attention_f32_chunk()))
         floats = tokens * nq * chunks * (d + 2)
         parts = None
@@ -292,7 +293,8 @@ def attention_simt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
 
 
 def gemm_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
-    """out[M, N] = x[M, K] . weight[N, K]^T in true float32 (CUDA-core FMA)."""
+    """out[M, N] = x[M, K] . weight[N, K]^T in float32: on the tensor cores from three bfloat16 of every float32, sums in float32
+    (`gemm_f32.cu`)."""
     m, k = x.shape
     n = weight.shape[0]
     _need(x, torch.float32, "gemm input")

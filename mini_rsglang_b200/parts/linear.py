@@ -1,7 +1,7 @@
 """Matrix products y = x . W^T (W stored [out, in], no bias).
 
-On the 32-bit path the product is the engine's own float32 kernel (CUDA-core FMA, no
-reduced-precision mode).  When serving in bfloat16, up to 128 rows (decoded tokens, short
+On the 32-bit path the product is the engine's own float32 kernel (tcgen05 over three
+bfloat16 of every float32, so that no bit of the inputs is given up; no reduced-precision mode).  When serving in bfloat16, up to 128 rows (decoded tokens, short
 portions) go through the engine's tcgen05 kernel, which streams the weights once with bulk
 tensor copies; more rows go through the library (cuBLAS through torch.mm, float32
 accumulation, reduced-precision reductions switched off), as the reference uses cuBLAS for

@@ -7,8 +7,8 @@
 // float32 addition in registers: 32-element sums into one of four ranges of K, the four ranges in order.  An element's bits depend
 // on K alone: not on M, not on the tile or the cut that the sizes chose, and a token's result does not change with what else is in the
 // batch.  Results that the parts cannot be trusted with are computed again in float64 from the inputs: those that are no number or
-// infinite, so that infinities and NaN are those of the sum of the products; those below 2^-60, whose smallest products may lie under
-// float32's range (`store_column`); and those of rows with an element below some 2^-110, which has bits under bfloat16's range (2^-133),
+// infinite, so that infinities and NaN are those of the sum of the products; those below 2^-100, whose smallest products lie near the end
+// of float32's range (`store_column`; products down to 2^-120 come as close to 64 bits as ordinary ones, 2^-125 a little less); and those of rows with an element below some 2^-110, which has bits under bfloat16's range (2^-133),
 // where the result is below 2^-60 or the other row has an element from 2^24 on (`mend_lost`).  Elsewhere K such bits are less than
 // K 2^-48 of the result.  Looking for them takes 0.4 to 0.8 us of a call of up to 128 rows (K = 1,024 to 3,072), none that shows of 777.
 //
@@ -102,7 +102,7 @@ __device__ __noinline__ float exact_dot(const float* __restrict__ a, const float
 // What a row's elements say of its results: some have bits under bfloat16's range; some are large enough for the other row's such bits
 // to show.  The whole warp.
 constexpr unsigned LOST = 1, LARGE = 2;
-constexpr float LEAST = 0x1p-60f;
+constexpr float LEAST = 0x1p-100f, LEAST_OF_LOST = 0x1p-60f;
 __device__ __noinline__ unsigned row_facts(const float* __restrict__ row, int K) {
     uint32_t rest = 0;
     float top = 0.0f;
@@ -131,7 +131,7 @@ __device__ __noinline__ void mend_lost(unsigned char* facts, const float* __rest
         const int row = task % (BM / 32) * 32 + lane, n = n0 + row, m = m0 + task / (BM / 32);
         const unsigned w = facts[row], a = facts[BM + m - m0];
         const bool lost = (w | a) & LOST, shows = ((w & LARGE) && (a & LOST)) || ((w & LOST) && (a & LARGE));
-        unsigned odd = __ballot_sync(0xffffffffu, n < N && lost && (shows || fabsf(C[(size_t)m * N + n]) < LEAST));
+        unsigned odd = __ballot_sync(0xffffffffu, n < N && lost && (shows || fabsf(C[(size_t)m * N + n]) < LEAST_OF_LOST));
         while (odd) {
             const int of = __ffs(odd) - 1;
             odd &= odd - 1;

@@ -224,6 +224,19 @@ def test_gemm_f32_of_factors_with_bits_under_the_parts_range(m, n, k):
     assert torch.equal(out[rows][:, ~odd], plain[rows][:, ~odd])
 
 
+@pytest.mark.parametrize("exponents", [(-30, -31), (-50, -49), (-50, -52), (-55, -60), (-62, -63), (-109, 3)])
+def test_gemm_f32_of_small_results(exponents):
+    """Results on both sides of 2^-100, below which they are computed again, down to 2^-125, and factors that just have their parts: the
+    error of ordinary ones, a rounding to a subnormal beside it."""
+    g = torch.Generator(device=DEV).manual_seed(2)
+    for k in (1, 300, 1024):
+        x, w = (torch.ldexp(torch.randn(rows, k, device=DEV, generator=g), torch.tensor(e, device=DEV)) for rows, e in zip((70, 300), exponents))
+        out = torch.empty(70, 300, device=DEV)
+        kernels.gemm_f32(x, w, out)
+        want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+        assert ((out.double() - want).abs() <= size * (2.0 ** -23 + (k / 32 + 4) * 2.0 ** -24) + 2.0 ** -149).all()
+
+
 @pytest.mark.parametrize("k", [1, 3, 32, 1024])
 def test_gemm_f32_of_factors_whose_parts_are_largest(k):
     """Factors just below 1 + 2^-8, whose second part is 2^-8 and whose third would be 2^-16 if the second were cut off: a product loses at most

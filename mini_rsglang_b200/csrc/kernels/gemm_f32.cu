@@ -8,9 +8,11 @@
 // on K alone: not on M, not on the tile or the cut that the sizes chose, and a token's result does not change with what else is in the
 // batch.  Results that the parts cannot be trusted with are computed again in float64 from the inputs: those that are no number or
 // infinite, so that infinities and NaN are those of the sum of the products; those below 2^-100, whose smallest products lie near the end
-// of float32's range (`store_column`; products down to 2^-120 come as close to 64 bits as ordinary ones, 2^-125 a little less); and those of rows with an element below some 2^-110, which has bits under bfloat16's range (2^-133),
-// where the result is below 2^-60 or the other row has an element from 2^24 on (`mend_lost`).  Elsewhere K such bits are less than
-// K 2^-48 of the result.  Looking for them takes 0.4 to 0.8 us of a call of up to 128 rows (K = 1,024 to 3,072), none that shows of 777.
+// of float32's range (`store_column`; products down to 2^-120 come as close to 64 bits as ordinary ones, 2^-125 a little less); and those of
+// rows with an element below some 2^-110, which has bits under bfloat16's range (2^-133), where the result is below 2^-60 or the other
+// row has an element from 2^24 on (`mend_lost`).  Elsewhere K such bits are less than K 2^-48 of the result.  Looking for them takes 0.4 to
+// 0.8 us of a call of up to 128 rows (K = 1,024 to 3,072), none that shows of 777; where one token has one, 777 rows take 102 us, where all
+// have, 111.
 //
 // What bounds it: the workers' instructions (a float32 into three bfloat16 is some twenty-five instructions for four elements, and the
 // sums), then shared memory (both matrices pass through it; parts of W lie in tensor memory, which took a step of 96 tokens from 0.80 to
